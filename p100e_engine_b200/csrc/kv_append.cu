@@ -2,9 +2,8 @@
 //
 // Cache bytes are fixed by the reference's formats and fp32 recipes (src/fast/kv_q8.cuh:20-49, src/fast/attn.cu:245-283 in
 // the reference project): every position written here is byte-identical to what the reference writes for the same inputs,
-// paged or contiguous.  The kernels are organised per token, not per head: one CTA takes a whole token row, computes the
-// token's cos / sin once, and its warps walk the row's heads (query heads with their gate halves, K heads, V heads), each
-// head staying inside one warp from the load to the cache bytes, so nothing but the cos / sin table crosses a block barrier.
+// paged or contiguous.  A head (query head with its gate half, K head, V head) stays inside one warp from the load to the cache
+// bytes; the warps of a CTA share a token's cos / sin table, the only thing that crosses a block barrier.
 #include "common.cuh"
 
 #include <cuda_bf16.h>
@@ -99,23 +98,43 @@ struct tok_args {
     unsigned * status;
 };
 constexpr int TOK_WARPS = 8;
-constexpr int MAXF4 = 8;   // float4 per lane of one head: D <= 1024
 
 // PREP: attention input prep of the decode path (reference semantics: attn_prep_k, src/fast/fused.cu:502-573): per q head
 // the gate half is copied out and q = rope(rmsnorm(q) * q_norm); per K head the same norm and rotation, then the cache bytes;
 // V heads go to the cache as they are.  !PREP: plain append of k, v rows (reference: kv_append, src/fast/attn.cu:245-283).
-// One CTA per token, one head per warp at a time.  The sum of squares keeps the defining order: per group of four values
-// x0*x0 + x1*x1 + x2*x2 + x3*x3, a 32-lane butterfly over every 32 consecutive groups, then the butterfly of those results.
-template <uint32_t KT, bool PREP, bool MR>
+// grid (tokens, groups of TOK_WARPS heads), one head per warp: a decode step has few tokens, so its time is one head's chain
+// of loads, norm, rotation and stores.  Measured in a recorded graph (24 + 4 heads, q8_0, 1 / 4 / 256 / 512 tokens): 3.4 / 3.7 /
+// 7.1 / 10.7 us; with all heads of a token in one CTA, four per warp one after the other, 9.0 / 9.1 / 10.2 / 18.6 us.  The plain
+// append of 32768 tokens: 98 us against 170 us (registers: 31 against 56).  The head's loads go out before the cos / sin of the token are
+// computed (32 threads, the slow range reduction of large angles), which every CTA of the token repeats: the values are the same.
+// NF = float4 per lane of one head that the code is laid out for: 2 (D <= 256) or 8 (D <= 1024).  The sum of squares keeps the
+// defining order: per group of four values x0*x0 + x1*x1 + x2*x2 + x3*x3, a 32-lane butterfly over every 32 consecutive
+// groups, then the butterfly of those results over 8 slots (absent slots are zeros and add nothing).
+template <uint32_t KT, bool PREP, bool MR, int NF>
 __global__ void __launch_bounds__(TOK_WARPS * 32) token_k(const tok_args a) {
     extern __shared__ float sm[];   // cos[half] | sin[half] | TOK_WARPS staged heads of D floats
     const int t = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int D = a.D, nb = D / 32, nf = D / 128, half = a.n_rot / 2;
     float * cs = sm, * st = sm + a.n_rot + w * D;
+    const int n_q = PREP && a.qg ? a.Hq : 0, it = blockIdx.y * TOK_WARPS + w;
+    const bool live = it < n_q + 2 * a.Hkv, is_q = it < n_q, is_v = it >= n_q + a.Hkv;
+    const int h = is_q ? it : is_v ? it - n_q - a.Hkv : it - n_q;
     int row;
     if constexpr (PREP) {
         const int ppos = a.pos ? a.pos[t] : a.p0 + t;
         row = a.crow ? a.crow[t] : a.p0 < 0 ? ppos : a.p0 + t;
+        float4 x[NF], gt[NF];
+        const bool rotated = live && !is_v;
+        if (rotated) {
+            const float4 * src = reinterpret_cast<const float4 *>(is_q ? a.qg + (size_t) t * a.ldq + (size_t) h * 2 * D
+                                                                       : a.k + (size_t) t * a.ldk + (size_t) h * D);
+#pragma unroll
+            for (int j = 0; j < NF; ++j) if (j < nf) x[j] = src[lane + 32 * j];
+            if (is_q) {
+#pragma unroll
+                for (int j = 0; j < NF; ++j) if (j < nf) gt[j] = src[D / 4 + lane + 32 * j];
+            }
+        }
         for (int j = threadIdx.x; j < half; j += TOK_WARPS * 32) {
             float theta;
             if constexpr (MR) theta = (float) mrope_position(a.mr, t, j) * powf(a.freq_base, -2.0f * j / a.n_rot);
@@ -123,80 +142,68 @@ __global__ void __launch_bounds__(TOK_WARPS * 32) token_k(const tok_args a) {
             cs[j] = cosf(theta);
             cs[half + j] = sinf(theta);
         }
-        __syncthreads();
-    } else {
-        row = (a.p0p ? *a.p0p : a.p0) + t;
-    }
-    unsigned long long roff = 0;
-    bool stored = row >= 0;
-    if (stored) {
-        const int32_t * tab = kv_tab(a.g, t);
-        if (tab && tab[row >> a.g.psh] < 0) { if (threadIdx.x == 0) atomicOr(a.status, ST_BAD_PAGE); stored = false; }
-        else roff = kv_off_tab(a.g, tab, row);
-    }
-    const int n_q = PREP && a.qg ? a.Hq : 0;
-    for (int it = w; it < n_q + 2 * a.Hkv; it += TOK_WARPS) {
-        const bool is_q = it < n_q, is_v = it >= n_q + a.Hkv;
-        const int h = is_q ? it : is_v ? it - n_q - a.Hkv : it - n_q;
-        if (!is_q && !stored) continue;
-        char * head = (is_v ? a.g.v : a.g.k) + roff + (unsigned long long) h * head_bytes(KT, D);
-        if (is_v || !PREP) {   // no norm, no rotation: 32 values per step straight from the activations
-            const float * src = is_v ? a.v + (size_t) t * a.ldv + (size_t) h * D : a.k + (size_t) t * a.ldk + (size_t) h * D;
-            float x[MAXF4 * 4];
-#pragma unroll
-            for (int b = 0; b < MAXF4 * 4; ++b) if (b < nb) x[b] = src[b * 32 + lane];
-#pragma unroll
-            for (int b = 0; b < MAXF4 * 4; ++b) if (b < nb) block_to_cache<KT>(x[b], lane, head, b, nb);
-            continue;
-        }
-        if constexpr (PREP) {
-            const float4 * src = reinterpret_cast<const float4 *>(is_q ? a.qg + (size_t) t * a.ldq + (size_t) h * 2 * D
-                                                                       : a.k + (size_t) t * a.ldk + (size_t) h * D);
-            float4 x[MAXF4];
-#pragma unroll
-            for (int j = 0; j < MAXF4; ++j) if (j < nf) x[j] = src[lane + 32 * j];
+        if (rotated) {
             if (is_q) {   // the gate half of the head moves on unchanged
                 float4 * gd = reinterpret_cast<float4 *>(a.gate + ((size_t) t * a.Hq + h) * D);
 #pragma unroll
-                for (int j = 0; j < MAXF4; ++j) if (j < nf) gd[lane + 32 * j] = src[D / 4 + lane + 32 * j];
+                for (int j = 0; j < NF; ++j) if (j < nf) gd[lane + 32 * j] = gt[j];
             }
-            float part[MAXF4];
+            float part[8];
 #pragma unroll
-            for (int j = 0; j < MAXF4; ++j) {
-                float ss = 0.0f;
-                if (j < nf) ss += x[j].x * x[j].x + x[j].y * x[j].y + x[j].z * x[j].z + x[j].w * x[j].w;
-                part[j] = lanes_sum(ss);
+            for (int j = 0; j < 8; ++j) {
+                part[j] = 0.0f;
+                if (j < NF && j < nf) part[j] = lanes_sum(0.0f + (x[j].x * x[j].x + x[j].y * x[j].y + x[j].z * x[j].z + x[j].w * x[j].w));
             }
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) {   // the butterfly of the per-32-group results (absent groups count as 0)
-                float nx[MAXF4];
+            for (int o = 4; o > 0; o >>= 1) {   // the butterfly of the per-32-group results
+                float nx[8];
 #pragma unroll
-                for (int j = 0; j < MAXF4; ++j) nx[j] = part[j] + part[j ^ o];
+                for (int j = 0; j < 8; ++j) nx[j] = part[j] + part[j ^ o];
 #pragma unroll
-                for (int j = 0; j < MAXF4; ++j) part[j] = nx[j];
+                for (int j = 0; j < 8; ++j) part[j] = nx[j];
             }
             const float sc = rsqrtf(part[0] / D + a.eps);
             const float4 * wt = reinterpret_cast<const float4 *>(is_q ? a.qn : a.kn);
 #pragma unroll
-            for (int j = 0; j < MAXF4; ++j)
+            for (int j = 0; j < NF; ++j)
                 if (j < nf) {
                     float4 o = x[j];
                     o.x *= sc; o.y *= sc; o.z *= sc; o.w *= sc;
                     if (wt) { const float4 ww = wt[lane + 32 * j]; o.x *= ww.x; o.y *= ww.y; o.z *= ww.z; o.w *= ww.w; }
                     reinterpret_cast<float4 *>(st)[lane + 32 * j] = o;
                 }
-            __syncwarp();
+        }
+        __syncthreads();
+    } else {
+        row = (a.p0p ? *a.p0p : a.p0) + t;
+    }
+    if (!live) return;
+    if constexpr (PREP) {
+        if (!is_v) {
             for (int j = lane; j < half; j += 32) rot_pair(st[j], st[j + half], cs[j], cs[half + j], st[j], st[j + half]);
             __syncwarp();
-            if (is_q) {
-                float4 * dst = reinterpret_cast<float4 *>(a.q + ((size_t) t * a.Hq + h) * D);
-#pragma unroll
-                for (int j = 0; j < MAXF4; ++j) if (j < nf) dst[lane + 32 * j] = reinterpret_cast<const float4 *>(st)[lane + 32 * j];
-            } else {
-                for (int b = 0; b < nb; ++b) block_to_cache<KT>(st[b * 32 + lane], lane, head, b, nb);
-            }
-            __syncwarp();   // the staged head is reused by this warp's next item
         }
+        if (is_q) {
+            float4 * dst = reinterpret_cast<float4 *>(a.q + ((size_t) t * a.Hq + h) * D);
+#pragma unroll
+            for (int j = 0; j < NF; ++j) if (j < nf) dst[lane + 32 * j] = reinterpret_cast<const float4 *>(st)[lane + 32 * j];
+            return;
+        }
+    }
+    if (row < 0) return;
+    const int32_t * tab = kv_tab(a.g, t);
+    if (tab && tab[row >> a.g.psh] < 0) { if (lane == 0) atomicOr(a.status, ST_BAD_PAGE); return; }
+    char * head = (is_v ? a.g.v : a.g.k) + kv_off_tab(a.g, tab, row) + (unsigned long long) h * head_bytes(KT, D);
+    if (PREP && !is_v) {
+#pragma unroll
+        for (int b = 0; b < NF * 4; ++b) if (b < nb) block_to_cache<KT>(st[b * 32 + lane], lane, head, b, nb);
+    } else {   // no norm, no rotation: straight from the activations
+        const float * src = is_v ? a.v + (size_t) t * a.ldv + (size_t) h * D : a.k + (size_t) t * a.ldk + (size_t) h * D;
+        float x[NF * 4];
+#pragma unroll
+        for (int b = 0; b < NF * 4; ++b) if (b < nb) x[b] = src[b * 32 + lane];
+#pragma unroll
+        for (int b = 0; b < NF * 4; ++b) if (b < nb) block_to_cache<KT>(x[b], lane, head, b, nb);
     }
 }
 
@@ -383,13 +390,16 @@ bool type_ok(uint32_t t) { return t == B200_KV_F16 || t == B200_KV_Q8_0 || t == 
 
 template <bool PREP>
 int token_launch(const tok_args & a, uint32_t type, int T, bool mrope, cudaStream_t s, const char * who) {
-    const size_t smem = ((size_t) a.n_rot + (size_t) TOK_WARPS * a.D) * sizeof(float);
-#define TOKEN(KT_) do { if (PREP && mrope) token_k<KT_, PREP, PREP><<<T, TOK_WARPS * 32, smem, s>>>(a); \
-                        else token_k<KT_, PREP, false><<<T, TOK_WARPS * 32, smem, s>>>(a); } while (0)
+    const size_t smem = PREP ? ((size_t) a.n_rot + (size_t) TOK_WARPS * a.D) * sizeof(float) : 0;
+    const dim3 grid(T, ((PREP && a.qg ? a.Hq : 0) + 2 * a.Hkv + TOK_WARPS - 1) / TOK_WARPS);
+#define TOKEN_NF(KT_, MR_) do { if (a.D <= 256) token_k<KT_, PREP, MR_, 2><<<grid, TOK_WARPS * 32, smem, s>>>(a); \
+                                else token_k<KT_, PREP, MR_, 8><<<grid, TOK_WARPS * 32, smem, s>>>(a); } while (0)
+#define TOKEN(KT_) do { if (PREP && mrope) TOKEN_NF(KT_, PREP); else TOKEN_NF(KT_, false); } while (0)
     if (type == B200_KV_F16) TOKEN(B200_KV_F16);
     else if (type == B200_KV_Q8_0) TOKEN(B200_KV_Q8_0);
     else TOKEN(B200_KV_Q4_0);
 #undef TOKEN
+#undef TOKEN_NF
     count_launch();
     return launch_status(who);
 }
