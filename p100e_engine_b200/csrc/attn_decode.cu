@@ -96,6 +96,23 @@ template <uint32_t KT> __device__ __forceinline__ int q_slot(int d) {
     } else return d;
 }
 
+// Chunk grids of the fixed-chunk modes, by absolute key index.  CH > 0: chunks of CH keys.  CH <= 0, the library default: 64 keys up
+// to position 4096, then 32 chunks per doubling (128 keys from 4096, 256 from 8192, ..) up to chunks of 64 << -CH keys.  A short context
+// is cut finely enough to fill the chip whatever the cache's capacity, and a long one into little more than one wave of equal units.
+// One row, q8_0, 4 kv heads: chunks of 512 keys everywhere take 22.3 / 24.8 / 69.1 us at 4096 / 16384 / 131072 keys, of 64 keys
+// 12.7 / 24.8 / 124.1 us.
+__host__ __device__ __forceinline__ int chunk_of(int CH, int p) {
+    if (CH > 0) return p / CH;
+    int k = 0;
+    while (k < -CH && (p >> (12 + k)) != 0) ++k;
+    return 32 * k + (p >> (6 + k));
+}
+__host__ __device__ __forceinline__ long long chunk_lo(int CH, int c) {
+    if (CH > 0) return (long long) c * CH;
+    const int k = c < 64 ? 0 : (c >> 5) - 1 < -CH ? (c >> 5) - 1 : -CH;
+    return (long long) (c - 32 * k) << (6 + k);
+}
+
 struct dec_args {
     const float * q;
     kv_view g;
@@ -105,12 +122,13 @@ struct dec_args {
     int p0;
     int q_len, n_slots, Hq;
     float qscale;                         // softmax scale * log2(e)
-    int CH, max_chunks;
+    int CH, max_chunks;                   // chunk grid (chunk_of / chunk_lo); chunks of the longest slot
+    int hk0, nhk;                         // kv heads of this launch: hk0 .. hk0 + nhk - 1 (all of them but in the allocation-free entry)
     unsigned * status;
     int n_ctx;                            // rows of a contiguous cache
     int tiled;                            // set by the launcher: whole tiles are fetched through the tensor maps
     const int2 * units;                   // work list written by decode_plan_k: (slot, chunk), longest first; nullptr = the
-    const int * n_units;                  // grid itself enumerates (slot, chunk) and units past a slot's end exit
+    const int * n_units;                  // CTAs enumerate (slot, chunk) themselves and skip units past a slot's end
     // even split (decode_split_k): the batch's 64-key tiles, slot after slot, are cut into one contiguous run per CTA
     const int4 * segs;                    // (slot, first key, end key, 0) in CTA order; a run that crosses a slot boundary has several
     const int * cta_seg;                  // [n_cta + 1] first segment of each CTA
@@ -122,7 +140,7 @@ struct dec_args {
 // partials are sized for max_chunks chunks) and to n_ctx for a contiguous cache.  A position beyond the limit is recorded
 // in the status word and its keys past the limit are left out.
 __device__ __forceinline__ int key_limit(const dec_args & a) {
-    const long long lim = (long long) a.max_chunks * a.CH;
+    const long long lim = chunk_lo(a.CH, a.max_chunks);
     const int l = (int) (lim < 0x7fffffffLL ? lim : 0x7fffffffLL);
     return a.g.pt ? l : min(l, a.n_ctx);
 }
@@ -203,10 +221,12 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
 
     // staging: the K rows and the V rows of the tiles form one sequence q = 2 * tile (K), 2 * tile + 1 (V) that walks a ring
     // of nslot half-tile slots.  The warp that is last to finish the Q K^T (P V) of a tile refills that tile's K (V) slot with
-    // item q + nslot, so a copy is in flight while the other half of the tile is being computed.  A tile that lies inside
-    // the slot's keys is one tiled copy through the cache's tensor map (box = 64 rows of this head, inside one page);
-    // otherwise the warp moves the 64 rows one by one, rows past the slot's last key replaced by that last key (always
-    // readable and finite, and masked in the softmax).
+    // item q + nslot, so a copy is in flight while the other half of the tile is being computed.  A tile is one tiled
+    // copy through the cache's tensor map (box = 64 rows of this head, inside one page), a slot's last, ragged tile too: what lies
+    // past its last key (stale rows of the page; zeros past the end of a contiguous cache) is masked in the softmax and
+    // enters P V as zeros.  One warp moving that tile row by row held its CTA for 30 us (q8_0) to 60 us (f16), longer than everything
+    // else in a call of 30011 keys (50.2 us in all).  Caches without a tensor map (small pages) are still moved that way, rows past the slot's
+    // last key replaced by that key.
     auto page_of = [&](int p, bool first) { return pg_staged && !first ? pgs[(p >> a.g.psh) - pg0] : tab[p >> a.g.psh]; };
     auto issue = [&](int q, int s, bool first) {   // s = q mod nslot; called by one whole warp
         if (q >= 2 * ntiles) return;
@@ -214,7 +234,7 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
         unsigned char * dst = stg + (size_t) s * TR::SLOT;
         const char * base = (q & 1) ? a.g.v : a.g.k;
         const int p_t = k_lo + it * TILE;
-        if (a.tiled && p_t + TILE <= n_slot) {
+        if (a.tiled) {
             if (lane == 0) {
                 int y = p_t, z = 0;
                 if (tab) {
@@ -501,13 +521,20 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
         };
         write_p();
         mbar_wait(bar_v, par_v, a.status);   // this tile's V rows
-        if constexpr (TR::SCALED) {   // V block scales, transposed to [block][key]
+        const int v_keys = k_hi - (k_lo + it * TILE);   // rows of the tile that hold keys: 64 or more but in the last tile
+        if constexpr (TR::SCALED) {   // V block scales, transposed to [block][key]; zero for rows past the last key (their bytes may be anything)
             const int key = tid >> 1, b0 = (tid & 1) * 4;
 #pragma unroll
             for (int b = b0; b < b0 + 4; ++b) {
                 const unsigned char * src = KT == B200_KV_Q8_0 ? Vs + key * SROW + 2 * b : Vs + key * SROW + 18 * b;
-                *reinterpret_cast<uint16_t *>(Sd + b * SDSTR + key * 2) = *reinterpret_cast<const uint16_t *>(src);
+                const uint16_t d = *reinterpret_cast<const uint16_t *>(src);
+                *reinterpret_cast<uint16_t *>(Sd + b * SDSTR + key * 2) = key < v_keys ? d : (uint16_t) 0;
             }
+        } else if (v_keys < TILE) {
+            unsigned char * vz = stg + (size_t) sv_now * TR::SLOT;
+            for (int i = tid; i < (TILE - v_keys) * 32; i += NTHR)
+                *reinterpret_cast<uint4 *>(vz + f16_slot_off(v_keys + (i >> 5), i & 31)) = make_uint4(0, 0, 0, 0);
+            umma::fence_async_smem();   // the slot's next fill comes through the async proxy
         }
         __syncthreads();   // P, the V scales, the warps' maxima and the flag are visible
         if constexpr (PARK) unpark();
@@ -685,37 +712,35 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
 
 #include "decode_tc.cuh"
 
-// The kernel: one unit per CTA (the grid enumerates (slot, chunk), directly or through the work list), or, with the even
-// split, every segment of the CTA's run one after the other.
+// The kernel.  Even split: every segment of the CTA's run one after the other.  Fixed chunks: units u = blockIdx.x, + gridDim.x, ..
+// with at most one resident wave of CTAs launched, the longest chunks first (work list, or the highest chunk index first), so that
+// several waves of short CTAs do not each pay their start-up and the tail is made of short units.
 template <uint32_t KT, int NT>
 __global__ void __launch_bounds__(NTHR, ctas_per_sm<KT, NT>())
 decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    // blockIdx.x = unit * Hkv + kv head: the heads of one (slot, key range) are neighbours in launch order, so the four
+    // unit number = index * heads + kv head: the heads of one (slot, key range) are neighbours in launch order, so the four
     // head rows of a position are fetched close together in time
-    const int hk = (int) (blockIdx.x % (unsigned) a.g.Hkv), ui = (int) (blockIdx.x / (unsigned) a.g.Hkv);
-    int s0 = 0, s1 = 1, slot = 0, k_lo = 0, k_cap = 0;
-    size_t unit = 0;
+    int hl = (int) (blockIdx.x % (unsigned) a.nhk), s0 = 0, s1 = 0, nch = a.max_chunks;
+    long long u_end = 0;
     if (a.segs) {
+        const int ui = (int) (blockIdx.x / (unsigned) a.nhk);
         if (ui >= *a.n_cta) return;
         s0 = a.cta_seg[ui]; s1 = a.cta_seg[ui + 1];
         if (s0 >= s1) return;
+    } else if (a.units) {
+        u_end = (long long) *a.n_units * a.nhk;
     } else {
-        int chunk;
-        if (a.units) {
-            if (ui >= *a.n_units) return;
-            const int2 u = a.units[ui];
-            slot = u.x; chunk = u.y;
-        } else {
-            slot = ui / a.max_chunks; chunk = ui - slot * a.max_chunks;
+        if (a.n_slots == 1) {
+            int n = 0;
+            for (int j = 0; j < a.q_len; ++j) n = max(n, row_pos(a, 0, j) + 1);
+            n = min(n, key_limit(a));
+            nch = n > 0 ? chunk_of(a.CH, n - 1) + 1 : 0;
+            // the chunks past the limit are the merge's business; a position beyond it is reported by the unit that runs
         }
-        int n = 0;
-        for (int j = 0; j < a.q_len; ++j) n = max(n, row_pos(a, slot, j) + 1);
-        k_lo = chunk * a.CH;
-        if (k_lo >= min(n, key_limit(a))) return;   // the chunk lies past the slot's keys
-        k_cap = k_lo + a.CH;
-        unit = ((size_t) slot * a.g.Hkv + hk) * a.max_chunks + chunk;
+        u_end = (long long) nch * a.n_slots * a.nhk;
     }
+    if (!a.segs && blockIdx.x >= u_end) return;
     // barriers of the copy ring, arrival counters and flags: made once per CTA
     if (threadIdx.x == 0) {
         uint64_t * full = reinterpret_cast<uint64_t *>(smem);
@@ -736,14 +761,31 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
         t_base = *t_slot;
     }
     int tiles = 0;
-    for (int sg = s0; sg < s1; ++sg) {
+    long long u = a.segs ? s0 : blockIdx.x;
+    const long long u_last = a.segs ? s1 : u_end, u_step = a.segs ? 1 : gridDim.x;
+    for (; u < u_last; u += u_step) {
+        int slot, k_lo, k_cap;
+        size_t unit;
         if (a.segs) {
-            const int4 e = a.segs[sg];
+            const int4 e = a.segs[u];
             slot = e.x; k_lo = e.y; k_cap = e.z;
-            unit = (size_t) sg * a.g.Hkv + hk;
+            unit = (size_t) u * a.nhk + hl;
+        } else {
+            hl = (int) (u % a.nhk);
+            const int i = (int) (u / a.nhk);
+            int chunk;
+            if (a.units) {
+                const int2 e = a.units[i];
+                slot = e.x; chunk = e.y;
+            } else {
+                slot = i % a.n_slots; chunk = nch - 1 - i / a.n_slots;
+            }
+            k_lo = (int) chunk_lo(a.CH, chunk);
+            k_cap = (int) min(0x7fffffffLL, chunk_lo(a.CH, chunk + 1));
+            unit = ((size_t) slot * a.nhk + hl) * a.max_chunks + chunk;
         }
-        if (sg > s0) __syncthreads();   // the previous segment's shared memory is no longer read
-        tiles += decode_unit<KT, NT>(a, nslot, mapK, mapV, smem, hk, slot, k_lo, k_cap, unit, tiles, t_base);
+        if (tiles) __syncthreads();   // the previous unit's shared memory is no longer read
+        tiles += decode_unit<KT, NT>(a, nslot, mapK, mapV, smem, a.hk0 + hl, slot, k_lo, k_cap, unit, tiles, t_base);
     }
     if constexpr (parks<KT, NT>()) {
         umma::fence_before_sync();
@@ -755,22 +797,25 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
     }
 }
 
-// Merge a row's chunk partials.  grid (rows, Hq), MERGE_GROUPS groups of 64 threads (one float4 of the head each): group w
-// sums the chunks w, w + G, .. in ascending order, the group sums are added in group order: a fixed order for a given number
-// of chunks, so a row's result does not depend on the rest of the call (the fixed-chunk modes run four groups).
+// Merge a row's chunk partials.  grid (rows, Hq), P groups of 64 threads (one float4 of the head each).  P > 1: chunk c belongs to
+// summation stream c mod MERGE_STREAMS, group w walks the streams w, w + P, .. (each in ascending order, its own accumulator),
+// and the streams are added in stream order: an order that depends on the number of chunks only, not on P nor on the rest of
+// the call.  P = 1: plain ascending order.
 //   out != nullptr : out = num / den (* sigmoid(gate)); rows that saw no key give zeros
 //   fo  != nullptr : unnormalised num, max in natural-log units, den (for a cross-GPU merge)
-// The even split leaves one to a few partials per row (one per CTA run that crosses the slot): there one group of 64 threads
-// per (row, head) keeps the launch to little more than one wave of small blocks.
-template <int MERGE_GROUPS>
-__global__ void __launch_bounds__(64 * MERGE_GROUPS) decode_merge_k(const dec_args a, const float * __restrict__ gate, float * __restrict__ out,
-                                                     float * __restrict__ fo, float * __restrict__ fm, float * __restrict__ fl,
-                                                     __half2 * __restrict__ qbuf) {
-    __shared__ float4 gnum[MERGE_GROUPS > 1 ? MERGE_GROUPS - 1 : 1][64];
-    __shared__ float gden[MERGE_GROUPS > 1 ? MERGE_GROUPS - 1 : 1];
-    const int lane4 = threadIdx.x & 63, grp = threadIdx.x >> 6;
-    const int h = blockIdx.y, row = blockIdx.x, slot = row / a.q_len, j = row - slot * a.q_len;
-    const int hk = h / GQA, hh = h - hk * GQA, r = j * GQA + hh, R = a.q_len * GQA;
+// The kernel is a chain of dependent loads (positions, maxima, partials), so what counts is how many partials are in flight:
+// merge_launch picks P from the number of partials a row can have.
+constexpr int MERGE_STREAMS = 16;
+template <int P>
+__global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const float * __restrict__ gate, float * __restrict__ out,
+                                                         float * __restrict__ fo, float * __restrict__ fm, float * __restrict__ fl,
+                                                         __half2 * __restrict__ qbuf) {
+    constexpr int SPG = P > 1 ? MERGE_STREAMS / P : 1;   // streams per group
+    __shared__ float4 snum[P > 1 ? MERGE_STREAMS : 1][64];
+    __shared__ float sden[P > 1 ? MERGE_STREAMS : 1], smax[2 * P];
+    const int tid = threadIdx.x, lane4 = tid & 63, grp = tid >> 6;
+    const int row = blockIdx.x, slot = row / a.q_len, j = row - slot * a.q_len;
+    const int hl = blockIdx.y / GQA, hh = blockIdx.y - hl * GQA, h = a.hk0 * GQA + blockIdx.y, r = j * GQA + hh, R = a.q_len * GQA;
     const int pos = min(row_pos(a, slot, j), key_limit(a) - 1);   // a row past the limit merges the chunks that exist
     // partials of the row's kv head: consecutive units of stride ustr from unit0 (a segment the row does not reach holds m = -inf)
     int nch;
@@ -778,36 +823,57 @@ __global__ void __launch_bounds__(64 * MERGE_GROUPS) decode_merge_k(const dec_ar
     if (a.segs) {
         const int2 sg = a.slot_seg[slot];
         nch = pos < 0 ? 0 : sg.y;
-        unit0 = (size_t) sg.x * a.g.Hkv + hk; ustr = a.g.Hkv;
+        unit0 = (size_t) sg.x * a.nhk + hl; ustr = a.nhk;
     } else {
-        nch = pos < 0 ? 0 : pos / a.CH + 1;
-        unit0 = ((size_t) slot * a.g.Hkv + hk) * a.max_chunks; ustr = 1;
+        nch = pos < 0 ? 0 : chunk_of(a.CH, pos) + 1;
+        unit0 = ((size_t) slot * a.nhk + hl) * a.max_chunks; ustr = 1;
     }
+    const float * pm = a.pm + unit0 * R + r, * pl = a.pl + unit0 * R + r;
+    const float4 * po = reinterpret_cast<const float4 *>(a.po + (unit0 * R + r) * DH) + lane4;
+    const size_t st = ustr * R;   // from one partial of the row to the next, in values (pm, pl) and head rows (po)
     float M = B200_NEG_INF;
-    for (int c = 0; c < nch; ++c) M = fmaxf(M, a.pm[(unit0 + c * ustr) * R + r]);
+    if constexpr (P > 1) {
+        for (int c = tid; c < nch; c += 64 * P) M = fmaxf(M, pm[c * st]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        if ((tid & 31) == 0) smax[tid >> 5] = M;
+        __syncthreads();
+        M = smax[0];
+#pragma unroll
+        for (int i = 1; i < 2 * P; ++i) M = fmaxf(M, smax[i]);
+    } else {
+        for (int c = 0; c < nch; ++c) M = fmaxf(M, pm[c * st]);
+    }
     float den = 0.0f;
     float4 num = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 4
-    for (int c = grp; c < nch; c += MERGE_GROUPS) {   // no early continue: the loads of several chunks are in flight together
-        const size_t u = unit0 + c * ustr;
-        const float ms = a.pm[u * R + r];
+    auto add = [&](int c, float4 & n, float & d) {   // no early continue: the loads of several chunks are in flight together
+        const float ms = pm[c * st];
         const float f = ms == B200_NEG_INF ? 0.0f : ex2f(ms - M);   // a chunk the row did not see holds zeros: adds nothing
-        den = fmaf(f, a.pl[u * R + r], den);
-        const float4 o = reinterpret_cast<const float4 *>(a.po + (u * R + r) * DH)[lane4];
-        num.x = fmaf(f, o.x, num.x); num.y = fmaf(f, o.y, num.y); num.z = fmaf(f, o.z, num.z); num.w = fmaf(f, o.w, num.w);
-    }
-    if constexpr (MERGE_GROUPS > 1) {
-        if (grp > 0) {
-            gnum[grp - 1][lane4] = num;
-            if (lane4 == 0) gden[grp - 1] = den;
+        d = fmaf(f, pl[c * st], d);
+        const float4 o = po[c * st * (DH / 4)];
+        n.x = fmaf(f, o.x, n.x); n.y = fmaf(f, o.y, n.y); n.z = fmaf(f, o.z, n.z); n.w = fmaf(f, o.w, n.w);
+    };
+    if constexpr (P == 1) {
+#pragma unroll 4
+        for (int c = 0; c < nch; ++c) add(c, num, den);
+    } else {
+#pragma unroll
+        for (int i = 0; i < SPG; ++i) {
+            const int s = grp + P * i;
+            float d = 0.0f;
+            float4 n = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+            for (int c = s; c < nch; c += MERGE_STREAMS) add(c, n, d);
+            snum[s][lane4] = n;
+            if (lane4 == 0) sden[s] = d;
         }
         __syncthreads();
         if (grp > 0) return;
-#pragma unroll
-        for (int w = 0; w < MERGE_GROUPS - 1; ++w) {
-            const float4 o = gnum[w][lane4];
+        const int ns = min(nch, MERGE_STREAMS);   // the other streams are empty
+        for (int s = 0; s < ns; ++s) {
+            const float4 o = snum[s][lane4];
             num.x += o.x; num.y += o.y; num.z += o.z; num.w += o.w;
-            den += gden[w];
+            den += sden[s];
         }
     }
     const size_t oi = ((size_t) row * a.Hq + h) * (DH / 4) + lane4;
@@ -944,49 +1010,49 @@ __global__ void merge_peers_k(const peer_parts pp, int n_seq, int me, unsigned e
     if (qbuf) a16_store_lanes8(y, qbuf, ((size_t) r * D + 4 * i) / 32, (size_t) R * D / 32, true);
 }
 
-// Work list of a batched call: every (slot, chunk) that holds at least one visible key, longest first.  Whole chunks
-// come first (all the same length), then the slots' last, shorter chunks in descending order of their tile count, so the
-// tail of the launch is made of the shortest units.  One block; writes units[] and *n_units.  The order of equal-length
-// units depends on the order of the atomics and does not affect any result (units are independent).
-constexpr int PLAN_THR = 256, PLAN_BUCKETS = 256;
+// Work list of a batched call: every (slot, chunk) that holds at least one visible key, longest first, so the tail of the
+// launch is made of the shortest units.  One block; writes units[] and *n_units.  The order of equal-length units depends on the
+// order of the atomics and does not affect any result (units are independent).
+constexpr int PLAN_THR = 1024, PLAN_BUCKETS = 256;
 __global__ void __launch_bounds__(PLAN_THR) decode_plan_k(const dec_args a, int2 * __restrict__ units, int * __restrict__ n_units) {
-    __shared__ int hist[PLAN_BUCKETS], total_full, cur_full;
-    const int tid = threadIdx.x;
-    const int tiles_per_chunk = a.CH / TILE;
+    __shared__ int hist[PLAN_BUCKETS];
+    const int tid = threadIdx.x, lim = key_limit(a);
+    const int top = a.CH > 0 ? a.CH / TILE : 1 << -a.CH;   // tiles of the longest chunk
     for (int i = tid; i < PLAN_BUCKETS; i += PLAN_THR) hist[i] = 0;
-    if (tid == 0) { total_full = 0; cur_full = 0; }
     __syncthreads();
-    const int lim = key_limit(a);
-    auto slot_keys = [&](int s) {
+    const long long pairs = (long long) a.n_slots * a.max_chunks;
+    // bucket of pair i (0 = longest class), -1 if the slot has no key in the chunk
+    auto bucket_of = [&](long long i) {
+        const int s = (int) (i % a.n_slots), c = (int) (i / a.n_slots);
         int n = 0;
         for (int j = 0; j < a.q_len; ++j) n = max(n, row_pos(a, s, j) + 1);
-        return min(n, lim);
+        n = min(n, lim);
+        const long long lo = chunk_lo(a.CH, c);
+        if (lo >= n) return -1;
+        const long long tiles = (min((long long) n, chunk_lo(a.CH, c + 1)) - lo + TILE - 1) / TILE;
+        return (int) min((long long) PLAN_BUCKETS - 1, (top - tiles) * PLAN_BUCKETS / top);
     };
-    // bucket of a last chunk: its tile count scaled into PLAN_BUCKETS classes, descending (bucket 0 = longest)
-    auto bucket_of = [&](int tail_keys) {
-        const int tiles = (tail_keys + TILE - 1) / TILE;   // 1 .. tiles_per_chunk - 1 (a whole chunk is not a tail) or tiles_per_chunk
-        const long long cls = (long long) (tiles_per_chunk - tiles) * PLAN_BUCKETS / max(tiles_per_chunk, 1);
-        return (int) min((long long) PLAN_BUCKETS - 1, max(0LL, cls));
-    };
-    for (int s = tid; s < a.n_slots; s += PLAN_THR) {
-        const int n = slot_keys(s), nfull = n / a.CH, tail = n - nfull * a.CH;
-        if (nfull) atomicAdd(&total_full, nfull);
-        if (tail) atomicAdd(&hist[bucket_of(tail)], 1);
+    for (long long i = tid; i < pairs; i += PLAN_THR) {
+        const int b = bucket_of(i);
+        if (b >= 0) atomicAdd(&hist[b], 1);
     }
     __syncthreads();
-    if (tid == 0) {   // exclusive scan of the tail classes, placed after the whole chunks
-        int run = total_full;
-        for (int i = 0; i < PLAN_BUCKETS; ++i) { const int c = hist[i]; hist[i] = run; run += c; }
-        *n_units = run;
-    }
-    __syncthreads();
-    for (int s = tid; s < a.n_slots; s += PLAN_THR) {
-        const int n = slot_keys(s), nfull = n / a.CH, tail = n - nfull * a.CH;
-        if (nfull) {
-            const int base = atomicAdd(&cur_full, nfull);
-            for (int c = 0; c < nfull; ++c) units[base + c] = make_int2(s, c);
+    if (tid < 32) {   // exclusive scan of the classes
+        int run = 0;
+        for (int base = 0; base < PLAN_BUCKETS; base += 32) {
+            const int v = hist[base + tid];
+            int x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (tid >= o) x += y; }
+            hist[base + tid] = run + x - v;
+            run += __shfl_sync(0xffffffffu, x, 31);
         }
-        if (tail) units[atomicAdd(&hist[bucket_of(tail)], 1)] = make_int2(s, nfull);
+        if (tid == 0) *n_units = run;
+    }
+    __syncthreads();
+    for (long long i = tid; i < pairs; i += PLAN_THR) {
+        const int b = bucket_of(i);
+        if (b >= 0) units[atomicAdd(&hist[b], 1)] = make_int2((int) (i % a.n_slots), (int) (i / a.n_slots));
     }
 }
 
@@ -994,9 +1060,10 @@ __global__ void __launch_bounds__(PLAN_THR) decode_plan_k(const dec_args a, int2
 // slots, slot after slot, form one sequence per kv head; CTA c of n_cta takes tiles [c W / n_cta, (c + 1) W / n_cta), so
 // every CTA has the same work to within one tile however ragged the contexts are, and all CTAs fit the machine at once.  A
 // run that crosses slot boundaries becomes several segments; each segment yields one partial.  n_cta = min(max_cta, W /
-// SPLIT_MIN_TILES) keeps runs from getting so short that start-up and the merge dominate.  One block; n_slots <= SPLIT_MAX_SLOTS.
-constexpr int SPLIT_THR = 1024, SPLIT_MAX_SLOTS = 2048, SPLIT_MAX_CTA = 1024, SPLIT_MIN_TILES = 4;
-__global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, int max_cta, int4 * __restrict__ segs, int * __restrict__ cta_seg,
+// min_tiles): the tcgen05 kernel walks tiles of 128 keys, so its runs hold at least two of these.  One block; n_slots <=
+// SPLIT_MAX_SLOTS.
+constexpr int SPLIT_THR = 1024, SPLIT_MAX_SLOTS = 2048, SPLIT_MAX_CTA = 1024;
+__global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, int max_cta, int min_tiles, int4 * __restrict__ segs, int * __restrict__ cta_seg,
                                                             int2 * __restrict__ slot_seg, int * __restrict__ n_cta_out) {
     __shared__ int pre[SPLIT_MAX_SLOTS + 1];     // tiles before slot s
     __shared__ int cseg[SPLIT_MAX_CTA + 1];      // segments before CTA c
@@ -1023,7 +1090,7 @@ __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, in
     }
     __syncthreads();
     const long long W = pre[a.n_slots];
-    const int n_cta = (int) max(1LL, min((long long) min(max_cta, SPLIT_MAX_CTA), W / SPLIT_MIN_TILES));
+    const int n_cta = (int) max(1LL, min((long long) min(max_cta, SPLIT_MAX_CTA), W / min_tiles));
     auto cut = [&](int c) { return (int) (W * c / n_cta); };
     // segments per CTA: the slots its run intersects
     int my_first = 0, my_cnt = 0;
@@ -1083,8 +1150,8 @@ __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, in
 }
 
 // ------------------------------------------------------------------------------------------------ host side ----
-constexpr int DEFAULT_CHUNK = 512;
-constexpr int MAX_DEFAULT_CHUNKS = 256;   // the default chunk grows with n_ctx so that a context never has more chunks than this
+constexpr int DEFAULT_CHUNK = 64;         // shortest chunk of the default grid
+constexpr int NOMINAL_NSPLIT = 256;       // what nsplit() reports while nothing is pinned
 int g_chunk = 0;            // 0 = not read yet; else B200ATTN_CHUNK or DEFAULT_CHUNK
 bool g_chunk_from_env = false;
 int g_nsplit_override = 0;  // set_nsplit: chunks per full context
@@ -1100,13 +1167,23 @@ int default_chunk() {
     if (!g_chunk) g_chunk = env_chunk(&g_chunk_from_env);
     return g_chunk;
 }
-// The chunk of a call that asks for the library default: a function of the cache's capacity only, so that a row's bits do
-// not depend on the batch it is decoded in.  set_nsplit(n) pins n chunks per full context; B200ATTN_CHUNK pins the keys.
-int fixed_chunk(int n_ctx) {
+// The chunk grid of a call that asks for the library default: a function of the cache's capacity and of settings only, so that a
+// row's bits do not depend on the batch it is decoded in.  set_nsplit(n) pins n chunks per full context; B200ATTN_CHUNK pins the keys;
+// else the default grid (CH <= 0), whose longest chunk is 512 keys up to a capacity of 131072 and n_ctx / 256 beyond.
+int default_grid(int n_ctx) {
     const int base = default_chunk();
     if (g_nsplit_override > 0) return round_tile(((long long) std::max(n_ctx, 1) + g_nsplit_override - 1) / g_nsplit_override);
     if (g_chunk_from_env) return base;
-    return std::max(base, round_tile(((long long) std::max(n_ctx, 1) + MAX_DEFAULT_CHUNKS - 1) / MAX_DEFAULT_CHUNKS));
+    int k = 3;
+    while (((long long) 256 * TILE << k) < n_ctx) ++k;
+    return -k;
+}
+// the longest chunk of a full context
+int fixed_chunk(int n_ctx) {
+    const int CH = default_grid(n_ctx);
+    if (CH > 0) return CH;
+    const int c = chunk_of(CH, std::max(n_ctx, 1) - 1);
+    return (int) (chunk_lo(CH, c + 1) - chunk_lo(CH, c));
 }
 
 // Split partials and the work list live in one library-owned buffer per (device, stream), as in the reference
@@ -1121,10 +1198,10 @@ int fixed_chunk(int n_ctx) {
 // call on the stream drops it.
 struct plan_key {
     const void * scr = nullptr, * pos = nullptr, * p0p = nullptr;
-    int p0 = 0, n_slots = 0, q_len = 0, max_chunks = 0, max_cta = 0, Hkv = 0, n_ctx = 0, paged = 0;
+    int p0 = 0, n_slots = 0, q_len = 0, CH = 0, max_chunks = 0, max_cta = 0, Hkv = 0, n_ctx = 0, paged = 0;
     size_t part_floats = 0;
     bool operator==(const plan_key & o) const {
-        return scr == o.scr && pos == o.pos && p0p == o.p0p && p0 == o.p0 && n_slots == o.n_slots && q_len == o.q_len &&
+        return scr == o.scr && pos == o.pos && p0p == o.p0p && p0 == o.p0 && n_slots == o.n_slots && q_len == o.q_len && CH == o.CH &&
                max_chunks == o.max_chunks && max_cta == o.max_cta && Hkv == o.Hkv && n_ctx == o.n_ctx && paged == o.paged &&
                part_floats == o.part_floats;
     }
@@ -1359,7 +1436,7 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
     if (max_n < 1) max_n = 1;
     g.tc = false;
     g.R = q_len * GQA;
-    g.split = chunk_keys < 0 && n_slots > 1 && n_slots <= SPLIT_MAX_SLOTS;   // one sequence is even as it is: no plan launch
+    g.split = chunk_keys < 0 && n_slots <= SPLIT_MAX_SLOTS;
     g.planned = false;
     g.max_cta = 0;
     if (g.split) {
@@ -1374,8 +1451,8 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
         g.list_ints = (g.list_ints + 3) & ~(size_t) 3;
         return true;
     }
-    g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) : fixed_chunk(n_ctx);
-    g.max_chunks = (max_n + g.CH - 1) / g.CH;
+    g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) : default_grid(n_ctx);
+    g.max_chunks = chunk_of(g.CH, max_n - 1) + 1;
     g.units = (size_t) n_slots * Hkv * g.max_chunks;
     if (g.units >= ((size_t) 1 << 31) || (size_t) n_slots * g.max_chunks >= ((size_t) 1 << 30)) return false;
     g.part_floats = g.units * g.R * (DH + 2);
@@ -1403,21 +1480,25 @@ struct merge_out { float * out; const float * gate; float * fo, * fm, * fl; void
 // the kernels of one call, partials and work list in `scr`
 int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo, int n_slots, int q_len, const int32_t * pos,
                   const int32_t * p0p, int p0, int Hq, float scale, const dec_geom & gm, float * scr, unsigned * st, cudaStream_t s,
-                  const char * who, bool reuse_plan = false) {
+                  const char * who, bool reuse_plan = false, int hk0 = 0, int nhk = 0) {
     dec_args a;
     a.q = q; a.g = view_of(*c);
-    a.po = scr; a.pm = scr + gm.units * gm.R * DH; a.pl = a.pm + gm.units * gm.R;
+    const int heads = nhk ? nhk : c->Hkv;
+    const size_t units = gm.units / c->Hkv * heads, part_floats = units * gm.R * (DH + 2);
+    a.po = scr; a.pm = scr + units * gm.R * DH; a.pl = a.pm + units * gm.R;
     a.pos = pos; a.p0p = p0p; a.p0 = p0;
     a.q_len = q_len; a.n_slots = n_slots; a.Hq = Hq;
     a.qscale = scale * LOG2E;
     a.CH = gm.CH; a.max_chunks = gm.max_chunks; a.status = st;
+    a.hk0 = hk0; a.nhk = heads;
     a.n_ctx = c->n_ctx; a.tiled = 0;
     a.units = nullptr; a.n_units = nullptr;
     a.segs = nullptr; a.cta_seg = nullptr; a.slot_seg = nullptr; a.n_cta = nullptr;
     int launches = 2;
-    unsigned blocks = (unsigned) gm.units;
+    // fixed chunks: at most one wave of CTAs, which walk the units
+    unsigned blocks = (unsigned) std::min<size_t>((size_t) n_slots * a.nhk * gm.max_chunks, (size_t) resident_ctas(c->type, q_len));
     if (gm.split) {
-        int * list = reinterpret_cast<int *>(scr + gm.part_floats);
+        int * list = reinterpret_cast<int *>(scr + part_floats);
         const size_t nseg = (size_t) gm.max_cta + n_slots;
         int4 * segs = reinterpret_cast<int4 *>(list);
         int2 * slot_seg = reinterpret_cast<int2 *>(list + 4 * nseg);
@@ -1425,16 +1506,18 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
         int * n_cta = cta_seg + gm.max_cta + 1;
         a.segs = segs; a.cta_seg = cta_seg; a.slot_seg = slot_seg; a.n_cta = n_cta;
         if (!reuse_plan) {   // else the lists of an earlier call of this step, same shape, same positions, are still there
-            decode_split_k<<<1, SPLIT_THR, 0, s>>>(a, gm.max_cta, segs, cta_seg, slot_seg, n_cta);
+            decode_split_k<<<1, SPLIT_THR, 0, s>>>(a, gm.max_cta, gm.tc ? 2 : 1, segs, cta_seg, slot_seg, n_cta);
             ++launches;
         }
         blocks = (unsigned) gm.max_cta * (unsigned) c->Hkv;
     } else if (gm.planned) {
-        int * list = reinterpret_cast<int *>(scr + gm.part_floats);
+        int * list = reinterpret_cast<int *>(scr + part_floats);
         a.n_units = list;
         a.units = reinterpret_cast<const int2 *>(list + 4);
-        decode_plan_k<<<1, PLAN_THR, 0, s>>>(a, reinterpret_cast<int2 *>(list + 4), list);
-        ++launches;
+        if (!reuse_plan) {
+            decode_plan_k<<<1, PLAN_THR, 0, s>>>(a, reinterpret_cast<int2 *>(list + 4), list);
+            ++launches;
+        }
     }
     int rc;
     if (gm.split && gm.tc) rc = launch_tc_nc(a, blocks, s);
@@ -1442,8 +1525,14 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     else if (c->type == B200_KV_Q8_0) rc = launch_part_nt<B200_KV_Q8_0>(a, blocks, s);
     else rc = launch_part_nt<B200_KV_Q4_0>(a, blocks, s);
     if (rc != B200_OK) return rc;
-    if (gm.split) decode_merge_k<1><<<dim3(n_slots * q_len, Hq), 64, 0, s>>>(a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
-    else decode_merge_k<4><<<dim3(n_slots * q_len, Hq), 256, 0, s>>>(a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    // Partials that a row of a typical slot has.  Measured on 24 rows x heads (q8_0, 16384 / 131072 keys): the 30 us that four groups of 64
+    // threads took to walk 256 partials one after the other become 5 us with 16 groups; with up to 8 partials one group of 64
+    // threads per row keeps a launch of thousands of rows to one wave.
+    const int parts = gm.split ? gm.max_cta / n_slots + 2 : gm.max_chunks;
+    const dim3 mg(n_slots * q_len, GQA * a.nhk);
+    if (gm.split && parts <= 8) decode_merge_k<1><<<mg, 64, 0, s>>>(a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    else if (parts <= 32) decode_merge_k<4><<<mg, 256, 0, s>>>(a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    else decode_merge_k<16><<<mg, 1024, 0, s>>>(a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
     count_launch(launches);
     return launch_status(who);
 }
@@ -1467,12 +1556,13 @@ int decode_impl(const float * q, const b200_kv_cache * c, const merge_out & mo, 
     unsigned * st = device_status_word();
     if (!st) return B200_ERR_CUDA;
     plan_key k;
-    k.scr = scr; k.pos = pos; k.p0p = p0p; k.p0 = p0; k.n_slots = n_slots; k.q_len = q_len; k.max_chunks = gm.max_chunks;
+    k.scr = scr; k.pos = pos; k.p0p = p0p; k.p0 = p0; k.n_slots = n_slots; k.q_len = q_len; k.CH = gm.CH; k.max_chunks = gm.max_chunks;
     k.max_cta = gm.max_cta; k.Hkv = c->Hkv; k.n_ctx = c->n_ctx; k.paged = c->pt != nullptr; k.part_floats = gm.part_floats;
     const bool in_step = e->step_mode && pos && (const char *) pos >= e->step_lo && (const char *) pos < e->step_hi;
-    const bool reuse = gm.split && in_step && e->plan_valid && k == e->key;
+    const bool listed = gm.split || gm.planned;
+    const bool reuse = listed && in_step && e->plan_valid && k == e->key;
     const int rc = decode_launch(q, c, mo, n_slots, q_len, pos, p0p, p0, Hq, scale, gm, scr, st, s, who, reuse);
-    e->plan_valid = gm.split && in_step && rc == B200_OK;   // any other call on the stream rewrites the scratch
+    e->plan_valid = listed && in_step && rc == B200_OK;   // any other call on the stream rewrites the scratch
     e->key = k;
     return rc;
 }
@@ -1521,15 +1611,24 @@ int decode_noalloc_impl(const float * q, const b200_kv_cache * c, float * out, c
     if (chk != B200_OK) return chk;
     dec_geom gm;
     const bool ok = decode_geometry(gm, c->type, n_slots, q_len, max_n, c->n_ctx, c->Hkv, chunk_keys, tc_eligible(*c, q_len));
-    const size_t need = ok ? gm.part_floats + gm.list_ints : 0;
-    if (!ok || need > NOALLOC_FLOATS)
-        B200_REFUSE(B200_ERR_SCRATCH, "%s: %zu bytes of split partials needed (slots %d x kv heads %d x chunks %d x rows %d), the built-in array holds %zu; "
-                    "use a larger chunk_keys or attn_decode_slots", who, need * sizeof(float), n_slots, c->Hkv, ok ? gm.max_chunks : -1, q_len * GQA, NOALLOC_BYTES);
+    // the kv heads go in as many groups as the array needs (the partials of a fixed chunk grid are independent of one another)
+    const size_t per_head = ok ? gm.part_floats / c->Hkv : 0;
+    int nhk = ok ? c->Hkv : 0;
+    if (ok && gm.part_floats + gm.list_ints > NOALLOC_FLOATS)
+        nhk = gm.split || gm.list_ints >= NOALLOC_FLOATS ? 0 : (int) ((NOALLOC_FLOATS - gm.list_ints) / per_head);
+    if (nhk < 1)
+        B200_REFUSE(B200_ERR_SCRATCH, "%s: %zu bytes of split partials needed (slots %d x kv heads %d x chunks %d x rows %d), the built-in array holds %zu for one kv head at "
+                    "least; use a larger chunk_keys or attn_decode_slots", who, (gm.part_floats + gm.list_ints) * sizeof(float), n_slots, c->Hkv, ok ? gm.max_chunks : -1,
+                    q_len * GQA, NOALLOC_BYTES);
     noalloc_dev e;
     const int src = noalloc_setup(e);
     if (src != B200_OK) return src;
     const merge_out mo = {out, gate, nullptr, nullptr, nullptr, nullptr};
-    return decode_launch(q, c, mo, n_slots, q_len, pos, nullptr, 0, Hq, scale, gm, e.partials, e.status, s, who);
+    for (int h0 = 0; h0 < c->Hkv; h0 += nhk) {
+        const int rc = decode_launch(q, c, mo, n_slots, q_len, pos, nullptr, 0, Hq, scale, gm, e.partials, e.status, s, who, false, h0, std::min(nhk, c->Hkv - h0));
+        if (rc != B200_OK) return rc;
+    }
+    return B200_OK;
 }
 
 }  // namespace b200
@@ -1562,7 +1661,7 @@ int b200_attn_fixed_chunk(int n_ctx) { return fixed_chunk(n_ctx); }
 
 int b200_attn_dec2_nsplit(int Hkv) {
     (void) Hkv;   // the reference derives its stream count from the SM count and Hkv; here the split follows the context
-    return g_nsplit_override > 0 ? g_nsplit_override : MAX_DEFAULT_CHUNKS;
+    return g_nsplit_override > 0 ? g_nsplit_override : NOMINAL_NSPLIT;
 }
 void b200_attn_dec2_set_nsplit(int n) { g_nsplit_override = n > 0 ? n : 0; }
 int b200_attn_step_begin(void * stream, const int32_t * positions, size_t bytes) {

@@ -1,0 +1,80 @@
+"""Decode attention where the key split can go wrong: ends of contexts inside a 64-key tile, with page rows past the end that
+hold anything; boundaries of the default chunk grid; one slot with the even split; the allocation-free entry in head groups."""
+import numpy as np
+import pytest
+
+from oracle import orc
+from tests import util
+from tests.util import D, HKV, HQ, SCALE, TYPES
+
+pytestmark = pytest.mark.gpu
+
+
+def _paged(cuda, kt, n, seed, hkv=HKV, extra_pages=0):
+    """one sequence of n positions in 256-row pages; every byte of the pool that is not a stored row is 0xff (f16 NaN)"""
+    import torch
+    from p100e_engine_b200 import fast
+    npg = (n + 255) // 256
+    pool = util.PagedPool(kt, npg + 1, psh=8, hkv=hkv, seed=seed)
+    pt = pool.take(n, npg + extra_pages)
+    pool_t = torch.full((pool.bytes,), 0xff, dtype=torch.uint8, device=cuda)
+    c = util.dev_cache(pool_t, pool, util.to_dev(pt, cuda), None, (npg + extra_pages) << 8)
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    for p in range(0, n, 8192):
+        T = min(8192, n - p)
+        assert fast.kv_append(c, torch.randn(T, hkv, D, generator=g, device=cuda), torch.randn(T, hkv, D, generator=g, device=cuda), p, T)
+    torch.cuda.synchronize()
+    pool.host[:pool.bytes] = pool_t.cpu().numpy()
+    return c, pool.host_cache(pt), pool_t
+
+
+@pytest.mark.parametrize("tname", ["q8_0", "f16", "q4_0"])
+@pytest.mark.parametrize("n", [1, 63, 65, 257, 4095, 4097, 8193, 16385 + 31])
+def test_ragged_ends_and_grid_boundaries(cuda, lib, tname, n):
+    """f16 products of f16 operands summed in fp32: held to the usual bar (2e-3 of the largest output, 1e-2 rms)"""
+    import torch
+    from p100e_engine_b200 import fast
+    c, hc, _keep = _paged(cuda, TYPES[tname], n, n)
+    for T in (1, 4):
+        if T > n:
+            continue
+        q = util.rng_normal(n + T, (T, HQ, D))
+        qd, pos = util.to_dev(q, cuda), torch.arange(n - T, n, dtype=torch.int32, device=cuda)
+        ref = orc.attention(q, hc, T, HQ, SCALE, p0=n - T)
+        a, b = (torch.full((T, HQ, D), float("nan"), device=cuda) for _ in range(2))
+        assert fast.attn_decode(qd, c, a, T, n - T, HQ, SCALE)                                   # default grid
+        assert fast.attn_decode_slots(qd, c, b, None, 1, T, pos, n, HQ, SCALE, -1)                # even split of one slot
+        torch.cuda.synchronize()
+        util.check_close(a.cpu().numpy(), ref, "default grid %s n=%d T=%d" % (tname, n, T))
+        util.check_close(b.cpu().numpy(), ref, "even split %s n=%d T=%d" % (tname, n, T))
+    assert fast.device_status() == 0
+
+
+def test_rows_do_not_depend_on_the_call_across_grid_boundaries(cuda, lib):
+    """row t of a call that straddles a boundary of the chunk grid == the one-row call, bit for bit, also as one of several
+    slots (work list) and through the allocation-free entry, whose kv heads then go in groups"""
+    import torch
+    from p100e_engine_b200 import fast
+    n = 12000
+    c, _, _keep = _paged(cuda, TYPES["q8_0"], n, 5, extra_pages=50)
+    q = util.to_dev(util.rng_normal(6, (4, HQ, D)), cuda)
+    for p0 in (4094, 8190, n - 4):
+        out, one = torch.zeros(4, HQ, D, device=cuda), torch.zeros(4, HQ, D, device=cuda)
+        assert fast.attn_decode(q, c, out, 4, p0, HQ, SCALE)
+        for t in range(4):
+            assert fast.attn_decode(q[t:t + 1], c, one[t:t + 1], 1, p0 + t, HQ, SCALE)
+        rows = torch.zeros(8, HQ, D, device=cuda)
+        pos8 = torch.tensor([p0 + t for t in range(4)] + [n - 1 - t for t in range(4)], dtype=torch.int32, device=cuda)
+        c.rtab = torch.zeros(8, dtype=torch.int32, device=cuda)
+        assert fast.attn_decode_rows(torch.cat([q, q]), c, rows, 8, pos8, HQ, SCALE)
+        pos4 = pos8[:4].contiguous()
+        free = torch.zeros(4, HQ, D, device=cuda)
+        assert fast.attn_decode_slots_noalloc(q, c, free, None, 1, 4, pos4, n, HQ, SCALE, 64) == 0    # 188 chunks: three heads fit
+        pinned = torch.zeros(4, HQ, D, device=cuda)
+        assert fast.attn_decode_slots(q, c, pinned, None, 1, 4, pos4, n, HQ, SCALE, 64)
+        torch.cuda.synchronize()
+        assert torch.equal(out, one), p0
+        assert torch.equal(rows[:4], out), p0
+        assert torch.equal(free, pinned), p0
+    assert fast.device_status() == 0
+    assert fast.noalloc_device_status() == 0
