@@ -130,7 +130,41 @@ struct pf_args {
     int T, p0, Hq, Hkv;
     float qscale;                 // softmax scale * log2(e)
     unsigned * status;
+    // even split (n_run > 0; one pass, no lim): see pf_cut
+    int n_run;                    // CTAs
+    int n_mtiles;                 // row tiles of a kv head
+    int head_steps;               // 128-key steps of a kv head, all row tiles together
+    float * po;                   // [2 n_run][128][256] unnormalised O of the pieces
+    float2 * pml;                 // [2 n_run][128] (maximum in log2 units, sum)
 };
+
+// Even split: the 128-key steps of all row tiles (kv head by kv head, row tile by row tile) form one sequence of
+// Hkv * head_steps; CTA c of n_run takes steps pf_cut(c) .. pf_cut(c + 1) - 1.  A row tile whose steps lie in several CTAs is left
+// as pieces, unnormalised, which prefill_merge_k adds up in key order: a CTA's piece that starts a row tile is number 2 c + 1, one that
+// continues a row tile number 2 c (a CTA has at most one of each).
+__host__ __device__ __forceinline__ int pf_tile_steps(int T, int p0, int m) {
+    const int n_last = m * BM + BM < T * GQA ? m * BM + BM - 1 : T * GQA - 1;
+    return (p0 + n_last / GQA + BP) / BP;   // ceil(visible keys / 128)
+}
+__device__ __forceinline__ int pf_cut(const pf_args & a, int c) { return (int) ((long long) a.Hkv * a.head_steps * c / a.n_run); }
+// row tile of a kv head that holds step `rem` of the head and the head's steps before that tile; called by a whole warp
+__device__ __forceinline__ int pf_find_tile(const pf_args & a, int rem, int & before) {
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    for (int m0 = 0;; m0 += 32) {
+        const int m = m0 + lane, own = m < a.n_mtiles ? pf_tile_steps(a.T, a.p0, m) : 0;
+        int x = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
+        const unsigned past = __ballot_sync(0xffffffffu, base + x > rem);
+        if (past || m0 + 32 >= a.n_mtiles) {
+            const int l = past ? __ffs(past) - 1 : 31;
+            before = base + __shfl_sync(0xffffffffu, x - own, l);
+            return m0 + l;
+        }
+        base += __shfl_sync(0xffffffffu, x, 31);
+    }
+}
 
 // 1 / (1 + 2^(-g log2 e)) with the hardware exponential and reciprocal (relative error ~1e-7 against expf and an IEEE divide)
 __device__ __forceinline__ float fast_sigmoid(float g) { return __fdividef(1.0f, 1.0f + ex2f(-g * LOG2E_PF)); }
@@ -152,21 +186,24 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
              * p_full = bars + 12, * pv_done = bars + 14, * o_done = bars + 16, * q_ready = bars + 17;
     uint32_t * tbase_p = reinterpret_cast<uint32_t *>(bars + 18);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int mtile = (int) gridDim.x - 1 - (int) blockIdx.x;   // heaviest (latest rows) first
-    const int hk = blockIdx.y;
-    const int R = a.T * GQA;                                    // rows of this kv head
-    const int n0 = mtile * BM;
-    const int t_last = min(n0 + BM - 1, R - 1) / GQA;           // last token of the tile
-    const int n_keys_vis = (a.lim ? a.lim[t_last] : a.p0 + t_last) + 1;   // keys any row of the tile can see (limits do not decrease with t)
-    // This pass covers keys kb .. ke-1.  A tile whose keys ended in an earlier pass has been written already; a tile
-    // whose keys go on past ke leaves its running state behind for the next pass.
-    if (n_keys_vis <= a.kb && a.kb > 0) return;
-    const bool carry_in = a.kb > 0;
-    const bool carry_out = n_keys_vis > a.ke;
-    const int n_keys_pass = max(0, min(n_keys_vis, a.ke) - a.kb);
-    const int ntiles = (n_keys_pass + BN - 1) / BN;             // 64-key images of this pass
-    const int nsteps = (ntiles + 1) / 2;                        // 128-key steps; the last one may hold a single image
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);     // as a warp-uniform value
+    const int R = a.T * GQA;                                    // rows of a kv head
+    // the segments of this CTA: one row tile, or (even split) the row tiles of its run of steps
+    int hk = blockIdx.y, mtile = (int) gridDim.x - 1 - (int) blockIdx.x;   // one tile per CTA: heaviest (latest rows) first
+    int st0 = 0, w = 0, w_end = 0;
+    if (a.n_run) {
+        w = pf_cut(a, (int) blockIdx.x); w_end = pf_cut(a, (int) blockIdx.x + 1);
+        hk = w / a.head_steps;
+        int before;
+        mtile = pf_find_tile(a, w - hk * a.head_steps, before);
+        st0 = w - hk * a.head_steps - before;
+    } else {
+        // This pass covers keys kb .. ke-1.  A tile whose keys ended in an earlier pass has been written already; a tile
+        // whose keys go on past ke leaves its running state behind for the next pass.
+        const int t_l = min(mtile * BM + BM - 1, R - 1) / GQA;
+        if ((a.lim ? a.lim[t_l] : a.p0 + t_l) < a.kb && a.kb > 0) return;
+    }
 
     if (tid == 0) {
         mbar_init(k_full, 1); mbar_init(k_free, 1); mbar_init(s_full, 1); mbar_init(s_free, NSOFT);
@@ -188,6 +225,20 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
     // tensor-memory lanes; for row-wise global accesses 8 lanes cover 128 bytes of one row, a warp instruction touches 4 rows
     const uint32_t lane_off = (uint32_t) ((warp & 3) * 32) << 16;
     const int sub = lane >> 3, col = 4 * (lane & 7);
+
+    int g = 0, gi = 0;   // steps and 64-key images of the earlier segments: the barriers' phases run on from one segment to the next
+    for (int seg = 0;; ++seg) {
+    const int n0 = mtile * BM;
+    const int t_last = min(n0 + BM - 1, R - 1) / GQA;           // last token of the tile
+    const int n_keys_vis = (a.lim ? a.lim[t_last] : a.p0 + t_last) + 1;   // keys any row of the tile can see (limits do not decrease with t)
+    const bool carry_in = a.kb > 0;
+    const bool carry_out = n_keys_vis > a.ke;
+    const int n_keys_pass = max(0, min(n_keys_vis, a.ke) - a.kb);
+    const int tile_steps = (n_keys_pass + BP - 1) / BP;
+    const int st1 = a.n_run ? min(tile_steps, st0 + w_end - w) : tile_steps;
+    const int nsteps = st1 - st0;                               // 128-key steps of this segment; a tile's last one may hold a single image
+    const int ntiles = min((n_keys_pass + BN - 1) / BN, 2 * st1) - 2 * st0;   // 64-key images of this segment
+    const bool piece = nsteps < tile_steps;                     // the tile is shared with other CTAs
     float m_ref = B200_NEG_INF, l = 0.0f;
 
     if (warp < W_PROD) {
@@ -272,7 +323,7 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
         if (tid == 0) mbar_arrive(q_ready);
     }
     const bool any_gate = a.gate || a.gate_b;
-    if (warp >= W_PROD && any_gate && !carry_out && (lane & 15) != 0) {
+    if (warp >= W_PROD && any_gate && !carry_out && !piece && (lane & 15) != 0) {
         // idle lanes of the producer and MMA warps pull this CTA's gate rows (contiguous per token: 6 heads) into L2
         const int t_first = n0 / GQA;
         const int esz = a.gate ? 4 : 2;
@@ -285,10 +336,10 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
     }
     if (warp == W_PROD) {
         // ---------------- producer: K in pairs of images (lane 0), V image by image through a ring (lane 16) ----------------
-        const unsigned char * src = a.tiles + (size_t) hk * a.n_tiles * (2 * IMG);
+        const unsigned char * src = a.tiles + ((size_t) hk * a.n_tiles + 2 * st0) * (2 * IMG);
         if (lane == 0) {
             for (int J = 0; J < nsteps; ++J) {
-                if (J >= 1) mbar_wait(k_free, (uint32_t) ((J - 1) & 1), a.status);   // Q K^T of step J-1 has read the pair
+                if (g + J >= 1) mbar_wait(k_free, (uint32_t) ((g + J - 1) & 1), a.status);   // Q K^T of step J-1 has read the pair
                 const int n_img = min(2, ntiles - 2 * J);
                 mbar_expect_tx(k_full, (uint32_t) n_img * IMG);
                 for (int h = 0; h < n_img; ++h)
@@ -296,59 +347,71 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
             }
         } else if (lane == 16) {
             for (int j = 0; j < ntiles; ++j) {
-                const int s = j % NSTG;
-                if (j >= NSTG) mbar_wait(&v_free[s], (uint32_t) ((j / NSTG - 1) & 1), a.status);   // P V of image j-NSTG has read the slot
+                const int s = (gi + j) % NSTG;
+                if (gi + j >= NSTG) mbar_wait(&v_free[s], (uint32_t) (((gi + j) / NSTG - 1) & 1), a.status);   // P V of image j-NSTG has read the slot
                 mbar_expect_tx(&v_full[s], IMG);
                 bulk_g2s(smem + SM_V + s * IMG, src + (size_t) j * (2 * IMG) + IMG, IMG, &v_full[s]);
             }
         }
     } else if (warp == W_MMA) {
         // ---------------- MMA issuer: Q K^T of step J+1 is queued before P V of step J ----------------
-        if (lane == 0) {
-            constexpr uint32_t id_qk = umma::idesc_f16(BM, BP, false, false);   // S[128 x 128] = Q (tensor memory) * K^T (K-major)
-            constexpr uint32_t id_pv = umma::idesc_f16(BM, DH, false, true);    // O[128 x 256] += P (K-major) * V (MN-major)
-            const uint32_t k_s = smem_u32(smem + SM_K);
-            auto issue_qk = [&](int J) {
-                mbar_wait(k_full, (uint32_t) (J & 1), a.status);
-                if (J >= 1) mbar_wait(s_free, (uint32_t) ((J - 1) & 1), a.status);   // the softmax threads hold S of step J-1 in registers
-                umma::fence_after_sync();
-                // K pair: K-major, 8-key groups 4096 apart (SBO), 8-dim chunks 128 apart (LBO); 16 dims = 256 bytes per k-step.
-                // A step with a single image multiplies whatever the second half of the buffer holds: those keys lie past
-                // every row of the tile and are masked.
-#pragma unroll 4
+        // All 32 lanes walk the loop and wait, so that addresses and descriptors are warp-uniform values (the MMA takes its
+        // operands from uniform registers); one elected lane issues.
+        __syncwarp();
+        const bool lead = umma::elect_one();
+        const uint32_t tb_u = __shfl_sync(0xffffffffu, tb, 0);
+        const uint32_t tS_u = tb_u, tO_u = tb_u + BP, tQ_u = tb_u + BP + DH;
+        const int ns_u = __shfl_sync(0xffffffffu, nsteps, 0), ni_u = __shfl_sync(0xffffffffu, ntiles, 0), g_u = __shfl_sync(0xffffffffu, g, 0);
+        int gj = __shfl_sync(0xffffffffu, gi, 0);   // images before the next P V
+        constexpr uint32_t id_qk = umma::idesc_f16(BM, BP, false, false);   // S[128 x 128] = Q (tensor memory) * K^T (K-major)
+        constexpr uint32_t id_pv = umma::idesc_f16(BM, DH, false, true);    // O[128 x 256] += P (K-major) * V (MN-major)
+        const uint32_t k_s = smem_u32(smem + SM_K), v_s0 = smem_u32(smem + SM_V), p_s0 = smem_u32(smem + SM_P);
+        auto issue_qk = [&](int J) {
+            const int G = g_u + J;
+            mbar_wait(k_full, (uint32_t) (G & 1), a.status);
+            if (G >= 1) mbar_wait(s_free, (uint32_t) ((G - 1) & 1), a.status);   // the softmax threads hold S of the step before in registers
+            umma::fence_after_sync();
+            // K pair: K-major, 8-key groups 4096 apart (SBO), 8-dim chunks 128 apart (LBO); 16 dims = 256 bytes per k-step.
+            // A step with a single image multiplies whatever the second half of the buffer holds: those keys lie past
+            // every row of the tile and are masked.
+            if (lead) {
+#pragma unroll
                 for (int ks = 0; ks < DH / 16; ++ks)
-                    umma::mma_ts(t_S, t_Q + ks * 8, umma::smem_desc(k_s + ks * 256, 128, 4096), id_qk, ks > 0);
+                    umma::mma_ts(tS_u, tQ_u + ks * 8, umma::smem_desc(k_s + ks * 256, 128, 4096), id_qk, ks > 0);
                 umma::commit(s_full);
                 umma::commit(k_free);
-            };
-            auto issue_pv = [&](int J) {
-                const int b = J & 1;
-                mbar_wait(&p_full[b], (uint32_t) ((J >> 1) & 1), a.status);
-                const uint32_t p_s = smem_u32(smem + SM_P + b * P_BYTES);
-                const int n_img = min(2, ntiles - 2 * J);
-                for (int h = 0; h < n_img; ++h) {
-                    const int j = 2 * J + h, st = j % NSTG;
-                    mbar_wait(&v_full[st], (uint32_t) ((j / NSTG) & 1), a.status);
-                    umma::fence_after_sync();
-                    const uint32_t v_s = smem_u32(smem + SM_V + st * IMG);
+            }
+        };
+        auto issue_pv = [&](int J) {
+            const int G = g_u + J, b = G & 1;
+            mbar_wait(&p_full[b], (uint32_t) ((G >> 1) & 1), a.status);
+            const int n_img = min(2, ni_u - 2 * J);
+            for (int h = 0; h < n_img; ++h, ++gj) {
+                const int st = gj % NSTG;
+                mbar_wait(&v_full[st], (uint32_t) ((gj / NSTG) & 1), a.status);
+                umma::fence_after_sync();
+                if (lead) {
+                    const uint32_t v_s = v_s0 + st * IMG, p_s = p_s0 + b * P_BYTES + h * 8 * 2048;
+                    const uint32_t acc0 = (carry_in || J > 0 || h > 0) ? 1u : 0u;
 #pragma unroll
                     for (int ks = 0; ks < BN / 16; ++ks)   // P: K-major, 8-key chunks 2048 apart; V: MN-major, 8-key groups 4096 apart (LBO),
                                                            // 8-dim chunks 128 apart (SBO)
-                        umma::mma_ss(t_O, umma::smem_desc(p_s + (h * 4 + ks) * 2 * 2048, 2048, 128),
-                                     umma::smem_desc(v_s + ks * 2 * 4096, 4096, 128), id_pv, (carry_in || j > 0 || ks > 0) ? 1u : 0u);
+                        umma::mma_ss(tO_u, umma::smem_desc(p_s + ks * 2 * 2048, 2048, 128),
+                                     umma::smem_desc(v_s + ks * 2 * 4096, 4096, 128), id_pv, ks > 0 ? 1u : acc0);
                     umma::commit(&v_free[st]);
                 }
-                umma::commit(&pv_done[b]);
-            };
-            mbar_wait(q_ready, 0, a.status);
-            umma::fence_after_sync();
-            if (nsteps > 0) issue_qk(0);
-            for (int J = 0; J < nsteps; ++J) {
-                if (J + 1 < nsteps) issue_qk(J + 1);
-                issue_pv(J);
             }
-            umma::commit(o_done);
+            if (lead) umma::commit(&pv_done[b]);
+        };
+        mbar_wait(q_ready, (uint32_t) (seg & 1), a.status);
+        umma::fence_after_sync();
+        if (ns_u > 0) issue_qk(0);
+        for (int J = 0; J < ns_u; ++J) {
+            if (J + 1 < ns_u) issue_qk(J + 1);
+            issue_pv(J);
         }
+        if (lead) umma::commit(o_done);
+        __syncwarp();
     } else {
         // ---------------- softmax: two threads per row ----------------
         // Thread (row r, half hf) owns keys 64 hf .. 64 hf + 63 of every step and, in the epilogue, output dims 128 hf ..
@@ -360,7 +423,8 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
         const int pair_bar = 2 + (warp & 3);
         float * xch = reinterpret_cast<float *>(smem + SM_XCH);
         for (int J = 0; J < nsteps; ++J) {
-            mbar_wait(s_full, (uint32_t) (J & 1), a.status);
+            const int G = g + J;
+            mbar_wait(s_full, (uint32_t) (G & 1), a.status);
             umma::fence_after_sync();
             uint32_t sr[2][32];
             umma::tmem_ld32(t_S + lane_off + 64 * hf, sr[0]);
@@ -368,7 +432,7 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
             umma::tmem_ld_wait();
             umma::fence_before_sync();
             mbar_arrive(s_free);   // S is in registers: the next Q K^T may overwrite it
-            const int k0 = a.kb + J * BP + 64 * hf;
+            const int k0 = a.kb + (st0 + J) * BP + 64 * hf;
             const bool diag = k0 + 63 > pos;   // some key of this half is masked for this row
             if (__any_sync(0xffffffffu, diag)) {
 #pragma unroll
@@ -400,7 +464,7 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
                     l *= f;
                 }
                 if (J > 0 || carry_in) {
-                    if (J > 0) mbar_wait(&pv_done[(J - 1) & 1], (uint32_t) (((J - 1) >> 1) & 1), a.status);   // P V of step J-1 has landed in O
+                    if (J > 0) mbar_wait(&pv_done[(G - 1) & 1], (uint32_t) (((G - 1) >> 1) & 1), a.status);   // P V of step J-1 has landed in O
                     umma::fence_after_sync();
 #pragma unroll 1
                     for (int c0 = hf * (DH / 2); c0 < (hf + 1) * (DH / 2); c0 += 32) {
@@ -416,9 +480,9 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
                 }
             }
             const float mref_safe = m_ref == B200_NEG_INF ? 0.0f : m_ref;
-            if (J >= 2) mbar_wait(&pv_done[J & 1], (uint32_t) (((J >> 1) - 1) & 1), a.status);   // P buffer no longer read
+            if (G >= 2) mbar_wait(&pv_done[G & 1], (uint32_t) (((G >> 1) - 1) & 1), a.status);   // P buffer no longer read
             // K-major P image of the step: key chunk kc (8 keys) at kc * 2048, row at 16 bytes; this thread's chunks are 8 hf ..
-            unsigned char * prow = smem + SM_P + (J & 1) * P_BYTES + (8 * hf) * 2048 + r * 16;
+            unsigned char * prow = smem + SM_P + (G & 1) * P_BYTES + (8 * hf) * 2048 + r * 16;
             float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int h = 0; h < 2; ++h)
@@ -438,7 +502,7 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
             l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
             umma::fence_async_smem();
             umma::fence_before_sync();
-            mbar_arrive(&p_full[J & 1]);
+            mbar_arrive(&p_full[G & 1]);
         }
         // ---------------- epilogue ----------------
         // final:   O / l, gate, store (f32 and / or bf16, a16 copy);  carry_out: unnormalised O, (maximum, sum) for the next pass;
@@ -446,14 +510,16 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
         xch[hf * BM + r] = l;
         asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
         l = xch[r] + xch[BM + r];
-        mbar_wait(o_done, 0, a.status);
+        mbar_wait(o_done, (uint32_t) (seg & 1), a.status);
         umma::fence_after_sync();
-        const bool raw = carry_out || a.pm;   // O leaves unnormalised
+        const bool raw = carry_out || a.pm || piece;   // O leaves unnormalised
+        const size_t slot = 2 * (size_t) blockIdx.x + (st0 == 0 ? 1 : 0);   // number of the piece
         const bool have_o = nsteps > 0 || carry_in;   // a tile that has seen no key at all (a sequence shard) holds nothing in O
         const float inv = raw ? 1.0f : (l > 0.0f ? 1.0f / l : 0.0f);
         if (n < R && hf == 0) {
             const size_t rowidx = (size_t) t_row * a.Hq + hk * GQA + (n - t_row * GQA);
-            if (carry_out) { a.ml[rowidx * 2] = m_ref; a.ml[rowidx * 2 + 1] = l; }
+            if (piece) a.pml[slot * BM + r] = make_float2(m_ref, l);
+            else if (carry_out) { a.ml[rowidx * 2] = m_ref; a.ml[rowidx * 2 + 1] = l; }
             else if (a.pm) { a.pm[rowidx] = m_ref * 0.6931471805599453f; a.pl[rowidx] = l; }
         }
         // A 32-column slab of O goes through a private shared-memory tile so that global accesses run along rows.
@@ -466,7 +532,7 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
             const int nr = n0 + (warp & 3) * 32 + 4 * q8 + sub;
             const int tr = nr / GQA, hr = nr - tr * GQA;
             live[q8] = nr < R;
-            orow[q8] = ((size_t) tr * a.Hq + hk * GQA + hr) * DH + col;
+            orow[q8] = piece ? (slot * BM + nr - n0) * DH + col : ((size_t) tr * a.Hq + hk * GQA + hr) * DH + col;
         }
         const bool gated = any_gate && !raw;
         auto gate_at = [&](size_t o) {
@@ -507,7 +573,7 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
                     y.z *= fast_sigmoid(gv[q8].z); y.w *= fast_sigmoid(gv[q8].w);
                 }
                 if (live[q8]) {
-                    if (raw || !a.out_b) *reinterpret_cast<float4 *>(a.out + orow[q8] + c0) = y;
+                    if (raw || !a.out_b) *reinterpret_cast<float4 *>((piece ? a.po : a.out) + orow[q8] + c0) = y;
                     if (!raw && a.out_b) {
                         const __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
                         *reinterpret_cast<uint2 *>(a.out_b + orow[q8] + c0) =
@@ -519,16 +585,83 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
             }
             __syncwarp();
         }
+        umma::fence_async_smem();   // the epilogue tiles lie where the next segment's K images are copied to
     }
     umma::fence_before_sync();
     __syncthreads();
+    umma::fence_after_sync();
+    g += nsteps; gi += ntiles;
+    w += nsteps;
+    if (w >= w_end) break;
+    st0 = 0;
+    if (++mtile == a.n_mtiles) { mtile = 0; ++hk; }
+    }
     if (warp == 0) umma::tmem_dealloc(tb, 512);
+}
+
+// Adds up the pieces of the row tiles that the even split cut, in key order, and finishes them like prefill_k does: 1/l, gate, f32 or
+// bf16 result, a16 copy.  grid (row tiles x 16, kv heads), a warp per row, eight values per lane: values 4 l .. 4 l + 3 of both 128-dim halves.
+__global__ void __launch_bounds__(256) prefill_merge_k(const pf_args a) {
+    const int m = blockIdx.x >> 4, hk = blockIdx.y, lane = threadIdx.x & 31;
+    const int r = (blockIdx.x & 15) * 8 + (threadIdx.x >> 5), n = m * BM + r;
+    // the CTAs that hold the tile's first and last step
+    int before = 0;
+    for (int m0 = 0; m0 < m; m0 += 32) before += m0 + lane < m ? pf_tile_steps(a.T, a.p0, m0 + lane) : 0;
+    before = __reduce_add_sync(0xffffffffu, before);
+    const long long W = (long long) a.Hkv * a.head_steps;
+    const int first = hk * a.head_steps + before, last = first + pf_tile_steps(a.T, a.p0, m) - 1;
+    auto cta_of = [&](int step) {
+        int c = (int) ((long long) step * a.n_run / W);
+        while (c + 1 < a.n_run && pf_cut(a, c + 1) <= step) ++c;
+        return c;
+    };
+    const int c0 = cta_of(first), c1 = cta_of(last);
+    if (c0 == c1 || n >= a.T * GQA) return;   // the whole tile ran in one CTA, which has written the result
+    auto piece = [&](int c) { return (size_t) (c == c0 ? 2 * c + 1 : 2 * c) * BM + r; };
+    float M = B200_NEG_INF;
+    for (int c = c0; c <= c1; ++c) M = fmaxf(M, a.pml[piece(c)].x);
+    float l = 0.0f;
+    float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f), y = x;
+#pragma unroll 4
+    for (int c = c0; c <= c1; ++c) {
+        const size_t i = piece(c);
+        const float2 ml = a.pml[i];
+        const float4 u = reinterpret_cast<const float4 *>(a.po + i * DH)[lane], v = reinterpret_cast<const float4 *>(a.po + i * DH)[32 + lane];
+        const float f = ml.x == B200_NEG_INF ? 0.0f : ex2f(ml.x - M);   // -inf: the row saw none of the piece's keys
+        l = fmaf(f, ml.y, l);
+        x.x = fmaf(f, u.x, x.x); x.y = fmaf(f, u.y, x.y); x.z = fmaf(f, u.z, x.z); x.w = fmaf(f, u.w, x.w);
+        y.x = fmaf(f, v.x, y.x); y.y = fmaf(f, v.y, y.y); y.z = fmaf(f, v.z, y.z); y.w = fmaf(f, v.w, y.w);
+    }
+    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+    const int t = n / GQA;
+    const size_t row = ((size_t) t * a.Hq + hk * GQA + (n - t * GQA)) * DH;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        float4 z = h ? y : x;
+        const size_t o = row + 128 * h + 4 * lane;
+        z.x *= inv; z.y *= inv; z.z *= inv; z.w *= inv;
+        if (a.gate || a.gate_b) {
+            float4 gv;
+            if (a.gate) gv = *reinterpret_cast<const float4 *>(a.gate + o);
+            else {
+                const uint2 u = *reinterpret_cast<const uint2 *>(a.gate_b + o);
+                gv = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+            }
+            z.x *= fast_sigmoid(gv.x); z.y *= fast_sigmoid(gv.y); z.z *= fast_sigmoid(gv.z); z.w *= fast_sigmoid(gv.w);
+        }
+        if (a.out_b) {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(z.x, z.y), hi = __floats2bfloat162_rn(z.z, z.w);
+            *reinterpret_cast<uint2 *>(a.out_b + o) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+        } else *reinterpret_cast<float4 *>(a.out + o) = z;
+        if (a.qbuf) a16_store_lanes8(z, a.qbuf, o / 32, (size_t) a.T * a.Hq * (DH / 32), true);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ host side ----
 constexpr size_t TILE_BYTES_PER_KEY = 2 * IMG / BN;   // K and V images: 1 KiB per key and kv head
 constexpr int DEFAULT_PASS_KEYS = 8192;               // keys per pass that attn_fold_scratch_bytes(T, Hkv, 0, 0) provides for
-constexpr size_t OWN_SCRATCH_TILE_CAP = (size_t) 256 << 20;   // library scratch holds tile images for at most this many bytes per pass
+constexpr size_t OWN_SCRATCH_TILE_CAP = (size_t) 640 << 20;   // library scratch holds tile images for at most this many bytes per pass,
+constexpr size_t OWN_SCRATCH_TILE_LOW = (size_t) 256 << 20;   // or this many where that much memory cannot be had
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t) 255; }
 size_t ml_bytes(int T, int Hkv) { return align256((size_t) T * Hkv * GQA * 2 * sizeof(float)); }
@@ -539,30 +672,49 @@ size_t tile_bytes(int keys, int Hkv) { return (size_t) ((keys + BP - 1) / BP * B
 // A later call that needs more gets a new buffer half as large again at least; the old one stays allocated until the
 // process exits, so nothing is freed under work in flight and no stream is synchronised.
 struct own_scratch { int dev = -1; cudaStream_t s = nullptr; void * p = nullptr; size_t cap = 0; };
-own_scratch g_own[64];
-int g_nown = 0;
+struct own_pool { own_scratch e[64]; int n = 0; };
+own_pool g_own, g_pieces;   // tile images and carried state; pieces of the even split
 std::mutex g_pf_mu;
 
-void * own_scratch_for(size_t bytes, cudaStream_t s, size_t * cap_out) {
+// under g_pf_mu
+void * own_scratch_for(own_pool & pool, size_t bytes, cudaStream_t s, size_t * cap_out) {
     int dev = 0;
     cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lk(g_pf_mu);
     own_scratch * e = nullptr;
-    for (int i = 0; i < g_nown; ++i) if (g_own[i].dev == dev && g_own[i].s == s) e = &g_own[i];
+    for (int i = 0; i < pool.n; ++i) if (pool.e[i].dev == dev && pool.e[i].s == s) e = &pool.e[i];
     if (!e) {
-        if (g_nown == 64) return nullptr;
-        e = &g_own[g_nown++];
+        if (pool.n == 64) return nullptr;
+        e = &pool.e[pool.n++];
         e->dev = dev; e->s = s;
     }
     if (bytes > e->cap) {
         const size_t want = std::max(bytes, e->cap + e->cap / 2);
         void * p = nullptr;
-        if (cudaMalloc(&p, want) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // no other thread's recording is disturbed
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t rc = cudaMalloc(&p, want);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (rc != cudaSuccess) { cudaGetLastError(); return nullptr; }
         e->p = p;
         e->cap = want;
     }
     *cap_out = e->cap;
     return e->p;
+}
+
+// CTAs of the even split for rows p0 .. p0 + T - 1 (n_mtiles row tiles per kv head); 0 = one row tile per CTA.  Row tiles that are fewer than
+// the SMs leave SMs idle for as long as the longest tile takes: they are cut, into at least two steps per CTA (the prologue and the hand-over of
+// a piece cost about two steps).  Measured, one layer of 4 kv heads, q8_0, with prep, tile images and merge: T = 48 behind 100003 keys (12 row tiles) 1658 ->
+// 422 us, T = 512 behind 16000 (96 row tiles) 319 -> 264 us.  More row tiles than SMs run one per CTA, the longest first.
+int split_ctas(int T, int p0, int n_mtiles, int Hkv, int sms, int * head_steps) {
+    const long long tiles = (long long) n_mtiles * Hkv;
+    if (tiles >= sms) return 0;
+    long long hs = 0;
+    for (int m = 0; m < n_mtiles; ++m) hs += pf_tile_steps(T, p0, m);
+    if (hs * Hkv >= 1 << 30) return 0;
+    *head_steps = (int) hs;
+    const long long n = std::min<long long>(sms, hs * Hkv / 2);
+    return n > tiles ? (int) n : 0;
 }
 
 struct pf_io {
@@ -590,9 +742,17 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
     const size_t carry = io.out ? 0 : align256((size_t) T * Hq * DH * sizeof(float));
     const size_t per_step = (size_t) BP * c->Hkv * TILE_BYTES_PER_KEY;
     const size_t full = tile_bytes(std::max(n_keys, 1), c->Hkv);
-    if (!scratch) {
-        const size_t want = fixed + carry + std::min(full, std::max(OWN_SCRATCH_TILE_CAP / per_step, (size_t) 1) * per_step) + 256;
-        scratch = own_scratch_for(want, s, &scratch_bytes);
+    // Launches that share a buffer of the library (per device and stream) are queued as one block: another thread's call on the same
+    // stream comes before or after all of them.
+    std::unique_lock<std::mutex> lk(g_pf_mu);
+    const bool own = !scratch;
+    if (own) {
+        size_t want = 0;
+        for (const size_t cap : {OWN_SCRATCH_TILE_CAP, OWN_SCRATCH_TILE_LOW}) {
+            want = fixed + carry + std::min(full, std::max(cap / per_step, (size_t) 1) * per_step) + 256;
+            scratch = own_scratch_for(g_own, want, s, &scratch_bytes);
+            if (scratch) break;
+        }
         if (!scratch) B200_REFUSE(B200_ERR_ALLOC, "%s: %zu bytes of scratch could not be allocated", who, want);
     } else if ((uintptr_t) scratch & 255) {
         B200_REFUSE(B200_ERR_SCRATCH, "%s: scratch must be 256-byte aligned", who);
@@ -627,6 +787,26 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
     a.T = T; a.p0 = p0; a.Hq = Hq; a.Hkv = c->Hkv; a.qscale = scale * LOG2E_PF; a.status = st;
     const kv_view g = view_of(*c);
     const int n_mtiles = (T * GQA + BM - 1) / BM;
+    // The pieces of the even split lie in a buffer of the library.  A recorded call whose scratch is the caller's must not depend on
+    // it (the recording may be replayed beside other calls).
+    a.n_run = 0; a.n_mtiles = n_mtiles; a.head_steps = 0; a.po = nullptr; a.pml = nullptr;
+    if (!multi && !io.lim && !io.pm) {
+        int sms = 148, head_steps = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const int n = split_ctas(T, p0, n_mtiles, c->Hkv, sms, &head_steps);
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (n > 0 && !own && cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
+        if (n > 0 && cap == cudaStreamCaptureStatusNone) {
+            size_t have = 0;
+            const size_t pml_bytes = align256((size_t) 2 * n * BM * sizeof(float2));
+            unsigned char * pieces = (unsigned char *) own_scratch_for(g_pieces, pml_bytes + (size_t) 2 * n * BM * DH * sizeof(float), s, &have);
+            if (pieces) {   // else one row tile per CTA
+                a.n_run = n; a.head_steps = head_steps;
+                a.pml = reinterpret_cast<float2 *>(pieces);
+                a.po = reinterpret_cast<float *>(pieces + pml_bytes);
+            }
+        }
+    }
     int launches = 0;
     long long kb = 0;
     do {   // at least one pass, also when no key is visible (a sequence shard that owns nothing yet): it writes the empty result
@@ -637,8 +817,12 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
         else if (c->type == B200_KV_Q8_0) kv_tiles_k<B200_KV_Q8_0><<<tg, 256, 0, s>>>(g, (int) kb, n_keys, tiles, n_tiles, st);
         else kv_tiles_k<B200_KV_Q4_0><<<tg, 256, 0, s>>>(g, (int) kb, n_keys, tiles, n_tiles, st);
         a.n_tiles = n_tiles; a.kb = (int) kb; a.ke = (int) ke;
-        prefill_k<<<dim3(n_mtiles, c->Hkv), NTHR_PF, SM_TOTAL, s>>>(a);
+        prefill_k<<<a.n_run ? dim3(a.n_run) : dim3(n_mtiles, c->Hkv), NTHR_PF, SM_TOTAL, s>>>(a);
         launches += 2;
+        if (a.n_run) {
+            prefill_merge_k<<<dim3(n_mtiles * (BM / 8), c->Hkv), 256, 0, s>>>(a);
+            ++launches;
+        }
         kb = ke;
     } while (kb < n_keys);
     count_launch(launches);

@@ -232,3 +232,33 @@ def test_rope_append_bf16_row_kernel_equals_head_kernel(cuda, lib, tname):
         outs.append((c.k.cpu().numpy().reshape(-1)[rows].copy(), c.v.cpu().numpy().reshape(-1)[rows].copy(), q_out.cpu().numpy().copy()))
     for a, b in zip(outs[0], outs[1]):
         assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+
+
+@pytest.mark.parametrize("tname", ["f16", "q8_0", "q4_0"])
+@pytest.mark.parametrize("T", [1, 7, 9])
+def test_rope_append_bf16_special_blocks(cuda, lib, tname, T):
+    """zero blocks, ties of the largest magnitude with either sign, infinities and NaN, at ends of a token group: same bytes from aligned
+    rows (16-byte loads, a block in four lanes) and from shifted ones (a value per lane)"""
+    import torch
+    from p100e_engine_b200 import fast
+    kt, hkv = TYPES[tname], 3
+    rng = np.random.default_rng(T)
+    x = rng.integers(-2, 3, (2, T, hkv, D)).astype(np.float32)            # many ties
+    x[:, 0, 0, :96] = 0.0
+    x[:, -1, 1, 64:96] = np.float32(1e-30)
+    x[:, -1, 2, 130], x[:, -1, 2, 170], x[:, -1, 2, 200] = np.inf, np.nan, -np.inf
+    outs = []
+    for shift in (0, 1):
+        bufs = []
+        for a in x:
+            flat = torch.zeros(a.size + 8, dtype=torch.bfloat16, device=cuda)
+            flat[shift:shift + a.size] = torch.from_numpy(a).reshape(-1).to(cuda).to(torch.bfloat16)
+            bufs.append(flat[shift:shift + a.size].view(T, hkv, D))
+        c = fast.kv_alloc(kt, T, hkv, D)
+        q = torch.zeros(T, 6 * hkv, D, dtype=torch.bfloat16, device=cuda)
+        assert fast.rope_append_bf16(q, bufs[0], bufs[1], torch.empty(T, 6 * hkv, D, device=cuda), c, 0, T, 6 * hkv, hkv, D, 64, 1e7)
+        torch.cuda.synchronize()
+        outs.append([t.cpu().numpy().reshape(-1).view(np.uint8).copy() for t in (c.k, c.v)])
+    assert fast.device_status() == 0
+    for a, b in zip(*outs):
+        assert np.array_equal(a, b)
