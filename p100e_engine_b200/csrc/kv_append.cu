@@ -302,6 +302,121 @@ __global__ void __launch_bounds__(ROPE_THR) rope_rows_k(const __nv_bfloat16 * __
     }
 }
 
+// The same for rows of 256 values, 64 of them rotary, 16-byte aligned: what the prefill entry points of the attention kernels get.
+// A CTA takes n_tok tokens (up to ROPE8_TOK, fewer when the tokens are few, so that the SMs are used); every thread computes
+// cos / sin of one (token, pair), so that the trigonometry (the longest chain of the kernel) occupies all threads once, then each warp
+// walks (token, head) rows: a lane holds values 8 l .. 8 l + 7 of the row from one 16-byte load, the pairs (j, j + 32) meet by one shuffle per
+// value, a 32-value block lies in four lanes and its bytes leave as 8- or 16-byte stores.  Against one token per CTA and one value per
+// lane (rope_rows_k), one bf16 prefill call of 4 kv heads: T = 77 40.9 -> 33.6 us, T = 8192 951 -> 924 us (eight tokens per CTA at T = 77:
+// 42.0 us, too few CTAs).
+constexpr int ROPE8_TOK = 8, ROPE8_THR = 256;
+template <uint32_t KT>
+__device__ __forceinline__ void lanes8_to_cache(const float (&x)[8], int lane, char * head) {
+    if constexpr (KT == B200_KV_F16) {
+        reinterpret_cast<uint4 *>(head)[lane] = make_uint4(pack_h2(x[0], x[1]), pack_h2(x[2], x[3]), pack_h2(x[4], x[5]), pack_h2(x[6], x[7]));
+    } else {
+        // the block's largest magnitude: bit patterns of |x| as unsigned integers, as in block_to_cache
+        unsigned top = 0;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) top = max(top, __float_as_uint(fabsf(x[e])));
+        const unsigned own = top;
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = max(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        const int b = lane >> 2;
+        if constexpr (KT == B200_KV_Q8_0) {
+            float id;
+            const float d = q8_scale(__uint_as_float(top), id);
+            uint32_t w[2] = {0u, 0u};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e >> 2] |= (uint32_t) (uint8_t) (int8_t) q8_quant(x[e], id) << (8 * (e & 3));
+            *reinterpret_cast<uint2 *>(head + 2 * NBLK + 8 * lane) = make_uint2(w[0], w[1]);
+            if ((lane & 3) == 0) reinterpret_cast<__half *>(head)[b] = __float2half(d);
+        } else {
+            // the first value of largest magnitude: in the lowest lane that holds the maximum, its first value that has it
+            float mine = 0.0f;
+#pragma unroll
+            for (int e = 7; e >= 0; --e) if (__float_as_uint(fabsf(x[e])) == own) mine = x[e];
+            const unsigned who = __ballot_sync(0xffffffffu, own == top) >> (4 * b) & 15u;
+            const float pick = __shfl_sync(0xffffffffu, mine, 4 * b + __ffs(who) - 1);
+            const float mx = top ? pick : 0.0f;
+            const float d = mx / -8.0f;
+            const float id = d != 0.0f ? 1.0f / d : 0.0f;
+            uint32_t nib = 0;   // this lane's eight nibbles
+#pragma unroll
+            for (int e = 0; e < 8; ++e) nib |= ((uint32_t) q4_quant(x[e], id) & 15u) << (4 * e);
+            const uint32_t hi = __shfl_xor_sync(0xffffffffu, nib, 2);   // values 16 further on
+            char * blk = head + 18 * b;
+            if ((lane & 2) == 0) {   // byte i = value i | value i + 16 << 4; this lane's bytes start at 8 (lane & 1)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const uint32_t l2 = nib >> (8 * e) & 255u, h2 = hi >> (8 * e) & 255u;
+                    *reinterpret_cast<uint16_t *>(blk + 2 + 8 * (lane & 1) + 2 * e) =
+                        (uint16_t) ((l2 & 15u) | (h2 & 15u) << 4 | (l2 >> 4) << 8 | (h2 >> 4) << 12);
+                }
+            }
+            if ((lane & 3) == 0) *reinterpret_cast<__half *>(blk) = __float2half(d);
+        }
+    }
+}
+template <uint32_t KT>
+__global__ void __launch_bounds__(ROPE8_THR) rope8_k(const __nv_bfloat16 * __restrict__ qg, const __nv_bfloat16 * __restrict__ k,
+                                                     const __nv_bfloat16 * __restrict__ v, float * __restrict__ q, float * __restrict__ cs_out,
+                                                     kv_view g, int p0, int rope0, int T, int n_tok, int Hq, int Hkv, float freq_base, unsigned * status) {
+    constexpr int N_ROT = 64, HALF = 32;
+    __shared__ __align__(16) float cs[ROPE8_TOK][N_ROT];   // cos[32] | sin[32]
+    const int t0 = blockIdx.x * n_tok, lane = threadIdx.x & 31, nt = min(n_tok, T - t0);
+    const int n_q = qg ? Hq : 0, items = n_q + (k ? 2 * Hkv : 0);   // rows of a token: query heads, K heads, V heads
+    auto src_of = [&](int i) {
+        const int t = t0 + i / items, h = i % items;
+        return h < n_q ? qg + ((size_t) t * Hq + h) * DH : h < n_q + Hkv ? k + ((size_t) t * Hkv + h - n_q) * DH : v + ((size_t) t * Hkv + h - n_q - Hkv) * DH;
+    };
+    const int first = threadIdx.x >> 5, n_it = nt * items;
+    uint4 nxt = make_uint4(0, 0, 0, 0);
+    if (first < n_it) nxt = __ldg(reinterpret_cast<const uint4 *>(src_of(first)) + lane);   // flies during the trigonometry
+    {
+        const int tt = threadIdx.x / HALF, j = threadIdx.x % HALF;
+        if (tt < nt) {
+            const float theta = (float) (rope0 + t0 + tt) * powf(freq_base, -2.0f * j / N_ROT);
+            const float c = cosf(theta), sn = sinf(theta);
+            cs[tt][j] = c; cs[tt][HALF + j] = sn;
+            if (cs_out) { cs_out[(size_t) (t0 + tt) * N_ROT + j] = c; cs_out[(size_t) (t0 + tt) * N_ROT + HALF + j] = sn; }
+        }
+    }
+    __syncthreads();
+    for (int i = first; i < n_it; i += ROPE8_THR / 32) {
+        float x[8];
+        bf16x8_to_f32(nxt, x);
+        if (i + ROPE8_THR / 32 < n_it) nxt = __ldg(reinterpret_cast<const uint4 *>(src_of(i + ROPE8_THR / 32)) + lane);
+        const int tt = i / items, h = i % items, t = t0 + tt;
+        if (h < n_q + Hkv) {   // lanes 0..3 hold the first values of the pairs, lanes 4..7 the second ones
+            float y[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] = __shfl_xor_sync(0xffffffffu, x[e], 4);
+            if (lane < 8) {
+                const float4 * c4 = reinterpret_cast<const float4 *>(cs[tt] + 8 * (lane & 3)), * s4 = c4 + HALF / 4;
+                const float4 ca = c4[0], cb = c4[1], sa = s4[0], sb = s4[1];
+                const float c[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w}, sn[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    float r0, r1;
+                    rot_pair(lane < 4 ? x[e] : y[e], lane < 4 ? y[e] : x[e], c[e], sn[e], r0, r1);
+                    x[e] = lane < 4 ? r0 : r1;
+                }
+            }
+        }
+        if (h < n_q) {
+            float4 * dst = reinterpret_cast<float4 *>(q + ((size_t) t * Hq + h) * DH) + 2 * lane;
+            dst[0] = make_float4(x[0], x[1], x[2], x[3]);
+            dst[1] = make_float4(x[4], x[5], x[6], x[7]);
+            continue;
+        }
+        const int row = p0 + t, hd = h - n_q, is_v = hd >= Hkv;
+        const int32_t * tab = kv_tab(g, t);
+        if (tab && tab[row >> g.psh] < 0) { if (lane == 0) atomicOr(status, ST_BAD_PAGE); continue; }
+        lanes8_to_cache<KT>(x, lane, (is_v ? g.v : g.k) + kv_off_tab(g, tab, row) + (unsigned long long) (is_v ? hd - Hkv : hd) * head_bytes(KT));
+    }
+}
+
 // -------------------------------------------------------------------------------------------------- fillers ----
 __device__ __forceinline__ uint32_t mix32(uint32_t x) {
     x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
@@ -451,6 +566,18 @@ int rope_append_launch(const uint16_t * q, const uint16_t * k, const uint16_t * 
     if (!st) return B200_ERR_CUDA;
     const kv_view g = view_of(*c);
     const __nv_bfloat16 * qb = (const __nv_bfloat16 *) q, * kb = (const __nv_bfloat16 *) k, * vb = (const __nv_bfloat16 *) v;
+    // rows that are read 16 bytes at a time, and cache rows that are written so (their base and strides are multiples of 16)
+    if (vec && D == DH && n_rot == 64 && aligned16(c->k) && aligned16(c->v) && (!c->pt || c->pstride % 16 == 0)) {
+        const int n_tok = std::max(1, std::min(ROPE8_TOK, T / 592));   // 592: four CTAs on each of 148 SMs
+        const unsigned blocks = (unsigned) ((T + n_tok - 1) / n_tok);
+#define ROPE8(KT_) rope8_k<KT_><<<blocks, ROPE8_THR, 0, s>>>(qb, kb, vb, q_out, cs_out, g, p0, rope0, T, n_tok, Hq, Hkv, freq_base, st)
+        if (c->type == B200_KV_F16) ROPE8(B200_KV_F16);
+        else if (c->type == B200_KV_Q8_0) ROPE8(B200_KV_Q8_0);
+        else ROPE8(B200_KV_Q4_0);
+#undef ROPE8
+        count_launch();
+        return launch_status(who);
+    }
     if (c->type == B200_KV_F16) rope_rows_k<B200_KV_F16><<<T, ROPE_THR, smem, s>>>(qb, kb, vb, q_out, cs_out, g, p0, rope0, Hq, Hkv, D, n_rot, freq_base, vec, st);
     else if (c->type == B200_KV_Q8_0) rope_rows_k<B200_KV_Q8_0><<<T, ROPE_THR, smem, s>>>(qb, kb, vb, q_out, cs_out, g, p0, rope0, Hq, Hkv, D, n_rot, freq_base, vec, st);
     else rope_rows_k<B200_KV_Q4_0><<<T, ROPE_THR, smem, s>>>(qb, kb, vb, q_out, cs_out, g, p0, rope0, Hq, Hkv, D, n_rot, freq_base, vec, st);
