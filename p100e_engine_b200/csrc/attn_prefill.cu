@@ -1,6 +1,6 @@
 // Chunked causal prefill attention over the paged f16 / q8_0 / q4_0 cache on the sm_100a tensor cores (tcgen05 + TMEM).
 //
-// Two kernels per call:
+// Two or three kernels per call:
 //   kv_tiles_k   dequantises the visible keys once into f16 "tile images" in scratch: per (kv head, 64-key tile) a
 //                32 KB K image and a 32 KB V image laid out exactly as the tensor core reads them from shared memory
 //                (un-swizzled canonical layout, see umma.cuh; 8-key groups 4 KB apart, so two images side by side form
@@ -14,6 +14,8 @@
 //                of a step runs; S is single-buffered (the next Q K^T starts when the softmax threads hold S in
 //                registers), P is double-buffered.  The running output is rescaled only when a row's maximum grows by
 //                more than 2^8 (P stays below 256 in f16).  Epilogue: O / l, optional sigmoid gate.
+//                A few rows behind a long history are fewer row tiles than SMs: then the steps of all row tiles are cut evenly over
+//                the SMs and prefill_merge_k adds up the pieces of a tile (pf_cut, split_ctas).
 // f16 operands (int8 * f16 scale is not representable in bf16's 8 significand bits), fp32 accumulation.
 // Long contexts run as several passes over consecutive key ranges (as many keys as the scratch holds tile images for):
 // a row tile whose keys continue in a later pass leaves its unnormalised O in the output buffer and (max, sum) beside it,
@@ -58,58 +60,74 @@ constexpr int SM_TOTAL = SM_BAR + 256;
 static_assert(SM_TOTAL <= 227 * 1024 && EPI_BYTES <= 2 * IMG, "prefill_k shared memory");
 
 // ---- pre-pass: cache rows -> f16 tile images -------------------------------------------------------------------
-// grid (n_tiles, Hkv), 256 threads; thread = (key, 8-dim chunk).  Image byte of (key, dim) = (key/8)*4096 + (dim/8)*128 +
+// grid (n_tiles, Hkv), 256 threads; thread = (key, 64 dims).  Image byte of (key, dim) = (key/8)*4096 + (dim/8)*128 +
 // (key%8)*16 + (dim%8)*2 for K (K-major B operand) and for V (MN-major B operand) alike.  Keys >= n_keys are zero.
+// Bound by HBM: 2 x 272 bytes read (q8_0) and 1 KiB written per key and head.  A thread has all its loads of K and V in flight at
+// once, behind one page lookup; eight rounds of 8-byte loads, each behind a lookup of its own, took a call of 48 rows behind 100003 keys
+// (four heads, 218 MB of rows in, 410 MB of images out) 423 us instead of 363, one of 512 rows behind 16000 263 us instead of 253.
+
+// 64 values of a head row (the blocks 2 part, 2 part + 1) as f16 pairs, each the stored integer times its block's scale, rounded once
+template <uint32_t KT> struct row_part {
+    uint4 d[KT == B200_KV_F16 ? 8 : 4];
+    uint32_t s[KT == B200_KV_Q4_0 ? 9 : 1];
+    __device__ __forceinline__ void load(const unsigned char * row, int part) {
+        if constexpr (KT == B200_KV_F16) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) d[u] = __ldg(reinterpret_cast<const uint4 *>(row + 128 * part) + u);
+        } else if constexpr (KT == B200_KV_Q8_0) {
+            s[0] = __ldg(reinterpret_cast<const uint32_t *>(row) + part);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) d[u] = __ldg(reinterpret_cast<const uint4 *>(row + 16 + 64 * part) + u);
+        } else {   // two blocks of {f16 scale, 16 bytes}: 36 bytes from a 4-byte boundary
+#pragma unroll
+            for (int u = 0; u < 9; ++u) s[u] = __ldg(reinterpret_cast<const uint32_t *>(row + 36 * part) + u);
+        }
+    }
+    // values 8 c .. 8 c + 7
+    __device__ __forceinline__ uint4 chunk(int c) const {
+        if constexpr (KT == B200_KV_F16) return d[c];
+        else if constexpr (KT == B200_KV_Q8_0) {
+            const uint32_t d2 = __byte_perm(s[0], 0u, c < 4 ? 0x1010 : 0x3232);
+            const uint32_t x = (&d[c >> 1].x)[2 * (c & 1)] ^ 0x80808080u, y = (&d[c >> 1].x)[2 * (c & 1) + 1] ^ 0x80808080u;
+            auto pair = [&](uint32_t w, uint32_t sel) { return hmul2_u32(hsub2_u32(__byte_perm(w, 0x64646464u, sel), 0x64806480u), d2); };
+            return make_uint4(pair(x, 0x5140), pair(x, 0x7362), pair(y, 0x5140), pair(y, 0x7362));
+        } else {
+            // block b = c / 4: scale in the low (b = 0) or high (b = 1) half of word 4 b + ..., its 16 bytes on a 2-byte (b = 0) or 4-byte boundary
+            const int b = c >> 2, j = c & 3;   // values 8 j .. of the block: bytes 8 (j & 1) .. + 7, low (j < 2) or high nibbles
+            const uint32_t d2 = b ? __byte_perm(s[4], 0u, 0x3232) : __byte_perm(s[0], 0u, 0x1010);
+            const int o = 2 * (j & 1);
+            uint32_t x, y;
+            if (b) { x = s[5 + o]; y = s[6 + o]; }
+            else { x = __funnelshift_r(s[o], s[o + 1], 16); y = __funnelshift_r(s[o + 1], s[o + 2], 16); }
+            if (j >= 2) { x >>= 4; y >>= 4; }
+            x &= 0x0f0f0f0fu; y &= 0x0f0f0f0fu;
+            auto pair = [&](uint32_t w, uint32_t sel) { return hmul2_u32(hsub2_u32(__byte_perm(w, 0x64646464u, sel), 0x64086408u), d2); };
+            return make_uint4(pair(x, 0x5140), pair(x, 0x7362), pair(y, 0x5140), pair(y, 0x7362));
+        }
+    }
+};
+
 template <uint32_t KT>
 __global__ void __launch_bounds__(256) kv_tiles_k(kv_view g, int kb, int n_keys, unsigned char * __restrict__ tiles, int n_tiles,
                                                   unsigned * status) {
     const int tile = blockIdx.x, hk = blockIdx.y;   // tile j of the pass holds keys kb + 64 j ..; keys >= n_keys are zero
-    unsigned char * kimg = tiles + ((size_t) hk * n_tiles + tile) * (2 * IMG);
-    unsigned char * vimg = kimg + IMG;
+    const int key = threadIdx.x & (BN - 1), part = threadIdx.x / BN, kk = kb + tile * BN + key;
+    unsigned char * kimg = tiles + ((size_t) hk * n_tiles + tile) * (2 * IMG) + (key >> 3) * 4096 + part * 1024 + (key & 7) * 16;
+    bool have = kk < n_keys;
     const int32_t * tab = kv_tab(g, 0);
-    for (int i = threadIdx.x; i < BN * 32; i += 256) {
-        const int key = i & (BN - 1), dc = i >> 6;
-        const int kk = kb + tile * BN + key;
-        uint4 ko = make_uint4(0, 0, 0, 0), vo = ko;
-        if (kk < n_keys) {
-            bool ok = true;
-            if (tab && tab[kk >> g.psh] < 0) { atomicOr(status, ST_BAD_PAGE); ok = false; }
-            if (ok) {
-                const unsigned long long off = kv_off_tab(g, tab, kk) + (unsigned long long) hk * head_bytes(KT);
-                const unsigned char * kr = (const unsigned char *) g.k + off, * vr = (const unsigned char *) g.v + off;
-                if constexpr (KT == B200_KV_F16) {
-                    ko = *reinterpret_cast<const uint4 *>(kr + dc * 16);
-                    vo = *reinterpret_cast<const uint4 *>(vr + dc * 16);
-                } else {
-                    float kf[8], vf[8];
-                    if constexpr (KT == B200_KV_Q8_0) {
-                        const float dk = __half2float(reinterpret_cast<const __half *>(kr)[dc >> 2]);
-                        const float dv = __half2float(reinterpret_cast<const __half *>(vr)[dc >> 2]);
-                        const uint2 qk = *reinterpret_cast<const uint2 *>(kr + 16 + dc * 8);
-                        const uint2 qv = *reinterpret_cast<const uint2 *>(vr + 16 + dc * 8);
-                        const int8_t * a = reinterpret_cast<const int8_t *>(&qk), * b = reinterpret_cast<const int8_t *>(&qv);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) { kf[e] = dk * (float) a[e]; vf[e] = dv * (float) b[e]; }
-                    } else {
-                        const int blk = dc >> 2, sub = dc & 3;   // dims 8 sub .. 8 sub + 7 of the block: bytes (8 sub) % 16 .., nibble sub / 2
-                        const unsigned char * kb = kr + blk * 18, * vb = vr + blk * 18;
-                        const float dk = __half2float(*reinterpret_cast<const __half *>(kb));
-                        const float dv = __half2float(*reinterpret_cast<const __half *>(vb));
-                        const int sh = (sub >> 1) * 4, b0 = 2 + (sub & 1) * 8;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            kf[e] = dk * (float) ((int) ((kb[b0 + e] >> sh) & 15) - 8);
-                            vf[e] = dv * (float) ((int) ((vb[b0 + e] >> sh) & 15) - 8);
-                        }
-                    }
-                    ko = make_uint4(pack_h2(kf[0], kf[1]), pack_h2(kf[2], kf[3]), pack_h2(kf[4], kf[5]), pack_h2(kf[6], kf[7]));
-                    vo = make_uint4(pack_h2(vf[0], vf[1]), pack_h2(vf[2], vf[3]), pack_h2(vf[4], vf[5]), pack_h2(vf[6], vf[7]));
-                }
-            }
-        }
-        *reinterpret_cast<uint4 *>(kimg + (key >> 3) * 4096 + dc * 128 + (key & 7) * 16) = ko;
-        *reinterpret_cast<uint4 *>(vimg + (key >> 3) * 4096 + dc * 128 + (key & 7) * 16) = vo;
+    int pg = 0;
+    if (have && tab && (pg = tab[kk >> g.psh]) < 0) { atomicOr(status, ST_BAD_PAGE); have = false; }
+    row_part<KT> k, v;
+    if (have) {
+        const unsigned long long off = (tab ? (unsigned long long) pg * g.pstride + (unsigned long long) (kk & ((1 << g.psh) - 1)) * g.rowb
+                                            : (unsigned long long) kk * g.rowb) + (unsigned long long) hk * head_bytes(KT);
+        k.load((const unsigned char *) g.k + off, part);
+        v.load((const unsigned char *) g.v + off, part);
     }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4 *>(kimg + c * 128) = have ? k.chunk(c) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4 *>(kimg + IMG + c * 128) = have ? v.chunk(c) : make_uint4(0, 0, 0, 0);
 }
 
 struct pf_args {
