@@ -718,6 +718,7 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
 template <uint32_t KT, int NT>
 __global__ void __launch_bounds__(NTHR, ctas_per_sm<KT, NT>())
 decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV) {
+    pdl_enter();
     extern __shared__ __align__(1024) unsigned char smem[];
     // unit number = index * heads + kv head: the heads of one (slot, key range) are neighbours in launch order, so the four
     // head rows of a position are fetched close together in time
@@ -810,6 +811,7 @@ template <int P>
 __global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const float * __restrict__ gate, float * __restrict__ out,
                                                          float * __restrict__ fo, float * __restrict__ fm, float * __restrict__ fl,
                                                          __half2 * __restrict__ qbuf) {
+    pdl_enter();
     constexpr int SPG = P > 1 ? MERGE_STREAMS / P : 1;   // streams per group
     __shared__ float4 snum[P > 1 ? MERGE_STREAMS : 1][64];
     __shared__ float sden[P > 1 ? MERGE_STREAMS : 1], smax[2 * P];
@@ -906,6 +908,7 @@ __global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const
 __global__ void merge_parts_k(const float * __restrict__ po, const float * __restrict__ pm, const float * __restrict__ pl,
                               int nparts, int R, int D, const float * __restrict__ gate, float * __restrict__ out, size_t so,
                               size_t sm, __half2 * __restrict__ qbuf) {
+    pdl_enter();
     const int r = blockIdx.x, i = threadIdx.x;
     float M = B200_NEG_INF;
     for (int s = 0; s < nparts; ++s) M = fmaxf(M, pm[s * sm + r]);
@@ -1015,6 +1018,7 @@ __global__ void merge_peers_k(const peer_parts pp, int n_seq, int me, unsigned e
 // order of the atomics and does not affect any result (units are independent).
 constexpr int PLAN_THR = 1024, PLAN_BUCKETS = 256;
 __global__ void __launch_bounds__(PLAN_THR) decode_plan_k(const dec_args a, int2 * __restrict__ units, int * __restrict__ n_units) {
+    pdl_enter();
     __shared__ int hist[PLAN_BUCKETS];
     const int tid = threadIdx.x, lim = key_limit(a);
     const int top = a.CH > 0 ? a.CH / TILE : 1 << -a.CH;   // tiles of the longest chunk
@@ -1065,6 +1069,7 @@ __global__ void __launch_bounds__(PLAN_THR) decode_plan_k(const dec_args a, int2
 constexpr int SPLIT_THR = 1024, SPLIT_MAX_SLOTS = 2048, SPLIT_MAX_CTA = 1024;
 __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, int max_cta, int min_tiles, int4 * __restrict__ segs, int * __restrict__ cta_seg,
                                                             int2 * __restrict__ slot_seg, int * __restrict__ n_cta_out) {
+    pdl_enter();
     __shared__ int pre[SPLIT_MAX_SLOTS + 1];     // tiles before slot s
     __shared__ int cseg[SPLIT_MAX_CTA + 1];      // segments before CTA c
     __shared__ int first_slot[SPLIT_MAX_CTA];
@@ -1390,7 +1395,9 @@ int launch_tc(const dec_args & a_in, unsigned blocks, cudaStream_t s) {
             return launch_status("attn_decode (shared memory attribute)");
         attr_done[dev & 63].store(true, std::memory_order_release);
     }
-    decode_tc_k<NC><<<blocks, TC_THR, sm, s>>>(a, mapK, mapV);
+    // a step of few rows is short enough for the gap before the kernel to count
+    if (a.n_slots * a.q_len <= 64) launch(decode_tc_k<NC>, blocks, TC_THR, sm, s, a, mapK, mapV);
+    else decode_tc_k<NC><<<blocks, TC_THR, sm, s>>>(a, mapK, mapV);
     return B200_OK;
 }
 int launch_tc_nc(const dec_args & a, unsigned blocks, cudaStream_t s) {
@@ -1506,7 +1513,7 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
         int * n_cta = cta_seg + gm.max_cta + 1;
         a.segs = segs; a.cta_seg = cta_seg; a.slot_seg = slot_seg; a.n_cta = n_cta;
         if (!reuse_plan) {   // else the lists of an earlier call of this step, same shape, same positions, are still there
-            decode_split_k<<<1, SPLIT_THR, 0, s>>>(a, gm.max_cta, gm.tc ? 2 : 1, segs, cta_seg, slot_seg, n_cta);
+            launch(decode_split_k, 1, SPLIT_THR, 0, s, a, gm.max_cta, gm.tc ? 2 : 1, segs, cta_seg, slot_seg, n_cta);
             ++launches;
         }
         blocks = (unsigned) gm.max_cta * (unsigned) c->Hkv;
@@ -1515,7 +1522,7 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
         a.n_units = list;
         a.units = reinterpret_cast<const int2 *>(list + 4);
         if (!reuse_plan) {
-            decode_plan_k<<<1, PLAN_THR, 0, s>>>(a, reinterpret_cast<int2 *>(list + 4), list);
+            launch(decode_plan_k, 1, PLAN_THR, 0, s, a, reinterpret_cast<int2 *>(list + 4), list);
             ++launches;
         }
     }
@@ -1530,9 +1537,9 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     // threads per row keeps a launch of thousands of rows to one wave.
     const int parts = gm.split ? gm.max_cta / n_slots + 2 : gm.max_chunks;
     const dim3 mg(n_slots * q_len, GQA * a.nhk);
-    if (gm.split && parts <= 8) decode_merge_k<1><<<mg, 64, 0, s>>>(a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
-    else if (parts <= 32) decode_merge_k<4><<<mg, 256, 0, s>>>(a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
-    else decode_merge_k<16><<<mg, 1024, 0, s>>>(a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    if (gm.split && parts <= 8) launch(decode_merge_k<1>, mg, 64, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    else if (parts <= 32) launch(decode_merge_k<4>, mg, 256, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    else launch(decode_merge_k<16>, mg, 1024, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
     count_launch(launches);
     return launch_status(who);
 }
@@ -1784,7 +1791,7 @@ int b200_attn_merge_gate(const float * part_o, const float * part_m, const float
     if (!part_o || !part_m || !part_l || !out || nparts < 1 || R < 1 || D % 4 || D < 4 || D > 4096 || !aligned16(part_o) ||
         !aligned16(out) || (gate && !aligned16(gate)))
         B200_REFUSE(B200_ERR_SHAPE, "attn_merge_gate: unsupported arguments");
-    merge_parts_k<<<R, D / 4, 0, (cudaStream_t) stream>>>(part_o, part_m, part_l, nparts, R, D, gate, out, (size_t) R * D, (size_t) R,
+    launch(merge_parts_k, R, D / 4, 0, (cudaStream_t) stream, part_o, part_m, part_l, nparts, R, D, gate, out, (size_t) R * D, (size_t) R,
                                                           nullptr);
     count_launch();
     return launch_status("attn_merge_gate");
@@ -1815,7 +1822,7 @@ static int seq_exchange_impl(void * nccl_comm, int n_seq, const float * send, fl
         const int rc = allgather(send, recv, part, 7 /* ncclFloat32 */, nccl_comm, s);
         if (rc != 0) B200_REFUSE(B200_ERR_CUDA, "%s: ncclAllGather returned %d", who, rc);
     }
-    merge_parts_k<<<R, D / 4, 0, s>>>(parts, parts + (size_t) R * D, parts + (size_t) R * D + R, n_seq, R, D, gate, out, part, part,
+    launch(merge_parts_k, R, D / 4, 0, s, parts, parts + (size_t) R * D, parts + (size_t) R * D + R, n_seq, R, D, gate, out, part, part,
                                       (__half2 *) qbuf);
     count_launch();
     return launch_status(who);

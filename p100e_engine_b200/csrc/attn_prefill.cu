@@ -110,6 +110,7 @@ template <uint32_t KT> struct row_part {
 template <uint32_t KT>
 __global__ void __launch_bounds__(256) kv_tiles_k(kv_view g, int kb, int n_keys, unsigned char * __restrict__ tiles, int n_tiles,
                                                   unsigned * status) {
+    pdl_enter();
     const int tile = blockIdx.x, hk = blockIdx.y;   // tile j of the pass holds keys kb + 64 j ..; keys >= n_keys are zero
     const int key = threadIdx.x & (BN - 1), part = threadIdx.x / BN, kk = kb + tile * BN + key;
     unsigned char * kimg = tiles + ((size_t) hk * n_tiles + tile) * (2 * IMG) + (key >> 3) * 4096 + part * 1024 + (key & 7) * 16;
@@ -198,6 +199,7 @@ __device__ __forceinline__ void bf16x8_widen(const uint4 u, float (&f)[8]) {
 }
 
 __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
+    pdl_enter();
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t * bars = reinterpret_cast<uint64_t *>(smem + SM_BAR);
     uint64_t * k_full = bars, * k_free = bars + 1, * s_full = bars + 2, * s_free = bars + 3, * v_full = bars + 4, * v_free = bars + 8,
@@ -620,6 +622,7 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
 // Adds up the pieces of the row tiles that the even split cut, in key order, and finishes them like prefill_k does: 1/l, gate, f32 or
 // bf16 result, a16 copy.  grid (row tiles x 16, kv heads), a warp per row, eight values per lane: values 4 l .. 4 l + 3 of both 128-dim halves.
 __global__ void __launch_bounds__(256) prefill_merge_k(const pf_args a) {
+    pdl_enter();
     const int m = blockIdx.x >> 4, hk = blockIdx.y, lane = threadIdx.x & 31;
     const int r = (blockIdx.x & 15) * 8 + (threadIdx.x >> 5), n = m * BM + r;
     // the CTAs that hold the tile's first and last step
@@ -838,7 +841,7 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
         prefill_k<<<a.n_run ? dim3(a.n_run) : dim3(n_mtiles, c->Hkv), NTHR_PF, SM_TOTAL, s>>>(a);
         launches += 2;
         if (a.n_run) {
-            prefill_merge_k<<<dim3(n_mtiles * (BM / 8), c->Hkv), 256, 0, s>>>(a);
+            launch(prefill_merge_k, dim3(n_mtiles * (BM / 8), c->Hkv), 256, 0, s, a);
             ++launches;
         }
         kb = ke;

@@ -205,6 +205,33 @@ __device__ __forceinline__ void a16_store_lanes8(const float4 x, __half2 * __res
     if (l == 0) qbuf[n_groups * 16 + group] = __floats2half2_rn(amax, sum);
 }
 
+// ---- launches of a chain ---------------------------------------------------------------------------------------
+// The kernels of a step follow one another on a stream and many last a few microseconds, so the gap between two of them (a
+// launch waits until its predecessor has drained and its memory is flushed, then its CTAs are set up) is a good part of the
+// time.  launch() marks the launch as a programmatic dependent: its CTAs may be set up while the predecessor still runs, and
+// pdl_enter(), the first statement of the kernels of these chains, holds them back until all earlier work of the stream is complete
+// and visible.  Nothing is read, written or allocated before it, so the order of effects is that of plain launches.  Every kernel
+// launched this way passes pdl_enter(), so completion is transitive along the stream.
+// Measured, us: 16 layers of one row at 4096 keys (recorded) 344 -> 314, 1 + 3 rows at 30011 keys 540 -> 434, four layers of 8 x 4 rows
+// 358 -> 345, of a 77-token prompt 139 -> 131.  Plain launches stay where the early CTAs are in the way: grids of many waves (two layers of
+// 64 x 4 rows 2029 -> 2057 with all of them early, 1887 -> 1881 without), the mma.sync decode kernel, whose one wave must spread evenly over
+// the SMs (four layers of one row at 131000 keys 364 -> 426), and prefill_k behind kv_tiles_k (48 rows at 100003 keys 421 -> 596).
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+constexpr size_t PDL_MAX_CTAS = 1024;
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = (size_t) grid.x * grid.y * grid.z < PDL_MAX_CTAS ? 1 : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // a failure is found by launch_status
+}
+
 inline bool aligned16(const void * p) { return ((uintptr_t) p & 15) == 0; }
 
 #define B200_REFUSE(code, ...) do { fprintf(stderr, "b200attn: " __VA_ARGS__); fprintf(stderr, "\n"); return (code); } while (0)

@@ -112,6 +112,7 @@ constexpr int TOK_WARPS = 8;
 // groups, then the butterfly of those results over 8 slots (absent slots are zeros and add nothing).
 template <uint32_t KT, bool PREP, bool MR, int NF>
 __global__ void __launch_bounds__(TOK_WARPS * 32) token_k(const tok_args a) {
+    pdl_enter();
     extern __shared__ float sm[];   // cos[half] | sin[half] | TOK_WARPS staged heads of D floats
     const int t = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int D = a.D, nb = D / 32, nf = D / 128, half = a.n_rot / 2;
@@ -233,6 +234,7 @@ __global__ void __launch_bounds__(ROPE_THR) rope_rows_k(const __nv_bfloat16 * __
                                                    const __nv_bfloat16 * __restrict__ v, float * __restrict__ q, float * __restrict__ cs_out,
                                                    kv_view g, int p0, int rope0, int Hq, int Hkv, int D, int n_rot, float freq_base,
                                                    int vec, unsigned * status) {
+    pdl_enter();
     extern __shared__ float smr[];   // cos[half] | sin[half] | K heads [Hkv][D]
     const int t = blockIdx.x, i = threadIdx.x, half = n_rot / 2, lane = i & 31, wid = i >> 5, nb = D / 32;
     float * cs = smr, * kb = smr + n_rot;
@@ -362,6 +364,7 @@ template <uint32_t KT>
 __global__ void __launch_bounds__(ROPE8_THR) rope8_k(const __nv_bfloat16 * __restrict__ qg, const __nv_bfloat16 * __restrict__ k,
                                                      const __nv_bfloat16 * __restrict__ v, float * __restrict__ q, float * __restrict__ cs_out,
                                                      kv_view g, int p0, int rope0, int T, int n_tok, int Hq, int Hkv, float freq_base, unsigned * status) {
+    pdl_enter();
     constexpr int N_ROT = 64, HALF = 32;
     __shared__ __align__(16) float cs[ROPE8_TOK][N_ROT];   // cos[32] | sin[32]
     const int t0 = blockIdx.x * n_tok, lane = threadIdx.x & 31, nt = min(n_tok, T - t0);
@@ -475,6 +478,7 @@ __device__ __forceinline__ float sigm(float v) { return 1.0f / (1.0f + expf(-v))
 __device__ __forceinline__ float silu(float v) { return v / (1.0f + expf(-v)); }
 
 __global__ void sigmoid_mul_k(float * __restrict__ x, const float * __restrict__ gt, int64_t n) {
+    pdl_enter();
     for (int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x)
         x[i] *= sigm(gt[i]);
 }
@@ -484,6 +488,7 @@ __global__ void sigmoid_mul_k(float * __restrict__ x, const float * __restrict__
 template <int OP>
 __global__ void __launch_bounds__(256) ew_k(const float * __restrict__ a, const float * __restrict__ b, float * __restrict__ y,
                                             __half2 * __restrict__ qbuf, int T, int n, int lda, int ldb) {
+    pdl_enter();
     const int n4 = n >> 2, segs = (n4 + 31) >> 5, lane = threadIdx.x & 31;
     const long long items = (long long) T * segs, stride = (long long) gridDim.x * (blockDim.x >> 5);
     for (long long it = (long long) blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < items; it += stride) {
@@ -507,8 +512,8 @@ template <bool PREP>
 int token_launch(const tok_args & a, uint32_t type, int T, bool mrope, cudaStream_t s, const char * who) {
     const size_t smem = PREP ? ((size_t) a.n_rot + (size_t) TOK_WARPS * a.D) * sizeof(float) : 0;
     const dim3 grid(T, ((PREP && a.qg ? a.Hq : 0) + 2 * a.Hkv + TOK_WARPS - 1) / TOK_WARPS);
-#define TOKEN_NF(KT_, MR_) do { if (a.D <= 256) token_k<KT_, PREP, MR_, 2><<<grid, TOK_WARPS * 32, smem, s>>>(a); \
-                                else token_k<KT_, PREP, MR_, 8><<<grid, TOK_WARPS * 32, smem, s>>>(a); } while (0)
+#define TOKEN_NF(KT_, MR_) do { if (a.D <= 256) launch(token_k<KT_, PREP, MR_, 2>, grid, TOK_WARPS * 32, smem, s, a); \
+                                else launch(token_k<KT_, PREP, MR_, 8>, grid, TOK_WARPS * 32, smem, s, a); } while (0)
 #define TOKEN(KT_) do { if (PREP && mrope) TOKEN_NF(KT_, PREP); else TOKEN_NF(KT_, false); } while (0)
     if (type == B200_KV_F16) TOKEN(B200_KV_F16);
     else if (type == B200_KV_Q8_0) TOKEN(B200_KV_Q8_0);
@@ -570,7 +575,7 @@ int rope_append_launch(const uint16_t * q, const uint16_t * k, const uint16_t * 
     if (vec && D == DH && n_rot == 64 && aligned16(c->k) && aligned16(c->v) && (!c->pt || c->pstride % 16 == 0)) {
         const int n_tok = std::max(1, std::min(ROPE8_TOK, T / 592));   // 592: four CTAs on each of 148 SMs
         const unsigned blocks = (unsigned) ((T + n_tok - 1) / n_tok);
-#define ROPE8(KT_) rope8_k<KT_><<<blocks, ROPE8_THR, 0, s>>>(qb, kb, vb, q_out, cs_out, g, p0, rope0, T, n_tok, Hq, Hkv, freq_base, st)
+#define ROPE8(KT_) launch(rope8_k<KT_>, blocks, ROPE8_THR, 0, s, qb, kb, vb, q_out, cs_out, g, p0, rope0, T, n_tok, Hq, Hkv, freq_base, st)
         if (c->type == B200_KV_F16) ROPE8(B200_KV_F16);
         else if (c->type == B200_KV_Q8_0) ROPE8(B200_KV_Q8_0);
         else ROPE8(B200_KV_Q4_0);
@@ -578,9 +583,9 @@ int rope_append_launch(const uint16_t * q, const uint16_t * k, const uint16_t * 
         count_launch();
         return launch_status(who);
     }
-    if (c->type == B200_KV_F16) rope_rows_k<B200_KV_F16><<<T, ROPE_THR, smem, s>>>(qb, kb, vb, q_out, cs_out, g, p0, rope0, Hq, Hkv, D, n_rot, freq_base, vec, st);
-    else if (c->type == B200_KV_Q8_0) rope_rows_k<B200_KV_Q8_0><<<T, ROPE_THR, smem, s>>>(qb, kb, vb, q_out, cs_out, g, p0, rope0, Hq, Hkv, D, n_rot, freq_base, vec, st);
-    else rope_rows_k<B200_KV_Q4_0><<<T, ROPE_THR, smem, s>>>(qb, kb, vb, q_out, cs_out, g, p0, rope0, Hq, Hkv, D, n_rot, freq_base, vec, st);
+    if (c->type == B200_KV_F16) launch(rope_rows_k<B200_KV_F16>, T, ROPE_THR, smem, s, qb, kb, vb, q_out, cs_out, g, p0, rope0, Hq, Hkv, D, n_rot, freq_base, vec, st);
+    else if (c->type == B200_KV_Q8_0) launch(rope_rows_k<B200_KV_Q8_0>, T, ROPE_THR, smem, s, qb, kb, vb, q_out, cs_out, g, p0, rope0, Hq, Hkv, D, n_rot, freq_base, vec, st);
+    else launch(rope_rows_k<B200_KV_Q4_0>, T, ROPE_THR, smem, s, qb, kb, vb, q_out, cs_out, g, p0, rope0, Hq, Hkv, D, n_rot, freq_base, vec, st);
     count_launch();
     return launch_status(who);
 }
@@ -688,7 +693,7 @@ int b200_sigmoid_mul(float * x, const float * g, int64_t n, void * stream) {
     if (n <= 0) return B200_OK;
     if (!x || !g) B200_REFUSE(B200_ERR_SHAPE, "sigmoid_mul: null argument");
     const int64_t blocks = (n + 255) / 256;
-    sigmoid_mul_k<<<(unsigned) (blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t) stream>>>(x, g, n);
+    launch(sigmoid_mul_k, (unsigned) (blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t) stream, x, g, n);
     count_launch();
     return launch_status("sigmoid_mul");
 }
@@ -702,8 +707,8 @@ int b200_ew_quant(int op, const float * a, const float * b, float * y, void * qb
         B200_REFUSE(B200_ERR_SHAPE, "ew_quant: unsupported op / shape / alignment");
     const long long items = (long long) T * ((n / 4 + 31) / 32);
     const unsigned blocks = (unsigned) std::min<long long>((items + 7) / 8, 148 * 8);
-    if (op == 0) ew_k<0><<<blocks, 256, 0, (cudaStream_t) stream>>>(a, b, y, (__half2 *) qbuf, T, n, lda, ldb);
-    else ew_k<1><<<blocks, 256, 0, (cudaStream_t) stream>>>(a, b, y, (__half2 *) qbuf, T, n, lda, ldb);
+    if (op == 0) launch(ew_k<0>, blocks, 256, 0, (cudaStream_t) stream, a, b, y, (__half2 *) qbuf, T, n, lda, ldb);
+    else launch(ew_k<1>, blocks, 256, 0, (cudaStream_t) stream, a, b, y, (__half2 *) qbuf, T, n, lda, ldb);
     count_launch();
     return launch_status("ew_quant");
 }

@@ -78,3 +78,27 @@ def test_rows_do_not_depend_on_the_call_across_grid_boundaries(cuda, lib):
         assert torch.equal(free, pinned), p0
     assert fast.device_status() == 0
     assert fast.noalloc_device_status() == 0
+
+
+@pytest.mark.parametrize("tname", ["q8_0", "f16", "q4_0"])
+@pytest.mark.parametrize("n_slots", [5, 2100, 8200])   # few units; a plan of runs; more slots than a plan holds
+def test_many_slots_of_fixed_chunks(cuda, lib, tname, n_slots):
+    """fixed chunks of many ragged slots, some of them without a key: every row equals the one-row call, bit for bit"""
+    import torch
+    from p100e_engine_b200 import fast
+    n, hkv = 400, 1
+    g = torch.Generator(device="cuda").manual_seed(n_slots)
+    c = fast.kv_alloc(TYPES[tname], n, hkv, D)
+    assert fast.kv_append(c, torch.randn(n, hkv, D, generator=g, device=cuda), torch.randn(n, hkv, D, generator=g, device=cuda), 0, n)
+    q = torch.randn(n_slots, 6 * hkv, D, generator=g, device=cuda)
+    pos = torch.randint(-1, n, (n_slots,), generator=g, device=cuda, dtype=torch.int32)
+    pos[:5] = torch.tensor([n - 1, 63, 64, -1, 0], dtype=torch.int32)
+    out = torch.full_like(q, float("nan"))
+    assert fast.attn_decode_slots(q, c, out, None, n_slots, 1, pos, n, 6 * hkv, SCALE, 64)
+    picked = list(range(5)) + list(range(5, n_slots, max(1, n_slots // 40)))
+    for i in picked:
+        one = torch.full_like(q[:1], float("nan"))
+        assert fast.attn_decode_slots(q[i:i + 1], c, one, None, 1, 1, pos[i:i + 1], n, 6 * hkv, SCALE, 64)
+        assert torch.equal(one, out[i:i + 1]), (i, int(pos[i]))
+    assert torch.isfinite(out).all()
+    assert fast.device_status() == 0
