@@ -127,9 +127,9 @@ struct dec_args {
     unsigned * status;
     int n_ctx;                            // rows of a contiguous cache
     int tiled;                            // set by the launcher: whole tiles are fetched through the tensor maps
-    const int2 * units;                   // work list written by decode_plan_k: (slot, chunk), longest first; nullptr = the
-    const int * n_units;                  // CTAs enumerate (slot, chunk) themselves and skip units past a slot's end
-    // even split (decode_split_k): the batch's 64-key tiles, slot after slot, are cut into one contiguous run per CTA
+    int chunked;                          // fixed chunks: every chunk of the grid leaves its own partial
+    // run plan (decode_split_k): the batch's 64-key tiles, slot after slot, are cut into one contiguous run per CTA; nullptr = fixed
+    // chunks without a plan (one slot, or few units: see decode_part_k)
     const int4 * segs;                    // (slot, first key, end key, 0) in CTA order; a run that crosses a slot boundary has several
     const int * cta_seg;                  // [n_cta + 1] first segment of each CTA
     const int2 * slot_seg;                // [n_slots] (first segment, segments) of each slot
@@ -172,15 +172,16 @@ __device__ __forceinline__ void tma_box4(void * dst, const CUtensorMap * map, in
                  ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar)) : "memory");
 }
 
-// One unit of work: the keys k_lo .. k_cap-1 (as far as the slot has them) of one slot and kv head, all its query rows;
-// writes the unnormalised partial (O, m, l) number `unit`.  Called by all threads of the CTA.  A CTA that runs several units
-// keeps its ring of copy slots, their barriers and the arrival counters going from one unit to the next: tiles_before is the
-// number of tiles its earlier units walked (two ring items each); the function returns this unit's tile count.
-// t_base: tensor-memory base of the parked accumulators.
-template <uint32_t KT, int NT>
+// One unit of work: the keys k_lo .. k_cap-1 (as far as the slot has them) of one slot and kv head, all its query rows; writes
+// the unnormalised partial (O, m, l) number `unit`, or with RUNS (planned runs of fixed chunks) one partial per chunk, unit,
+// unit + 1, ..: sums and references start afresh at every chunk, so a chunk's bits do not depend on where a unit begins or
+// ends. Called by all threads of the CTA.  A CTA that runs several units keeps its ring of copy slots, their barriers and the
+// arrival counters going from one unit to the next: tiles_before is the number of tiles its earlier units walked (two ring
+// items each); the function returns this unit's tile count. t_base: tensor-memory base of the parked accumulators.
+template <uint32_t KT, int NT, bool RUNS>
 __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, const CUtensorMap & mapK, const CUtensorMap & mapV,
                                            unsigned char * smem, const int hk, const int slot, const int k_lo, const int k_cap,
-                                           const size_t unit, const int tiles_before, const uint32_t t_base) {
+                                           unsigned unit, const int tiles_before, const uint32_t t_base) {
     using TR = traits<KT>;
     constexpr int HB = TR::HB, SROW = TR::SROW;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -380,6 +381,63 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
     int rmin = 0x7fffffff;   // the mask is only evaluated in tiles that reach past some row's last key or the chunk's end
     for (int j = 0; j < a.q_len; ++j) rmin = min(rmin, row_pos(a, slot, j));
     const int mask_from = min(k_hi, rmin + 1);
+
+    // writes partial `unit` from the accumulators
+    auto flush = [&]() {
+        // l: sum over the lanes that share this row pair (same t), then over the warps
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float l = l_run[i][e];
+                l += __shfl_xor_sync(0xffffffffu, l, 4);
+                l += __shfl_xor_sync(0xffffffffu, l, 8);
+                l += __shfl_xor_sync(0xffffffffu, l, 16);
+                if (g == 0) wl[w * NT * 8 + 8 * i + 2 * t + e] = l;
+            }
+        __syncthreads();
+        if (w == 0 && g == 0) {
+#pragma unroll
+            for (int i = 0; i < NT; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int r = 8 * i + 2 * t + e;
+                    if (r < R) {
+                        a.pm[(size_t) unit * R + r] = m_run[i][e];
+                        a.pl[(size_t) unit * R + r] = (wl[r] + wl[NT * 8 + r]) + (wl[2 * NT * 8 + r] + wl[3 * NT * 8 + r]);
+                    }
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = 8 * i + 2 * t + e;
+                if (r >= R) continue;
+                float * dst = a.po + ((size_t) unit * R + r) * DH;
+                if constexpr (KT == B200_KV_F16) {
+#pragma unroll
+                    for (int mt = 0; mt < 4; ++mt) {
+                        dst[64 * w + 16 * mt + g] = O[mt][i][e];
+                        dst[64 * w + 16 * mt + g + 8] = O[mt][i][2 + e];
+                    }
+                } else if constexpr (KT == B200_KV_Q8_0) {
+#pragma unroll
+                    for (int y = 0; y < 2; ++y)
+                        *reinterpret_cast<float4 *>(dst + 64 * w + 32 * y + 4 * g) =
+                            make_float4(O[2 * y][i][e], O[2 * y][i][2 + e], O[2 * y + 1][i][e], O[2 * y + 1][i][2 + e]);
+                } else {
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) {
+                        *reinterpret_cast<float2 *>(dst + 64 * w + 32 * y + 2 * g) = make_float2(O[2 * y][i][e], O[2 * y][i][2 + e]);
+                        *reinterpret_cast<float2 *>(dst + 64 * w + 32 * y + 16 + 2 * g) = make_float2(O[2 * y + 1][i][e], O[2 * y + 1][i][2 + e]);
+                    }
+                }
+            }
+    };
+    auto end_from = [&](int key) { return (int) min((long long) k_hi, chunk_lo(a.CH, chunk_of(a.CH, key) + 1)); };
+    int part_end = 0;
+    if constexpr (RUNS) part_end = end_from(k_lo);   // first key that the partial being summed does not cover
 
     // ring position of the tile's K item (2 it) and V item (2 it + 1): slot index and the parity of its use count
     int last_v = 0, sv_prev = 0;
@@ -652,96 +710,58 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
         }
         last_v = arrive(1);
         sv_prev = sv_now;
+        if (RUNS && k_lo + (it + 1) * TILE >= part_end) {
+            flush();
+            if (it + 1 < ntiles) {   // the next chunk starts afresh
+                ++unit;
+                part_end = end_from(part_end);
+#pragma unroll
+                for (int i = 0; i < NT; ++i) {
+                    m_run[i][0] = m_run[i][1] = B200_NEG_INF;
+                    l_run[i][0] = l_run[i][1] = 0.0f;
+#pragma unroll
+                    for (int mt = 0; mt < 4; ++mt) O[mt][i][0] = O[mt][i][1] = O[mt][i][2] = O[mt][i][3] = 0.0f;
+                }
+            }
+        }
         if constexpr (PARK) park();
     }
-    if constexpr (PARK) unpark();
-
-    // ---------------- write the unit's partial ----------------
-    // l: sum over the lanes that share this row pair (same t), then over the warps
-#pragma unroll
-    for (int i = 0; i < NT; ++i)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            float l = l_run[i][e];
-            l += __shfl_xor_sync(0xffffffffu, l, 4);
-            l += __shfl_xor_sync(0xffffffffu, l, 8);
-            l += __shfl_xor_sync(0xffffffffu, l, 16);
-            if (g == 0) wl[w * NT * 8 + 8 * i + 2 * t + e] = l;
-        }
-    __syncthreads();
-    if (w == 0 && g == 0) {
-#pragma unroll
-        for (int i = 0; i < NT; ++i)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int r = 8 * i + 2 * t + e;
-                if (r < R) {
-                    a.pm[unit * R + r] = m_run[i][e];
-                    a.pl[unit * R + r] = (wl[r] + wl[NT * 8 + r]) + (wl[2 * NT * 8 + r] + wl[3 * NT * 8 + r]);
-                }
-            }
+    if constexpr (!RUNS) {
+        if constexpr (PARK) unpark();
+        flush();
     }
-#pragma unroll
-    for (int i = 0; i < NT; ++i)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int r = 8 * i + 2 * t + e;
-            if (r >= R) continue;
-            float * dst = a.po + (unit * R + r) * DH;
-            if constexpr (KT == B200_KV_F16) {
-#pragma unroll
-                for (int mt = 0; mt < 4; ++mt) {
-                    dst[64 * w + 16 * mt + g] = O[mt][i][e];
-                    dst[64 * w + 16 * mt + g + 8] = O[mt][i][2 + e];
-                }
-            } else if constexpr (KT == B200_KV_Q8_0) {
-#pragma unroll
-                for (int y = 0; y < 2; ++y)
-                    *reinterpret_cast<float4 *>(dst + 64 * w + 32 * y + 4 * g) =
-                        make_float4(O[2 * y][i][e], O[2 * y][i][2 + e], O[2 * y + 1][i][e], O[2 * y + 1][i][2 + e]);
-            } else {
-#pragma unroll
-                for (int y = 0; y < 2; ++y) {
-                    *reinterpret_cast<float2 *>(dst + 64 * w + 32 * y + 2 * g) = make_float2(O[2 * y][i][e], O[2 * y][i][2 + e]);
-                    *reinterpret_cast<float2 *>(dst + 64 * w + 32 * y + 16 + 2 * g) = make_float2(O[2 * y + 1][i][e], O[2 * y + 1][i][2 + e]);
-                }
-            }
-        }
     return ntiles;
 }
 
 #include "decode_tc.cuh"
 
-// The kernel.  Even split: every segment of the CTA's run one after the other.  Fixed chunks: units u = blockIdx.x, + gridDim.x, ..
-// with at most one resident wave of CTAs launched, the longest chunks first (work list, or the highest chunk index first), so that
-// several waves of short CTAs do not each pay their start-up and the tail is made of short units.
-template <uint32_t KT, int NT>
+// The kernel.  With a run plan: every segment of the CTA's run one after the other.  Fixed chunks without a plan (one slot;
+// few units; more slots than a plan holds): units u = index, + CTAs of the kv head, .., one chunk each, the highest chunk
+// index first, so that the long chunks start first and the short ones fill the tail.  (One long context as contiguous runs,
+// cut at chunk boundaries like the plans: 401 us against 364 for four layers of 131000 keys, because a CTA got either 8 or 16
+// tiles.)
+template <uint32_t KT, int NT, bool RUNS>
 __global__ void __launch_bounds__(NTHR, ctas_per_sm<KT, NT>())
 decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV) {
     pdl_enter();
     extern __shared__ __align__(1024) unsigned char smem[];
-    // unit number = index * heads + kv head: the heads of one (slot, key range) are neighbours in launch order, so the four
+    // kv head = block index mod heads: the heads of one (slot, key range) are neighbours in launch order, so the four
     // head rows of a position are fetched close together in time
-    int hl = (int) (blockIdx.x % (unsigned) a.nhk), s0 = 0, s1 = 0, nch = a.max_chunks;
-    long long u_end = 0;
+    const int hl = (int) (blockIdx.x % (unsigned) a.nhk), ui = (int) (blockIdx.x / (unsigned) a.nhk);
+    int s0, s1, nch = a.max_chunks;
     if (a.segs) {
-        const int ui = (int) (blockIdx.x / (unsigned) a.nhk);
         if (ui >= *a.n_cta) return;
         s0 = a.cta_seg[ui]; s1 = a.cta_seg[ui + 1];
-        if (s0 >= s1) return;
-    } else if (a.units) {
-        u_end = (long long) *a.n_units * a.nhk;
     } else {
-        if (a.n_slots == 1) {
+        if (a.n_slots == 1) {   // the chunks the slot has (a position beyond the limit is reported by the unit that runs)
             int n = 0;
             for (int j = 0; j < a.q_len; ++j) n = max(n, row_pos(a, 0, j) + 1);
             n = min(n, key_limit(a));
             nch = n > 0 ? chunk_of(a.CH, n - 1) + 1 : 0;
-            // the chunks past the limit are the merge's business; a position beyond it is reported by the unit that runs
         }
-        u_end = (long long) nch * a.n_slots * a.nhk;
+        s0 = ui; s1 = (int) min((long long) nch * a.n_slots, 0x7fffffffLL);
     }
-    if (!a.segs && blockIdx.x >= u_end) return;
+    if (s0 >= s1) return;
     // barriers of the copy ring, arrival counters and flags: made once per CTA
     if (threadIdx.x == 0) {
         uint64_t * full = reinterpret_cast<uint64_t *>(smem);
@@ -762,31 +782,24 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
         t_base = *t_slot;
     }
     int tiles = 0;
-    long long u = a.segs ? s0 : blockIdx.x;
-    const long long u_last = a.segs ? s1 : u_end, u_step = a.segs ? 1 : gridDim.x;
-    for (; u < u_last; u += u_step) {
-        int slot, k_lo, k_cap;
-        size_t unit;
+    const int step = a.segs ? 1 : (int) (gridDim.x / (unsigned) a.nhk);
+    for (int u = s0; u < s1; u += step) {
+        int slot, chunk = -1, k_lo, k_cap;
+        unsigned unit;
         if (a.segs) {
             const int4 e = a.segs[u];
             slot = e.x; k_lo = e.y; k_cap = e.z;
-            unit = (size_t) u * a.nhk + hl;
+            unit = (unsigned) u * a.nhk + hl;
+            if constexpr (RUNS) chunk = chunk_of(a.CH, k_lo);
         } else {
-            hl = (int) (u % a.nhk);
-            const int i = (int) (u / a.nhk);
-            int chunk;
-            if (a.units) {
-                const int2 e = a.units[i];
-                slot = e.x; chunk = e.y;
-            } else {
-                slot = i % a.n_slots; chunk = nch - 1 - i / a.n_slots;
-            }
-            k_lo = (int) chunk_lo(a.CH, chunk);
+            slot = u % a.n_slots; chunk = nch - 1 - u / a.n_slots;
+            k_lo = (int) min(0x7fffffffLL, chunk_lo(a.CH, chunk));
             k_cap = (int) min(0x7fffffffLL, chunk_lo(a.CH, chunk + 1));
-            unit = ((size_t) slot * a.nhk + hl) * a.max_chunks + chunk;
         }
+        if (chunk >= 0) unit = ((unsigned) slot * a.nhk + hl) * a.max_chunks + chunk;   // below 2^31 (decode_geometry)
         if (tiles) __syncthreads();   // the previous unit's shared memory is no longer read
-        tiles += decode_unit<KT, NT>(a, nslot, mapK, mapV, smem, a.hk0 + hl, slot, k_lo, k_cap, unit, tiles, t_base);
+        tiles += decode_unit<KT, NT, RUNS>(a, nslot, mapK, mapV, smem, a.hk0 + hl, slot, k_lo, k_cap, unit, tiles, t_base);
+        if (u > 0x7fffffff - step) break;
     }
     if constexpr (parks<KT, NT>()) {
         umma::fence_before_sync();
@@ -822,7 +835,7 @@ __global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const
     // partials of the row's kv head: consecutive units of stride ustr from unit0 (a segment the row does not reach holds m = -inf)
     int nch;
     size_t unit0, ustr;
-    if (a.segs) {
+    if (!a.chunked) {
         const int2 sg = a.slot_seg[slot];
         nch = pos < 0 ? 0 : sg.y;
         unit0 = (size_t) sg.x * a.nhk + hl; ustr = a.nhk;
@@ -1013,66 +1026,22 @@ __global__ void merge_peers_k(const peer_parts pp, int n_seq, int me, unsigned e
     if (qbuf) a16_store_lanes8(y, qbuf, ((size_t) r * D + 4 * i) / 32, (size_t) R * D / 32, true);
 }
 
-// Work list of a batched call: every (slot, chunk) that holds at least one visible key, longest first, so the tail of the
-// launch is made of the shortest units.  One block; writes units[] and *n_units.  The order of equal-length units depends on the
-// order of the atomics and does not affect any result (units are independent).
-constexpr int PLAN_THR = 1024, PLAN_BUCKETS = 256;
-__global__ void __launch_bounds__(PLAN_THR) decode_plan_k(const dec_args a, int2 * __restrict__ units, int * __restrict__ n_units) {
-    pdl_enter();
-    __shared__ int hist[PLAN_BUCKETS];
-    const int tid = threadIdx.x, lim = key_limit(a);
-    const int top = a.CH > 0 ? a.CH / TILE : 1 << -a.CH;   // tiles of the longest chunk
-    for (int i = tid; i < PLAN_BUCKETS; i += PLAN_THR) hist[i] = 0;
-    __syncthreads();
-    const long long pairs = (long long) a.n_slots * a.max_chunks;
-    // bucket of pair i (0 = longest class), -1 if the slot has no key in the chunk
-    auto bucket_of = [&](long long i) {
-        const int s = (int) (i % a.n_slots), c = (int) (i / a.n_slots);
-        int n = 0;
-        for (int j = 0; j < a.q_len; ++j) n = max(n, row_pos(a, s, j) + 1);
-        n = min(n, lim);
-        const long long lo = chunk_lo(a.CH, c);
-        if (lo >= n) return -1;
-        const long long tiles = (min((long long) n, chunk_lo(a.CH, c + 1)) - lo + TILE - 1) / TILE;
-        return (int) min((long long) PLAN_BUCKETS - 1, (top - tiles) * PLAN_BUCKETS / top);
-    };
-    for (long long i = tid; i < pairs; i += PLAN_THR) {
-        const int b = bucket_of(i);
-        if (b >= 0) atomicAdd(&hist[b], 1);
-    }
-    __syncthreads();
-    if (tid < 32) {   // exclusive scan of the classes
-        int run = 0;
-        for (int base = 0; base < PLAN_BUCKETS; base += 32) {
-            const int v = hist[base + tid];
-            int x = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (tid >= o) x += y; }
-            hist[base + tid] = run + x - v;
-            run += __shfl_sync(0xffffffffu, x, 31);
-        }
-        if (tid == 0) *n_units = run;
-    }
-    __syncthreads();
-    for (long long i = tid; i < pairs; i += PLAN_THR) {
-        const int b = bucket_of(i);
-        if (b >= 0) units[atomicAdd(&hist[b], 1)] = make_int2((int) (i % a.n_slots), (int) (i / a.n_slots));
-    }
-}
-
-// Even split of a batch over the resident CTAs (used when the chunk is chosen from the batch).  The 64-key tiles of all
-// slots, slot after slot, form one sequence per kv head; CTA c of n_cta takes tiles [c W / n_cta, (c + 1) W / n_cta), so
-// every CTA has the same work to within one tile however ragged the contexts are, and all CTAs fit the machine at once.  A
-// run that crosses slot boundaries becomes several segments; each segment yields one partial.  n_cta = min(max_cta, W /
-// min_tiles): the tcgen05 kernel walks tiles of 128 keys, so its runs hold at least two of these.  One block; n_slots <=
-// SPLIT_MAX_SLOTS.
-constexpr int SPLIT_THR = 1024, SPLIT_MAX_SLOTS = 2048, SPLIT_MAX_CTA = 1024;
+// Even split of a batch over the resident CTAs (used when the chunk is chosen from the batch).  The 64-key tiles of all slots,
+// slot after slot, form one sequence per kv head; CTA c of n_cta takes tiles [c W / n_cta, (c + 1) W / n_cta), so every CTA
+// has the same work to within one tile however ragged the contexts are, and all CTAs fit the machine at once.  A run that
+// crosses slot boundaries becomes several segments; each segment yields one partial.  n_cta = min(max_cta, W / min_tiles): the
+// tcgen05 kernel walks tiles of 128 keys, so its runs hold at least two of these.  Fixed chunks (chunked): the same runs,
+// their ends moved to the nearest chunk boundary, so that a CTA streams neighbouring chunks of one slot instead of starting
+// afresh for each chunk of a work list (four layers of 8 rows of 700 .. 16384 keys, f16: 389 -> 341 us).  One block; n_slots
+// <= PLAN_MAX_SLOTS.
+constexpr int SPLIT_THR = 1024, SPLIT_MAX_SLOTS = 2048, PLAN_MAX_SLOTS = 8192, SPLIT_MAX_CTA = 1024;
 __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, int max_cta, int min_tiles, int4 * __restrict__ segs, int * __restrict__ cta_seg,
                                                             int2 * __restrict__ slot_seg, int * __restrict__ n_cta_out) {
     pdl_enter();
-    __shared__ int pre[SPLIT_MAX_SLOTS + 1];     // tiles before slot s
+    __shared__ int pre[PLAN_MAX_SLOTS + 1];      // tiles before slot s
     __shared__ int cseg[SPLIT_MAX_CTA + 1];      // segments before CTA c
-    __shared__ int first_slot[SPLIT_MAX_CTA];
+    __shared__ int scut[SPLIT_MAX_CTA + 1];      // first tile of CTA c
+    __shared__ short first_slot[SPLIT_MAX_CTA];
     const int tid = threadIdx.x, lim = key_limit(a);
     auto slot_keys = [&](int s) {
         int n = 0;
@@ -1096,7 +1065,20 @@ __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, in
     __syncthreads();
     const long long W = pre[a.n_slots];
     const int n_cta = (int) max(1LL, min((long long) min(max_cta, SPLIT_MAX_CTA), W / min_tiles));
-    auto cut = [&](int c) { return (int) (W * c / n_cta); };
+    if (tid <= n_cta) {
+        int x = (int) (W * tid / n_cta);
+        if (a.chunked && tid > 0 && tid < n_cta) {
+            int l = 0, r = a.n_slots;               // last slot with pre[s] <= x
+            while (r - l > 1) { const int m = (l + r) >> 1; if (pre[m] <= x) l = m; else r = m; }
+            const int len = pre[l + 1] - pre[l], off = x - pre[l];   // x < W, so off < len
+            const int c = chunk_of(a.CH, off * TILE);
+            const int lo = (int) (chunk_lo(a.CH, c) / TILE), hi = (int) min((long long) len, chunk_lo(a.CH, c + 1) / TILE);
+            x = pre[l] + (off - lo <= hi - off ? lo : hi);
+        }
+        scut[tid] = x;
+    }
+    __syncthreads();
+    auto cut = [&](int c) { return scut[c]; };
     // segments per CTA: the slots its run intersects
     int my_first = 0, my_cnt = 0;
     if (tid < n_cta) {
@@ -1109,7 +1091,7 @@ __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, in
             int e = l;
             while (e < a.n_slots && pre[e] < hi) { if (pre[e + 1] > pre[e] && pre[e + 1] > lo) ++my_cnt; ++e; }
         }
-        first_slot[tid] = my_first;
+        first_slot[tid] = (short) my_first;
         cseg[tid + 1] = my_cnt;
     }
     if (tid == 0) cseg[0] = 0;
@@ -1137,6 +1119,7 @@ __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, in
             segs[o++] = make_int4(s, t0 * TILE, t1 * TILE, 0);
         }
     }
+    if (a.chunked) return;   // a chunk's partial has its own place
     // the segments of a slot are consecutive: from the CTA that holds its first tile to the one that holds its last
     for (int s = tid; s < a.n_slots; s += SPLIT_THR) {
         if (pre[s + 1] <= pre[s]) { slot_seg[s] = make_int2(0, 0); continue; }
@@ -1321,7 +1304,7 @@ template <uint32_t KT, int NT> size_t smem_bytes(int nslot) {
            (traits<KT>::SCALED ? NBLK * NT * 4 * sizeof(float4) : 0);
 }
 
-template <uint32_t KT, int NT>
+template <uint32_t KT, int NT, bool RUNS>
 int launch_part(const dec_args & a_in, unsigned blocks, cudaStream_t s) {
     dec_args a = a_in;
     CUtensorMap mapK, mapV;
@@ -1345,19 +1328,23 @@ int launch_part(const dec_args & a_in, unsigned blocks, cudaStream_t s) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_done[dev & 63].load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(decode_part_k<KT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm) != cudaSuccess)
+        if (cudaFuncSetAttribute(decode_part_k<KT, NT, RUNS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm) != cudaSuccess)
             return launch_status("attn_decode (shared memory attribute)");
-        cudaFuncSetAttribute(decode_part_k<KT, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        cudaFuncSetAttribute(decode_part_k<KT, NT, RUNS>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         attr_done[dev & 63].store(true, std::memory_order_release);
     }
-    decode_part_k<KT, NT><<<blocks, NTHR, sm, s>>>(a, nslot, mapK, mapV);
+    decode_part_k<KT, NT, RUNS><<<blocks, NTHR, sm, s>>>(a, nslot, mapK, mapV);
     return B200_OK;
 }
 
+template <uint32_t KT, bool RUNS>
+int launch_part_runs(const dec_args & a, unsigned blocks, cudaStream_t s) {
+    const int nt = (a.q_len * GQA + 7) / 8;
+    return nt == 1 ? launch_part<KT, 1, RUNS>(a, blocks, s) : nt == 2 ? launch_part<KT, 2, RUNS>(a, blocks, s) : launch_part<KT, 3, RUNS>(a, blocks, s);
+}
 template <uint32_t KT>
 int launch_part_nt(const dec_args & a, unsigned blocks, cudaStream_t s) {
-    const int nt = (a.q_len * GQA + 7) / 8;
-    return nt == 1 ? launch_part<KT, 1>(a, blocks, s) : nt == 2 ? launch_part<KT, 2>(a, blocks, s) : launch_part<KT, 3>(a, blocks, s);
+    return a.chunked && a.segs ? launch_part_runs<KT, true>(a, blocks, s) : launch_part_runs<KT, false>(a, blocks, s);
 }
 
 // whole tiles can be fetched through tensor maps: pages of at least 64 rows, 16-byte row strides, strides inside the map's fields
@@ -1435,8 +1422,11 @@ int auto_chunk(long long total_keys, int Hkv) {
 
 // geometry of a call: chunk, chunks per slot, partial floats, work-list ints
 //   split   (chunk chosen from the batch, up to SPLIT_MAX_SLOTS slots): one contiguous run of tiles per resident CTA
-//   planned (fixed chunk, more units than a wave): the grid's units ordered longest first through a work list
-//   else    the grid enumerates (slot, chunk)
+//   planned (fixed chunks of several slots, more units than a wave): the same runs, cut at chunk boundaries
+//   else    see decode_part_k
+size_t run_list_ints(int max_cta, int n_slots) {
+    return (4 * ((size_t) max_cta + n_slots) + 2 * (size_t) n_slots + max_cta + 2 + 3) & ~(size_t) 3;
+}
 struct dec_geom { int CH, max_chunks, R, max_cta; size_t units, part_floats, list_ints; bool planned, split, tc; };
 
 bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int max_n, int n_ctx, int Hkv, int chunk_keys, bool tc = false) {
@@ -1454,8 +1444,7 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
         const size_t nseg = (size_t) g.max_cta + n_slots;
         g.units = nseg * Hkv;
         g.part_floats = g.units * g.R * (DH + 2);
-        g.list_ints = 4 * nseg + 2 * (size_t) n_slots + g.max_cta + 2;
-        g.list_ints = (g.list_ints + 3) & ~(size_t) 3;
+        g.list_ints = run_list_ints(g.max_cta, n_slots);
         return true;
     }
     g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) : default_grid(n_ctx);
@@ -1463,9 +1452,10 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
     g.units = (size_t) n_slots * Hkv * g.max_chunks;
     if (g.units >= ((size_t) 1 << 31) || (size_t) n_slots * g.max_chunks >= ((size_t) 1 << 30)) return false;
     g.part_floats = g.units * g.R * (DH + 2);
-    // a work list pays once the launch is longer than one wave of resident CTAs; shorter launches enumerate the grid
-    g.planned = n_slots > 1 && g.units > (size_t) 2 * sm_count();
-    g.list_ints = g.planned ? 2 * (size_t) n_slots * g.max_chunks + 4 : 0;
+    // a plan pays once the launch is longer than one wave of resident CTAs; shorter launches enumerate the grid
+    g.planned = n_slots > 1 && n_slots <= PLAN_MAX_SLOTS && g.units > (size_t) 2 * sm_count();
+    g.max_cta = std::max(1, std::min(SPLIT_MAX_CTA, resident_ctas(type, q_len) / Hkv));
+    g.list_ints = g.planned ? run_list_ints(g.max_cta, n_slots) : 0;
     return true;
 }
 
@@ -1499,12 +1489,12 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     a.CH = gm.CH; a.max_chunks = gm.max_chunks; a.status = st;
     a.hk0 = hk0; a.nhk = heads;
     a.n_ctx = c->n_ctx; a.tiled = 0;
-    a.units = nullptr; a.n_units = nullptr;
+    a.chunked = gm.split ? 0 : 1;
     a.segs = nullptr; a.cta_seg = nullptr; a.slot_seg = nullptr; a.n_cta = nullptr;
     int launches = 2;
-    // fixed chunks: at most one wave of CTAs, which walk the units
-    unsigned blocks = (unsigned) std::min<size_t>((size_t) n_slots * a.nhk * gm.max_chunks, (size_t) resident_ctas(c->type, q_len));
-    if (gm.split) {
+    // fixed chunks without a plan: at most one wave of CTAs, a multiple of the heads
+    unsigned blocks = (unsigned) std::min<size_t>((size_t) n_slots * gm.max_chunks, (size_t) gm.max_cta) * (unsigned) a.nhk;
+    if (gm.split || gm.planned) {
         int * list = reinterpret_cast<int *>(scr + part_floats);
         const size_t nseg = (size_t) gm.max_cta + n_slots;
         int4 * segs = reinterpret_cast<int4 *>(list);
@@ -1516,15 +1506,7 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
             launch(decode_split_k, 1, SPLIT_THR, 0, s, a, gm.max_cta, gm.tc ? 2 : 1, segs, cta_seg, slot_seg, n_cta);
             ++launches;
         }
-        blocks = (unsigned) gm.max_cta * (unsigned) c->Hkv;
-    } else if (gm.planned) {
-        int * list = reinterpret_cast<int *>(scr + part_floats);
-        a.n_units = list;
-        a.units = reinterpret_cast<const int2 *>(list + 4);
-        if (!reuse_plan) {
-            launch(decode_plan_k, 1, PLAN_THR, 0, s, a, reinterpret_cast<int2 *>(list + 4), list);
-            ++launches;
-        }
+        blocks = (unsigned) gm.max_cta * (unsigned) a.nhk;
     }
     int rc;
     if (gm.split && gm.tc) rc = launch_tc_nc(a, blocks, s);
@@ -1704,11 +1686,11 @@ int b200_attn_reserve(uint32_t kv_type, int max_slots, int q_len, int max_n, int
         B200_REFUSE(B200_ERR_SHAPE, "attn_reserve: unsupported arguments");
     dec_geom gm;
     if (!decode_geometry(gm, kv_type, max_slots, q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, chunk_keys)) B200_REFUSE(B200_ERR_SHAPE, "attn_reserve: too many chunks");
-    size_t need = gm.part_floats + std::max(gm.list_ints, 2 * (size_t) max_slots * gm.max_chunks + 4);
+    size_t need = gm.part_floats + std::max(gm.list_ints, run_list_ints(gm.max_cta, max_slots));
     if (chunk_keys < 0 && !gm.split) {
         // a fixed chunk chosen from the batch: smaller batches take smaller chunks; their unit count stays under this bound
         const size_t u = 2 * 8 * (size_t) sm_count() + (size_t) max_slots * Hkv;
-        need = std::max(need, u * q_len * GQA * (DH + 2) + 2 * u + 4);
+        need = std::max(need, u * q_len * GQA * (DH + 2) + run_list_ints(gm.max_cta, max_slots));
     }
     if (!scratch_for((cudaStream_t) stream, need, 0)) B200_REFUSE(B200_ERR_ALLOC, "attn_reserve: %zu floats could not be allocated", need);
     return B200_OK;
