@@ -727,7 +727,7 @@ void * own_scratch_for(own_pool & pool, size_t bytes, cudaStream_t s, size_t * c
 // the SMs leave SMs idle for as long as the longest tile takes: they are cut, into at least two steps per CTA (the prologue and the hand-over of
 // a piece cost about two steps).  Measured, one layer of 4 kv heads, q8_0, with prep, tile images and merge: T = 48 behind 100003 keys (12 row tiles) 1658 ->
 // 422 us, T = 512 behind 16000 (96 row tiles) 319 -> 264 us.  More row tiles than SMs run one per CTA, the longest first.
-int split_ctas(int T, int p0, int n_mtiles, int Hkv, int sms, int * head_steps) {
+int split_ctas(int T, int p0, int n_mtiles, int Hkv, int sms, size_t image_bytes, int * head_steps) {
     const long long tiles = (long long) n_mtiles * Hkv;
     if (tiles >= sms) return 0;
     long long hs = 0;
@@ -735,6 +735,11 @@ int split_ctas(int T, int p0, int n_mtiles, int Hkv, int sms, int * head_steps) 
     if (hs * Hkv >= 1 << 30) return 0;
     *head_steps = (int) hs;
     const long long n = std::min<long long>(sms, hs * Hkv / 2);
+    // Images that L2 does not hold (126 MB, shared with everything else) are read from HBM by every row tile that is elsewhere in the keys at
+    // the time: the same number of runs for every tile keeps the tiles of a head at the same keys, if that leaves few SMs idle.
+    // 48 rows behind 100003 keys (410 MB of images, three tiles a head): 368 -> 300 us.  512 rows behind 16000 (66 MB) would get 96 runs: not taken.
+    const long long same = sms / tiles * tiles;
+    if (image_bytes > ((size_t) 64 << 20) && n == sms && same > tiles && same * 8 >= 7LL * sms) return (int) same;
     return n > tiles ? (int) n : 0;
 }
 
@@ -814,7 +819,7 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
     if (!multi && !io.lim && !io.pm) {
         int sms = 148, head_steps = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int n = split_ctas(T, p0, n_mtiles, c->Hkv, sms, &head_steps);
+        const int n = split_ctas(T, p0, n_mtiles, c->Hkv, sms, full, &head_steps);
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (n > 0 && !own && cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
         if (n > 0 && cap == cudaStreamCaptureStatusNone) {
