@@ -160,7 +160,7 @@ int b200_attn_step_end(void *stream);
 int b200_attn_dec_tc(void);
 void b200_attn_dec_set_tc(int on);
 
-/* Library-owned scratch of the decode entry points (split partials and the work list), one buffer per (device, stream)
+/* Library-owned scratch of the decode entry points (split partials and the run plan), one buffer per (device, stream)
  * like the reference's (attn_dec2.cu:452-464,503-517).  The reference-compatible entry points size it on their first call
  * for the largest call they accept on that cache (B200_ATTN_MAX_ROWS rows over n_ctx keys); for the batched entry points
  * call b200_attn_reserve once with the largest batch (n_ctx = the caches' capacity; it only matters for chunk_keys == 0).

@@ -1174,7 +1174,7 @@ int fixed_chunk(int n_ctx) {
     return (int) (chunk_lo(CH, c + 1) - chunk_lo(CH, c));
 }
 
-// Split partials and the work list live in one library-owned buffer per (device, stream), as in the reference
+// Split partials and the run plan live in one library-owned buffer per (device, stream), as in the reference
 // (src/fast/attn_dec2.cu:452-464,503-517): sized on the first call or by b200_attn_reserve, and from then on calls that
 // fit neither allocate nor synchronise, and the pointer does not move (recorded work stays valid).  A call that needs more
 // gets a new, larger buffer; the old one is kept allocated until the process exits, so nothing that was recorded against
@@ -1474,7 +1474,7 @@ int decode_check(const float * q, const b200_kv_cache * c, const float * out, co
 
 struct merge_out { float * out; const float * gate; float * fo, * fm, * fl; void * qbuf; };
 
-// the kernels of one call, partials and work list in `scr`
+// the kernels of one call, partials and run plan in `scr`
 int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo, int n_slots, int q_len, const int32_t * pos,
                   const int32_t * p0p, int p0, int Hq, float scale, const dec_geom & gm, float * scr, unsigned * st, cudaStream_t s,
                   const char * who, bool reuse_plan = false, int hk0 = 0, int nhk = 0) {
