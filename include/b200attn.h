@@ -143,7 +143,7 @@ int b200_attn_dec2_reload_env(void);
 int b200_attn_chunk_keys(void);        /* the smallest default chunk (keys): B200ATTN_CHUNK or 64 */
 int b200_attn_fixed_chunk(int n_ctx);  /* the longest chunk the entry points above use for a cache of n_ctx positions */
 /* Kernel choice of the batched entry points with chunk_keys = -1 (even split of the batch): q8_0 caches whose tiles can be
- * fetched through tensor maps (pages of at least 64 positions), with two to four rows per slot, run on the tcgen05 kernel
+ * fetched through tensor maps (pages of at least 64 positions), two or more slots of two to four rows each, run on the tcgen05 kernel
  * (one CTA per SM, K widened into tensor memory, V into an f16 image in shared memory); everything else on the mma.sync
  * kernel.  set_tc(0) keeps the mma.sync kernel everywhere, set_tc(1) restores the default, set_tc(-1) re-reads
  * B200ATTN_TC (0 = off); tc() reports the setting.  Both kernels meet the same tolerance; their results are not bitwise
@@ -163,7 +163,7 @@ void b200_attn_dec_set_tc(int on);
 /* Library-owned scratch of the decode entry points (split partials and the run plan), one buffer per (device, stream)
  * like the reference's (attn_dec2.cu:452-464,503-517).  The reference-compatible entry points size it on their first call
  * for the largest call they accept on that cache (B200_ATTN_MAX_ROWS rows over n_ctx keys); for the batched entry points
- * call b200_attn_reserve once with the largest batch (n_ctx = the caches' capacity; it only matters for chunk_keys == 0).
+ * call b200_attn_reserve once with the largest batch (n_ctx = the caches' capacity; it only matters for chunk_keys <= 0).
  * Afterwards calls that fit allocate nothing, synchronise nothing, and the buffer does not move, so recorded work stays
  * valid.  A call that needs more than was reserved gets a new, larger buffer (cudaMalloc, no synchronisation); the old one
  * stays allocated until the process exits, so earlier recorded work never reads freed memory.  Two calls on the same
@@ -180,6 +180,7 @@ int b200_attn_reserve(uint32_t kv_type, int max_slots, int q_len, int max_n, int
  * chunk_keys: keys per split (multiple of 64); 0 = the default grid (a function of the cache's capacity); -1 = an even
  * split of the whole batch: the batch's 64-key tiles, slot after slot, are cut into one contiguous run per resident CTA, so
  * ragged contexts load every SM equally (up to 2048 slots; larger batches take a chunk chosen from the batch size).
+ * A single slot with -1 takes the chunks of attn_decode (same bits, K integer times fp32 scale).
  * With chunk_keys >= 0 each row's result depends only on its own keys and on the chunk, never on the other rows of the call
  * (bitwise); with -1 the split points depend on the batch, so results of different batches agree to rounding only. */
 int b200_attn_decode_slots(const float *q, const b200_kv_cache *c, float *out, const float *gate, int n_slots,

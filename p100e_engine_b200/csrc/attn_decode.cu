@@ -1421,9 +1421,13 @@ int auto_chunk(long long total_keys, int Hkv) {
 }
 
 // geometry of a call: chunk, chunks per slot, partial floats, work-list ints
-//   split   (chunk chosen from the batch, up to SPLIT_MAX_SLOTS slots): one contiguous run of tiles per resident CTA
+//   split   (chunk chosen from the batch, two to SPLIT_MAX_SLOTS slots): one contiguous run of tiles per resident CTA
 //   planned (fixed chunks of several slots, more units than a wave): the same runs, cut at chunk boundaries
 //   else    see decode_part_k
+// One slot with chunk_keys < 0 takes the position grid: K stays integer times fp32 scale (decode_tc_k rounds q * d to f16) and short
+// chunks have reference maxima of their own.  Error against 64-bit attention over the stored rows, q8_0, 1 / 2 / 4 rows at 30011 keys:
+// 3.6e-4 / 3.6e-4 / 3.5e-4; on decode_tc_k 2 / 4 rows 4.2e-4 / 4.2e-4; one run per CTA of an f16 cache, 4 rows at 131000 keys 3.00e-4
+// against 2.96e-4.
 size_t run_list_ints(int max_cta, int n_slots) {
     return (4 * ((size_t) max_cta + n_slots) + 2 * (size_t) n_slots + max_cta + 2 + 3) & ~(size_t) 3;
 }
@@ -1433,7 +1437,7 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
     if (max_n < 1) max_n = 1;
     g.tc = false;
     g.R = q_len * GQA;
-    g.split = chunk_keys < 0 && n_slots <= SPLIT_MAX_SLOTS;
+    g.split = chunk_keys < 0 && n_slots > 1 && n_slots <= SPLIT_MAX_SLOTS;
     g.planned = false;
     g.max_cta = 0;
     if (g.split) {
@@ -1447,7 +1451,7 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
         g.list_ints = run_list_ints(g.max_cta, n_slots);
         return true;
     }
-    g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) : default_grid(n_ctx);
+    g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 && n_slots > 1 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) : default_grid(n_ctx);
     g.max_chunks = chunk_of(g.CH, max_n - 1) + 1;
     g.units = (size_t) n_slots * Hkv * g.max_chunks;
     if (g.units >= ((size_t) 1 << 31) || (size_t) n_slots * g.max_chunks >= ((size_t) 1 << 30)) return false;
@@ -1687,7 +1691,9 @@ int b200_attn_reserve(uint32_t kv_type, int max_slots, int q_len, int max_n, int
     dec_geom gm;
     if (!decode_geometry(gm, kv_type, max_slots, q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, chunk_keys)) B200_REFUSE(B200_ERR_SHAPE, "attn_reserve: too many chunks");
     size_t need = gm.part_floats + std::max(gm.list_ints, run_list_ints(gm.max_cta, max_slots));
-    if (chunk_keys < 0 && !gm.split) {
+    dec_geom g1;   // one slot may take more partials than a small batch
+    if (chunk_keys < 0 && decode_geometry(g1, kv_type, 1, q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, chunk_keys)) need = std::max(need, g1.part_floats + g1.list_ints);
+    if (chunk_keys < 0 && max_slots > 1 && !gm.split) {
         // a fixed chunk chosen from the batch: smaller batches take smaller chunks; their unit count stays under this bound
         const size_t u = 2 * 8 * (size_t) sm_count() + (size_t) max_slots * Hkv;
         need = std::max(need, u * q_len * GQA * (DH + 2) + run_list_ints(gm.max_cta, max_slots));

@@ -1,0 +1,92 @@
+"""One slot through the batched entry point with chunk_keys = -1: the same bits as the row entry points, and no further from 64-bit attention
+than fixed chunks on the same kernel."""
+import numpy as np
+import pytest
+
+from tests.util import D, SCALE, TYPES
+
+pytestmark = pytest.mark.gpu
+HKV, HQ = 2, 12
+
+
+def _dequant(raw, tname, n):
+    """stored rows in 64 bits [n][Hkv][D]"""
+    import torch
+    if tname == "f16":
+        return raw.view(torch.float16).view(n, HKV, D).double()
+    if tname == "q8_0":
+        r = raw.view(n, HKV, 272)
+        return (r[..., 16:].contiguous().view(torch.int8).double().view(n, HKV, 8, 32) *
+                r[..., :16].contiguous().view(torch.float16).double()[..., None]).view(n, HKV, D)
+    r = raw.view(n, HKV, 8, 18)
+    b = r[..., 2:].to(torch.int32)
+    return (torch.cat([(b & 15) - 8, (b >> 4) - 8], -1).double() * r[..., :2].contiguous().view(torch.float16).double()).view(n, HKV, D)
+
+
+def _attention64(q, c, tname, n, p0):
+    import torch
+    k, v = _dequant(c.k, tname, n), _dequant(c.v, tname, n)
+    T, out = q.shape[0], torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    hidden = torch.arange(n, device=q.device)[None, None] > (p0 + torch.arange(T, device=q.device))[:, None, None]
+    for h in range(HKV):
+        s = torch.einsum("tgd,nd->tgn", q[:, 6 * h:6 * h + 6].double(), k[:, h]) * SCALE
+        out[:, 6 * h:6 * h + 6] = torch.einsum("tgn,nd->tgd", s.masked_fill(hidden, float("-inf")).softmax(-1), v[:, h])
+    return out
+
+
+@pytest.mark.parametrize("tname", ["q8_0", "f16", "q4_0"])
+@pytest.mark.parametrize("n", [100, 5000, 30011])
+@pytest.mark.parametrize("T", [1, 2, 4])
+def test_one_slot_keeps_the_precision_of_fixed_chunks(cuda, lib, tname, n, T):
+    import torch
+    from p100e_engine_b200 import fast
+    c = fast.kv_alloc(TYPES[tname], n, HKV, D)
+    g = torch.Generator(device="cuda").manual_seed(n + T)
+    rn = lambda *s: torch.randn(*s, generator=g, device=cuda)
+    assert fast.kv_append(c, rn(n, HKV, D), rn(n, HKV, D), 0, n)
+    p0 = n - T
+    pos = torch.arange(p0, n, dtype=torch.int32, device=cuda)
+    err = np.zeros(2)
+    for _ in range(3):
+        q = rn(T, HQ, D)
+        one, rows, fixed = (torch.full((T, HQ, D), float("nan"), device=cuda) for _ in range(3))
+        assert fast.attn_decode_slots(q, c, one, None, 1, T, pos, n, HQ, SCALE, -1)
+        assert fast.attn_decode(q, c, rows, T, p0, HQ, SCALE)
+        assert fast.attn_decode_slots(q, c, fixed, None, 1, T, pos, n, HQ, SCALE, 512)
+        torch.cuda.synchronize()
+        assert torch.equal(one, rows)
+        ref = _attention64(q, c, tname, n, p0)
+        err += [float((o.double() - ref).norm() / ref.norm()) for o in (one, fixed)]
+    print("%s n=%d T=%d: one slot %.3e, chunks of 512 %.3e" % (tname, n, T, *(err / 3)))
+    assert fast.device_status() == 0
+    # the roundings of P are those of another set of reference maxima: three draws of T x 12 rows x 256 values scatter by a percent or two
+    assert err[0] <= 1.03 * err[1]
+
+
+@pytest.mark.parametrize("q_len", [2, 4])
+def test_verify_kernel_error(cuda, lib, q_len):
+    """two slots of the same rows on the verify kernel (K rounded to f16) and on the mma.sync kernel (K integer): both within the f16 bound"""
+    import torch
+    from p100e_engine_b200 import fast
+    n = 30011
+    c = fast.kv_alloc(TYPES["q8_0"], n, HKV, D)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rn = lambda *s: torch.randn(*s, generator=g, device=cuda)
+    assert fast.kv_append(c, rn(n, HKV, D), rn(n, HKV, D), 0, n)
+    q = rn(2 * q_len, HQ, D)
+    pos = torch.arange(n - q_len, n, dtype=torch.int32, device=cuda).repeat(2)
+    ref = torch.cat([_attention64(x, c, "q8_0", n, n - q_len) for x in (q[:q_len], q[q_len:])])
+    err = []
+    try:
+        for tc in (1, 0):
+            lib.b200_attn_dec_set_tc(tc)
+            out = torch.full((2 * q_len, HQ, D), float("nan"), device=cuda)
+            assert fast.attn_decode_slots(q, c, out, None, 2, q_len, pos, n, HQ, SCALE, -1)
+            torch.cuda.synchronize()
+            err.append(float((out.double() - ref).norm() / ref.norm()))
+    finally:
+        lib.b200_attn_dec_set_tc(-1)
+    print("q_len %d: verify kernel %.3e, mma.sync kernel %.3e" % (q_len, *err))
+    assert fast.device_status() == 0
+    # three f16 roundings (K, P, V scaled) of 2^-12 rms at most each, sums over independent errors
+    assert max(err) < 3 ** 0.5 * 2.0 ** -11
