@@ -1179,21 +1179,27 @@ int fixed_chunk(int n_ctx) {
 // fit neither allocate nor synchronise, and the pointer does not move (recorded work stays valid).  A call that needs more
 // gets a new, larger buffer; the old one is kept allocated until the process exits, so nothing that was recorded against
 // it ever reads freed memory, and no stream is synchronised.
-// The even split of a batch depends on the rows' positions only, which a model step does not change from layer to layer.
+// A run plan depends on the rows' positions only, which a model step does not change from layer to layer.
 // Between b200_attn_step_begin(stream, positions, bytes) and the next one (or b200_attn_step_end) the plan that the first
 // batched call of a given shape, with its positions inside the declared array, leaves in the stream's scratch is used again by
 // the following calls of the same shape instead of being recomputed: what identifies the plan is kept here, and any other
-// call on the stream drops it.
+// call on the stream drops it.  A recorded call's plan does not exist until the recording is replayed, and a replay comes with
+// positions of its own, so a plan serves only calls of the recording it was recorded in (`rec`), or only calls outside of any.  Plans
+// of recorded calls and of the others have a place each at the front of the buffer, away from all partials: a replay between two
+// calls of a step leaves their plan alone.
 struct plan_key {
+    unsigned long long rec = 0;
+
     const void * scr = nullptr, * pos = nullptr, * p0p = nullptr;
     int p0 = 0, n_slots = 0, q_len = 0, CH = 0, max_chunks = 0, max_cta = 0, Hkv = 0, n_ctx = 0, paged = 0;
     size_t part_floats = 0;
     bool operator==(const plan_key & o) const {
-        return scr == o.scr && pos == o.pos && p0p == o.p0p && p0 == o.p0 && n_slots == o.n_slots && q_len == o.q_len && CH == o.CH &&
+        return rec == o.rec && scr == o.scr && pos == o.pos && p0p == o.p0p && p0 == o.p0 && n_slots == o.n_slots && q_len == o.q_len && CH == o.CH &&
                max_chunks == o.max_chunks && max_cta == o.max_cta && Hkv == o.Hkv && n_ctx == o.n_ctx && paged == o.paged &&
                part_floats == o.part_floats;
     }
 };
+constexpr int SCR_PLAN_INTS = 6 * PLAN_MAX_SLOTS + 5 * SPLIT_MAX_CTA + 4;   // run_list_ints(SPLIT_MAX_CTA, PLAN_MAX_SLOTS)
 struct scratch {
     int dev = -1; cudaStream_t s = nullptr; float * p = nullptr; size_t cap = 0;
     bool step_mode = false, plan_valid = false;
@@ -1204,7 +1210,10 @@ scratch g_scr[64];
 int g_nscr = 0;
 std::mutex g_mu;
 
+// `floats`: partials of the call (0: no buffer is needed)
 scratch * scratch_entry(cudaStream_t s, size_t floats, size_t floats_hint) {
+    if (floats) floats += 2 * SCR_PLAN_INTS;
+    if (floats_hint) floats_hint += 2 * SCR_PLAN_INTS;
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(g_mu);
@@ -1431,6 +1440,14 @@ int auto_chunk(long long total_keys, int Hkv) {
 size_t run_list_ints(int max_cta, int n_slots) {
     return (4 * ((size_t) max_cta + n_slots) + 2 * (size_t) n_slots + max_cta + 2 + 3) & ~(size_t) 3;
 }
+static_assert(SCR_PLAN_INTS % 4 == 0 && SCR_PLAN_INTS >= 4 * (SPLIT_MAX_CTA + PLAN_MAX_SLOTS) + 2 * PLAN_MAX_SLOTS + SPLIT_MAX_CTA + 2, "a plan fits its place");
+// the recording the stream takes part in, 0 if none; false = unknown
+bool recording_of(cudaStream_t s, unsigned long long & id) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamGetCaptureInfo(s, &st, &id) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (st == cudaStreamCaptureStatusNone) id = 0;
+    return st != cudaStreamCaptureStatusInvalidated;
+}
 struct dec_geom { int CH, max_chunks, R, max_cta; size_t units, part_floats, list_ints; bool planned, split, tc; };
 
 bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int max_n, int n_ctx, int Hkv, int chunk_keys, bool tc = false) {
@@ -1478,9 +1495,9 @@ int decode_check(const float * q, const b200_kv_cache * c, const float * out, co
 
 struct merge_out { float * out; const float * gate; float * fo, * fm, * fl; void * qbuf; };
 
-// the kernels of one call, partials and run plan in `scr`
+// the kernels of one call, partials in `scr`, run plan in `list` (nullptr: behind the partials)
 int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo, int n_slots, int q_len, const int32_t * pos,
-                  const int32_t * p0p, int p0, int Hq, float scale, const dec_geom & gm, float * scr, unsigned * st, cudaStream_t s,
+                  const int32_t * p0p, int p0, int Hq, float scale, const dec_geom & gm, float * scr, int * list, unsigned * st, cudaStream_t s,
                   const char * who, bool reuse_plan = false, int hk0 = 0, int nhk = 0) {
     dec_args a;
     a.q = q; a.g = view_of(*c);
@@ -1499,7 +1516,7 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     // fixed chunks without a plan: at most one wave of CTAs, a multiple of the heads
     unsigned blocks = (unsigned) std::min<size_t>((size_t) n_slots * gm.max_chunks, (size_t) gm.max_cta) * (unsigned) a.nhk;
     if (gm.split || gm.planned) {
-        int * list = reinterpret_cast<int *>(scr + part_floats);
+        if (!list) list = reinterpret_cast<int *>(scr + part_floats);
         const size_t nseg = (size_t) gm.max_cta + n_slots;
         int4 * segs = reinterpret_cast<int4 *>(list);
         int2 * slot_seg = reinterpret_cast<int2 *>(list + 4 * nseg);
@@ -1542,10 +1559,9 @@ int decode_impl(const float * q, const b200_kv_cache * c, const merge_out & mo, 
     if (mo.qbuf && (!mo.out || ((uintptr_t) mo.qbuf & 3))) B200_REFUSE(B200_ERR_SHAPE, "%s: the a16 buffer needs out and 4-byte alignment", who);
     dec_geom gm;
     if (!decode_geometry(gm, c->type, n_slots, q_len, max_n, c->n_ctx, c->Hkv, chunk_keys, tc_eligible(*c, q_len))) B200_REFUSE(B200_ERR_SHAPE, "%s: too many chunks", who);
-    const size_t need = gm.part_floats + gm.list_ints;
-    scratch * e = scratch_entry(s, need, hint_floats);
-    if (!e || !e->p) B200_REFUSE(B200_ERR_ALLOC, "%s: split scratch (%zu floats) could not be allocated", who, need);
-    float * scr = e->p;
+    scratch * e = scratch_entry(s, gm.part_floats, hint_floats);
+    if (!e || !e->p) B200_REFUSE(B200_ERR_ALLOC, "%s: split scratch (%zu floats) could not be allocated", who, gm.part_floats);
+    float * scr = e->p + 2 * SCR_PLAN_INTS;
     unsigned * st = device_status_word();
     if (!st) return B200_ERR_CUDA;
     plan_key k;
@@ -1553,9 +1569,11 @@ int decode_impl(const float * q, const b200_kv_cache * c, const merge_out & mo, 
     k.max_cta = gm.max_cta; k.Hkv = c->Hkv; k.n_ctx = c->n_ctx; k.paged = c->pt != nullptr; k.part_floats = gm.part_floats;
     const bool in_step = e->step_mode && pos && (const char *) pos >= e->step_lo && (const char *) pos < e->step_hi;
     const bool listed = gm.split || gm.planned;
-    const bool reuse = listed && in_step && e->plan_valid && k == e->key;
-    const int rc = decode_launch(q, c, mo, n_slots, q_len, pos, p0p, p0, Hq, scale, gm, scr, st, s, who, reuse);
-    e->plan_valid = listed && in_step && rc == B200_OK;   // any other call on the stream rewrites the scratch
+    const bool known = !listed || recording_of(s, k.rec);
+    const bool reuse = listed && in_step && known && e->plan_valid && k == e->key;
+    int * list = reinterpret_cast<int *>(e->p) + (!known || k.rec ? SCR_PLAN_INTS : 0);
+    const int rc = decode_launch(q, c, mo, n_slots, q_len, pos, p0p, p0, Hq, scale, gm, scr, list, st, s, who, reuse);
+    e->plan_valid = listed && in_step && known && rc == B200_OK;
     e->key = k;
     return rc;
 }
@@ -1618,7 +1636,7 @@ int decode_noalloc_impl(const float * q, const b200_kv_cache * c, float * out, c
     if (src != B200_OK) return src;
     const merge_out mo = {out, gate, nullptr, nullptr, nullptr, nullptr};
     for (int h0 = 0; h0 < c->Hkv; h0 += nhk) {
-        const int rc = decode_launch(q, c, mo, n_slots, q_len, pos, nullptr, 0, Hq, scale, gm, e.partials, e.status, s, who, false, h0, std::min(nhk, c->Hkv - h0));
+        const int rc = decode_launch(q, c, mo, n_slots, q_len, pos, nullptr, 0, Hq, scale, gm, e.partials, nullptr, e.status, s, who, false, h0, std::min(nhk, c->Hkv - h0));
         if (rc != B200_OK) return rc;
     }
     return B200_OK;
@@ -1690,13 +1708,13 @@ int b200_attn_reserve(uint32_t kv_type, int max_slots, int q_len, int max_n, int
         B200_REFUSE(B200_ERR_SHAPE, "attn_reserve: unsupported arguments");
     dec_geom gm;
     if (!decode_geometry(gm, kv_type, max_slots, q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, chunk_keys)) B200_REFUSE(B200_ERR_SHAPE, "attn_reserve: too many chunks");
-    size_t need = gm.part_floats + std::max(gm.list_ints, run_list_ints(gm.max_cta, max_slots));
+    size_t need = gm.part_floats;
     dec_geom g1;   // one slot may take more partials than a small batch
-    if (chunk_keys < 0 && decode_geometry(g1, kv_type, 1, q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, chunk_keys)) need = std::max(need, g1.part_floats + g1.list_ints);
+    if (chunk_keys < 0 && decode_geometry(g1, kv_type, 1, q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, chunk_keys)) need = std::max(need, g1.part_floats);
     if (chunk_keys < 0 && max_slots > 1 && !gm.split) {
         // a fixed chunk chosen from the batch: smaller batches take smaller chunks; their unit count stays under this bound
         const size_t u = 2 * 8 * (size_t) sm_count() + (size_t) max_slots * Hkv;
-        need = std::max(need, u * q_len * GQA * (DH + 2) + run_list_ints(gm.max_cta, max_slots));
+        need = std::max(need, u * q_len * GQA * (DH + 2));
     }
     if (!scratch_for((cudaStream_t) stream, need, 0)) B200_REFUSE(B200_ERR_ALLOC, "attn_reserve: %zu floats could not be allocated", need);
     return B200_OK;
@@ -1714,7 +1732,7 @@ int b200_attn_decode2(const float * q, const b200_kv_cache * c, float * out, int
     size_t hint = 0;
     if (c && c->Hkv > 0) {
         dec_geom gm;
-        if (decode_geometry(gm, c->type, B200_ATTN_MAX_ROWS, 1, n_ctx, n_ctx, c->Hkv, 0)) hint = gm.part_floats + gm.list_ints;
+        if (decode_geometry(gm, c->type, B200_ATTN_MAX_ROWS, 1, n_ctx, n_ctx, c->Hkv, 0)) hint = gm.part_floats;
     }
     const merge_out mo = {out, nullptr, nullptr, nullptr, nullptr, nullptr};
     // rows of one sequence at consecutive positions share the pass over its KV (up to 4 rows per slot)
@@ -1737,7 +1755,7 @@ int b200_attn_decode_dev(const float * q, const b200_kv_cache * c, float * out, 
     size_t hint = 0;
     if (c && c->Hkv > 0) {
         dec_geom gm;
-        if (decode_geometry(gm, c->type, B200_ATTN_MAX_ROWS, 1, n_ctx, n_ctx, c->Hkv, 0)) hint = gm.part_floats + gm.list_ints;
+        if (decode_geometry(gm, c->type, B200_ATTN_MAX_ROWS, 1, n_ctx, n_ctx, c->Hkv, 0)) hint = gm.part_floats;
     }
     const merge_out mo = {out, nullptr, nullptr, nullptr, nullptr, nullptr};
     if (T <= B200_MAX_QLEN)
