@@ -1192,10 +1192,11 @@ struct plan_key {
 
     const void * scr = nullptr, * pos = nullptr, * p0p = nullptr;
     int p0 = 0, n_slots = 0, q_len = 0, CH = 0, max_chunks = 0, max_cta = 0, Hkv = 0, n_ctx = 0, paged = 0;
+    int split = 0, tc = 0;   // an even split has slot_seg, a plan of fixed chunks has not; they can agree in all the rest
     size_t part_floats = 0;
     bool operator==(const plan_key & o) const {
         return rec == o.rec && scr == o.scr && pos == o.pos && p0p == o.p0p && p0 == o.p0 && n_slots == o.n_slots && q_len == o.q_len && CH == o.CH &&
-               max_chunks == o.max_chunks && max_cta == o.max_cta && Hkv == o.Hkv && n_ctx == o.n_ctx && paged == o.paged &&
+               max_chunks == o.max_chunks && max_cta == o.max_cta && Hkv == o.Hkv && n_ctx == o.n_ctx && paged == o.paged && split == o.split && tc == o.tc &&
                part_floats == o.part_floats;
     }
 };
@@ -1567,6 +1568,7 @@ int decode_impl(const float * q, const b200_kv_cache * c, const merge_out & mo, 
     plan_key k;
     k.scr = scr; k.pos = pos; k.p0p = p0p; k.p0 = p0; k.n_slots = n_slots; k.q_len = q_len; k.CH = gm.CH; k.max_chunks = gm.max_chunks;
     k.max_cta = gm.max_cta; k.Hkv = c->Hkv; k.n_ctx = c->n_ctx; k.paged = c->pt != nullptr; k.part_floats = gm.part_floats;
+    k.split = gm.split; k.tc = gm.tc;
     const bool in_step = e->step_mode && pos && (const char *) pos >= e->step_lo && (const char *) pos < e->step_hi;
     const bool listed = gm.split || gm.planned;
     const bool known = !listed || recording_of(s, k.rec);

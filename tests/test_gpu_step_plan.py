@@ -146,3 +146,35 @@ def test_two_layers_of_one_recording_share_a_plan(cuda, lib):
         b.replay(g)
         b.s.synchronize()
         assert all(torch.equal(o, want) for o in outs)
+
+
+def test_even_split_and_fixed_chunks_of_one_geometry(cuda, lib):
+    """f16, 4 kv heads, two slots of up to 2432 keys in 64-key chunks: as many partials as the even split over 74 CTAs per head, the same
+    chunk and the same chunk count.  Each kind computes its own plan."""
+    import torch
+    from p100e_engine_b200 import fast
+    n = 2432
+    c = fast.kv_alloc(TYPES["f16"], n, HKV, D)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rn = lambda *s: torch.randn(*s, generator=g, device=cuda)
+    assert fast.kv_append(c, rn(n, HKV, D), rn(n, HKV, D), 0, n)
+    q, pos = rn(2, HQ, D), torch.tensor([n - 1, 2400], dtype=torch.int32, device=cuda)
+
+    def call(chunk):
+        out = torch.full((2, HQ, D), float("nan"), device=cuda)
+        n0 = lib.b200_launch_count()
+        assert fast.attn_decode_slots(q, c, out, None, 2, 1, pos, n, HQ, SCALE, chunk)
+        launches = lib.b200_launch_count() - n0
+        torch.cuda.synchronize()
+        return out, launches
+
+    want = {chunk: call(chunk)[0] for chunk in (64, -1)}
+    assert fast.attn_step_begin(pos)
+    try:
+        for chunk, launches in ((64, 3), (64, 2), (-1, 3), (-1, 2), (64, 3)):
+            out, k = call(chunk)
+            assert k == launches, chunk
+            assert torch.equal(out, want[chunk]), chunk
+    finally:
+        assert fast.attn_step_end()
+    assert fast.device_status() == 0
