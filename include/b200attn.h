@@ -132,16 +132,18 @@ int b200_attn_decode_rows(const float *q, const b200_kv_cache *c, float *out, in
 int b200_attn_decode2(const float *q, const b200_kv_cache *c, float *out, int T, int p0, const int32_t *p0_dev, int Hq,
                       float scale, void *stream, const int32_t *pos_rows);
 /* attn_dec2_nsplit / attn_dec2_set_nsplit / attn_dec2_reload_env (attn_dec2.cuh:19-21).  The reference splits the keys
- * into a fixed number of interleaved streams; this library splits them into consecutive chunks of a grid that depends on
- * the key's position and the cache's capacity only: 64 keys up to position 4096, then 32 chunks per doubling (128 keys from
- * 4096, 256 from 8192, ..) up to chunks of max(512, n_ctx / 256) keys.  set_nsplit(n > 0) pins n equal chunks per full context
- * instead (chunk = n_ctx / n rounded up to 64; 0 restores the default), nsplit reports that number (256 while nothing is pinned),
- * reload_env re-reads B200ATTN_CHUNK (a fixed chunk in keys, for every n_ctx) and returns 1 if the setting changed. */
+ * into a fixed number of interleaved streams; this library splits them into consecutive chunks that depend on the key's
+ * position and the cache's capacity only.  The row entry points above take the position grid: 64 keys up to position 4096,
+ * then 32 chunks per doubling (128 keys from 4096, 256 from 8192, ..) up to chunks of 512 keys, beyond a capacity of 131072 of n_ctx / 256
+ * rounded up to a power of two.  The batched entry points with chunk_keys = 0 take equal chunks of b200_attn_fixed_chunk(n_ctx)
+ * = max(b200_attn_chunk_keys(), n_ctx / 256 rounded up to 64).  set_nsplit(n > 0) pins n equal chunks per full context for both
+ * (chunk = n_ctx / n rounded up to 64; 0 restores the defaults), nsplit reports that number (256 while nothing is pinned),
+ * reload_env re-reads B200ATTN_CHUNK (a fixed chunk in keys for both, for every n_ctx) and returns 1 if the setting changed. */
 int b200_attn_dec2_nsplit(int Hkv);
 void b200_attn_dec2_set_nsplit(int n);
 int b200_attn_dec2_reload_env(void);
-int b200_attn_chunk_keys(void);        /* the smallest default chunk (keys): B200ATTN_CHUNK or 64 */
-int b200_attn_fixed_chunk(int n_ctx);  /* the longest chunk the entry points above use for a cache of n_ctx positions */
+int b200_attn_chunk_keys(void);        /* the smallest default chunk of the batched entry points (keys): B200ATTN_CHUNK or 512 */
+int b200_attn_fixed_chunk(int n_ctx);  /* the chunk the batched entry points use for a cache of n_ctx positions */
 /* Kernel choice of the batched entry points with chunk_keys = -1 (even split of the batch): q8_0 caches whose tiles can be
  * fetched through tensor maps (pages of at least 64 positions), two or more slots of two to four rows each, run on the tcgen05 kernel
  * (one CTA per SM, K widened into tensor memory, V into an f16 image in shared memory); everything else on the mma.sync
@@ -166,7 +168,8 @@ void b200_attn_dec_set_tc(int on);
 /* Library-owned scratch of the decode entry points (split partials and the run plan), one buffer per (device, stream)
  * like the reference's (attn_dec2.cu:452-464,503-517).  The reference-compatible entry points size it on their first call
  * for the largest call they accept on that cache (B200_ATTN_MAX_ROWS rows over n_ctx keys); for the batched entry points
- * call b200_attn_reserve once with the largest batch (n_ctx = the caches' capacity; it only matters for chunk_keys <= 0).
+ * call b200_attn_reserve once with the largest batch (n_ctx = the caches' capacity; it only matters for chunk_keys <= 0).  With chunk_keys <= 0
+ * the reservation also covers the row entry points for up to max_slots rows.
  * Afterwards calls that fit allocate nothing, synchronise nothing, and the buffer does not move, so recorded work stays
  * valid.  A call that needs more than was reserved gets a new, larger buffer (cudaMalloc, no synchronisation); the old one
  * stays allocated until the process exits, so earlier recorded work never reads freed memory.  Two calls on the same
@@ -180,7 +183,7 @@ int b200_attn_reserve(uint32_t kv_type, int max_slots, int q_len, int max_n, int
  * pt + rtab[slot * q_len] (rtab == NULL: one table for all).  The q_len rows of a slot share one pass over its KV.
  * gate != NULL: out = attn * sigmoid(gate) fused into the split merge (ew_quant(EW_SIGMOID_MUL), fused.cu:479-496;
  * k::sigmoid_mul, src/kernels.cu:85-93).  max_n: upper bound of pos[r] + 1 over the call (sizes the grid).
- * chunk_keys: keys per split (multiple of 64); 0 = the default grid (a function of the cache's capacity); -1 = an even
+ * chunk_keys: keys per split (multiple of 64); 0 = b200_attn_fixed_chunk(n_ctx) (a function of the cache's capacity); -1 = an even
  * split of the whole batch: the batch's 64-key tiles, slot after slot, are cut into one contiguous run per resident CTA, so
  * ragged contexts load every SM equally (up to 2048 slots; larger batches take a chunk chosen from the batch size).
  * A single slot with -1 takes the chunks of attn_decode (same bits, K integer times fp32 scale).
@@ -194,8 +197,8 @@ int b200_attn_decode_slots(const float *q, const b200_kv_cache *c, float *out, c
  * allocator calls after start-up.  This entry point calls no cudaMalloc, cudaFree or
  * other allocating routine, ever: the split partials go to a fixed 16 MiB array that is part of the library image on
  * every GPU that loads it.  Arguments, results and bits are those of b200_attn_decode_slots.
- *   - Limit: n_slots * chunks(max_n) * 6 * q_len * 258 floats (the partials of one kv head) must fit in 16 MiB; beyond that the
- *     call returns B200_ERR_SCRATCH with nothing launched (raise chunk_keys, or use b200_attn_decode_slots).  A call whose kv
+ *   - Limit: n_slots * ceil(max_n / chunk) * 6 * q_len * 258 floats (the partials of one kv head) must fit in 16 MiB; with
+ *     chunk_keys = -1 and several slots those of all heads (n_slots + CTAs of a head partials per head).  Beyond that the call returns B200_ERR_SCRATCH with nothing launched (raise chunk_keys, or use b200_attn_decode_slots).  A call whose kv
  *     heads do not fit together runs them in groups, one after the other.
  *   - The first call on each device looks up the array's device address (with that device current); make that first call
  *     before any stream capture begins.

@@ -96,8 +96,8 @@ template <uint32_t KT> __device__ __forceinline__ int q_slot(int d) {
     } else return d;
 }
 
-// Chunk grids of the fixed-chunk modes, by absolute key index.  CH > 0: chunks of CH keys.  CH <= 0, the library default: 64 keys up
-// to position 4096, then 32 chunks per doubling (128 keys from 4096, 256 from 8192, ..) up to chunks of 64 << -CH keys.  A short context
+// Chunk grids of the fixed-chunk modes, by absolute key index.  CH > 0: chunks of CH keys.  CH <= 0, the grid of the row entry
+// points (position_grid): 64 keys up to position 4096, then 32 chunks per doubling (128 keys from 4096, 256 from 8192, ..) up to chunks of 64 << -CH keys.  A short context
 // is cut finely enough to fill the chip whatever the cache's capacity, and a long one into little more than one wave of equal units.
 // One row, q8_0, 4 kv heads: chunks of 512 keys everywhere take 22.3 / 24.8 / 69.1 us at 4096 / 16384 / 131072 keys, of 64 keys
 // 12.7 / 24.8 / 124.1 us.
@@ -1138,8 +1138,8 @@ __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, in
 }
 
 // ------------------------------------------------------------------------------------------------ host side ----
-constexpr int DEFAULT_CHUNK = 64;         // shortest chunk of the default grid
-constexpr int NOMINAL_NSPLIT = 256;       // what nsplit() reports while nothing is pinned
+constexpr int DEFAULT_CHUNK = 512;
+constexpr int MAX_DEFAULT_CHUNKS = 256;   // the default chunk grows with n_ctx so that a context never has more chunks than this
 int g_chunk = 0;            // 0 = not read yet; else B200ATTN_CHUNK or DEFAULT_CHUNK
 bool g_chunk_from_env = false;
 int g_nsplit_override = 0;  // set_nsplit: chunks per full context
@@ -1155,23 +1155,27 @@ int default_chunk() {
     if (!g_chunk) g_chunk = env_chunk(&g_chunk_from_env);
     return g_chunk;
 }
-// The chunk grid of a call that asks for the library default: a function of the cache's capacity and of settings only, so that a
-// row's bits do not depend on the batch it is decoded in.  set_nsplit(n) pins n chunks per full context; B200ATTN_CHUNK pins the keys;
-// else the default grid (CH <= 0), whose longest chunk is 512 keys up to a capacity of 131072 and n_ctx / 256 beyond.
-int default_grid(int n_ctx) {
+// Chunks of the calls that name none: functions of the cache's capacity and of settings only, so that a row's bits do not depend on the
+// batch it is decoded in.  set_nsplit(n) pins n chunks per full context, B200ATTN_CHUNK pins the keys, for both grids.
+int pinned_chunk(int n_ctx) {
     const int base = default_chunk();
     if (g_nsplit_override > 0) return round_tile(((long long) std::max(n_ctx, 1) + g_nsplit_override - 1) / g_nsplit_override);
-    if (g_chunk_from_env) return base;
+    return g_chunk_from_env ? base : 0;
+}
+// Batched entry points with chunk_keys = 0.  A batch fills the chip with long chunks, and every chunk costs its partials: with the
+// position grid 64 slots x 4 rows at 4096 keys (q8_0, 4 kv heads) take 441 us against 214, 8 x 1 rows 37 against 29, and eight times the scratch.
+int fixed_chunk(int n_ctx) {
+    const int pinned = pinned_chunk(n_ctx);
+    return pinned ? pinned : std::max(default_chunk(), round_tile(((long long) std::max(n_ctx, 1) + MAX_DEFAULT_CHUNKS - 1) / MAX_DEFAULT_CHUNKS));
+}
+// Row entry points (attn_decode and its kin, at most 8 rows) and one slot with chunk_keys = -1: the position grid, whose longest chunk is
+// 512 keys up to a capacity of 131072 and n_ctx / 256 rounded up to a power of two beyond.
+int position_grid(int n_ctx) {
+    const int pinned = pinned_chunk(n_ctx);
+    if (pinned) return pinned;
     int k = 3;
     while (((long long) 256 * TILE << k) < n_ctx) ++k;
     return -k;
-}
-// the longest chunk of a full context
-int fixed_chunk(int n_ctx) {
-    const int CH = default_grid(n_ctx);
-    if (CH > 0) return CH;
-    const int c = chunk_of(CH, std::max(n_ctx, 1) - 1);
-    return (int) (chunk_lo(CH, c + 1) - chunk_lo(CH, c));
 }
 
 // Split partials and the run plan live in one library-owned buffer per (device, stream), as in the reference
@@ -1434,7 +1438,7 @@ int auto_chunk(long long total_keys, int Hkv) {
 //   split   (chunk chosen from the batch, two to SPLIT_MAX_SLOTS slots): one contiguous run of tiles per resident CTA
 //   planned (fixed chunks of several slots, more units than a wave): the same runs, cut at chunk boundaries
 //   else    see decode_part_k
-// One slot with chunk_keys < 0 takes the position grid: K stays integer times fp32 scale (decode_tc_k rounds q * d to f16) and short
+// rows: a call of the row entry points (chunk_keys = 0: the position grid).  One slot with chunk_keys < 0 takes the position grid: K stays integer times fp32 scale (decode_tc_k rounds q * d to f16) and short
 // chunks have reference maxima of their own.  Error against 64-bit attention over the stored rows, q8_0, 1 / 2 / 4 rows at 30011 keys:
 // 3.6e-4 / 3.6e-4 / 3.5e-4; on decode_tc_k 2 / 4 rows 4.2e-4 / 4.2e-4; one run per CTA of an f16 cache, 4 rows at 131000 keys 3.00e-4
 // against 2.96e-4.
@@ -1451,7 +1455,7 @@ bool recording_of(cudaStream_t s, unsigned long long & id) {
 }
 struct dec_geom { int CH, max_chunks, R, max_cta; size_t units, part_floats, list_ints; bool planned, split, tc; };
 
-bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int max_n, int n_ctx, int Hkv, int chunk_keys, bool tc = false) {
+bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int max_n, int n_ctx, int Hkv, int chunk_keys, bool tc = false, bool rows = false) {
     if (max_n < 1) max_n = 1;
     g.tc = false;
     g.R = q_len * GQA;
@@ -1469,7 +1473,8 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
         g.list_ints = run_list_ints(g.max_cta, n_slots);
         return true;
     }
-    g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 && n_slots > 1 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) : default_grid(n_ctx);
+    g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 && n_slots > 1 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) :
+           rows || chunk_keys < 0 ? position_grid(n_ctx) : fixed_chunk(n_ctx);
     g.max_chunks = chunk_of(g.CH, max_n - 1) + 1;
     g.units = (size_t) n_slots * Hkv * g.max_chunks;
     if (g.units >= ((size_t) 1 << 31) || (size_t) n_slots * g.max_chunks >= ((size_t) 1 << 30)) return false;
@@ -1551,15 +1556,15 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
 }  // namespace
 
 // q [rows][Hq][256]; rows = n_slots * q_len. Exactly one of (pos), (p0p), (p0) gives the positions.
-// hint_floats: size the library scratch for at least this much when it has to be (re)allocated.
+// hint_floats: size the library scratch for at least this much when it has to be (re)allocated.  rows: a call of the row entry points (decode_geometry).
 int decode_impl(const float * q, const b200_kv_cache * c, const merge_out & mo, int n_slots, int q_len, const int32_t * pos,
                 const int32_t * p0p, int p0, int max_n, int Hq, float scale, int chunk_keys, cudaStream_t s, const char * who,
-                size_t hint_floats = 0) {
+                size_t hint_floats = 0, bool rows = false) {
     const int chk = decode_check(q, c, mo.out, mo.gate, n_slots, q_len, Hq, who);
     if (chk != B200_OK) return chk;
     if (mo.qbuf && (!mo.out || ((uintptr_t) mo.qbuf & 3))) B200_REFUSE(B200_ERR_SHAPE, "%s: the a16 buffer needs out and 4-byte alignment", who);
     dec_geom gm;
-    if (!decode_geometry(gm, c->type, n_slots, q_len, max_n, c->n_ctx, c->Hkv, chunk_keys, tc_eligible(*c, q_len))) B200_REFUSE(B200_ERR_SHAPE, "%s: too many chunks", who);
+    if (!decode_geometry(gm, c->type, n_slots, q_len, max_n, c->n_ctx, c->Hkv, chunk_keys, tc_eligible(*c, q_len), rows)) B200_REFUSE(B200_ERR_SHAPE, "%s: too many chunks", who);
     scratch * e = scratch_entry(s, gm.part_floats, hint_floats);
     if (!e || !e->p) B200_REFUSE(B200_ERR_ALLOC, "%s: split scratch (%zu floats) could not be allocated", who, gm.part_floats);
     float * scr = e->p + 2 * SCR_PLAN_INTS;
@@ -1624,7 +1629,8 @@ int decode_noalloc_impl(const float * q, const b200_kv_cache * c, float * out, c
     if (chk != B200_OK) return chk;
     dec_geom gm;
     const bool ok = decode_geometry(gm, c->type, n_slots, q_len, max_n, c->n_ctx, c->Hkv, chunk_keys, tc_eligible(*c, q_len));
-    // the kv heads go in as many groups as the array needs (the partials of a fixed chunk grid are independent of one another)
+    // fixed chunks need no plan; beyond that the kv heads go in as many groups as the array needs (their partials are independent of one another)
+    if (ok && gm.planned && gm.part_floats <= NOALLOC_FLOATS && gm.part_floats + gm.list_ints > NOALLOC_FLOATS) { gm.planned = false; gm.list_ints = 0; }
     const size_t per_head = ok ? gm.part_floats / c->Hkv : 0;
     int nhk = ok ? c->Hkv : 0;
     if (ok && gm.part_floats + gm.list_ints > NOALLOC_FLOATS)
@@ -1674,7 +1680,7 @@ int b200_attn_fixed_chunk(int n_ctx) { return fixed_chunk(n_ctx); }
 
 int b200_attn_dec2_nsplit(int Hkv) {
     (void) Hkv;   // the reference derives its stream count from the SM count and Hkv; here the split follows the context
-    return g_nsplit_override > 0 ? g_nsplit_override : NOMINAL_NSPLIT;
+    return g_nsplit_override > 0 ? g_nsplit_override : MAX_DEFAULT_CHUNKS;
 }
 void b200_attn_dec2_set_nsplit(int n) { g_nsplit_override = n > 0 ? n : 0; }
 int b200_attn_step_begin(void * stream, const int32_t * positions, size_t bytes) {
@@ -1711,8 +1717,9 @@ int b200_attn_reserve(uint32_t kv_type, int max_slots, int q_len, int max_n, int
     dec_geom gm;
     if (!decode_geometry(gm, kv_type, max_slots, q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, chunk_keys)) B200_REFUSE(B200_ERR_SHAPE, "attn_reserve: too many chunks");
     size_t need = gm.part_floats;
-    dec_geom g1;   // one slot may take more partials than a small batch
-    if (chunk_keys < 0 && decode_geometry(g1, kv_type, 1, q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, chunk_keys)) need = std::max(need, g1.part_floats);
+    dec_geom g1;   // the position grid (row entry points; one slot with -1) may take more partials than a small batch of equal chunks or runs
+    if (chunk_keys <= 0 && decode_geometry(g1, kv_type, std::min(max_slots, B200_ATTN_MAX_ROWS), q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, 0, false, true))
+        need = std::max(need, g1.part_floats);
     if (chunk_keys < 0 && max_slots > 1 && !gm.split) {
         // a fixed chunk chosen from the batch: smaller batches take smaller chunks; their unit count stays under this bound
         const size_t u = 2 * 8 * (size_t) sm_count() + (size_t) max_slots * Hkv;
@@ -1734,13 +1741,13 @@ int b200_attn_decode2(const float * q, const b200_kv_cache * c, float * out, int
     size_t hint = 0;
     if (c && c->Hkv > 0) {
         dec_geom gm;
-        if (decode_geometry(gm, c->type, B200_ATTN_MAX_ROWS, 1, n_ctx, n_ctx, c->Hkv, 0)) hint = gm.part_floats;
+        if (decode_geometry(gm, c->type, B200_ATTN_MAX_ROWS, 1, n_ctx, n_ctx, c->Hkv, 0, false, true)) hint = gm.part_floats;
     }
     const merge_out mo = {out, nullptr, nullptr, nullptr, nullptr, nullptr};
     // rows of one sequence at consecutive positions share the pass over its KV (up to 4 rows per slot)
     if (!pos_rows && T <= B200_MAX_QLEN)
-        return decode_impl(q, c, mo, 1, T, nullptr, p0_dev, p0, max_n, Hq, scale, 0, (cudaStream_t) stream, "attn_decode", hint);
-    return decode_impl(q, c, mo, T, 1, pos_rows, p0_dev, p0, max_n, Hq, scale, 0, (cudaStream_t) stream, "attn_decode", hint);
+        return decode_impl(q, c, mo, 1, T, nullptr, p0_dev, p0, max_n, Hq, scale, 0, (cudaStream_t) stream, "attn_decode", hint, true);
+    return decode_impl(q, c, mo, T, 1, pos_rows, p0_dev, p0, max_n, Hq, scale, 0, (cudaStream_t) stream, "attn_decode", hint, true);
 }
 
 int b200_attn_decode(const float * q, const b200_kv_cache * c, float * out, int T, int p0, int Hq, float scale, void * stream) {
@@ -1757,12 +1764,12 @@ int b200_attn_decode_dev(const float * q, const b200_kv_cache * c, float * out, 
     size_t hint = 0;
     if (c && c->Hkv > 0) {
         dec_geom gm;
-        if (decode_geometry(gm, c->type, B200_ATTN_MAX_ROWS, 1, n_ctx, n_ctx, c->Hkv, 0)) hint = gm.part_floats;
+        if (decode_geometry(gm, c->type, B200_ATTN_MAX_ROWS, 1, n_ctx, n_ctx, c->Hkv, 0, false, true)) hint = gm.part_floats;
     }
     const merge_out mo = {out, nullptr, nullptr, nullptr, nullptr, nullptr};
     if (T <= B200_MAX_QLEN)
-        return decode_impl(q, c, mo, 1, T, nullptr, p0_dev, 0, max_n, Hq, scale, 0, (cudaStream_t) stream, "attn_decode_dev", hint);
-    return decode_impl(q, c, mo, T, 1, nullptr, p0_dev, 0, max_n, Hq, scale, 0, (cudaStream_t) stream, "attn_decode_dev", hint);
+        return decode_impl(q, c, mo, 1, T, nullptr, p0_dev, 0, max_n, Hq, scale, 0, (cudaStream_t) stream, "attn_decode_dev", hint, true);
+    return decode_impl(q, c, mo, T, 1, nullptr, p0_dev, 0, max_n, Hq, scale, 0, (cudaStream_t) stream, "attn_decode_dev", hint, true);
 }
 int b200_attn_decode_rows(const float * q, const b200_kv_cache * c, float * out, int T, const int32_t * pos, int Hq, float scale,
                           void * stream) {

@@ -52,7 +52,7 @@ def test_ragged_ends_and_grid_boundaries(cuda, lib, tname, n):
 
 def test_rows_do_not_depend_on_the_call_across_grid_boundaries(cuda, lib):
     """row t of a call that straddles a boundary of the chunk grid == the one-row call, bit for bit, also as one of several
-    slots (work list) and through the allocation-free entry, whose kv heads then go in groups"""
+    slots (a run plan) and through the allocation-free entry, whose kv heads then go in groups"""
     import torch
     from p100e_engine_b200 import fast
     n = 12000
@@ -102,3 +102,55 @@ def test_many_slots_of_fixed_chunks(cuda, lib, tname, n_slots):
         assert torch.equal(one, out[i:i + 1]), (i, int(pos[i]))
     assert torch.isfinite(out).all()
     assert fast.device_status() == 0
+
+
+@pytest.mark.parametrize("tname,n_slots,q_len,n,hkv", [
+    ("q8_0", 64, 1, 4096, 1), ("f16", 16, 4, 8192, 1), ("q4_0", 100, 4, 512, 4), ("q8_0", 100, 4, 512, 1), ("q8_0", 64, 4, 1024, 2),
+    ("q4_0", 300, 1, 1024, 2), ("q8_0", 64, 1, 4096, 4), ("q8_0", 1353, 1, 1024, 1)])
+def test_default_chunk_of_batches(cuda, lib, tname, n_slots, q_len, n, hkv):
+    """chunk_keys = 0 is the chunk that b200_attn_fixed_chunk names: 512 keys here, few enough partials for the allocation-free entry, even
+    where they fill its array to the last value and leave no room for a run plan"""
+    import torch
+    from p100e_engine_b200 import fast
+    g = torch.Generator(device="cuda").manual_seed(n_slots)
+    rn = lambda *s: torch.randn(*s, generator=g, device=cuda)
+    c = fast.kv_alloc(TYPES[tname], n, hkv, D)
+    assert fast.kv_append(c, rn(n, hkv, D), rn(n, hkv, D), 0, n)
+    assert lib.b200_attn_fixed_chunk(n) == lib.b200_attn_chunk_keys() == 512
+    rows, hq = n_slots * q_len, 6 * hkv
+    q = rn(rows, hq, D)
+    last = torch.randint(q_len - 1, n, (n_slots, 1), generator=g, device=cuda, dtype=torch.int32)
+    pos = (last - q_len + 1 + torch.arange(q_len, device=cuda, dtype=torch.int32)).reshape(-1).contiguous()
+    outs = [torch.full((rows, hq, D), float("nan"), device=cuda) for _ in range(3)]
+    assert fast.attn_decode_slots(q, c, outs[0], None, n_slots, q_len, pos, n, hq, SCALE, 0)
+    assert fast.attn_decode_slots(q, c, outs[1], None, n_slots, q_len, pos, n, hq, SCALE, 512)
+    assert fast.attn_decode_slots_noalloc(q, c, outs[2], None, n_slots, q_len, pos, n, hq, SCALE, 0) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    assert fast.device_status() == 0 and fast.noalloc_device_status() == 0
+
+
+@pytest.mark.parametrize("chunk", [0, -1])
+def test_reservation_covers_the_position_grid(cuda, lib, chunk):
+    """after attn_reserve for 8 slots, one slot with -1 and the row entry points are recorded without a call before (a recording cannot allocate)"""
+    import torch
+    from p100e_engine_b200 import fast
+    n, hkv = 4096, 4
+    c = fast.kv_alloc(TYPES["q8_0"], n, hkv, D)
+    assert fast.kv_fill_random(c, 0, n, 3)
+    c.rtab = None
+    q, pos = torch.randn(8, 6 * hkv, D, device=cuda), torch.arange(n - 8, n, dtype=torch.int32, device=cuda)
+    a, b = torch.zeros_like(q), torch.zeros_like(q)
+    assert fast.attn_decode_rows(q, c, torch.zeros_like(q), 8, pos, 6 * hkv, SCALE)          # kernels loaded
+    assert fast.attn_decode_slots(q, c, torch.zeros_like(q), None, 1, 4, pos, n, 6 * hkv, SCALE, -1)
+    want = torch.zeros_like(q)
+    assert fast.attn_decode_rows(q, c, want, 8, pos, 6 * hkv, SCALE)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    assert fast.attn_reserve(TYPES["q8_0"], 8, 4, n, n, hkv, chunk, s=side)
+    with torch.cuda.graph(graph, stream=side):
+        assert fast.attn_decode_rows(q, c, a, 8, pos, 6 * hkv, SCALE)
+        assert fast.attn_decode_slots(q, c, b, None, 1, 4, pos, n, 6 * hkv, SCALE, -1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(a, want) and torch.equal(b[:4], want[:4])
