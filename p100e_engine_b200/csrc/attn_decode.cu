@@ -814,13 +814,13 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
 // Merge a row's chunk partials.  grid (rows, Hq), P groups of 64 threads (one float4 of the head each).  P > 1: chunk c belongs to
 // summation stream c mod MERGE_STREAMS, group w walks the streams w, w + P, .. (each in ascending order, its own accumulator),
 // and the streams are added in stream order: an order that depends on the number of chunks only, not on P nor on the rest of
-// the call.  P = 1: plain ascending order.
+// the call.  P = 1: ascending order, for fixed chunks with the roundings of one chunk per stream (at most MERGE_STREAMS chunks).
 //   out != nullptr : out = num / den (* sigmoid(gate)); rows that saw no key give zeros
 //   fo  != nullptr : unnormalised num, max in natural-log units, den (for a cross-GPU merge)
 // The kernel is a chain of dependent loads (positions, maxima, partials), so what counts is how many partials are in flight:
-// merge_launch picks P from the number of partials a row can have.
+// decode_launch picks P from the number of partials a row can have and the size of the grid.
 constexpr int MERGE_STREAMS = 16;
-template <int P>
+template <int P, bool CHUNKED>
 __global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const float * __restrict__ gate, float * __restrict__ out,
                                                          float * __restrict__ fo, float * __restrict__ fm, float * __restrict__ fl,
                                                          __half2 * __restrict__ qbuf) {
@@ -835,7 +835,7 @@ __global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const
     // partials of the row's kv head: consecutive units of stride ustr from unit0 (a segment the row does not reach holds m = -inf)
     int nch;
     size_t unit0, ustr;
-    if (!a.chunked) {
+    if constexpr (!CHUNKED) {
         const int2 sg = a.slot_seg[slot];
         nch = pos < 0 ? 0 : sg.y;
         unit0 = (size_t) sg.x * a.nhk + hl; ustr = a.nhk;
@@ -870,7 +870,15 @@ __global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const
     };
     if constexpr (P == 1) {
 #pragma unroll 4
-        for (int c = 0; c < nch; ++c) add(c, num, den);
+        for (int c = 0; c < nch; ++c) {
+            if constexpr (CHUNKED) {
+                float d = 0.0f;
+                float4 n = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                add(c, n, d);
+                num.x += n.x; num.y += n.y; num.z += n.z; num.w += n.w;
+                den += d;
+            } else add(c, num, den);
+        }
     } else {
 #pragma unroll
         for (int i = 0; i < SPG; ++i) {
@@ -1541,14 +1549,19 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     else if (c->type == B200_KV_Q8_0) rc = launch_part_nt<B200_KV_Q8_0>(a, blocks, s);
     else rc = launch_part_nt<B200_KV_Q4_0>(a, blocks, s);
     if (rc != B200_OK) return rc;
-    // Partials that a row of a typical slot has.  Measured on 24 rows x heads (q8_0, 16384 / 131072 keys): the 30 us that four groups of 64
-    // threads took to walk 256 partials one after the other become 5 us with 16 groups; with up to 8 partials one group of 64
-    // threads per row keeps a launch of thousands of rows to one wave.
-    const int parts = gm.split ? gm.max_cta / n_slots + 2 : gm.max_chunks;
+    // Groups of 64 threads per (row, head), by the partials that a row of a typical slot has and by the grid.  Few partials: one group, as
+    // long as the grid would not fit the SMs at once with four (8 CTAs of 256 threads each); many partials on a grid of one wave (two CTAs of 1024
+    // threads per SM): sixteen.  Measured, us, with 1 / 4 / 16 groups: 8 partials on 24 CTAs 6.6 / 5.2 / 5.1, on 6144 17.3 / 36.2 / 127.5;
+    // 64 partials on 24 CTAs - / 11.5 / 6.2, on 1536 - / 33.7 / 46.1; 256 partials on 384 CTAs - / 34.1 / 26.8.
+    const int parts = gm.split ? gm.max_cta / n_slots + 2 : gm.max_chunks, sms = sm_count();
     const dim3 mg(n_slots * q_len, GQA * a.nhk);
-    if (gm.split && parts <= 8) launch(decode_merge_k<1>, mg, 64, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
-    else if (parts <= 32) launch(decode_merge_k<4>, mg, 256, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
-    else launch(decode_merge_k<16>, mg, 1024, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    const long long grid = (long long) mg.x * mg.y;
+    const bool one = gm.split ? parts <= 8 : parts <= 4 || (parts <= MERGE_STREAMS && grid > 8LL * sms);
+    const bool sixteen = parts > 32 && (grid <= 2LL * sms || (parts > 128 && grid <= 8LL * sms));
+    const unsigned threads = one ? 64 : sixteen ? 1024 : 256;
+    auto * merge = gm.split ? (one ? decode_merge_k<1, false> : sixteen ? decode_merge_k<16, false> : decode_merge_k<4, false>)
+                            : (one ? decode_merge_k<1, true> : sixteen ? decode_merge_k<16, true> : decode_merge_k<4, true>);
+    launch(merge, mg, threads, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
     count_launch(launches);
     return launch_status(who);
 }

@@ -154,3 +154,26 @@ def test_reservation_covers_the_position_grid(cuda, lib, chunk):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(a, want) and torch.equal(b[:4], want[:4])
+
+
+@pytest.mark.parametrize("n_slots,chunks", [(2, 4), (2, 5), (60, 16), (200, 16), (60, 17), (20, 40), (60, 40), (60, 150), (200, 150)])
+def test_merge_forms_agree(cuda, lib, n_slots, chunks):
+    """the merge runs one, four or sixteen groups of threads per row and head, by partials and grid: the bits of a row are those of the row
+    alone (24 heads x 1 row: the smallest grid)"""
+    import torch
+    from p100e_engine_b200 import fast
+    n, hkv = 64 * chunks, 4
+    c = fast.kv_alloc(TYPES["q8_0"], n, hkv, D)
+    g = torch.Generator(device="cuda").manual_seed(chunks)
+    rn = lambda *s: torch.randn(*s, generator=g, device=cuda)
+    assert fast.kv_append(c, rn(n, hkv, D), rn(n, hkv, D), 0, n)
+    q, gate = rn(n_slots, 6 * hkv, D), rn(n_slots, 6 * hkv * D)
+    pos = torch.randint(0, n, (n_slots,), generator=g, device=cuda, dtype=torch.int32)
+    pos[0], pos[1] = n - 1, -1
+    out = torch.full_like(q, float("nan"))
+    assert fast.attn_decode_slots(q, c, out, gate, n_slots, 1, pos, n, 6 * hkv, SCALE, 64)
+    for i in {0, 1, n_slots // 2, n_slots - 1}:
+        one = torch.full_like(q[:1], float("nan"))
+        assert fast.attn_decode_slots(q[i:i + 1], c, one, gate[i:i + 1], 1, 1, pos[i:i + 1], n, 6 * hkv, SCALE, 64)
+        assert torch.equal(one, out[i:i + 1]), (i, int(pos[i]))
+    assert fast.device_status() == 0
