@@ -1040,7 +1040,9 @@ __global__ void merge_peers_k(const peer_parts pp, int n_seq, int me, unsigned e
 // crosses slot boundaries becomes several segments; each segment yields one partial.  n_cta = min(max_cta, W / min_tiles): the
 // tcgen05 kernel walks tiles of 128 keys, so its runs hold at least two of these.  Fixed chunks (chunked): the same runs,
 // their ends moved to the nearest chunk boundary, so that a CTA streams neighbouring chunks of one slot instead of starting
-// afresh for each chunk of a work list (four layers of 8 rows of 700 .. 16384 keys, f16: 389 -> 341 us).  One block; n_slots
+// afresh for each chunk of a work list (four layers of 8 rows of 700 .. 16384 keys, f16: 389 -> 341 us).  As many
+// chunks as CTAs or fewer: one chunk each, without a plan where the host can tell (cut by tiles, CTAs without a chunk lie between the others and leave SMs
+// idle: 512 chunks of 512 keys, q4_0, one head, 888 CTAs: 53.8 us a call, 37.3 with a CTA per chunk).  One block; n_slots
 // <= PLAN_MAX_SLOTS.
 constexpr int SPLIT_THR = 1024, SPLIT_MAX_SLOTS = 2048, PLAN_MAX_SLOTS = 8192, SPLIT_MAX_CTA = 1024;
 __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, int max_cta, int min_tiles, int4 * __restrict__ segs, int * __restrict__ cta_seg,
@@ -1050,15 +1052,25 @@ __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, in
     __shared__ int cseg[SPLIT_MAX_CTA + 1];      // segments before CTA c
     __shared__ int scut[SPLIT_MAX_CTA + 1];      // first tile of CTA c
     __shared__ short first_slot[SPLIT_MAX_CTA];
+    __shared__ int n_chunks;
     const int tid = threadIdx.x, lim = key_limit(a);
     auto slot_keys = [&](int s) {
         int n = 0;
         for (int j = 0; j < a.q_len; ++j) n = max(n, row_pos(a, s, j) + 1);
         return min(n, lim);
     };
-    for (int s = tid; s < a.n_slots; s += SPLIT_THR) pre[s + 1] = (slot_keys(s) + TILE - 1) / TILE;
-    if (tid == 0) pre[0] = 0;
+    int my_chunks = 0;
+    for (int s = tid; s < a.n_slots; s += SPLIT_THR) {
+        const int n = slot_keys(s);
+        pre[s + 1] = (n + TILE - 1) / TILE;
+        if (a.chunked && n > 0) my_chunks += chunk_of(a.CH, n - 1) + 1;
+    }
+    if (tid == 0) { pre[0] = 0; n_chunks = 0; }
     __syncthreads();
+    if (a.chunked) {
+        my_chunks = __reduce_add_sync(0xffffffffu, my_chunks);
+        if ((tid & 31) == 0 && my_chunks) atomicAdd(&n_chunks, my_chunks);
+    }
     if (tid < 32) {   // inclusive scan of pre[1..n_slots], 32 entries at a time with a running carry
         int carry = 0;
         for (int base = 1; base <= a.n_slots; base += 32) {
@@ -1072,6 +1084,18 @@ __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, in
     }
     __syncthreads();
     const long long W = pre[a.n_slots];
+    if (a.chunked && n_chunks <= max_cta) {   // a CTA per chunk, in any order
+        if (tid == 0) cseg[0] = 0;
+        __syncthreads();
+        for (int s = tid; s < a.n_slots; s += SPLIT_THR) {
+            const int n = (pre[s + 1] - pre[s]) * TILE, k = n > 0 ? chunk_of(a.CH, n - 1) + 1 : 0;
+            int o = k ? atomicAdd(&cseg[0], k) : 0;
+            for (int c = 0; c < k; ++c, ++o) segs[o] = make_int4(s, (int) chunk_lo(a.CH, c), (int) min((long long) n, chunk_lo(a.CH, c + 1)), 0);
+        }
+        for (int c = tid; c <= n_chunks; c += SPLIT_THR) cta_seg[c] = c;
+        if (tid == 0) *n_cta_out = n_chunks;
+        return;
+    }
     const int n_cta = (int) max(1LL, min((long long) min(max_cta, SPLIT_MAX_CTA), W / min_tiles));
     if (tid <= n_cta) {
         int x = (int) (W * tid / n_cta);
@@ -1487,9 +1511,9 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
     g.units = (size_t) n_slots * Hkv * g.max_chunks;
     if (g.units >= ((size_t) 1 << 31) || (size_t) n_slots * g.max_chunks >= ((size_t) 1 << 30)) return false;
     g.part_floats = g.units * g.R * (DH + 2);
-    // a plan pays once the launch is longer than one wave of resident CTAs; shorter launches enumerate the grid
-    g.planned = n_slots > 1 && n_slots <= PLAN_MAX_SLOTS && g.units > (size_t) 2 * sm_count();
     g.max_cta = std::max(1, std::min(SPLIT_MAX_CTA, resident_ctas(type, q_len) / Hkv));
+    // a plan pays once there are more chunks than resident CTAs; fewer are enumerated
+    g.planned = n_slots > 1 && n_slots <= PLAN_MAX_SLOTS && (size_t) n_slots * g.max_chunks > (size_t) g.max_cta;
     g.list_ints = g.planned ? run_list_ints(g.max_cta, n_slots) : 0;
     return true;
 }

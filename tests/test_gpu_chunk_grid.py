@@ -177,3 +177,27 @@ def test_merge_forms_agree(cuda, lib, n_slots, chunks):
         assert fast.attn_decode_slots(q[i:i + 1], c, one, gate[i:i + 1], 1, 1, pos[i:i + 1], n, 6 * hkv, SCALE, 64)
         assert torch.equal(one, out[i:i + 1]), (i, int(pos[i]))
     assert fast.device_status() == 0
+
+
+@pytest.mark.parametrize("tname", ["q8_0", "f16"])
+@pytest.mark.parametrize("longest", [64, 1000, 4096])
+def test_short_slots_in_a_long_cache(cuda, lib, tname, longest):
+    """room for more chunks than CTAs, slots that fill few of them: a CTA per chunk (64, 1000 keys) or runs of chunks"""
+    import torch
+    from p100e_engine_b200 import fast
+    n, hkv, n_slots = 4096, 1, 300
+    c = fast.kv_alloc(TYPES[tname], n, hkv, D)
+    g = torch.Generator(device="cuda").manual_seed(longest)
+    rn = lambda *s: torch.randn(*s, generator=g, device=cuda)
+    assert fast.kv_append(c, rn(n, hkv, D), rn(n, hkv, D), 0, n)
+    q = rn(n_slots, 6 * hkv, D)
+    pos = torch.randint(-1, 64, (n_slots,), generator=g, device=cuda, dtype=torch.int32)
+    pos[7:300:19] = longest - 1
+    pos[11], pos[299] = -1, longest - 30
+    out = torch.full_like(q, float("nan"))
+    assert fast.attn_decode_slots(q, c, out, None, n_slots, 1, pos, n, 6 * hkv, SCALE, 64)
+    for i in (0, 7, 8, 11, 26, 150, 298, 299):
+        one = torch.full_like(q[:1], float("nan"))
+        assert fast.attn_decode_slots(q[i:i + 1], c, one, None, 1, 1, pos[i:i + 1], n, 6 * hkv, SCALE, 64)
+        assert torch.equal(one, out[i:i + 1]), (i, int(pos[i]))
+    assert torch.isfinite(out).all() and fast.device_status() == 0

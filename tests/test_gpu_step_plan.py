@@ -69,7 +69,7 @@ class _Batch:
             g.replay()
 
 
-KINDS = [("f16", "rows", 1), ("q8_0", 64, 1), ("q8_0", 256, 4), ("f16", -1, 1), ("q8_0", -1, 4)]   # -1 with 4 rows of q8_0: the verify kernel
+KINDS = [("f16", "rows", 1), ("q8_0", 64, 1), ("q8_0", 64, 4), ("f16", -1, 1), ("q8_0", -1, 4)]   # -1 with 4 rows of q8_0: the verify kernel
 
 
 @pytest.mark.parametrize("tname,kind,q_len", KINDS)
