@@ -214,13 +214,15 @@ __device__ __forceinline__ void a16_store_lanes8(const float4 x, __half2 * __res
 // launched this way passes pdl_enter(), so completion is transitive along the stream.
 // Measured, us: 16 layers of one row at 4096 keys (recorded) 344 -> 314, 1 + 3 rows at 30011 keys 540 -> 434, four layers of 8 x 4 rows
 // 358 -> 345, of a 77-token prompt 139 -> 131.  Plain launches stay where the early CTAs are in the way: grids of many waves (two layers of
-// 64 x 4 rows 2029 -> 2057 with all of them early, 1887 -> 1881 without), the mma.sync decode kernel, whose one wave must spread evenly over
+// 64 x 4 rows 2029 -> 2057 with all of them early, no difference without), the mma.sync decode kernel, whose one wave must spread evenly over
 // the SMs (four layers of one row at 131000 keys 364 -> 426), and prefill_k behind kv_tiles_k (48 rows at 100003 keys 421 -> 596).
+// The line is four CTAs per SM of a B200.  Late / early: rope_rows_k of 600 tokens 11.5 / 14.1 us, of 256 4.8 / 4.4; a merge of 768 CTAs behind the verify
+// kernel (8 x 4 rows at 4096 keys, with prep, in a step) 37.8 / 41.7, of 384 (two heads) 32.0 / 30.7 when launched call by call.
 __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-constexpr size_t PDL_MAX_CTAS = 1024;
+constexpr size_t PDL_MAX_CTAS = 4 * 148;
 template <typename... P, typename... A>
 inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&... args) {
     cudaLaunchAttribute at[1];
