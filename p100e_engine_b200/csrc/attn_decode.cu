@@ -133,7 +133,7 @@ struct dec_args {
     const int4 * segs;                    // (slot, first key, end key, 0) in CTA order; a run that crosses a slot boundary has several
     const int * cta_seg;                  // [n_cta + 1] first segment of each CTA
     const int2 * slot_seg;                // [n_slots] (first segment, segments) of each slot
-    const int * n_cta;                    // CTAs (per kv head) that hold work
+    const int * n_cta;                    // CTAs (per kv head) that hold work; < 0: -n_cta segments, CTA c takes c, c + CTAs of the head, ..
 };
 
 // keys of a slot that the call may touch: 1 + its largest row position, held to the caller's max_n (the grid and the
@@ -748,10 +748,14 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
     // kv head = block index mod heads: the heads of one (slot, key range) are neighbours in launch order, so the four
     // head rows of a position are fetched close together in time
     const int hl = (int) (blockIdx.x % (unsigned) a.nhk), ui = (int) (blockIdx.x / (unsigned) a.nhk);
-    int s0, s1, nch = a.max_chunks;
+    int s0, s1, nch = a.max_chunks, step = (int) (gridDim.x / (unsigned) a.nhk);
     if (a.segs) {
-        if (ui >= *a.n_cta) return;
-        s0 = a.cta_seg[ui]; s1 = a.cta_seg[ui + 1];
+        const int n = *a.n_cta;
+        if (RUNS && n < 0) { s0 = ui; s1 = -n; }
+        else {
+            if (ui >= n) return;
+            s0 = a.cta_seg[ui]; s1 = a.cta_seg[ui + 1]; step = 1;
+        }
     } else {
         if (a.n_slots == 1) {   // the chunks the slot has (a position beyond the limit is reported by the unit that runs)
             int n = 0;
@@ -782,7 +786,6 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
         t_base = *t_slot;
     }
     int tiles = 0;
-    const int step = a.segs ? 1 : (int) (gridDim.x / (unsigned) a.nhk);
     for (int u = s0; u < s1; u += step) {
         int slot, chunk = -1, k_lo, k_cap;
         unsigned unit;
@@ -1042,10 +1045,13 @@ __global__ void merge_peers_k(const peer_parts pp, int n_seq, int me, unsigned e
 // their ends moved to the nearest chunk boundary, so that a CTA streams neighbouring chunks of one slot instead of starting
 // afresh for each chunk of a work list (four layers of 8 rows of 700 .. 16384 keys, f16: 389 -> 341 us).  As many
 // chunks as CTAs or fewer: one chunk each, without a plan where the host can tell (cut by tiles, CTAs without a chunk lie between the others and leave SMs
-// idle: 512 chunks of 512 keys, q4_0, one head, 888 CTAs: 53.8 us a call, 37.3 with a CTA per chunk).  One block; n_slots
+// idle: 512 chunks of 512 keys, q4_0, one head, 888 CTAs: 53.8 us a call, 37.3 with a CTA per chunk).  Few slots of a quantised cache with chunks
+// of two tiles on average or more (list_cap): a list of all chunks, the highest first, over more CTAs than are resident.  There the chip is busy with
+// arithmetic, and what counts is that an SM gets its next chunk when it has room: 8 rows at 100003 keys, q4_0, two heads 182.9 us in runs, 158.5
+// in a list; f16, four heads, 30011 keys 136.7 and 158.4.  One block; n_slots
 // <= PLAN_MAX_SLOTS.
-constexpr int SPLIT_THR = 1024, SPLIT_MAX_SLOTS = 2048, PLAN_MAX_SLOTS = 8192, SPLIT_MAX_CTA = 1024;
-__global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, int max_cta, int min_tiles, int4 * __restrict__ segs, int * __restrict__ cta_seg,
+constexpr int SPLIT_THR = 1024, SPLIT_MAX_SLOTS = 2048, PLAN_MAX_SLOTS = 8192, SPLIT_MAX_CTA = 1024, LIST_SLOTS = 8, LIST_MAX = 8192;
+__global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, int max_cta, int list_cap, int min_tiles, int4 * __restrict__ segs, int * __restrict__ cta_seg,
                                                             int2 * __restrict__ slot_seg, int * __restrict__ n_cta_out) {
     pdl_enter();
     __shared__ int pre[PLAN_MAX_SLOTS + 1];      // tiles before slot s
@@ -1084,16 +1090,26 @@ __global__ void __launch_bounds__(SPLIT_THR) decode_split_k(const dec_args a, in
     }
     __syncthreads();
     const long long W = pre[a.n_slots];
-    if (a.chunked && n_chunks <= max_cta) {   // a CTA per chunk, in any order
-        if (tid == 0) cseg[0] = 0;
-        __syncthreads();
-        for (int s = tid; s < a.n_slots; s += SPLIT_THR) {
-            const int n = (pre[s + 1] - pre[s]) * TILE, k = n > 0 ? chunk_of(a.CH, n - 1) + 1 : 0;
-            int o = k ? atomicAdd(&cseg[0], k) : 0;
-            for (int c = 0; c < k; ++c, ++o) segs[o] = make_int4(s, (int) chunk_lo(a.CH, c), (int) min((long long) n, chunk_lo(a.CH, c + 1)), 0);
+    if (a.chunked && (n_chunks <= max_cta || (n_chunks <= list_cap && W >= 2LL * n_chunks))) {   // a list of chunks
+        if (a.n_slots <= LIST_SLOTS) {
+            if (tid < a.n_slots) { const int n = (pre[tid + 1] - pre[tid]) * TILE; cseg[tid] = n > 0 ? chunk_of(a.CH, n - 1) + 1 : 0; }
+            __syncthreads();
+            for (int s = 0; s < a.n_slots; ++s)
+                for (int c = tid; c < cseg[s]; c += SPLIT_THR) {
+                    int o = 0;   // chunks of a higher index, and of this index in earlier slots
+                    for (int r = 0; r < a.n_slots; ++r) o += max(0, cseg[r] - 1 - c) + (r < s && cseg[r] > c);
+                    segs[o] = make_int4(s, (int) chunk_lo(a.CH, c), (int) min((long long) (pre[s + 1] - pre[s]) * TILE, chunk_lo(a.CH, c + 1)), 0);
+                }
+        } else {   // a CTA each: in any order
+            if (tid == 0) cseg[0] = 0;
+            __syncthreads();
+            for (int s = tid; s < a.n_slots; s += SPLIT_THR) {
+                const int n = (pre[s + 1] - pre[s]) * TILE, k = n > 0 ? chunk_of(a.CH, n - 1) + 1 : 0;
+                int o = k ? atomicAdd(&cseg[0], k) : 0;
+                for (int c = 0; c < k; ++c, ++o) segs[o] = make_int4(s, (int) chunk_lo(a.CH, c), (int) min((long long) n, chunk_lo(a.CH, c + 1)), 0);
+            }
         }
-        for (int c = tid; c <= n_chunks; c += SPLIT_THR) cta_seg[c] = c;
-        if (tid == 0) *n_cta_out = n_chunks;
+        if (tid == 0) *n_cta_out = -n_chunks;
         return;
     }
     const int n_cta = (int) max(1LL, min((long long) min(max_cta, SPLIT_MAX_CTA), W / min_tiles));
@@ -1236,7 +1252,7 @@ struct plan_key {
                part_floats == o.part_floats;
     }
 };
-constexpr int SCR_PLAN_INTS = 6 * PLAN_MAX_SLOTS + 5 * SPLIT_MAX_CTA + 4;   // run_list_ints(SPLIT_MAX_CTA, PLAN_MAX_SLOTS)
+constexpr int SCR_PLAN_INTS = 6 * PLAN_MAX_SLOTS + 5 * SPLIT_MAX_CTA + 4;   // the longest plan (run_list_ints)
 struct scratch {
     int dev = -1; cudaStream_t s = nullptr; float * p = nullptr; size_t cap = 0;
     bool step_mode = false, plan_valid = false;
@@ -1474,10 +1490,10 @@ int auto_chunk(long long total_keys, int Hkv) {
 // chunks have reference maxima of their own.  Error against 64-bit attention over the stored rows, q8_0, 1 / 2 / 4 rows at 30011 keys:
 // 3.6e-4 / 3.6e-4 / 3.5e-4; on decode_tc_k 2 / 4 rows 4.2e-4 / 4.2e-4; one run per CTA of an f16 cache, 4 rows at 131000 keys 3.00e-4
 // against 2.96e-4.
-size_t run_list_ints(int max_cta, int n_slots) {
-    return (4 * ((size_t) max_cta + n_slots) + 2 * (size_t) n_slots + max_cta + 2 + 3) & ~(size_t) 3;
-}
-static_assert(SCR_PLAN_INTS % 4 == 0 && SCR_PLAN_INTS >= 4 * (SPLIT_MAX_CTA + PLAN_MAX_SLOTS) + 2 * PLAN_MAX_SLOTS + SPLIT_MAX_CTA + 2, "a plan fits its place");
+//   the plan holds `segs` segments, the runs' or (listed) every chunk
+size_t run_list_ints(size_t segs, int max_cta, int n_slots) { return (4 * segs + 2 * (size_t) n_slots + max_cta + 2 + 3) & ~(size_t) 3; }
+static_assert(SCR_PLAN_INTS % 4 == 0 && SCR_PLAN_INTS >= 4 * (SPLIT_MAX_CTA + PLAN_MAX_SLOTS) + 2 * PLAN_MAX_SLOTS + SPLIT_MAX_CTA + 2 &&
+              SCR_PLAN_INTS >= 4 * LIST_MAX + 2 * LIST_SLOTS + SPLIT_MAX_CTA + 4, "a plan fits its place");
 // the recording the stream takes part in, 0 if none; false = unknown
 bool recording_of(cudaStream_t s, unsigned long long & id) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -1485,7 +1501,7 @@ bool recording_of(cudaStream_t s, unsigned long long & id) {
     if (st == cudaStreamCaptureStatusNone) id = 0;
     return st != cudaStreamCaptureStatusInvalidated;
 }
-struct dec_geom { int CH, max_chunks, R, max_cta; size_t units, part_floats, list_ints; bool planned, split, tc; };
+struct dec_geom { int CH, max_chunks, R, max_cta, list_cap; size_t units, segs, part_floats, list_ints; bool planned, split, tc; };
 
 bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int max_n, int n_ctx, int Hkv, int chunk_keys, bool tc = false, bool rows = false) {
     if (max_n < 1) max_n = 1;
@@ -1493,16 +1509,16 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
     g.R = q_len * GQA;
     g.split = chunk_keys < 0 && n_slots > 1 && n_slots <= SPLIT_MAX_SLOTS;
     g.planned = false;
-    g.max_cta = 0;
+    g.max_cta = g.list_cap = 0;
     if (g.split) {
         g.CH = TILE;
         g.max_chunks = (max_n + TILE - 1) / TILE;
         g.tc = tc && type == B200_KV_Q8_0 && q_len >= 2;   // the tensor-core kernel: one CTA per SM
         g.max_cta = std::max(1, std::min(SPLIT_MAX_CTA, (g.tc ? sm_count() : resident_ctas(type, q_len)) / Hkv));
-        const size_t nseg = (size_t) g.max_cta + n_slots;
-        g.units = nseg * Hkv;
+        g.segs = (size_t) g.max_cta + n_slots;
+        g.units = g.segs * Hkv;
         g.part_floats = g.units * g.R * (DH + 2);
-        g.list_ints = run_list_ints(g.max_cta, n_slots);
+        g.list_ints = run_list_ints(g.segs, g.max_cta, n_slots);
         return true;
     }
     g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 && n_slots > 1 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) :
@@ -1514,7 +1530,9 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
     g.max_cta = std::max(1, std::min(SPLIT_MAX_CTA, resident_ctas(type, q_len) / Hkv));
     // a plan pays once there are more chunks than resident CTAs; fewer are enumerated
     g.planned = n_slots > 1 && n_slots <= PLAN_MAX_SLOTS && (size_t) n_slots * g.max_chunks > (size_t) g.max_cta;
-    g.list_ints = g.planned ? run_list_ints(g.max_cta, n_slots) : 0;
+    if (g.planned && type != B200_KV_F16 && n_slots <= LIST_SLOTS && n_slots * g.max_chunks <= LIST_MAX) g.list_cap = n_slots * g.max_chunks;
+    g.segs = std::max((size_t) g.max_cta + n_slots, (size_t) g.list_cap);
+    g.list_ints = g.planned ? run_list_ints(g.segs, g.max_cta, n_slots) : 0;
     return true;
 }
 
@@ -1555,17 +1573,17 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     unsigned blocks = (unsigned) std::min<size_t>((size_t) n_slots * gm.max_chunks, (size_t) gm.max_cta) * (unsigned) a.nhk;
     if (gm.split || gm.planned) {
         if (!list) list = reinterpret_cast<int *>(scr + part_floats);
-        const size_t nseg = (size_t) gm.max_cta + n_slots;
         int4 * segs = reinterpret_cast<int4 *>(list);
-        int2 * slot_seg = reinterpret_cast<int2 *>(list + 4 * nseg);
-        int * cta_seg = list + 4 * nseg + 2 * (size_t) n_slots;
+        int2 * slot_seg = reinterpret_cast<int2 *>(list + 4 * gm.segs);
+        int * cta_seg = list + 4 * gm.segs + 2 * (size_t) n_slots;
         int * n_cta = cta_seg + gm.max_cta + 1;
         a.segs = segs; a.cta_seg = cta_seg; a.slot_seg = slot_seg; a.n_cta = n_cta;
         if (!reuse_plan) {   // else the lists of an earlier call of this step, same shape, same positions, are still there
-            launch(decode_split_k, 1, SPLIT_THR, 0, s, a, gm.max_cta, gm.tc ? 2 : 1, segs, cta_seg, slot_seg, n_cta);
+            launch(decode_split_k, 1, SPLIT_THR, 0, s, a, gm.max_cta, gm.list_cap, gm.tc ? 2 : 1, segs, cta_seg, slot_seg, n_cta);
             ++launches;
         }
-        blocks = (unsigned) gm.max_cta * (unsigned) a.nhk;
+        // a list is dealt out to up to four waves of CTAs; CTAs without a chunk come last and leave at once
+        blocks = (unsigned) (gm.list_cap ? std::min(gm.list_cap, 4 * gm.max_cta) : gm.max_cta) * (unsigned) a.nhk;
     }
     int rc;
     if (gm.split && gm.tc) rc = launch_tc_nc(a, blocks, s);

@@ -201,3 +201,30 @@ def test_short_slots_in_a_long_cache(cuda, lib, tname, longest):
         assert fast.attn_decode_slots(q[i:i + 1], c, one, None, 1, 1, pos[i:i + 1], n, 6 * hkv, SCALE, 64)
         assert torch.equal(one, out[i:i + 1]), (i, int(pos[i]))
     assert torch.isfinite(out).all() and fast.device_status() == 0
+
+
+@pytest.mark.parametrize("tname", ["q8_0", "q4_0", "f16"])
+@pytest.mark.parametrize("chunk,n_slots", [(512, 8), (512, 9), (256, 3), (64, 8), (128, 8)])
+def test_long_slots_in_fixed_chunks(cuda, lib, tname, chunk, n_slots):
+    """more chunks than CTAs (f16: 296 CTAs of one head, q8_0 and q4_0: 888), whole ones and ragged last ones: listed (up to eight slots of a quantised
+    cache) or in runs; also through the row entry point, whose chunks grow with the position"""
+    import torch
+    from p100e_engine_b200 import fast
+    n, hkv = 70000, 1
+    c = fast.kv_alloc(TYPES[tname], n, hkv, D)
+    assert fast.kv_fill_random(c, 0, n, chunk)
+    g = torch.Generator(device="cuda").manual_seed(n_slots)
+    q = torch.randn(n_slots, 6 * hkv, D, generator=g, device=cuda)
+    pos = torch.tensor([n - 1, 65535, 65536, n - 1, -1, 63, 40000, n - 5, n - 1][:n_slots], dtype=torch.int32, device=cuda)
+    out, one = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    assert fast.attn_decode_slots(q, c, out, None, n_slots, 1, pos, n, 6 * hkv, SCALE, chunk)
+    for i in range(n_slots):
+        assert fast.attn_decode_slots(q[i:i + 1], c, one[i:i + 1], None, 1, 1, pos[i:i + 1], n, 6 * hkv, SCALE, chunk)
+    torch.cuda.synchronize()
+    assert torch.equal(one, out)
+    if n_slots == 8:
+        assert fast.attn_decode_rows(q, c, out, 8, pos, 6 * hkv, SCALE)
+        for i in (0, 1, 2, 5, 6):
+            assert fast.attn_decode(q[i:i + 1], c, one[i:i + 1], 1, int(pos[i]), 6 * hkv, SCALE)
+            assert torch.equal(one[i], out[i]), i
+    assert torch.isfinite(out).all() and fast.device_status() == 0
