@@ -134,7 +134,7 @@ int b200_attn_decode2(const float *q, const b200_kv_cache *c, float *out, int T,
 /* attn_dec2_nsplit / attn_dec2_set_nsplit / attn_dec2_reload_env (attn_dec2.cuh:19-21).  The reference splits the keys
  * into a fixed number of interleaved streams; this library splits them into consecutive chunks that depend on the key's
  * position and the cache's capacity only.  The row entry points above take the position grid: 64 keys up to position 4096,
- * then 32 chunks per doubling (128 keys from 4096, 256 from 8192, ..) up to chunks of 512 keys, beyond a capacity of 131072 of n_ctx / 256
+ * then 32 chunks per doubling (128 keys from 4096, 256 from 8192, ..) up to chunks of 512 keys, beyond a capacity of 229376 of n_ctx / 448
  * rounded up to a power of two.  The batched entry points with chunk_keys = 0 take equal chunks of b200_attn_fixed_chunk(n_ctx)
  * = max(b200_attn_chunk_keys(), n_ctx / 256 rounded up to 64).  set_nsplit(n > 0) pins n equal chunks per full context for both
  * (chunk = n_ctx / n rounded up to 64; 0 restores the defaults), nsplit reports that number (256 while nothing is pinned),

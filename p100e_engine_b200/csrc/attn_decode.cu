@@ -1217,12 +1217,14 @@ int fixed_chunk(int n_ctx) {
     return pinned ? pinned : std::max(default_chunk(), round_tile(((long long) std::max(n_ctx, 1) + MAX_DEFAULT_CHUNKS - 1) / MAX_DEFAULT_CHUNKS));
 }
 // Row entry points (attn_decode and its kin, at most 8 rows) and one slot with chunk_keys = -1: the position grid, whose longest chunk is
-// 512 keys up to a capacity of 131072 and n_ctx / 256 rounded up to a power of two beyond.
+// 512 keys up to a capacity of 229376 and n_ctx / 448 rounded up to a power of two beyond.  One row, 4 heads, chunks of up to 512 / 1024 keys: q4_0 at
+// 65664 of 131328 keys 44.7 / 54.5 us, q8_0 48.6 / 61.1 (the longest CTA walks 8 or 16 tiles); q4_0 at 262141 of 262144 125.9 / 115.1, at half of it
+// 70.2 / 76.2.
 int position_grid(int n_ctx) {
     const int pinned = pinned_chunk(n_ctx);
     if (pinned) return pinned;
     int k = 3;
-    while (((long long) 256 * TILE << k) < n_ctx) ++k;
+    while (((long long) 448 * TILE << k) < n_ctx) ++k;
     return -k;
 }
 

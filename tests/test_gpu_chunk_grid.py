@@ -228,3 +228,27 @@ def test_long_slots_in_fixed_chunks(cuda, lib, tname, chunk, n_slots):
             assert fast.attn_decode(q[i:i + 1], c, one[i:i + 1], 1, int(pos[i]), 6 * hkv, SCALE)
             assert torch.equal(one[i], out[i]), i
     assert torch.isfinite(out).all() and fast.device_status() == 0
+
+
+@pytest.mark.parametrize("n_ctx", [131072, 131328, 229376, 229632])
+def test_rows_around_capacities_where_the_grid_changes(cuda, lib, n_ctx):
+    """row t of a call == the one-row call where the longest chunk doubles; against an even split of two slots (rounding: the usual bar)"""
+    import torch
+    from p100e_engine_b200 import fast
+    n, hkv = 70000, 1
+    c = fast.kv_alloc(TYPES["q4_0"], n_ctx, hkv, D)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for p in range(0, n, 10000):
+        assert fast.kv_append(c, torch.randn(10000, hkv, D, generator=g, device=cuda), torch.randn(10000, hkv, D, generator=g, device=cuda), p, 10000)
+    q = torch.randn(4, 6 * hkv, D, generator=g, device=cuda)
+    out, one, two = torch.zeros_like(q), torch.zeros_like(q), torch.zeros(8, 6 * hkv, D, device=cuda)
+    for p0 in (n - 4, 65534, 32766):
+        assert fast.attn_decode(q, c, out, 4, p0, 6 * hkv, SCALE)
+        for t in range(4):
+            assert fast.attn_decode(q[t:t + 1], c, one[t:t + 1], 1, p0 + t, 6 * hkv, SCALE)
+        pos = torch.arange(p0, p0 + 4, dtype=torch.int32, device=cuda).repeat(2)
+        assert fast.attn_decode_slots(torch.cat([q, q]), c, two, None, 2, 4, pos, n, 6 * hkv, SCALE, -1)
+        torch.cuda.synchronize()
+        assert torch.equal(out, one), p0
+        util.check_close(out.cpu().numpy(), two[:4].cpu().numpy(), "n_ctx %d p0 %d" % (n_ctx, p0))
+    assert fast.device_status() == 0
