@@ -724,9 +724,12 @@ void * own_scratch_for(own_pool & pool, size_t bytes, cudaStream_t s, size_t * c
 }
 
 // CTAs of the even split for rows p0 .. p0 + T - 1 (n_mtiles row tiles per kv head); 0 = one row tile per CTA.  Row tiles that are fewer than
-// the SMs leave SMs idle for as long as the longest tile takes: they are cut, into at least two steps per CTA (the prologue and the hand-over of
-// a piece cost about two steps).  Measured, one layer of 4 kv heads, q8_0, with prep, tile images and merge: T = 48 behind 100003 keys (12 row tiles) 1658 ->
-// 422 us, T = 512 behind 16000 (96 row tiles) 319 -> 264 us.  More row tiles than SMs run one per CTA, the longest first.
+// the SMs leave SMs idle for as long as the longest tile takes: they are cut, into at least two steps per CTA, if that is shorter by the
+// time model below, in tenths of a microsecond, fitted to 396 shapes (T 5 .. 3000 behind 0 .. 65000 keys, q8_0, 1 / 2 / 4 heads) timed both ways in
+// turn: a step 1.4 us, each further row tile in a CTA's run 15 us (prologue and epilogue), pieces and their merge 8 us.  Measured, us, one row tile
+// per CTA / cut: 4 heads, T = 48 behind 40000 keys 586 / 124, T = 512 behind 20000 323 / 256; but T = 512 behind nothing 28 / 49, 2 heads, T = 1500
+// behind nothing 39 / 112 (the first runs cross six tiles of one step): those are left whole.  The choice is within 3 % of the better one on all
+// but six of the shapes, 10 % off at worst.
 int split_ctas(int T, int p0, int n_mtiles, int Hkv, int sms, size_t image_bytes, int * head_steps) {
     const long long tiles = (long long) n_mtiles * Hkv;
     if (tiles >= sms) return 0;
@@ -734,13 +737,30 @@ int split_ctas(int T, int p0, int n_mtiles, int Hkv, int sms, size_t image_bytes
     for (int m = 0; m < n_mtiles; ++m) hs += pf_tile_steps(T, p0, m);
     if (hs * Hkv >= 1 << 30) return 0;
     *head_steps = (int) hs;
-    const long long n = std::min<long long>(sms, hs * Hkv / 2);
+    long long n = std::min<long long>(sms, hs * Hkv / 2);
     // Images that L2 does not hold (126 MB, shared with everything else) are read from HBM by every row tile that is elsewhere in the keys at
     // the time: the same number of runs for every tile keeps the tiles of a head at the same keys, if that leaves few SMs idle.
     // 48 rows behind 100003 keys (410 MB of images, three tiles a head): 368 -> 300 us.  512 rows behind 16000 (66 MB) would get 96 runs: not taken.
     const long long same = sms / tiles * tiles;
-    if (image_bytes > ((size_t) 64 << 20) && n == sms && same > tiles && same * 8 >= 7LL * sms) return (int) same;
-    return n > tiles ? (int) n : 0;
+    const bool aligned = image_bytes > ((size_t) 64 << 20) && n == sms && same > tiles && same * 8 >= 7LL * sms;
+    if (aligned) n = same;
+    if (n <= tiles) return 0;
+    // longest tile, longest run, most row tiles in a run
+    const long long W = hs * Hkv, longest = pf_tile_steps(T, p0, n_mtiles - 1);
+    long long run = 0, segs = 0, end = 0;
+    int m = -1;   // row tile that holds the last step looked at; `end`: steps up to its end
+    for (long long c = 0; c < n; ++c) {
+        const long long a = W * c / n, b = W * (c + 1) / n;
+        while (end <= a) { m = m + 1 == n_mtiles ? 0 : m + 1; end += pf_tile_steps(T, p0, m); }
+        long long k = 1;
+        while (end < b) { m = m + 1 == n_mtiles ? 0 : m + 1; end += pf_tile_steps(T, p0, m); ++k; }
+        run = std::max(run, b - a);
+        segs = std::max(segs, k);
+    }
+    // images beyond L2 with the tiles at different keys: every step is read from HBM, 128 KB at 6.5 TB/s (512 rows behind 65000 keys, 4 heads:
+    // 948 / 977 us)
+    const long long steps_us10 = std::max(14 * run, image_bytes > ((size_t) 144 << 20) && !aligned ? W / 5 : 0);
+    return 100 * run <= 88 * longest && 14 * longest > steps_us10 + 150 * (segs - 1) + 80 ? (int) n : 0;
 }
 
 struct pf_io {

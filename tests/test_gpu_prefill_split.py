@@ -28,6 +28,9 @@ def _filled(kt, n, cuda, seed, hkv):
     ("f16", 1, 4031, 43),        # tile of 128 rows + tile of 130: ends inside an image
     ("q8_0", 1, 0, 700),         # causal ramp: tiles of 1 .. 6 steps, rows that see none of a piece's keys
     ("q8_0", 3, 1000, 130),
+    ("q8_0", 2, 2685, 174),      # runs that start at the last step of a tile, which its first rows do not see
+    ("f16", 2, 3055, 174),
+    ("q4_0", 1, 40, 1500),       # left whole: the first runs would cross many tiles of one step
 ])
 def test_cut_row_tiles_vs_oracle(cuda, lib, tname, hkv, p0, T):
     import torch
