@@ -692,35 +692,37 @@ size_t tile_bytes(int keys, int Hkv) { return (size_t) ((keys + BP - 1) / BP * B
 // first use for the call at hand (tile images capped at OWN_SCRATCH_TILE_CAP per pass; longer contexts take more passes).
 // A later call that needs more gets a new buffer half as large again at least; the old one stays allocated until the
 // process exits, so nothing is freed under work in flight and no stream is synchronised.
-struct own_scratch { int dev = -1; cudaStream_t s = nullptr; void * p = nullptr; size_t cap = 0; };
+// Launches that share a buffer are queued as one block under its lock: another thread's call on the same stream comes before or after all of
+// them.  Calls on other streams and devices do not wait for it (a launch may block on a full queue).
+struct own_scratch { int dev = -1; cudaStream_t s = nullptr; void * p = nullptr; size_t cap = 0; std::mutex mu; };
 struct own_pool { own_scratch e[64]; int n = 0; };
 own_pool g_own, g_pieces;   // tile images and carried state; pieces of the even split
-std::mutex g_pf_mu;
+std::mutex g_pf_mu;         // the pools' lists
 
-// under g_pf_mu
-void * own_scratch_for(own_pool & pool, size_t bytes, cudaStream_t s, size_t * cap_out) {
+// the buffer of (current device, stream), nullptr if the pool is full
+own_scratch * own_entry(own_pool & pool, cudaStream_t s) {
     int dev = 0;
     cudaGetDevice(&dev);
-    own_scratch * e = nullptr;
-    for (int i = 0; i < pool.n; ++i) if (pool.e[i].dev == dev && pool.e[i].s == s) e = &pool.e[i];
-    if (!e) {
-        if (pool.n == 64) return nullptr;
-        e = &pool.e[pool.n++];
-        e->dev = dev; e->s = s;
-    }
-    if (bytes > e->cap) {
-        const size_t want = std::max(bytes, e->cap + e->cap / 2);
-        void * p = nullptr;
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // no other thread's recording is disturbed
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        const cudaError_t rc = cudaMalloc(&p, want);
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        if (rc != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        e->p = p;
-        e->cap = want;
-    }
-    *cap_out = e->cap;
-    return e->p;
+    std::lock_guard<std::mutex> lk(g_pf_mu);
+    for (int i = 0; i < pool.n; ++i) if (pool.e[i].dev == dev && pool.e[i].s == s) return &pool.e[i];
+    if (pool.n == 64) return nullptr;
+    own_scratch * e = &pool.e[pool.n++];
+    e->dev = dev; e->s = s;
+    return e;
+}
+// at least `bytes` in the buffer, under its lock
+bool own_grow(own_scratch * e, size_t bytes) {
+    if (bytes <= e->cap) return true;
+    const size_t want = std::max(bytes, e->cap + e->cap / 2);
+    void * p = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // no other thread's recording is disturbed
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t rc = cudaMalloc(&p, want);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (rc != cudaSuccess) { cudaGetLastError(); return false; }
+    e->p = p;
+    e->cap = want;
+    return true;
 }
 
 // CTAs of the even split for rows p0 .. p0 + T - 1 (n_mtiles row tiles per kv head); 0 = one row tile per CTA.  Row tiles that are fewer than
@@ -788,16 +790,15 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
     const size_t carry = io.out ? 0 : align256((size_t) T * Hq * DH * sizeof(float));
     const size_t per_step = (size_t) BP * c->Hkv * TILE_BYTES_PER_KEY;
     const size_t full = tile_bytes(std::max(n_keys, 1), c->Hkv);
-    // Launches that share a buffer of the library (per device and stream) are queued as one block: another thread's call on the same
-    // stream comes before or after all of them.
-    std::unique_lock<std::mutex> lk(g_pf_mu);
+    std::unique_lock<std::mutex> lk, lk_pieces;
     const bool own = !scratch;
     if (own) {
+        own_scratch * e = own_entry(g_own, s);
+        if (e) lk = std::unique_lock<std::mutex>(e->mu);
         size_t want = 0;
         for (const size_t cap : {OWN_SCRATCH_TILE_CAP, OWN_SCRATCH_TILE_LOW}) {
             want = fixed + carry + std::min(full, std::max(cap / per_step, (size_t) 1) * per_step) + 256;
-            scratch = own_scratch_for(g_own, want, s, &scratch_bytes);
-            if (scratch) break;
+            if (e && own_grow(e, want)) { scratch = e->p; scratch_bytes = e->cap; break; }
         }
         if (!scratch) B200_REFUSE(B200_ERR_ALLOC, "%s: %zu bytes of scratch could not be allocated", who, want);
     } else if ((uintptr_t) scratch & 255) {
@@ -843,10 +844,11 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (n > 0 && !own && cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
         if (n > 0 && cap == cudaStreamCaptureStatusNone) {
-            size_t have = 0;
             const size_t pml_bytes = align256((size_t) 2 * n * BM * sizeof(float2));
-            unsigned char * pieces = (unsigned char *) own_scratch_for(g_pieces, pml_bytes + (size_t) 2 * n * BM * DH * sizeof(float), s, &have);
-            if (pieces) {   // else one row tile per CTA
+            own_scratch * e = own_entry(g_pieces, s);
+            if (e) lk_pieces = std::unique_lock<std::mutex>(e->mu);
+            if (e && own_grow(e, pml_bytes + (size_t) 2 * n * BM * DH * sizeof(float))) {   // else one row tile per CTA
+                unsigned char * pieces = (unsigned char *) e->p;
                 a.n_run = n; a.head_steps = head_steps;
                 a.pml = reinterpret_cast<float2 *>(pieces);
                 a.po = reinterpret_cast<float *>(pieces + pml_bytes);

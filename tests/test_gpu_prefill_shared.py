@@ -1,0 +1,75 @@
+"""Prefill calls that could meet in a buffer of the library: several host threads, streams and recordings."""
+import threading
+
+import pytest
+
+from tests.util import D, SCALE, TYPES
+
+pytestmark = pytest.mark.gpu
+HKV, HQ = 2, 12
+SHAPES = [(48, 6000), (5, 9000), (130, 4000)]   # rows, history: cut row tiles
+
+
+class _Call:
+    """one prefill call with inputs of its own; scratch: "library", or "caller" for the smallest that takes the context in one pass"""
+
+    def __init__(self, cuda, seed, shape, scratch):
+        import torch
+        from p100e_engine_b200 import fast
+        self.T, self.p0 = shape
+        n = self.T + self.p0
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        self.c = fast.kv_alloc(TYPES["q8_0"], n, HKV, D)
+        assert fast.kv_fill_random(self.c, 0, n, seed)
+        self.q, self.gate = torch.randn(self.T, HQ, D, generator=g, device=cuda), torch.randn(self.T, HQ * D, generator=g, device=cuda)
+        self.out = torch.full((self.T, HQ, D), float("nan"), device=cuda)
+        self.nb = fast.attn_fold_scratch_bytes(self.T, HKV, n) if scratch == "caller" else 0
+        self.scratch = torch.empty(self.nb, dtype=torch.uint8, device=cuda) if self.nb else None
+        self.want = None
+
+    def __call__(self, s=None):
+        from p100e_engine_b200 import fast
+        assert fast.attn_prefill_gated(self.q, self.c, self.out, self.gate, self.T, self.p0, HQ, SCALE, self.scratch, self.nb, s=s)
+
+    def alone(self):
+        import torch
+        self()
+        torch.cuda.synchronize()
+        self.want = self.out.clone()
+        self.out.fill_(float("nan"))
+        torch.cuda.synchronize()
+
+
+def _in_threads(calls, streams, rounds=40):
+    import torch
+    failed = []
+
+    def work(call, stream):
+        try:
+            torch.cuda.set_device(0)
+            for _ in range(rounds):
+                call(stream)
+        except BaseException as e:
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=x) for x in zip(calls, streams)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
+    for c in calls:
+        assert torch.equal(c.out, c.want)
+
+
+@pytest.mark.parametrize("scratch", ["library", "caller"])
+def test_threads_on_one_stream_and_on_several(cuda, lib, scratch):
+    import torch
+    from p100e_engine_b200 import fast
+    calls = [_Call(cuda, i, SHAPES[i % 3], scratch) for i in range(4)]
+    for c in calls:
+        c.alone()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    _in_threads(calls, [a, a, b, b])
+    assert fast.device_status() == 0
