@@ -266,9 +266,11 @@ int b200_seq_merge_peers_a16(const void *const *parts, void *const *flags, int n
  * the cache must already hold 0..p0+T-1.  Uses library scratch: one buffer per (device, stream), allocated on first use,
  * at most 640 MiB of tile images per pass (256 MiB where that cannot be had) plus 8 bytes per row and head; a longer context takes
  * several passes; a call that needs more than earlier ones gets a new buffer and the old one stays allocated (nothing is freed or
- * synchronised).  Calls of this family with fewer row tiles (128 rows of a kv head) than the GPU has SMs also keep up to 39 MiB per (device,
- * stream) for the partial sums of row tiles that are cut between CTAs; without that memory, and where a call with the caller's scratch
- * is being recorded, a tile runs in one CTA. */
+ * synchronised).  Calls of this family with fewer row tiles (128 rows of a kv head) than the GPU has SMs may cut row tiles between
+ * CTAs; the partial sums (up to 39 MiB) lie behind the tile images, in the library's scratch or in the caller's where it has room for
+ * all visible keys and for them.  A call with less of the caller's scratch takes a library buffer for them (one per device and stream,
+ * passed on between streams by an event), or, while it is being recorded or without that memory, runs a row tile per CTA.  The two
+ * forms agree to rounding; which one a call takes depends on its sizes, the number of SMs and the above. */
 int b200_attn_prefill(const float *q, const b200_kv_cache *c, float *out, int T, int p0, int Hq, float scale, void *stream);
 int b200_attn_prefill_variant(const float *q, const b200_kv_cache *c, float *out, int T, int p0, int Hq, float scale,
                               void *stream, int variant);

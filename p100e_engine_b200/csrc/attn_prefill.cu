@@ -694,9 +694,14 @@ size_t tile_bytes(int keys, int Hkv) { return (size_t) ((keys + BP - 1) / BP * B
 // process exits, so nothing is freed under work in flight and no stream is synchronised.
 // Launches that share a buffer are queued as one block under its lock: another thread's call on the same stream comes before or after all of
 // them.  Calls on other streams and devices do not wait for it (a launch may block on a full queue).
-struct own_scratch { int dev = -1; cudaStream_t s = nullptr; void * p = nullptr; size_t cap = 0; std::mutex mu; };
+struct own_scratch {
+    int dev = -1; cudaStream_t s = nullptr; void * p = nullptr; size_t cap = 0;
+    std::mutex mu;
+    unsigned long long user = 0; cudaEvent_t done = nullptr;   // g_pieces: the last stream that used the buffer and its last use
+};
 struct own_pool { own_scratch e[64]; int n = 0; };
-own_pool g_own, g_pieces;   // tile images and carried state; pieces of the even split
+own_pool g_own;      // tile images, carried state and pieces of calls without scratch of their own
+own_pool g_pieces;   // pieces of calls with the caller's scratch that has no room for them
 std::mutex g_pf_mu;         // the pools' lists
 
 // the buffer of (current device, stream), nullptr if the pool is full
@@ -723,6 +728,32 @@ bool own_grow(own_scratch * e, size_t bytes) {
     e->p = p;
     e->cap = want;
     return true;
+}
+
+// Pieces for a call whose scratch is the caller's.  Such a call must not depend on what else runs on the GPU: a recorded one may be replayed
+// anywhere, so it gets none; and a stream handle may stand for several streams (cudaStreamPerThread; the handle of a destroyed stream, given out
+// again), so the buffer goes from one stream to the next through an event.  On success the buffer is locked and `user` is the stream's id.
+own_scratch * pieces_acquire(size_t bytes, cudaStream_t s, std::unique_lock<std::mutex> & lk, unsigned long long & user) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (cap != cudaStreamCaptureStatusNone) return nullptr;
+    if (cudaStreamGetId(s, &user) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    own_scratch * e = own_entry(g_pieces, s);
+    if (!e) return nullptr;
+    lk = std::unique_lock<std::mutex>(e->mu);
+    bool ok = true;
+    if (!e->done) {
+        ok = cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming) == cudaSuccess;
+        e->user = user;
+    } else if (e->user != user) ok = cudaStreamWaitEvent(s, e->done, 0) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    if (ok && own_grow(e, bytes)) return e;
+    lk.unlock();
+    return nullptr;
+}
+void pieces_release(own_scratch * e, cudaStream_t s, unsigned long long user) {
+    if (cudaEventRecord(e->done, s) != cudaSuccess) cudaGetLastError();
+    e->user = user;
 }
 
 // CTAs of the even split for rows p0 .. p0 + T - 1 (n_mtiles row tiles per kv head); 0 = one row tile per CTA.  Row tiles that are fewer than
@@ -790,15 +821,27 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
     const size_t carry = io.out ? 0 : align256((size_t) T * Hq * DH * sizeof(float));
     const size_t per_step = (size_t) BP * c->Hkv * TILE_BYTES_PER_KEY;
     const size_t full = tile_bytes(std::max(n_keys, 1), c->Hkv);
-    std::unique_lock<std::mutex> lk, lk_pieces;
+    // row tiles cut between n_run CTAs (calls of one pass): pieces behind the images
+    int dev = 0, sms = 148, head_steps = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int n_mtiles = (T * GQA + BM - 1) / BM;
+    const int n_run = io.lim || io.pm ? 0 : split_ctas(T, p0, n_mtiles, c->Hkv, sms, full, &head_steps);
+    const size_t pml_bytes = align256((size_t) 2 * n_run * BM * sizeof(float2)), piece_bytes = n_run ? pml_bytes + (size_t) 2 * n_run * BM * DH * sizeof(float) : 0;
+    std::unique_lock<std::mutex> lk;
     const bool own = !scratch;
     if (own) {
         own_scratch * e = own_entry(g_own, s);
         if (e) lk = std::unique_lock<std::mutex>(e->mu);
         size_t want = 0;
         for (const size_t cap : {OWN_SCRATCH_TILE_CAP, OWN_SCRATCH_TILE_LOW}) {
-            want = fixed + carry + std::min(full, std::max(cap / per_step, (size_t) 1) * per_step) + 256;
-            if (e && own_grow(e, want)) { scratch = e->p; scratch_bytes = e->cap; break; }
+            const size_t images = std::min(full, std::max(cap / per_step, (size_t) 1) * per_step);
+            for (const size_t extra : {images == full ? piece_bytes : 0, (size_t) 0}) {
+                want = fixed + carry + images + extra + 256;
+                if (e && own_grow(e, want)) { scratch = e->p; scratch_bytes = e->cap; break; }
+                if (!extra) break;
+            }
+            if (scratch) break;
         }
         if (!scratch) B200_REFUSE(B200_ERR_ALLOC, "%s: %zu bytes of scratch could not be allocated", who, want);
     } else if ((uintptr_t) scratch & 255) {
@@ -815,8 +858,6 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
     unsigned * st = device_status_word();
     if (!st) return B200_ERR_CUDA;
     static std::atomic<bool> attr_done[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
     if (!attr_done[dev & 63].load(std::memory_order_acquire)) {
         if (cudaFuncSetAttribute(prefill_k, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_TOTAL) != cudaSuccess)
             return launch_status("attn_prefill (shared memory attribute)");
@@ -833,26 +874,17 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
     a.tiles = tiles;
     a.T = T; a.p0 = p0; a.Hq = Hq; a.Hkv = c->Hkv; a.qscale = scale * LOG2E_PF; a.status = st;
     const kv_view g = view_of(*c);
-    const int n_mtiles = (T * GQA + BM - 1) / BM;
-    // The pieces of the even split lie in a buffer of the library.  A recorded call whose scratch is the caller's must not depend on
-    // it (the recording may be replayed beside other calls).
-    a.n_run = 0; a.n_mtiles = n_mtiles; a.head_steps = 0; a.po = nullptr; a.pml = nullptr;
-    if (!multi && !io.lim && !io.pm) {
-        int sms = 148, head_steps = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int n = split_ctas(T, p0, n_mtiles, c->Hkv, sms, full, &head_steps);
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (n > 0 && !own && cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
-        if (n > 0 && cap == cudaStreamCaptureStatusNone) {
-            const size_t pml_bytes = align256((size_t) 2 * n * BM * sizeof(float2));
-            own_scratch * e = own_entry(g_pieces, s);
-            if (e) lk_pieces = std::unique_lock<std::mutex>(e->mu);
-            if (e && own_grow(e, pml_bytes + (size_t) 2 * n * BM * DH * sizeof(float))) {   // else one row tile per CTA
-                unsigned char * pieces = (unsigned char *) e->p;
-                a.n_run = n; a.head_steps = head_steps;
-                a.pml = reinterpret_cast<float2 *>(pieces);
-                a.po = reinterpret_cast<float *>(pieces + pml_bytes);
-            }
+    a.n_run = 0; a.n_mtiles = n_mtiles; a.head_steps = head_steps; a.po = nullptr; a.pml = nullptr;
+    own_scratch * lent = nullptr;
+    unsigned long long user = 0;
+    if (n_run && !multi) {
+        unsigned char * pieces = nullptr;
+        if (scratch_bytes >= fixed + full + piece_bytes) pieces = base + fixed + full;
+        else if (!own && (lent = pieces_acquire(piece_bytes, s, lk, user)) != nullptr) pieces = (unsigned char *) lent->p;
+        if (pieces) {   // else one row tile per CTA
+            a.n_run = n_run;
+            a.pml = reinterpret_cast<float2 *>(pieces);
+            a.po = reinterpret_cast<float *>(pieces + pml_bytes);
         }
     }
     int launches = 0;
@@ -873,6 +905,7 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
         }
         kb = ke;
     } while (kb < n_keys);
+    if (lent) pieces_release(lent, s, user);
     count_launch(launches);
     return launch_status(who);
 }

@@ -73,3 +73,66 @@ def test_threads_on_one_stream_and_on_several(cuda, lib, scratch):
     a, b = torch.cuda.Stream(), torch.cuda.Stream()
     _in_threads(calls, [a, a, b, b])
     assert fast.device_status() == 0
+
+
+def test_threads_on_the_per_thread_stream(cuda, lib):
+    """cudaStreamPerThread is one handle and a stream per thread"""
+    from p100e_engine_b200 import fast
+    calls = [_Call(cuda, i, SHAPES[i % 3], "caller") for i in range(3)]
+    for c in calls:
+        c.alone()
+    _in_threads(calls, [2, 2, 2])
+    assert fast.device_status() == 0
+
+
+def test_replay_elsewhere_beside_a_call_on_the_recording_stream(cuda, lib):
+    """a recorded call with the library's scratch, replayed on another stream, and a call with the caller's scratch on the stream it was recorded
+    on share nothing"""
+    import torch
+    from p100e_engine_b200 import fast
+    rec, own = _Call(cuda, 1, SHAPES[0], "library"), _Call(cuda, 2, SHAPES[1], "caller")
+    rec.alone()
+    own.alone()
+    a, b, graph = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(a):
+        rec(a)                                   # sizes the stream's scratch
+        a.synchronize()
+        with torch.cuda.graph(graph, stream=a):
+            rec(a)
+    torch.cuda.synchronize()
+    for _ in range(30):
+        with torch.cuda.stream(b):
+            graph.replay()
+        own(a)
+    torch.cuda.synchronize()
+    assert torch.equal(rec.out, rec.want) and torch.equal(own.out, own.want)
+    assert fast.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_room_in_the_callers_scratch(cuda, lib, shape):
+    """with room for images and partial sums a call is the same, recorded or not, with the library's scratch or its own; without, a recorded
+    call runs a row tile per CTA: the same attention, to f16 operands and fp32 sums (2e-3 of the largest output)"""
+    import torch
+    from p100e_engine_b200 import fast
+    call = _Call(cuda, 3, shape, "library")
+    call.alone()
+    n = shape[0] + shape[1]
+    small = fast.attn_fold_scratch_bytes(shape[0], HKV, n)
+    for nb in (small, small + (40 << 20)):
+        call.nb, call.scratch = nb, torch.empty(nb, dtype=torch.uint8, device=cuda)
+        call.out.fill_(float("nan"))
+        call()
+        torch.cuda.synchronize()
+        assert torch.equal(call.out, call.want)
+        side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            call(side)
+        call.out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        if nb == small:
+            assert (call.out - call.want).abs().max() <= 2e-3 * call.want.abs().max()
+        else:
+            assert torch.equal(call.out, call.want)
+    assert fast.device_status() == 0
