@@ -26,6 +26,7 @@
 // Reference counterparts: attn_fold (src/fast/attn_fold.cu:562-649: per chunk dequantise to f16 in scratch, HFMA2 tile
 // GEMMs on CUDA cores), attn_prefill (src/fast/attn.cu:457-499, fp32 CUDA cores).
 #include "umma.cuh"
+#include "grow.h"
 
 #include <cuda_bf16.h>
 
@@ -683,6 +684,7 @@ constexpr size_t TILE_BYTES_PER_KEY = 2 * IMG / BN;   // K and V images: 1 KiB p
 constexpr int DEFAULT_PASS_KEYS = 8192;               // keys per pass that attn_fold_scratch_bytes(T, Hkv, 0, 0) provides for
 constexpr size_t OWN_SCRATCH_TILE_CAP = (size_t) 640 << 20;   // library scratch holds tile images for at most this many bytes per pass,
 constexpr size_t OWN_SCRATCH_TILE_LOW = (size_t) 256 << 20;   // or this many where that much memory cannot be had
+constexpr size_t OWN_SCRATCH_PIECES = (size_t) 40 << 20;      // pieces of the even split: 2 x 148 of 128 rows of 1032 bytes
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t) 255; }
 size_t ml_bytes(int T, int Hkv) { return align256((size_t) T * Hkv * GQA * 2 * sizeof(float)); }
@@ -690,12 +692,13 @@ size_t tile_bytes(int keys, int Hkv) { return (size_t) ((keys + BP - 1) / BP * B
 
 // Library scratch of the prefill entry points that take none from the caller: one buffer per (device, stream), sized on
 // first use for the call at hand (tile images capped at OWN_SCRATCH_TILE_CAP per pass; longer contexts take more passes).
-// A later call that needs more gets a new buffer half as large again at least; the old one stays allocated until the
-// process exits, so nothing is freed under work in flight and no stream is synchronised.
+// A later call that needs more gets a new buffer (grow_buffer); the old one stays allocated until the process exits, so nothing is freed
+// under work in flight and no stream is synchronised.
 // Launches that share a buffer are queued as one block under its lock: another thread's call on the same stream comes before or after all of
 // them.  Calls on other streams and devices do not wait for it (a launch may block on a full queue).
 struct own_scratch {
-    int dev = -1; cudaStream_t s = nullptr; void * p = nullptr; size_t cap = 0;
+    int dev = -1; cudaStream_t s = nullptr;
+    grow_buffer b;
     std::mutex mu;
     unsigned long long user = 0; cudaEvent_t done = nullptr;   // g_pieces: the last stream that used the buffer and its last use
 };
@@ -717,17 +720,15 @@ own_scratch * own_entry(own_pool & pool, cudaStream_t s) {
 }
 // at least `bytes` in the buffer, under its lock
 bool own_grow(own_scratch * e, size_t bytes) {
-    if (bytes <= e->cap) return true;
-    const size_t want = std::max(bytes, e->cap + e->cap / 2);
-    void * p = nullptr;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // no other thread's recording is disturbed
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t rc = cudaMalloc(&p, want);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (rc != cudaSuccess) { cudaGetLastError(); return false; }
-    e->p = p;
-    e->cap = want;
-    return true;
+    return e->b.need(bytes, OWN_SCRATCH_TILE_CAP + OWN_SCRATCH_PIECES, [](size_t want) {
+        void * p = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // no other thread's recording is disturbed
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t rc = cudaMalloc(&p, want);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (rc != cudaSuccess) { cudaGetLastError(); return (void *) nullptr; }
+        return p;
+    });
 }
 
 // Pieces for a call whose scratch is the caller's.  Such a call must not depend on what else runs on the GPU: a recorded one may be replayed
@@ -838,7 +839,7 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
             const size_t images = std::min(full, std::max(cap / per_step, (size_t) 1) * per_step);
             for (const size_t extra : {images == full ? piece_bytes : 0, (size_t) 0}) {
                 want = fixed + carry + images + extra + 256;
-                if (e && own_grow(e, want)) { scratch = e->p; scratch_bytes = e->cap; break; }
+                if (e && own_grow(e, want)) { scratch = e->b.p; scratch_bytes = e->b.cap; break; }
                 if (!extra) break;
             }
             if (scratch) break;
@@ -848,9 +849,11 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
         B200_REFUSE(B200_ERR_SCRATCH, "%s: scratch must be 256-byte aligned", who);
     }
     // one pass if the tile images of every visible key fit (no running O is needed then), else as many keys per pass as fit
-    size_t steps_fit = scratch_bytes > fixed ? (scratch_bytes - fixed) / per_step : 0;
+    // (of the library's buffer no more than its cap, whatever an earlier call made of it: the passes depend on this call alone)
+    const size_t most = own ? std::max(OWN_SCRATCH_TILE_CAP / per_step, (size_t) 1) : (size_t) 1 << 40;
+    size_t steps_fit = std::min(most, scratch_bytes > fixed ? (scratch_bytes - fixed) / per_step : 0);
     bool multi = steps_fit * per_step < full;
-    if (multi) steps_fit = scratch_bytes > fixed + carry ? (scratch_bytes - fixed - carry) / per_step : 0;
+    if (multi) steps_fit = std::min(most, scratch_bytes > fixed + carry ? (scratch_bytes - fixed - carry) / per_step : 0);
     if (steps_fit < 1)
         B200_REFUSE(B200_ERR_SCRATCH, "%s: scratch too small (%zu bytes given; %zu needed for one 128-key step, %zu for a single pass over %d keys)",
                     who, scratch_bytes, fixed + carry + per_step, fixed + full, n_keys);
@@ -880,7 +883,7 @@ int prefill_run(const pf_io & io, const b200_kv_cache * c, int T, int p0, int n_
     if (n_run && !multi) {
         unsigned char * pieces = nullptr;
         if (scratch_bytes >= fixed + full + piece_bytes) pieces = base + fixed + full;
-        else if (!own && (lent = pieces_acquire(piece_bytes, s, lk, user)) != nullptr) pieces = (unsigned char *) lent->p;
+        else if (!own && (lent = pieces_acquire(piece_bytes, s, lk, user)) != nullptr) pieces = (unsigned char *) lent->b.p;
         if (pieces) {   // else one row tile per CTA
             a.n_run = n_run;
             a.pml = reinterpret_cast<float2 *>(pieces);

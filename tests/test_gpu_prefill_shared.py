@@ -136,3 +136,26 @@ def test_room_in_the_callers_scratch(cuda, lib, shape):
         else:
             assert torch.equal(call.out, call.want)
     assert fast.device_status() == 0
+
+
+def test_an_earlier_larger_call_does_not_change_a_call(cuda, lib):
+    """165000 keys of four heads are more images than one pass of the library's scratch holds; a call with 20000 rows in between needs a little
+    more of it, which makes the buffer larger, not the passes"""
+    import torch
+    from p100e_engine_b200 import fast
+    n, T, hkv, hq = 165000, 5, 4, 24
+    c = fast.kv_alloc(TYPES["q4_0"], n, hkv, D)
+    assert fast.kv_fill_random(c, 0, n, 5)
+    q = torch.randn(T, hq, D, device=cuda, generator=torch.Generator(device="cuda").manual_seed(1))
+    big = torch.zeros(20000, hq, D, device=cuda)
+    big_out, outs = torch.empty_like(big), [torch.full((T, hq, D), float("nan"), device=cuda) for _ in range(2)]
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for i in range(2):
+        n0 = lib.b200_launch_count()
+        assert fast.attn_prefill(q, c, outs[i], T, n - T, hq, SCALE, s=s)
+        assert lib.b200_launch_count() - n0 == 4     # two passes
+        assert fast.attn_prefill(big, c, big_out, big.shape[0], n - big.shape[0], hq, SCALE, s=s)
+    s.synchronize()
+    assert torch.equal(outs[0], outs[1])
+    assert fast.device_status() == 0
