@@ -98,6 +98,8 @@ struct tok_args {
     unsigned * status;
 };
 constexpr int TOK_WARPS = 8;
+// floats of a token's cos / sin table; n_rot is even, the heads behind it are read and written four floats at a time
+__host__ __device__ __forceinline__ int tok_cs_floats(int n_rot) { return (n_rot + 3) & ~3; }
 
 // PREP: attention input prep of the decode path (reference semantics: attn_prep_k, src/fast/fused.cu:502-573): per q head
 // the gate half is copied out and q = rope(rmsnorm(q) * q_norm); per K head the same norm and rotation, then the cache bytes;
@@ -113,10 +115,10 @@ constexpr int TOK_WARPS = 8;
 template <uint32_t KT, bool PREP, bool MR, int NF>
 __global__ void __launch_bounds__(TOK_WARPS * 32) token_k(const tok_args a) {
     pdl_enter();
-    extern __shared__ float sm[];   // cos[half] | sin[half] | TOK_WARPS staged heads of D floats
+    extern __shared__ __align__(16) float sm[];   // cos[half] | sin[half] | TOK_WARPS staged heads of D floats, 16-byte aligned
     const int t = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int D = a.D, nb = D / 32, nf = D / 128, half = a.n_rot / 2;
-    float * cs = sm, * st = sm + a.n_rot + w * D;
+    float * cs = sm, * st = sm + tok_cs_floats(a.n_rot) + w * D;
     const int n_q = PREP && a.qg ? a.Hq : 0, it = blockIdx.y * TOK_WARPS + w;
     const bool live = it < n_q + 2 * a.Hkv, is_q = it < n_q, is_v = it >= n_q + a.Hkv;
     const int h = is_q ? it : is_v ? it - n_q - a.Hkv : it - n_q;
@@ -510,7 +512,7 @@ bool type_ok(uint32_t t) { return t == B200_KV_F16 || t == B200_KV_Q8_0 || t == 
 
 template <bool PREP>
 int token_launch(const tok_args & a, uint32_t type, int T, bool mrope, cudaStream_t s, const char * who) {
-    const size_t smem = PREP ? ((size_t) a.n_rot + (size_t) TOK_WARPS * a.D) * sizeof(float) : 0;
+    const size_t smem = PREP ? ((size_t) tok_cs_floats(a.n_rot) + (size_t) TOK_WARPS * a.D) * sizeof(float) : 0;
     const dim3 grid(T, ((PREP && a.qg ? a.Hq : 0) + 2 * a.Hkv + TOK_WARPS - 1) / TOK_WARPS);
 #define TOKEN_NF(KT_, MR_) do { if (a.D <= 256) launch(token_k<KT_, PREP, MR_, 2>, grid, TOK_WARPS * 32, smem, s, a); \
                                 else launch(token_k<KT_, PREP, MR_, 8>, grid, TOK_WARPS * 32, smem, s, a); } while (0)
@@ -656,7 +658,7 @@ int b200_attn_prep(const float * qg, const float * k, const float * v, const flo
     if (ldv <= 0) ldv = Hkv * D;
     if (!c || !k || !v || !pos || (qg && (!q || !gate))) B200_REFUSE(B200_ERR_SHAPE, "attn_prep: null argument");
     if (ldq < Hq * 2 * D || ldk < Hkv * D || ldv < Hkv * D || ldq % 4 || ldk % 4) B200_REFUSE(B200_ERR_SHAPE, "attn_prep: bad row strides");
-    if (!type_ok(c->type) || !c->k || c->D != D || c->Hkv != Hkv || D % 128 || D > 1024 || n_rot > D || n_rot % 2 ||
+    if (!type_ok(c->type) || !c->k || c->D != D || c->Hkv != Hkv || D % 128 || D > 1024 || n_rot > D || n_rot < 0 || n_rot % 2 ||
         !aligned16(qg) || !aligned16(k) || !aligned16(q) || !aligned16(gate) || (q_norm && !aligned16(q_norm)) ||
         (k_norm && !aligned16(k_norm)) || (p0 >= 0 && !c->pt && p0 + T > c->n_ctx))
         B200_REFUSE(B200_ERR_SHAPE, "attn_prep: unsupported shape / cache / alignment (D=%d Hkv=%d n_rot=%d)", D, Hkv, n_rot);
@@ -670,7 +672,7 @@ int b200_attn_prep_rows(const float * qg, const float * k, const float * v, cons
                         int T, int Hq, int Hkv, int D, int n_rot, float freq_base, float eps, void * stream) {
     if (T <= 0) return B200_OK;
     if (!c || !k || !v || !rope_pos || !cache_row || (qg && (!q || !gate))) B200_REFUSE(B200_ERR_SHAPE, "attn_prep_rows: null argument");
-    if (!type_ok(c->type) || !c->k || c->D != D || c->Hkv != Hkv || D % 128 || D > 1024 || n_rot > D || n_rot % 2 ||
+    if (!type_ok(c->type) || !c->k || c->D != D || c->Hkv != Hkv || D % 128 || D > 1024 || n_rot > D || n_rot < 0 || n_rot % 2 ||
         !aligned16(qg) || !aligned16(k) || !aligned16(q) || !aligned16(gate) || (q_norm && !aligned16(q_norm)) ||
         (k_norm && !aligned16(k_norm)))
         B200_REFUSE(B200_ERR_SHAPE, "attn_prep_rows: unsupported shape / cache / alignment (D=%d Hkv=%d n_rot=%d)", D, Hkv, n_rot);

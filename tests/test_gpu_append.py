@@ -262,3 +262,33 @@ def test_rope_append_bf16_special_blocks(cuda, lib, tname, T):
     assert fast.device_status() == 0
     for a, b in zip(*outs):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("tname", ["q8_0", "q4_0", "f16"])
+@pytest.mark.parametrize("dim,n_rot", [(256, 62), (256, 66), (256, 2), (256, 0), (512, 62), (512, 66), (128, 126)])
+def test_attn_prep_rotary_widths(cuda, lib, tname, dim, n_rot):
+    """rotary widths that are no multiple of four floats, in front of the staged heads in shared memory; against the CPU restatement with the
+    bounds of the 64-wide case"""
+    import torch
+    from p100e_engine_b200 import fast
+    kt, T, p0, base, eps, hq, hkv = TYPES[tname], 3, 100, 1e7, 1e-6, 6, 2
+    qg, k, v = util.rng_normal(1, (T, hq, 2 * dim)), util.rng_normal(2, (T, hkv, dim)), util.rng_normal(3, (T, hkv, dim))
+    qn, kn = (util.rng_normal(4 + i, (dim,)) * 0.1 + 1.0 for i in range(2))
+    pos = np.arange(p0, p0 + T, dtype=np.int32)
+    oc = orc.Cache.contiguous(kt, 256, hkv, dim)
+    q_o, gate_o = orc.attn_prep(qg, k, v, qn, kn, pos, oc, p0, T, hq, hkv, dim, n_rot, base, eps)
+    dev = [util.to_dev(x, cuda) for x in (qg, k, v, qn, kn, pos)]
+    for rows in (False, True):
+        c = fast.kv_alloc(kt, 256, hkv, dim)
+        q, gate = torch.zeros(T, hq, dim, device=cuda), torch.zeros(T, hq * dim, device=cuda)
+        if rows:
+            assert fast.attn_prep_rows(*dev[:5], dev[5], dev[5], q, gate, c, T, hq, hkv, dim, n_rot, base, eps)
+        else:
+            assert fast.attn_prep(*dev, q, gate, c, p0, T, hq, hkv, dim, n_rot, base, eps)
+        torch.cuda.synchronize()
+        assert np.array_equal(gate.cpu().numpy(), gate_o)
+        np.testing.assert_allclose(q.cpu().numpy(), q_o, rtol=1e-5, atol=2e-4 + 1.2e-7 * (p0 + T))
+        assert np.array_equal(c.v.cpu().numpy(), oc.v)
+        assert (c.k.cpu().numpy() != oc.k).mean() < 1e-2
+    assert not fast.attn_prep(*dev, q, gate, c, p0, T, hq, hkv, dim, -2, base, eps)
+    assert fast.device_status() == 0
