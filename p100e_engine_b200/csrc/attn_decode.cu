@@ -817,7 +817,7 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
 // Merge a row's chunk partials.  grid (rows, Hq), P groups of 64 threads (one float4 of the head each).  P > 1: chunk c belongs to
 // summation stream c mod MERGE_STREAMS, group w walks the streams w, w + P, .. (each in ascending order, its own accumulator),
 // and the streams are added in stream order: an order that depends on the number of chunks only, not on P nor on the rest of
-// the call.  P = 1: ascending order, for fixed chunks with the roundings of one chunk per stream (at most MERGE_STREAMS chunks).
+// the call.  P = 1: ascending order, for fixed chunks (CHUNKED) with the roundings of one chunk per stream (at most MERGE_STREAMS chunks).
 //   out != nullptr : out = num / den (* sigmoid(gate)); rows that saw no key give zeros
 //   fo  != nullptr : unnormalised num, max in natural-log units, den (for a cross-GPU merge)
 // The kernel is a chain of dependent loads (positions, maxima, partials), so what counts is how many partials are in flight:
@@ -838,7 +838,7 @@ __global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const
     // partials of the row's kv head: consecutive units of stride ustr from unit0 (a segment the row does not reach holds m = -inf)
     int nch;
     size_t unit0, ustr;
-    if constexpr (!CHUNKED) {
+    if (P == 1 ? !CHUNKED : !a.chunked) {   // (known at compile time, <16> keeps 39 registers and fewer loads in flight: 7.6 us for 6.6)
         const int2 sg = a.slot_seg[slot];
         nch = pos < 0 ? 0 : sg.y;
         unit0 = (size_t) sg.x * a.nhk + hl; ustr = a.nhk;
@@ -1254,7 +1254,8 @@ struct plan_key {
                part_floats == o.part_floats;
     }
 };
-constexpr int SCR_PLAN_INTS = 6 * PLAN_MAX_SLOTS + 5 * SPLIT_MAX_CTA + 4;   // the longest plan (run_list_ints)
+// the longest plan (run_list_ints), in whole 256-byte units
+constexpr int SCR_PLAN_INTS = (6 * PLAN_MAX_SLOTS + 5 * SPLIT_MAX_CTA + 4 + 63) / 64 * 64;
 struct scratch {
     int dev = -1; cudaStream_t s = nullptr; float * p = nullptr; size_t cap = 0;
     bool step_mode = false, plan_valid = false;
@@ -1494,7 +1495,7 @@ int auto_chunk(long long total_keys, int Hkv) {
 // against 2.96e-4.
 //   the plan holds `segs` segments, the runs' or (listed) every chunk
 size_t run_list_ints(size_t segs, int max_cta, int n_slots) { return (4 * segs + 2 * (size_t) n_slots + max_cta + 2 + 3) & ~(size_t) 3; }
-static_assert(SCR_PLAN_INTS % 4 == 0 && SCR_PLAN_INTS >= 4 * (SPLIT_MAX_CTA + PLAN_MAX_SLOTS) + 2 * PLAN_MAX_SLOTS + SPLIT_MAX_CTA + 2 &&
+static_assert(SCR_PLAN_INTS >= 4 * (SPLIT_MAX_CTA + PLAN_MAX_SLOTS) + 2 * PLAN_MAX_SLOTS + SPLIT_MAX_CTA + 2 &&
               SCR_PLAN_INTS >= 4 * LIST_MAX + 2 * LIST_SLOTS + SPLIT_MAX_CTA + 4, "a plan fits its place");
 // the recording the stream takes part in, 0 if none; false = unknown
 bool recording_of(cudaStream_t s, unsigned long long & id) {
@@ -1603,8 +1604,7 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     const bool one = gm.split ? parts <= 8 : parts <= 4 || (parts <= MERGE_STREAMS && grid > 8LL * sms);
     const bool sixteen = parts > 32 && (grid <= 2LL * sms || (parts > 128 && grid <= 8LL * sms));
     const unsigned threads = one ? 64 : sixteen ? 1024 : 256;
-    auto * merge = gm.split ? (one ? decode_merge_k<1, false> : sixteen ? decode_merge_k<16, false> : decode_merge_k<4, false>)
-                            : (one ? decode_merge_k<1, true> : sixteen ? decode_merge_k<16, true> : decode_merge_k<4, true>);
+    auto * merge = sixteen ? decode_merge_k<16, false> : !one ? decode_merge_k<4, false> : gm.split ? decode_merge_k<1, false> : decode_merge_k<1, true>;
     launch(merge, mg, threads, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
     count_launch(launches);
     return launch_status(who);

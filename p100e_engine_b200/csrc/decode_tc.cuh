@@ -77,7 +77,6 @@ template <int NC>
 __global__ void __launch_bounds__(TC_THR, 1)
 decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV) {
     pdl_enter();
-    pdl_enter();
     extern __shared__ __align__(1024) unsigned char smem[];
     constexpr int HB = TC_HB, BUF = UT * HB;
     const int tid = threadIdx.x, lane = tid & 31;
