@@ -186,7 +186,7 @@ int b200_attn_reserve(uint32_t kv_type, int max_slots, int q_len, int max_n, int
  * chunk_keys: keys per split (multiple of 64); 0 = b200_attn_fixed_chunk(n_ctx) (a function of the cache's capacity); -1 = an even
  * split of the whole batch: the batch's 64-key tiles, slot after slot, are cut into one contiguous run per resident CTA, so
  * ragged contexts load every SM equally (up to 2048 slots; larger batches take a chunk chosen from the batch size).
- * A single slot with -1 takes the chunks of attn_decode (same bits, K integer times fp32 scale).
+ * A single slot with -1 is cut into chunks chosen from max_n and the kv heads, without a plan (K integer times fp32 scale).
  * With chunk_keys >= 0 each row's result depends only on its own keys and on the chunk, never on the other rows of the call
  * (bitwise); with -1 the split points depend on the batch, so results of different batches agree to rounding only. */
 int b200_attn_decode_slots(const float *q, const b200_kv_cache *c, float *out, const float *gate, int n_slots,

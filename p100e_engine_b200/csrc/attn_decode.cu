@@ -1216,7 +1216,7 @@ int fixed_chunk(int n_ctx) {
     const int pinned = pinned_chunk(n_ctx);
     return pinned ? pinned : std::max(default_chunk(), round_tile(((long long) std::max(n_ctx, 1) + MAX_DEFAULT_CHUNKS - 1) / MAX_DEFAULT_CHUNKS));
 }
-// Row entry points (attn_decode and its kin, at most 8 rows) and one slot with chunk_keys = -1: the position grid, whose longest chunk is
+// Row entry points (attn_decode and its kin, at most 8 rows): the position grid, whose longest chunk is
 // 512 keys up to a capacity of 229376 and n_ctx / 448 rounded up to a power of two beyond.  One row, 4 heads, chunks of up to 512 / 1024 keys: q4_0 at
 // 65664 of 131328 keys 44.7 / 54.5 us, q8_0 48.6 / 61.1 (the longest CTA walks 8 or 16 tiles); q4_0 at 262141 of 262144 125.9 / 115.1, at half of it
 // 70.2 / 76.2.
@@ -1485,14 +1485,23 @@ int auto_chunk(long long total_keys, int Hkv) {
     return c;
 }
 
+// One slot: the position grid up to auto_chunk's chunk, which short contexts need to fill the chip; a long one in equal chunks.  4 rows of
+// 2 heads, q8_0, 30011 keys: 29.9 us, with the row entry points' grid (chunks of up to 512 keys) 36.5; 131000 keys 66.9 and 62.1.
+int single_grid(int max_n, int Hkv) {
+    const int c = auto_chunk(max_n / 2, Hkv);
+    int k = 0;
+    while (TILE << k < c) ++k;
+    return max_n > 65536 ? c : -k;
+}
+
 // geometry of a call: chunk, chunks per slot, partial floats, work-list ints
 //   split   (chunk chosen from the batch, two to SPLIT_MAX_SLOTS slots): one contiguous run of tiles per resident CTA
 //   planned (fixed chunks of several slots, more units than a wave): the same runs, cut at chunk boundaries
 //   else    see decode_part_k
-// rows: a call of the row entry points (chunk_keys = 0: the position grid).  One slot with chunk_keys < 0 takes the position grid: K stays integer times fp32 scale (decode_tc_k rounds q * d to f16) and short
-// chunks have reference maxima of their own.  Error against 64-bit attention over the stored rows, q8_0, 1 / 2 / 4 rows at 30011 keys:
-// 3.6e-4 / 3.6e-4 / 3.5e-4; on decode_tc_k 2 / 4 rows 4.2e-4 / 4.2e-4; one run per CTA of an f16 cache, 4 rows at 131000 keys 3.00e-4
-// against 2.96e-4.
+// rows: a call of the row entry points (chunk_keys = 0: the position grid).
+// One slot with chunk_keys < 0 (single_grid) stays on decode_part_k, which keeps K integer times fp32 scale (decode_tc_k rounds q * d to f16), in
+// chunks that are nowhere longer than auto_chunk's: their error is that of their reference maxima.  Against 64-bit attention over the stored rows,
+// q8_0, 4 rows at 30011 keys: 3.5e-4, on decode_tc_k 4.2e-4.
 //   the plan holds `segs` segments, the runs' or (listed) every chunk
 size_t run_list_ints(size_t segs, int max_cta, int n_slots) { return (4 * segs + 2 * (size_t) n_slots + max_cta + 2 + 3) & ~(size_t) 3; }
 static_assert(SCR_PLAN_INTS >= 4 * (SPLIT_MAX_CTA + PLAN_MAX_SLOTS) + 2 * PLAN_MAX_SLOTS + SPLIT_MAX_CTA + 2 &&
@@ -1525,7 +1534,7 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
         return true;
     }
     g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 && n_slots > 1 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) :
-           rows || chunk_keys < 0 ? position_grid(n_ctx) : fixed_chunk(n_ctx);
+           chunk_keys < 0 ? single_grid(max_n, Hkv) : rows ? position_grid(n_ctx) : fixed_chunk(n_ctx);
     g.max_chunks = chunk_of(g.CH, max_n - 1) + 1;
     g.units = (size_t) n_slots * Hkv * g.max_chunks;
     if (g.units >= ((size_t) 1 << 31) || (size_t) n_slots * g.max_chunks >= ((size_t) 1 << 30)) return false;
@@ -1774,9 +1783,16 @@ int b200_attn_reserve(uint32_t kv_type, int max_slots, int q_len, int max_n, int
     dec_geom gm;
     if (!decode_geometry(gm, kv_type, max_slots, q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, chunk_keys)) B200_REFUSE(B200_ERR_SHAPE, "attn_reserve: too many chunks");
     size_t need = gm.part_floats;
-    dec_geom g1;   // the position grid (row entry points; one slot with -1) may take more partials than a small batch of equal chunks or runs
+    dec_geom g1;   // the position grid of the row entry points, and one slot with -1, may take more partials than a small batch of equal chunks or runs
     if (chunk_keys <= 0 && decode_geometry(g1, kv_type, std::min(max_slots, B200_ATTN_MAX_ROWS), q_len, max_n, n_ctx > 0 ? n_ctx : max_n, Hkv, 0, false, true))
         need = std::max(need, g1.part_floats);
+    // one slot of any length up to max_n: most chunks where its chunk is about to double, and at the end of single_grid's fine chunks
+    for (long long c = 256; chunk_keys < 0 && c <= 4096; c *= 2)
+        for (const long long cap : {(long long) max_n, std::min(65536LL, (long long) max_n)}) {
+            const int n1 = (int) std::max(1LL, std::min(cap, (c + 1) * 16 * sm_count() / Hkv));
+            if (decode_geometry(g1, kv_type, 1, q_len, n1, n1, Hkv, -1)) need = std::max(need, g1.part_floats);
+        }
+    if (chunk_keys < 0 && max_slots == 1 && decode_geometry(g1, kv_type, 1, q_len, max_n, max_n, Hkv, -1)) need = std::max(need, g1.part_floats);
     if (chunk_keys < 0 && max_slots > 1 && !gm.split) {
         // a fixed chunk chosen from the batch: smaller batches take smaller chunks; their unit count stays under this bound
         const size_t u = 2 * 8 * (size_t) sm_count() + (size_t) max_slots * Hkv;

@@ -143,8 +143,9 @@ def test_reservation_covers_the_position_grid(cuda, lib, chunk):
     a, b = torch.zeros_like(q), torch.zeros_like(q)
     assert fast.attn_decode_rows(q, c, torch.zeros_like(q), 8, pos, 6 * hkv, SCALE)          # kernels loaded
     assert fast.attn_decode_slots(q, c, torch.zeros_like(q), None, 1, 4, pos, n, 6 * hkv, SCALE, -1)
-    want = torch.zeros_like(q)
+    want, want1 = torch.zeros_like(q), torch.zeros_like(q)
     assert fast.attn_decode_rows(q, c, want, 8, pos, 6 * hkv, SCALE)
+    assert fast.attn_decode_slots(q, c, want1, None, 1, 4, pos, n, 6 * hkv, SCALE, -1)
     side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
     torch.cuda.synchronize()
     assert fast.attn_reserve(TYPES["q8_0"], 8, 4, n, n, hkv, chunk, s=side)
@@ -153,7 +154,7 @@ def test_reservation_covers_the_position_grid(cuda, lib, chunk):
         assert fast.attn_decode_slots(q, c, b, None, 1, 4, pos, n, 6 * hkv, SCALE, -1)
     graph.replay()
     torch.cuda.synchronize()
-    assert torch.equal(a, want) and torch.equal(b[:4], want[:4])
+    assert torch.equal(a, want) and torch.equal(b[:4], want1[:4])
 
 
 @pytest.mark.parametrize("n_slots,chunks", [(2, 4), (2, 5), (60, 16), (200, 16), (60, 17), (20, 40), (60, 40), (60, 150), (200, 150)])
