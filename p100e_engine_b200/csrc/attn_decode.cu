@@ -5,8 +5,8 @@
 //   staging   the K rows and the V rows of a tile (one kv head, 64 positions) are each fetched by ONE tiled TMA copy through a
 //             tensor map of the cache (x = row bytes, y = position in page, z = page) into a ring of half-tile slots,
 //             completion counted on mbarriers; rows keep their cache format in shared memory.  The warp that is last to
-//             finish with a slot issues its refill.  f16 rows go through a rank-4 map with the 128-byte swizzle.  Ragged
-//             last tiles and pages under 64 rows are staged row by row through registers instead.
+//             finish with a slot issues its refill.  f16 rows go through a rank-4 map with the 128-byte swizzle.  What a
+//             ragged last tile holds past the last key is masked; pages under 64 rows are staged row by row through registers instead.
 //   QK^T      warp w owns keys 16w..16w+15 of the tile: keys on the MMA M axis, the slot's 6 * q_len query rows on N
 //             (all GQA heads and verify rows share one pass over the KV bytes).  int8 / nibbles are widened to f16
 //             exactly in registers (byte permute + one f16x2 subtract), products accumulate in fp32 on the tensor
@@ -20,7 +20,7 @@
 // The chunk grid is fixed by absolute key index, and a chunk's arithmetic never depends on the other rows of the call:
 // a row's result is a function of its own keys and of chunk_keys only (row t of a T-row call == the 1-row call).
 //
-// Batched calls that let the library choose the split (chunk_keys < 0) cut the batch evenly over the CTAs that fit the GPU
+// Batched calls of several slots that let the library choose the split (chunk_keys < 0) cut the batch evenly over the CTAs that fit the GPU
 // (decode_split_k; one plan per model step when the caller declares the step, b200_attn_step_begin).  There q8_0 caches
 // with two to four rows per slot run on a second kernel, decode_tc_k (decode_tc.cuh): tcgen05 MMAs with K in tensor
 // memory and V as an f16 image in shared memory, one CTA per SM.  Everything else, and every fixed-chunk call, runs on
@@ -736,7 +736,7 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
 #include "decode_tc.cuh"
 
 // The kernel.  With a run plan: every segment of the CTA's run one after the other.  Fixed chunks without a plan (one slot;
-// few units; more slots than a plan holds): units u = index, + CTAs of the kv head, .., one chunk each, the highest chunk
+// no more chunks than CTAs; more slots than a plan holds): units u = index, + CTAs of the kv head, .., one chunk each, the highest chunk
 // index first, so that the long chunks start first and the short ones fill the tail.  (One long context as contiguous runs,
 // cut at chunk boundaries like the plans: 401 us against 364 for four layers of 131000 keys, because a CTA got either 8 or 16
 // tiles.)
@@ -1246,11 +1246,11 @@ struct plan_key {
 
     const void * scr = nullptr, * pos = nullptr, * p0p = nullptr;
     int p0 = 0, n_slots = 0, q_len = 0, CH = 0, max_chunks = 0, max_cta = 0, Hkv = 0, n_ctx = 0, paged = 0;
-    int split = 0, tc = 0;   // an even split has slot_seg, a plan of fixed chunks has not; they can agree in all the rest
+    int list_cap = 0, split = 0, tc = 0;   // an even split has slot_seg, a plan of fixed chunks has not; they can agree in all the rest
     size_t part_floats = 0;
     bool operator==(const plan_key & o) const {
         return rec == o.rec && scr == o.scr && pos == o.pos && p0p == o.p0p && p0 == o.p0 && n_slots == o.n_slots && q_len == o.q_len && CH == o.CH &&
-               max_chunks == o.max_chunks && max_cta == o.max_cta && Hkv == o.Hkv && n_ctx == o.n_ctx && paged == o.paged && split == o.split && tc == o.tc &&
+               max_chunks == o.max_chunks && max_cta == o.max_cta && Hkv == o.Hkv && n_ctx == o.n_ctx && paged == o.paged && list_cap == o.list_cap && split == o.split && tc == o.tc &&
                part_floats == o.part_floats;
     }
 };
@@ -1639,7 +1639,7 @@ int decode_impl(const float * q, const b200_kv_cache * c, const merge_out & mo, 
     plan_key k;
     k.scr = scr; k.pos = pos; k.p0p = p0p; k.p0 = p0; k.n_slots = n_slots; k.q_len = q_len; k.CH = gm.CH; k.max_chunks = gm.max_chunks;
     k.max_cta = gm.max_cta; k.Hkv = c->Hkv; k.n_ctx = c->n_ctx; k.paged = c->pt != nullptr; k.part_floats = gm.part_floats;
-    k.split = gm.split; k.tc = gm.tc;
+    k.list_cap = gm.list_cap; k.split = gm.split; k.tc = gm.tc;
     const bool in_step = e->step_mode && pos && (const char *) pos >= e->step_lo && (const char *) pos < e->step_hi;
     const bool listed = gm.split || gm.planned;
     const bool known = !listed || recording_of(s, k.rec);
