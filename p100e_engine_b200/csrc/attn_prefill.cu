@@ -759,11 +759,11 @@ void pieces_release(own_scratch * e, cudaStream_t s, unsigned long long user) {
 
 // CTAs of the even split for rows p0 .. p0 + T - 1 (n_mtiles row tiles per kv head); 0 = one row tile per CTA.  Row tiles that are fewer than
 // the SMs leave SMs idle for as long as the longest tile takes: they are cut, into at least two steps per CTA, if that is shorter by the
-// time model below, in tenths of a microsecond, fitted to 396 shapes (T 5 .. 3000 behind 0 .. 65000 keys, q8_0, 1 / 2 / 4 heads) timed both ways in
-// turn: a step 1.4 us, each further row tile in a CTA's run 15 us (prologue and epilogue), pieces and their merge 8 us.  Measured, us, one row tile
-// per CTA / cut: 4 heads, T = 48 behind 40000 keys 586 / 124, T = 512 behind 20000 323 / 256; but T = 512 behind nothing 28 / 49, 2 heads, T = 1500
-// behind nothing 39 / 112 (the first runs cross six tiles of one step): those are left whole.  The choice is within 3 % of the better one on all
-// but six of the shapes, 10 % off at worst.
+// time model below, in tenths of a microsecond, fitted to 1457 calls (T 5 .. 3000 behind 0 .. 65000 keys, q8_0 and q4_0, 1 / 2 / 4 heads, f32 and bf16
+// forms) timed both ways in turn: a step 1.3 us, each further row tile in a CTA's run 8 us (prologue and epilogue), pieces and their merge 1 us and
+// 0.06 us a CTA.  Measured, us, one row tile per CTA / cut: 4 heads, T = 48 behind 40000 keys 586 / 124, T = 512 behind 20000 323 / 256, T = 16
+// behind 700 (bf16) 38 / 28; but T = 512 behind nothing 28 / 49, 2 heads, T = 1500 behind nothing 39 / 112 (the first runs cross six tiles of one
+// step): those are left whole.  The choice is within 5 % of the better one on all but 31 of the calls, 13 % off at worst.
 int split_ctas(int T, int p0, int n_mtiles, int Hkv, int sms, size_t image_bytes, int * head_steps) {
     const long long tiles = (long long) n_mtiles * Hkv;
     if (tiles >= sms) return 0;
@@ -793,8 +793,8 @@ int split_ctas(int T, int p0, int n_mtiles, int Hkv, int sms, size_t image_bytes
     }
     // images beyond L2 with the tiles at different keys: every step is read from HBM, 128 KB at 6.5 TB/s (512 rows behind 65000 keys, 4 heads:
     // 948 / 977 us)
-    const long long steps_us10 = std::max(14 * run, image_bytes > ((size_t) 144 << 20) && !aligned ? W / 5 : 0);
-    return 100 * run <= 88 * longest && 14 * longest > steps_us10 + 150 * (segs - 1) + 80 ? (int) n : 0;
+    const long long steps_us10 = std::max(13 * run, image_bytes > ((size_t) 144 << 20) && !aligned ? W / 5 : 0);
+    return 100 * run <= 86 * longest && 13 * longest > steps_us10 + 80 * (segs - 1) + 10 + 6 * n / 10 ? (int) n : 0;
 }
 
 struct pf_io {
