@@ -548,7 +548,7 @@ class Workload:
         """per-layer device times of the step's parts from CUDA events on this rank (eager launches, the slots in one batch, no
         overlap between parts), and the host's time to issue a layer"""
         torch, fast = self.torch, self.fast
-        names = ["attn_prep", "split plan / work list + attention kernel + merge of the partials"]
+        names = ["attn_prep", "split plan + attention kernel + merge of the partials"]
         if self.merge is not None:
             import torch.distributed as dist
             from p100e_engine_b200 import dist as Dm
@@ -730,7 +730,7 @@ def run_b200(args):
                  "clocks": clocks, "gpu_launches": int(launches), "out_fingerprint": fingerprint,
                  "e2e": {"value": total_bytes / (e2e_ms * 1e-3) / 1e9, "unit": "GB/s", "ms_per_step": e2e_ms,
                          "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
-                 "roofline": {"bound": "hbm", "kernel": kname + " (+ split plan / work list, merge of the partials) per layer call", "achieved": achieved,
+                 "roofline": {"bound": "hbm", "kernel": kname + " (+ split plan, merge of the partials) per layer call", "achieved": achieved,
                               "peak": peak, "peak_source": "measured" if peaks else "fallback", "unit": "GB/s",
                               "frac": achieved / peak,
                               "traffic": int(tr["dram_bytes_per_kv_byte"] * wl.kv_bytes_layer) if tr else None,

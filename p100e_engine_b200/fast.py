@@ -131,7 +131,7 @@ def seq_exchange_merge_a16(nccl_comm, n_seq, send, recv, R, D, gate, out, qbuf, 
 
 def attn_step_begin(positions, nbytes=None, s=None):
     """the device array `positions` stays as it is until the next call: batched calls on the stream whose pos argument lies
-    inside it reuse the even split within the step"""
+    inside it share one run plan within the step, in one recording or outside of any"""
     if nbytes is None:
         nbytes = positions.numel() * positions.element_size()
     return L.load().b200_attn_step_begin(_stream(s), L.ptr(positions), nbytes) == L.OK
