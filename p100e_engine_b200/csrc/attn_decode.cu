@@ -814,31 +814,51 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
     }
 }
 
-// Merge a row's chunk partials.  grid (rows, Hq), P groups of 64 threads (one float4 of the head each).  P > 1: chunk c belongs to
-// summation stream c mod MERGE_STREAMS, group w walks the streams w, w + P, .. (each in ascending order, its own accumulator),
-// and the streams are added in stream order: an order that depends on the number of chunks only, not on P nor on the rest of
-// the call.  P = 1: ascending order, for fixed chunks (CHUNKED) with the roundings of one chunk per stream (at most MERGE_STREAMS chunks).
+// Merge a row's chunk partials.  Chunk c belongs to summation stream c mod MERGE_STREAMS; a stream is summed in ascending order in an
+// accumulator of its own and the streams are added in stream order: an order that depends on the number of chunks only, not on the
+// rest of the call.
 //   out != nullptr : out = num / den (* sigmoid(gate)); rows that saw no key give zeros
 //   fo  != nullptr : unnormalised num, max in natural-log units, den (for a cross-GPU merge)
-// The kernel is a chain of dependent loads (positions, maxima, partials), so what counts is how many partials are in flight:
-// decode_launch picks P from the number of partials a row can have and the size of the grid.
+// What both kernels below do once a row's partials are summed: lanes hold four dims each, oi = float4 index of the result.
+__device__ __forceinline__ void merge_finish(const dec_args & a, float4 num, float den, float M, size_t oi, size_t row, int h, bool live, bool first, float4 gv,
+                                             const float * gate, float * out, float * fo, float * fm, float * fl, __half2 * qbuf, size_t rows) {
+    if (fo && live) {   // public partials are plain sums: take the internal 2^PSHIFT out (exact)
+        constexpr float U = 1.0f / 256.0f;
+        static_assert(PSHIFT == 8.0f, "U must be 2^-PSHIFT");
+        reinterpret_cast<float4 *>(fo)[oi] = make_float4(num.x * U, num.y * U, num.z * U, num.w * U);
+        if (first) { fm[row * a.Hq + h] = M * LN2; fl[row * a.Hq + h] = den * U; }
+    }
+    if (out) {
+        float4 y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (den > 0.0f) {
+            const float inv = 1.0f / den;
+            y = make_float4(num.x * inv, num.y * inv, num.z * inv, num.w * inv);
+            if (gate) {
+                y.x *= 1.0f / (1.0f + expf(-gv.x)); y.y *= 1.0f / (1.0f + expf(-gv.y));
+                y.z *= 1.0f / (1.0f + expf(-gv.z)); y.w *= 1.0f / (1.0f + expf(-gv.w));
+            }
+        }
+        if (live) reinterpret_cast<float4 *>(out)[oi] = y;
+        // the projection that follows attention reads its input in the a16 format: emitted here, from registers
+        if (qbuf) a16_store_lanes8(y, qbuf, oi >> 3, rows * (a.Hq * (DH / 32)), live);
+    }
+}
+
+// Few partials on a grid that fills the GPU: grid (rows, Hq), 64 threads of one float4 each, the partials one after the other.  CHUNKED: the
+// roundings of one chunk per stream (at most MERGE_STREAMS chunks).
 constexpr int MERGE_STREAMS = 16;
-template <int P, bool CHUNKED>
-__global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const float * __restrict__ gate, float * __restrict__ out,
-                                                         float * __restrict__ fo, float * __restrict__ fm, float * __restrict__ fl,
-                                                         __half2 * __restrict__ qbuf) {
+template <bool CHUNKED>
+__global__ void __launch_bounds__(64) decode_merge_k(const dec_args a, const float * __restrict__ gate, float * __restrict__ out, float * __restrict__ fo,
+                                                     float * __restrict__ fm, float * __restrict__ fl, __half2 * __restrict__ qbuf) {
     pdl_enter();
-    constexpr int SPG = P > 1 ? MERGE_STREAMS / P : 1;   // streams per group
-    __shared__ float4 snum[P > 1 ? MERGE_STREAMS : 1][64];
-    __shared__ float sden[P > 1 ? MERGE_STREAMS : 1], smax[2 * P];
-    const int tid = threadIdx.x, lane4 = tid & 63, grp = tid >> 6;
+    const int lane4 = threadIdx.x;
     const int row = blockIdx.x, slot = row / a.q_len, j = row - slot * a.q_len;
     const int hl = blockIdx.y / GQA, hh = blockIdx.y - hl * GQA, h = a.hk0 * GQA + blockIdx.y, r = j * GQA + hh, R = a.q_len * GQA;
     const int pos = min(row_pos(a, slot, j), key_limit(a) - 1);   // a row past the limit merges the chunks that exist
     // partials of the row's kv head: consecutive units of stride ustr from unit0 (a segment the row does not reach holds m = -inf)
     int nch;
     size_t unit0, ustr;
-    if (P == 1 ? !CHUNKED : !a.chunked) {   // (known at compile time, <16> keeps 39 registers and fewer loads in flight: 7.6 us for 6.6)
+    if constexpr (!CHUNKED) {
         const int2 sg = a.slot_seg[slot];
         nch = pos < 0 ? 0 : sg.y;
         unit0 = (size_t) sg.x * a.nhk + hl; ustr = a.nhk;
@@ -850,81 +870,114 @@ __global__ void __launch_bounds__(64 * P) decode_merge_k(const dec_args a, const
     const float4 * po = reinterpret_cast<const float4 *>(a.po + (unit0 * R + r) * DH) + lane4;
     const size_t st = ustr * R;   // from one partial of the row to the next, in values (pm, pl) and head rows (po)
     float M = B200_NEG_INF;
-    if constexpr (P > 1) {
-        for (int c = tid; c < nch; c += 64 * P) M = fmaxf(M, pm[c * st]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-        if ((tid & 31) == 0) smax[tid >> 5] = M;
-        __syncthreads();
-        M = smax[0];
-#pragma unroll
-        for (int i = 1; i < 2 * P; ++i) M = fmaxf(M, smax[i]);
-    } else {
-        for (int c = 0; c < nch; ++c) M = fmaxf(M, pm[c * st]);
-    }
+    for (int c = 0; c < nch; ++c) M = fmaxf(M, pm[c * st]);
     float den = 0.0f;
     float4 num = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    auto add = [&](int c, float4 & n, float & d) {   // no early continue: the loads of several chunks are in flight together
-        const float ms = pm[c * st];
-        const float f = ms == B200_NEG_INF ? 0.0f : ex2f(ms - M);   // a chunk the row did not see holds zeros: adds nothing
-        d = fmaf(f, pl[c * st], d);
+#pragma unroll 4
+    for (int c = 0; c < nch; ++c) {   // no early continue: the loads of several chunks are in flight together
+        const float ms = pm[c * st], lc = pl[c * st];
         const float4 o = po[c * st * (DH / 4)];
-        n.x = fmaf(f, o.x, n.x); n.y = fmaf(f, o.y, n.y); n.z = fmaf(f, o.z, n.z); n.w = fmaf(f, o.w, n.w);
-    };
-    if constexpr (P == 1) {
-#pragma unroll 4
-        for (int c = 0; c < nch; ++c) {
-            if constexpr (CHUNKED) {
-                float d = 0.0f;
-                float4 n = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                add(c, n, d);
-                num.x += n.x; num.y += n.y; num.z += n.z; num.w += n.w;
-                den += d;
-            } else add(c, num, den);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < SPG; ++i) {
-            const int s = grp + P * i;
-            float d = 0.0f;
-            float4 n = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 4
-            for (int c = s; c < nch; c += MERGE_STREAMS) add(c, n, d);
-            snum[s][lane4] = n;
-            if (lane4 == 0) sden[s] = d;
-        }
-        __syncthreads();
-        if (grp > 0) return;
-        const int ns = min(nch, MERGE_STREAMS);   // the other streams are empty
-        for (int s = 0; s < ns; ++s) {
-            const float4 o = snum[s][lane4];
-            num.x += o.x; num.y += o.y; num.z += o.z; num.w += o.w;
-            den += sden[s];
+        const float f = ms == B200_NEG_INF ? 0.0f : ex2f(ms - M);   // a chunk the row did not see holds zeros: adds nothing
+        if constexpr (CHUNKED) {
+            den += __fmul_rn(f, lc);
+            num.x += __fmul_rn(f, o.x); num.y += __fmul_rn(f, o.y); num.z += __fmul_rn(f, o.z); num.w += __fmul_rn(f, o.w);
+        } else {
+            den = fmaf(f, lc, den);
+            num.x = fmaf(f, o.x, num.x); num.y = fmaf(f, o.y, num.y); num.z = fmaf(f, o.z, num.z); num.w = fmaf(f, o.w, num.w);
         }
     }
     const size_t oi = ((size_t) row * a.Hq + h) * (DH / 4) + lane4;
-    if (fo) {   // public partials are plain sums: take the internal 2^PSHIFT out (exact)
-        constexpr float U = 1.0f / 256.0f;
-        static_assert(PSHIFT == 8.0f, "U must be 2^-PSHIFT");
-        reinterpret_cast<float4 *>(fo)[oi] = make_float4(num.x * U, num.y * U, num.z * U, num.w * U);
-        if (lane4 == 0) { fm[(size_t) row * a.Hq + h] = M * LN2; fl[(size_t) row * a.Hq + h] = den * U; }
+    const float4 gv = gate ? reinterpret_cast<const float4 *>(gate)[oi] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    merge_finish(a, num, den, M, oi, row, h, true, lane4 == 0, gv, gate, out, fo, fm, fl, qbuf, gridDim.x);
+}
+
+// Everything else: grid (rows, Hq, 256 / 64), a thread per (stream, four dims) of a 64-dim slice.  Bound by a chain of dependent loads
+// (position, number of partials, maxima, partials) with nothing else to hide it, so all loads that can go out do so at once: the gate, the
+// position and the first AHEAD partials of every stream, which lie inside the scratch whether the row has them or not and are left out
+// once the position is known.  Against CTAs of up to 1024 threads per (row, head) that loaded one after the other (64 registers: one such CTA
+// on an SM): 16 layers of one row at 4096 keys 311 -> 283 us, four layers of one row at 131000 keys (q4_0) 321 -> 305, 16 layers of 1 + 3 rows at
+// 30011 keys 609 -> 592, four layers of 8 rows of up to 16384 keys 337 -> 330.
+constexpr int MERGE_DL = 16, MERGE_THR = MERGE_STREAMS * MERGE_DL;
+template <int AHEAD>
+__global__ void __launch_bounds__(MERGE_THR, AHEAD > 4 ? 2 : 4) decode_merge_streams_k(const dec_args a, const float * __restrict__ gate, float * __restrict__ out,
+                                                                    float * __restrict__ fo, float * __restrict__ fm, float * __restrict__ fl,
+                                                                    __half2 * __restrict__ qbuf) {
+    pdl_enter();
+    __shared__ float4 snum[MERGE_STREAMS][MERGE_DL];
+    __shared__ float sden[MERGE_STREAMS], smax[MERGE_THR / 32];
+    const int tid = threadIdx.x, dl = tid & (MERGE_DL - 1), s = tid / MERGE_DL;
+    const int row = blockIdx.x, slot = row / a.q_len, j = row - slot * a.q_len;
+    const int hl = blockIdx.y / GQA, hh = blockIdx.y - hl * GQA, h = a.hk0 * GQA + blockIdx.y, r = j * GQA + hh, R = a.q_len * GQA;
+    const size_t oi = ((size_t) row * a.Hq + h) * (DH / 4) + blockIdx.z * MERGE_DL + dl;
+    float4 gv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (gate && s < 2) gv = reinterpret_cast<const float4 *>(gate)[oi];   // the first warp finishes the row
+    size_t unit0, ustr;
+    int most;   // partials that may be read
+    if (a.chunked) {
+        most = a.max_chunks;
+        unit0 = ((size_t) slot * a.nhk + hl) * a.max_chunks; ustr = 1;
+    } else {
+        const int2 sg = a.slot_seg[slot];
+        most = sg.y;
+        unit0 = (size_t) sg.x * a.nhk + hl; ustr = a.nhk;
     }
-    if (out) {
-        float4 y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (den > 0.0f) {
-            const float inv = 1.0f / den;
-            y = make_float4(num.x * inv, num.y * inv, num.z * inv, num.w * inv);
-            if (gate) {
-                const float4 gv = reinterpret_cast<const float4 *>(gate)[oi];
-                y.x *= 1.0f / (1.0f + expf(-gv.x)); y.y *= 1.0f / (1.0f + expf(-gv.y));
-                y.z *= 1.0f / (1.0f + expf(-gv.z)); y.w *= 1.0f / (1.0f + expf(-gv.w));
-            }
+    // the stream's next partial; from one partial of the row to the next, ustr * R values (pm, pl) and head rows (po)
+    const size_t i0 = (unit0 + s * ustr) * R + r, st = MERGE_STREAMS * ustr * R;
+    const float * pm = a.pm + i0;
+    const ptrdiff_t to_pl = a.pl - a.pm;
+    const float4 * po = reinterpret_cast<const float4 *>(a.po + i0 * DH) + blockIdx.z * MERGE_DL + dl;
+    float ms[AHEAD], ls[AHEAD];
+    float4 o[AHEAD];
+    auto fetch = [&](int c0, int n) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            ms[u] = B200_NEG_INF; ls[u] = 0.0f; o[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (c0 + u * MERGE_STREAMS < n) { ms[u] = *pm; ls[u] = pm[to_pl]; o[u] = *po; }
+            pm += st; po += st * (DH / 4);
         }
-        reinterpret_cast<float4 *>(out)[oi] = y;
-        // the projection that follows attention reads its input in the a16 format: emitted here, from registers
-        if (qbuf) a16_store_lanes8(y, qbuf, (size_t) row * (a.Hq * (DH / 32)) + h * (DH / 32) + (lane4 >> 3),
-                                   (size_t) gridDim.x * (a.Hq * (DH / 32)), true);
+    };
+    fetch(s, most);
+    const int pos = min(row_pos(a, slot, j), key_limit(a) - 1);   // a row past the limit merges the chunks that exist
+    const int nch = pos < 0 ? 0 : a.chunked ? chunk_of(a.CH, pos) + 1 : most;
+    float M = B200_NEG_INF;
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+        if (s + u * MERGE_STREAMS >= nch) { ms[u] = B200_NEG_INF; ls[u] = 0.0f; o[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+        M = fmaxf(M, ms[u]);
     }
+    for (int c = AHEAD * MERGE_STREAMS + tid; c < nch; c += MERGE_THR) M = fmaxf(M, a.pm[(unit0 + c * ustr) * R + r]);
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, k));
+    if ((tid & 31) == 0) smax[tid >> 5] = M;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < MERGE_THR / 32; ++i) M = fmaxf(M, smax[i]);
+    float d = 0.0f;
+    float4 n = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int c0 = s;;) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const float f = ms[u] == B200_NEG_INF ? 0.0f : ex2f(ms[u] - M);   // a chunk the row did not see holds zeros: adds nothing
+            d = fmaf(f, ls[u], d);
+            n.x = fmaf(f, o[u].x, n.x); n.y = fmaf(f, o[u].y, n.y); n.z = fmaf(f, o[u].z, n.z); n.w = fmaf(f, o[u].w, n.w);
+        }
+        c0 += AHEAD * MERGE_STREAMS;
+        if (c0 >= nch) break;
+        fetch(c0, nch);
+    }
+    snum[s][dl] = n;
+    if (dl == 0) sden[s] = d;
+    __syncthreads();
+    if (tid >= 32) return;   // both halves of the first warp add up the streams, the first one writes
+    float den = 0.0f;
+    float4 num = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int ns = min(nch, MERGE_STREAMS);   // the other streams are empty
+    for (int k = 0; k < ns; ++k) {
+        const float4 v = snum[k][dl];
+        num.x += v.x; num.y += v.y; num.z += v.z; num.w += v.w;
+        den += sden[k];
+    }
+    merge_finish(a, num, den, M, oi, row, h, tid < MERGE_DL, blockIdx.z == 0 && dl == 0, gv, gate, out, fo, fm, fl, qbuf, gridDim.x);
 }
 
 // Merge of caller-provided partials (cross-GPU sequence split): part s has O [R][D] at po + s * so, m (natural log) [R] at
@@ -1603,18 +1656,15 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     else if (c->type == B200_KV_Q8_0) rc = launch_part_nt<B200_KV_Q8_0>(a, blocks, s);
     else rc = launch_part_nt<B200_KV_Q4_0>(a, blocks, s);
     if (rc != B200_OK) return rc;
-    // Groups of 64 threads per (row, head), by the partials that a row of a typical slot has and by the grid.  Few partials: one group, as
-    // long as the grid would not fit the SMs at once with four (8 CTAs of 256 threads each); many partials on a grid of one wave (two CTAs of 1024
-    // threads per SM): sixteen.  Measured, us, with 1 / 4 / 16 groups: 8 partials on 24 CTAs 6.6 / 5.2 / 5.1, on 6144 17.3 / 36.2 / 127.5;
-    // 64 partials on 24 CTAs - / 11.5 / 6.2, on 1536 - / 33.7 / 46.1; 256 partials on 384 CTAs - / 34.1 / 26.8.
+    // Few partials (of a typical slot): one group of threads per (row, head), for fixed chunks on grids beyond eight CTAs per SM up to one
+    // chunk per stream.  Measured, us, with one group / 256 threads: 8 partials on 24 (row, head) pairs 6.6 / 5.2, on 6144 17.3 / 36.2.  Eight partials of a stream
+    // at once cost occupancy: 118 partials of 48 pairs (16 layers, 609 at the start) 595, with four 601; up to 128 of 192 pairs 341 and 331.
     const int parts = gm.split ? gm.max_cta / n_slots + 2 : gm.max_chunks, sms = sm_count();
     const dim3 mg(n_slots * q_len, GQA * a.nhk);
     const long long grid = (long long) mg.x * mg.y;
     const bool one = gm.split ? parts <= 8 : parts <= 4 || (parts <= MERGE_STREAMS && grid > 8LL * sms);
-    const bool sixteen = parts > 32 && (grid <= 2LL * sms || (parts > 128 && grid <= 8LL * sms));
-    const unsigned threads = one ? 64 : sixteen ? 1024 : 256;
-    auto * merge = sixteen ? decode_merge_k<16, false> : !one ? decode_merge_k<4, false> : gm.split ? decode_merge_k<1, false> : decode_merge_k<1, true>;
-    launch(merge, mg, threads, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    if (one) launch(gm.split ? decode_merge_k<false> : decode_merge_k<true>, mg, 64, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    else launch(parts > 4 * MERGE_STREAMS && grid * (DH / 4 / MERGE_DL) <= 2LL * sms ? decode_merge_streams_k<8> : decode_merge_streams_k<4>, dim3(mg.x, mg.y, DH / 4 / MERGE_DL), MERGE_THR, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
     count_launch(launches);
     return launch_status(who);
 }
