@@ -7,13 +7,16 @@
 //                one 128-key operand), so the main kernel fetches a tile with one bulk copy.
 //   prefill_k    one CTA per (128 query rows of one kv head): rows n = 6 t + hh (token t, head hh of the GQA group) on
 //                the MMA M axis, keys in steps of 128 (a pair of images).  Per step: S = Q K^T as 16 MMAs m128n128k16
-//                (Q from tensor memory, fp32 S in tensor memory), online softmax in base 2 with two threads per row
-//                (64 keys each, no shuffles), P to shared memory as f16, O += P V as 8 MMAs m128n256k16 accumulated in
-//                tensor memory.  Warp roles: 8 softmax warps, 1 bulk-copy producer warp, 1 MMA-issue warp.  The MMA
+//                (Q from tensor memory and shared memory, half of the dims each; fp32 S in tensor memory), online softmax in base 2
+//                with two threads per row (64 keys each, no shuffles), P to tensor memory as f16, O += P V as 8 MMAs m128n256k16
+//                accumulated in tensor memory.  Warp roles: 8 softmax warps, 1 bulk-copy producer warp, 1 MMA-issue warp.  The MMA
 //                queue alternates Q K^T of step J+1 and P V of step J, so the tensor pipe has work while the softmax
 //                of a step runs; S is single-buffered (the next Q K^T starts when the softmax threads hold S in
-//                registers), P is double-buffered.  The running output is rescaled only when a row's maximum grows by
-//                more than 2^8 (P stays below 256 in f16).  Epilogue: O / l, optional sigmoid gate.
+//                registers), P is freed and filled in halves of 64 keys.  The running output is rescaled only when a row's maximum
+//                grows by more than 2^8 (P stays below 256 in f16).  Epilogue: O / l, optional sigmoid gate.
+//                What bounds a step is shared memory (128 bytes per clk): K and V images in and out 256 KB and half of Q out 32 KB are 2304 clk, measured
+//                2300 (1.4 us at 1.65 GHz; the MMAs take 2048).  With P in shared memory (64 KB in and out) and all of Q in tensor memory it
+//                was 2515; tensor memory is full now: S 128, O 256, Q 64, P 64 columns.
 //                A few rows behind a long history are fewer row tiles than SMs: then the steps of all row tiles are cut evenly over
 //                the SMs and prefill_merge_k adds up the pieces of a tile (pf_cut, split_ctas).
 // f16 operands (int8 * f16 scale is not representable in bf16's 8 significand bits), fp32 accumulation.
@@ -41,24 +44,26 @@ constexpr int BM = 128;                 // query rows per CTA
 constexpr int BN = 64;                  // keys per tile image
 constexpr int BP = 2 * BN;              // keys per step: S tile = 128 rows x 128 keys
 constexpr int IMG = BN * DH * 2;        // bytes of one tile image (32 KB)
-constexpr int P_BYTES = BM * BP * 2;    // 32 KB
-constexpr int Q_BYTES = BM * DH * 2;    // 64 KB
-constexpr int EPI_BYTES = 8 * 32 * 33 * 4;   // per softmax warp a 32 x 33 float tile for the row-wise epilogue
+constexpr int Q_BYTES = BM * DH / 2 * 2;    // 32 KB: half of the dims
+constexpr int EPI_STR = DH / 2 + 4;     // floats per row of the epilogue's tiles: 32 rows x 128 dims per softmax warp (+ 4: rows on different banks)
+constexpr int EPI_BYTES = 8 * 32 * EPI_STR * 4;
 constexpr int NSOFT = 256;              // softmax threads: two per query row (key halves of a tile, dim halves of the output)
 constexpr int NTHR_PF = NSOFT + 64;     // 8 softmax warps + producer + MMA issuer
 constexpr int W_PROD = NSOFT / 32, W_MMA = W_PROD + 1;
 constexpr float LOG2E_PF = 1.4426950408889634f;
 constexpr float RESCALE_GAP = 8.0f;     // rescale O when a row maximum grows by more than this (log2 units)
 
-constexpr int NSTG = 3;                         // V ring depth (64-key images)
-constexpr int SM_K = 0;                         // one pair of K images (the epilogue tiles reuse it)
-constexpr int SM_EPI = SM_K;
-constexpr int SM_V = SM_K + 2 * IMG;            // NSTG images
-constexpr int SM_P = SM_V + NSTG * IMG;         // 2 buffers
-constexpr int SM_XCH = SM_P + 2 * P_BYTES;      // [2][128] floats exchanged between the two threads of a row
+// Two pairs of K images and one pair of V images whose halves are copied and freed by themselves: every copy has 1500 clk or more before it
+// is waited for.  One pair of K images left 1024 clk for its 64 KB (48 rows behind 100003 keys, images from HBM: a step 1.84 us, 1.65 with two).
+// A ring of single images that frees K by halves needs Q K^T in two m128n64k16, which take longer than half of an m128n128k16: 1.75 us for 1.5.
+constexpr int SM_K = 0;
+constexpr int SM_V = SM_K + 4 * IMG;
+constexpr int SM_Q = SM_V + 2 * IMG;            // dims 128 .. 255 of the query rows
+constexpr int SM_EPI = SM_K;                    // the epilogue tiles lie over K and V
+constexpr int SM_XCH = SM_Q + Q_BYTES;          // [2][128] floats exchanged between the two threads of a row
 constexpr int SM_BAR = SM_XCH + 1024;           // mbarriers + tmem base
 constexpr int SM_TOTAL = SM_BAR + 256;
-static_assert(SM_TOTAL <= 227 * 1024 && EPI_BYTES <= 2 * IMG, "prefill_k shared memory");
+static_assert(SM_TOTAL <= 227 * 1024 && EPI_BYTES <= SM_Q, "prefill_k shared memory");
 
 // ---- pre-pass: cache rows -> f16 tile images -------------------------------------------------------------------
 // grid (n_tiles, Hkv), 256 threads; thread = (key, 64 dims).  Image byte of (key, dim) = (key/8)*4096 + (dim/8)*128 +
@@ -186,8 +191,13 @@ __device__ __forceinline__ int pf_find_tile(const pf_args & a, int rem, int & be
     }
 }
 
+__device__ __forceinline__ float rcpf(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 // 1 / (1 + 2^(-g log2 e)) with the hardware exponential and reciprocal (relative error ~1e-7 against expf and an IEEE divide)
-__device__ __forceinline__ float fast_sigmoid(float g) { return __fdividef(1.0f, 1.0f + ex2f(-g * LOG2E_PF)); }
+__device__ __forceinline__ float fast_sigmoid(float g) { return rcpf(1.0f + ex2f(-g * LOG2E_PF)); }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t * bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -203,9 +213,9 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
     pdl_enter();
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t * bars = reinterpret_cast<uint64_t *>(smem + SM_BAR);
-    uint64_t * k_full = bars, * k_free = bars + 1, * s_full = bars + 2, * s_free = bars + 3, * v_full = bars + 4, * v_free = bars + 8,
-             * p_full = bars + 12, * pv_done = bars + 14, * o_done = bars + 16, * q_ready = bars + 17;
-    uint32_t * tbase_p = reinterpret_cast<uint32_t *>(bars + 18);
+    uint64_t * k_full = bars, * k_free = bars + 2, * v_full = bars + 4, * v_free = bars + 6, * p_full = bars + 8, * pv_done = bars + 10,   // two each
+             * s_full = bars + 12, * s_free = bars + 13, * o_done = bars + 14, * q_ready = bars + 15;
+    uint32_t * tbase_p = reinterpret_cast<uint32_t *>(bars + 16);
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);     // as a warp-uniform value
@@ -227,9 +237,11 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
     }
 
     if (tid == 0) {
-        mbar_init(k_full, 1); mbar_init(k_free, 1); mbar_init(s_full, 1); mbar_init(s_free, NSOFT);
-        for (int b = 0; b < NSTG; ++b) { mbar_init(&v_full[b], 1); mbar_init(&v_free[b], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&p_full[b], NSOFT); mbar_init(&pv_done[b], 1); }
+        mbar_init(s_full, 1); mbar_init(s_free, NSOFT);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&k_full[b], 1); mbar_init(&k_free[b], 1); mbar_init(&v_full[b], 1); mbar_init(&v_free[b], 1);
+            mbar_init(&p_full[b], NSOFT / 2); mbar_init(&pv_done[b], 1);
+        }
         mbar_init(o_done, 1);
         mbar_init(q_ready, 1);
         mbar_fence_init();
@@ -240,14 +252,15 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tb = *tbase_p;
-    const uint32_t t_S = tb, t_O = tb + BP, t_Q = tb + BP + DH;   // S at columns 0..127, O at 128..383, Q (f16 pairs) at 384..511
+    const uint32_t t_S = tb, t_O = tb + BP, t_Q = t_O + DH, t_P = t_Q + DH / 4;   // S at columns 0..127, O at 128..383, Q (dims 0..127 as f16 pairs) at 384.., P (128 keys) at 448..
 
     // row bookkeeping of the softmax threads, shared by the prologue, the loop and the epilogue: a warp owns the 32 rows of its
     // tensor-memory lanes; for row-wise global accesses 8 lanes cover 128 bytes of one row, a warp instruction touches 4 rows
     const uint32_t lane_off = (uint32_t) ((warp & 3) * 32) << 16;
     const int sub = lane >> 3, col = 4 * (lane & 7);
 
-    int g = 0, gi = 0;   // steps and 64-key images of the earlier segments: the barriers' phases run on from one segment to the next
+    // steps of the earlier segments and those of them that had a second V image: the barriers' phases run on from one segment to the next
+    int g = 0, g2 = 0;
     for (int seg = 0;; ++seg) {
     const int n0 = mtile * BM;
     const int t_last = min(n0 + BM - 1, R - 1) / GQA;           // last token of the tile
@@ -264,39 +277,74 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
 
     if (warp < W_PROD) {
         // Q rows -> f16, scaled by softmax scale * log2(e), into tensor memory as the A operand of Q K^T: lane = row,
-        // column c holds dims 2c, 2c+1.  The two threads of a row take 128 dims each, 64 dims per slab.
+        // column c holds dims 2c, 2c+1.  The two threads of a row take 128 dims each.  A warp reads 256 bytes of a row with 16 lanes (all of
+        // its half of a bf16 row, half of it of an f32 row), two rows per load and 16 loads in flight, and turns them by way of a tile of its own
+        // where the K images of the second step go, chunk c of row i at c ^ (i & 7): with each lane reading along its own row a load touched 32 rows (4.5 us of
+        // prologue on a busy chip; as one bulk copy per row 9 us, of which 128 copies took 6 to issue).
         const int r = tid & (BM - 1), hf = tid >> 7, n = n0 + r;
         const int t = n / GQA, hh = n - t * GQA;
         const size_t rowidx = (size_t) t * a.Hq + hk * GQA + hh;
         const float sc = a.qscale;
-        if (a.q) {
-            const float4 * src = n < R ? reinterpret_cast<const float4 *>(a.q + rowidx * DH) : nullptr;
-#pragma unroll 1
-            for (int d0 = hf * (DH / 2); d0 < (hf + 1) * (DH / 2); d0 += 64) {
-                float4 x[16];
+        unsigned char * qt = smem + SM_K + ((g + 1) & 1) * (2 * IMG) + warp * 8192;
+        const int esz = a.q ? 4 : 2;
+        const char * qsrc = a.q ? reinterpret_cast<const char *>(a.q) : reinterpret_cast<const char *>(a.qb);
+        auto ahead = [&](uint4 (&x)[16], int part) {   // bytes 256 part .. of the warp's half rows
 #pragma unroll
-                for (int u = 0; u < 16; ++u) x[u] = src ? __ldg(src + d0 / 4 + u) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            for (int u = 0; u < 16; ++u) {
+                const int nr = n0 + (warp & 3) * 32 + 2 * u + (lane >> 4), tr = nr / GQA, hr = nr - tr * GQA;
+                x[u] = nr < R ? __ldg(reinterpret_cast<const uint4 *>(qsrc + (((size_t) tr * a.Hq + hk * GQA + hr) * DH + hf * (DH / 2)) * esz + 256 * part) + (lane & 15))
+                              : make_uint4(0, 0, 0, 0);
+            }
+        };
+        auto put = [&](const uint4 (&x)[16]) {
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                const int i = 2 * u + (lane >> 4);
+                *reinterpret_cast<uint4 *>(qt + i * 256 + (((lane & 15) ^ (i & 7)) << 4)) = x[u];
+            }
+            __syncwarp();
+        };
+        auto chunk = [&](int c) { return *reinterpret_cast<const uint4 *>(qt + lane * 256 + ((c ^ (lane & 7)) << 4)); };
+        auto put_q = [&](const uint32_t (&w)[32], int part) {   // 64 dims of the thread's row, f16 pairs: to tensor memory, or K-major to shared memory
+            if (hf == 0) umma::tmem_st32(t_Q + lane_off + 32 * part, w);
+            else
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<uint4 *>(smem + SM_Q + (8 * part + c) * 2048 + r * 16) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+        };
+        uint4 x[16];
+        ahead(x, 0);
+        if (a.q) {
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                put(x);
+                if (part == 0) ahead(x, 1);
                 uint32_t w[32];
 #pragma unroll
-                for (int u = 0; u < 16; ++u) { w[2 * u] = pack_h2(x[u].x * sc, x[u].y * sc); w[2 * u + 1] = pack_h2(x[u].z * sc, x[u].w * sc); }
-                umma::tmem_st32(t_Q + lane_off + d0 / 2, w);
+                for (int u = 0; u < 16; ++u) {
+                    const uint4 v = chunk(u);
+                    w[2 * u] = pack_h2(__uint_as_float(v.x) * sc, __uint_as_float(v.y) * sc);
+                    w[2 * u + 1] = pack_h2(__uint_as_float(v.z) * sc, __uint_as_float(v.w) * sc);
+                }
+                put_q(w, part);
             }
         } else {
             // bf16 rows as the projection wrote them: widen, rotate the 32 pairs (j, j + 32) of the first 64 dims with the
             // token's cos / sin (same expressions and roundings as the append kernel), scale, round to f16
-            const uint4 * src = n < R ? reinterpret_cast<const uint4 *>(a.qb + rowidx * DH) : nullptr;
+            const float4 * cs4 = reinterpret_cast<const float4 *>(a.cs + (size_t) t * 64);
+            put(x);
 #pragma unroll 1
-            for (int d0 = hf * (DH / 2); d0 < (hf + 1) * (DH / 2); d0 += 64) {
+            for (int part = 0; part < 2; ++part) {
                 float f[64];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     float e8[8];
-                    bf16x8_widen(src ? __ldg(src + d0 / 8 + u) : make_uint4(0, 0, 0, 0), e8);
+                    bf16x8_widen(chunk(8 * part + u), e8);
 #pragma unroll
                     for (int e = 0; e < 8; ++e) f[8 * u + e] = e8[e];
                 }
-                if (d0 == 0 && src) {
-                    const float4 * cs4 = reinterpret_cast<const float4 *>(a.cs + (size_t) t * 64);
+                if (hf == 0 && part == 0 && n < R) {
 #pragma unroll
                     for (int u = 0; u < 8; ++u) {
                         const float4 c4 = __ldg(cs4 + u), s4 = __ldg(cs4 + 8 + u);
@@ -308,13 +356,14 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
                 uint32_t w[32];
 #pragma unroll
                 for (int u = 0; u < 32; ++u) w[u] = pack_h2(f[2 * u] * sc, f[2 * u + 1] * sc);
-                umma::tmem_st32(t_Q + lane_off + d0 / 2, w);
+                put_q(w, part);
             }
         }
         if (carry_in) {
             // the running O of the earlier passes goes back into tensor memory (read row-wise, handed over through a
-            // per-warp tile in the P buffers, which nothing uses before the barrier below), with the row's maximum and sum
-            float * tile = reinterpret_cast<float *>(smem + SM_P) + warp * (32 * 33);
+            // per-warp tile in the same place), with the row's maximum and sum
+            asm volatile("bar.sync 1, %0;" ::"n"(NSOFT) : "memory");   // every warp is done with its tile of query values
+            float * tile = reinterpret_cast<float *>(smem + SM_K + ((g + 1) & 1) * (2 * IMG)) + warp * (32 * 33);
             const int c_lo = hf * (DH / 2), c_hi = c_lo + DH / 2;
 #pragma unroll 1
             for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
@@ -340,38 +389,30 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
         }
         umma::tmem_st_wait();
         umma::fence_before_sync();
+        umma::fence_async_smem();   // K images are copied to where the tiles lay
         asm volatile("bar.sync 1, %0;" ::"n"(NSOFT) : "memory");   // the softmax warps: every Q (and O) row is in place
         if (tid == 0) mbar_arrive(q_ready);
     }
     const bool any_gate = a.gate || a.gate_b;
-    if (warp >= W_PROD && any_gate && !carry_out && !piece && (lane & 15) != 0) {
-        // idle lanes of the producer and MMA warps pull this CTA's gate rows (contiguous per token: 6 heads) into L2
-        const int t_first = n0 / GQA;
-        const int esz = a.gate ? 4 : 2;
-        const char * g0 = a.gate ? reinterpret_cast<const char *>(a.gate + ((size_t) t_first * a.Hq + hk * GQA) * DH)
-                                 : reinterpret_cast<const char *>(a.gate_b + ((size_t) t_first * a.Hq + hk * GQA) * DH);
-        const int idx = (warp - W_PROD) * 30 + lane - 1 - (lane > 16);
-        for (int t = t_first; t <= t_last; ++t)
-            for (int ln = idx; ln < GQA * DH * esz / 128; ln += 60)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(g0 + (size_t) (t - t_first) * a.Hq * DH * esz + ln * 128));
-    }
     if (warp == W_PROD) {
-        // ---------------- producer: K in pairs of images (lane 0), V image by image through a ring (lane 16) ----------------
+        // ---------------- producer: K in pairs of images (lane 0), V image by image (lane 16) ----------------
         const unsigned char * src = a.tiles + ((size_t) hk * a.n_tiles + 2 * st0) * (2 * IMG);
         if (lane == 0) {
             for (int J = 0; J < nsteps; ++J) {
-                if (g + J >= 1) mbar_wait(k_free, (uint32_t) ((g + J - 1) & 1), a.status);   // Q K^T of step J-1 has read the pair
+                const int G = g + J, b = G & 1;
+                if (J == 1) mbar_wait(q_ready, (uint32_t) (seg & 1), a.status);   // the query rows have passed through this pair's place
+                if (G >= 2) mbar_wait(&k_free[b], (uint32_t) (((G >> 1) - 1) & 1), a.status);   // Q K^T of step J-2 has read the pair
                 const int n_img = min(2, ntiles - 2 * J);
-                mbar_expect_tx(k_full, (uint32_t) n_img * IMG);
+                mbar_expect_tx(&k_full[b], (uint32_t) n_img * IMG);
                 for (int h = 0; h < n_img; ++h)
-                    bulk_g2s(smem + SM_K + h * IMG, src + (size_t) (2 * J + h) * (2 * IMG), IMG, k_full);
+                    bulk_g2s(smem + SM_K + (2 * b + h) * IMG, src + (size_t) (2 * J + h) * (2 * IMG), IMG, &k_full[b]);
             }
         } else if (lane == 16) {
             for (int j = 0; j < ntiles; ++j) {
-                const int s = (gi + j) % NSTG;
-                if (gi + j >= NSTG) mbar_wait(&v_free[s], (uint32_t) (((gi + j) / NSTG - 1) & 1), a.status);   // P V of image j-NSTG has read the slot
-                mbar_expect_tx(&v_full[s], IMG);
-                bulk_g2s(smem + SM_V + s * IMG, src + (size_t) j * (2 * IMG) + IMG, IMG, &v_full[s]);
+                const int h = j & 1, u = (h ? g2 : g) + (j >> 1);   // earlier uses of the slot
+                if (u >= 1) mbar_wait(&v_free[h], (uint32_t) ((u - 1) & 1), a.status);   // P V of the image before has read the slot
+                mbar_expect_tx(&v_full[h], IMG);
+                bulk_g2s(smem + SM_V + h * IMG, src + (size_t) j * (2 * IMG) + IMG, IMG, &v_full[h]);
             }
         }
     } else if (warp == W_MMA) {
@@ -381,48 +422,49 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
         __syncwarp();
         const bool lead = umma::elect_one();
         const uint32_t tb_u = __shfl_sync(0xffffffffu, tb, 0);
-        const uint32_t tS_u = tb_u, tO_u = tb_u + BP, tQ_u = tb_u + BP + DH;
+        const uint32_t tS_u = tb_u, tO_u = tb_u + BP, tQ_u = tO_u + DH, tP_u = tQ_u + DH / 4;
         const int ns_u = __shfl_sync(0xffffffffu, nsteps, 0), ni_u = __shfl_sync(0xffffffffu, ntiles, 0), g_u = __shfl_sync(0xffffffffu, g, 0);
-        int gj = __shfl_sync(0xffffffffu, gi, 0);   // images before the next P V
+        const int g2_u = __shfl_sync(0xffffffffu, g2, 0);
         constexpr uint32_t id_qk = umma::idesc_f16(BM, BP, false, false);   // S[128 x 128] = Q (tensor memory) * K^T (K-major)
         constexpr uint32_t id_pv = umma::idesc_f16(BM, DH, false, true);    // O[128 x 256] += P (K-major) * V (MN-major)
-        const uint32_t k_s = smem_u32(smem + SM_K), v_s0 = smem_u32(smem + SM_V), p_s0 = smem_u32(smem + SM_P);
+        const uint32_t k_s0 = smem_u32(smem + SM_K), v_s0 = smem_u32(smem + SM_V), q_s = smem_u32(smem + SM_Q);
         auto issue_qk = [&](int J) {
-            const int G = g_u + J;
-            mbar_wait(k_full, (uint32_t) (G & 1), a.status);
+            const int G = g_u + J, b = G & 1;
+            mbar_wait(&k_full[b], (uint32_t) ((G >> 1) & 1), a.status);
             if (G >= 1) mbar_wait(s_free, (uint32_t) ((G - 1) & 1), a.status);   // the softmax threads hold S of the step before in registers
             umma::fence_after_sync();
             // K pair: K-major, 8-key groups 4096 apart (SBO), 8-dim chunks 128 apart (LBO); 16 dims = 256 bytes per k-step.
             // A step with a single image multiplies whatever the second half of the buffer holds: those keys lie past
             // every row of the tile and are masked.
             if (lead) {
+                const uint32_t k_s = k_s0 + b * (2 * IMG);
 #pragma unroll
-                for (int ks = 0; ks < DH / 16; ++ks)
+                for (int ks = 0; ks < DH / 32; ++ks)
                     umma::mma_ts(tS_u, tQ_u + ks * 8, umma::smem_desc(k_s + ks * 256, 128, 4096), id_qk, ks > 0);
+#pragma unroll
+                for (int ks = 0; ks < DH / 32; ++ks)   // Q: 8-row groups 128 apart (SBO), 8-dim chunks 2048 apart (LBO)
+                    umma::mma_ss(tS_u, umma::smem_desc(q_s + ks * 2 * 2048, 2048, 128), umma::smem_desc(k_s + (DH / 32 + ks) * 256, 128, 4096), id_qk, 1u);
                 umma::commit(s_full);
-                umma::commit(k_free);
+                umma::commit(&k_free[b]);
             }
         };
         auto issue_pv = [&](int J) {
-            const int G = g_u + J, b = G & 1;
-            mbar_wait(&p_full[b], (uint32_t) ((G >> 1) & 1), a.status);
-            const int n_img = min(2, ni_u - 2 * J);
-            for (int h = 0; h < n_img; ++h, ++gj) {
-                const int st = gj % NSTG;
-                mbar_wait(&v_full[st], (uint32_t) ((gj / NSTG) & 1), a.status);
+            const int G = g_u + J, n_img = min(2, ni_u - 2 * J);
+            for (int h = 0; h < n_img; ++h) {
+                mbar_wait(&p_full[h], (uint32_t) (G & 1), a.status);
+                mbar_wait(&v_full[h], (uint32_t) (((h ? g2_u : g_u) + J) & 1), a.status);
                 umma::fence_after_sync();
                 if (lead) {
-                    const uint32_t v_s = v_s0 + st * IMG, p_s = p_s0 + b * P_BYTES + h * 8 * 2048;
+                    const uint32_t v_s = v_s0 + h * IMG;
                     const uint32_t acc0 = (carry_in || J > 0 || h > 0) ? 1u : 0u;
 #pragma unroll
-                    for (int ks = 0; ks < BN / 16; ++ks)   // P: K-major, 8-key chunks 2048 apart; V: MN-major, 8-key groups 4096 apart (LBO),
-                                                           // 8-dim chunks 128 apart (SBO)
-                        umma::mma_ss(tO_u, umma::smem_desc(p_s + ks * 2 * 2048, 2048, 128),
-                                     umma::smem_desc(v_s + ks * 2 * 4096, 4096, 128), id_pv, ks > 0 ? 1u : acc0);
-                    umma::commit(&v_free[st]);
+                    for (int ks = 0; ks < BN / 16; ++ks)   // V: MN-major, 8-key groups 4096 apart (LBO), 8-dim chunks 128 apart (SBO)
+                        umma::mma_ts(tO_u, tP_u + 32 * h + ks * 8, umma::smem_desc(v_s + ks * 2 * 4096, 4096, 128), id_pv, ks > 0 ? 1u : acc0);
+                    umma::commit(&v_free[h]);
+                    umma::commit(&pv_done[h]);
                 }
             }
-            if (lead) umma::commit(&pv_done[b]);
+            if (n_img < 2 && lead) umma::commit(&pv_done[1]);   // the half without keys
         };
         mbar_wait(q_ready, (uint32_t) (seg & 1), a.status);
         umma::fence_after_sync();
@@ -485,7 +527,7 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
                     l *= f;
                 }
                 if (J > 0 || carry_in) {
-                    if (J > 0) mbar_wait(&pv_done[(G - 1) & 1], (uint32_t) (((G - 1) >> 1) & 1), a.status);   // P V of step J-1 has landed in O
+                    if (J > 0) mbar_wait(&pv_done[1], (uint32_t) ((G - 1) & 1), a.status);   // P V of step J-1 has landed in O
                     umma::fence_after_sync();
 #pragma unroll 1
                     for (int c0 = hf * (DH / 2); c0 < (hf + 1) * (DH / 2); c0 += 32) {
@@ -501,40 +543,66 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
                 }
             }
             const float mref_safe = m_ref == B200_NEG_INF ? 0.0f : m_ref;
-            if (G >= 2) mbar_wait(&pv_done[G & 1], (uint32_t) (((G >> 1) - 1) & 1), a.status);   // P buffer no longer read
-            // K-major P image of the step: key chunk kc (8 keys) at kc * 2048, row at 16 bytes; this thread's chunks are 8 hf ..
-            unsigned char * prow = smem + SM_P + (G & 1) * P_BYTES + (8 * hf) * 2048 + r * 16;
+            if (G >= 1) mbar_wait(&pv_done[hf], (uint32_t) ((G - 1) & 1), a.status);   // this half of P is no longer read
+            // P as f16 pairs into tensor memory: lane = row, this thread's 64 keys in columns 32 hf ..
             float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+            for (int h = 0; h < 2; ++h) {
+                uint32_t w[16];
 #pragma unroll
-                for (int c8 = 0; c8 < 4; ++c8) {
-                    uint32_t w4[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        // ex2(-inf) = 0: masked keys need no special case (mref_safe is finite)
-                        const float p0 = ex2f(__uint_as_float(sr[h][c8 * 8 + 2 * e]) - mref_safe);
-                        const float p1 = ex2f(__uint_as_float(sr[h][c8 * 8 + 2 * e + 1]) - mref_safe);
-                        l4[e] += p0 + p1;
-                        w4[e] = pack_h2(p0, p1);
-                    }
-                    *reinterpret_cast<uint4 *>(prow + (4 * h + c8) * 2048) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                for (int e = 0; e < 16; ++e) {
+                    // ex2(-inf) = 0: masked keys need no special case (mref_safe is finite)
+                    const float p0 = ex2f(__uint_as_float(sr[h][2 * e]) - mref_safe);
+                    const float p1 = ex2f(__uint_as_float(sr[h][2 * e + 1]) - mref_safe);
+                    l4[e & 3] += p0 + p1;
+                    w[e] = pack_h2(p0, p1);
                 }
+                umma::tmem_st16(t_P + lane_off + 32 * hf + 16 * h, w);
+            }
             l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
-            umma::fence_async_smem();
+            umma::tmem_st_wait();
             umma::fence_before_sync();
-            mbar_arrive(&p_full[G & 1]);
+            mbar_arrive(&p_full[hf]);
         }
         // ---------------- epilogue ----------------
         // final:   O / l, gate, store (f32 and / or bf16, a16 copy);  carry_out: unnormalised O, (maximum, sum) for the next pass;
         // partial: unnormalised O with the maximum in natural-log units and the sum, for a merge across sequence shards
+        const bool raw = carry_out || a.pm || piece;   // O leaves unnormalised
+        const bool gated = any_gate && !raw, gate16 = a.gate == nullptr;
+        const size_t slot = 2 * (size_t) blockIdx.x + (st0 == 0 ? 1 : 0);   // number of the piece
+        // A warp owns 32 rows x 128 dims.  Its lanes read them back from a private shared-memory tile along the rows: in step i, lane l holds values
+        // 4 (l mod 16) .. and 64 + 4 (l mod 16) .. of row 2 i + l / 16.  The gate values go out four steps ahead, raw (a conversion right behind
+        // each load made the loads wait for one another: 12 us an epilogue instead of 3).
+        const int lr = lane >> 4, lc = 4 * (lane & 15);
+        auto row_at = [&](int i) {   // offset of the lane's first values in a result or gate array, or -1 past the last row
+            const int nr = n0 + (warp & 3) * 32 + 2 * i + lr;
+            const int tr = nr / GQA, hr = nr - tr * GQA;
+            return nr < R ? (long long) ((size_t) tr * a.Hq + hk * GQA + hr) * DH + hf * (DH / 2) + lc : -1ll;
+        };
+        constexpr int AHEAD = 4, STEPS = 16;
+        float4 gn[AHEAD][2];
+        auto gate_ahead = [&](int i0) {   // rows past the last one: the first values of the array
+            if (gate16) {
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i) {
+                    const __nv_bfloat16 * p = a.gate_b + max(row_at(i0 + i), 0ll);
+                    const float2 u = __ldg(reinterpret_cast<const float2 *>(p)), v = __ldg(reinterpret_cast<const float2 *>(p + 64));
+                    gn[i][0].x = u.x; gn[i][0].y = u.y; gn[i][1].x = v.x; gn[i][1].y = v.y;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i) {
+                    const float * p = a.gate + max(row_at(i0 + i), 0ll);
+                    gn[i][0] = __ldg(reinterpret_cast<const float4 *>(p)); gn[i][1] = __ldg(reinterpret_cast<const float4 *>(p + 64));
+                }
+            }
+        };
+        if (gated) gate_ahead(0);
         xch[hf * BM + r] = l;
         asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
         l = xch[r] + xch[BM + r];
         mbar_wait(o_done, (uint32_t) (seg & 1), a.status);
         umma::fence_after_sync();
-        const bool raw = carry_out || a.pm || piece;   // O leaves unnormalised
-        const size_t slot = 2 * (size_t) blockIdx.x + (st0 == 0 ? 1 : 0);   // number of the piece
         const bool have_o = nsteps > 0 || carry_in;   // a tile that has seen no key at all (a sequence shard) holds nothing in O
         const float inv = raw ? 1.0f : (l > 0.0f ? 1.0f / l : 0.0f);
         if (n < R && hf == 0) {
@@ -543,75 +611,84 @@ __global__ void __launch_bounds__(NTHR_PF, 1) prefill_k(const pf_args a) {
             else if (carry_out) { a.ml[rowidx * 2] = m_ref; a.ml[rowidx * 2 + 1] = l; }
             else if (a.pm) { a.pm[rowidx] = m_ref * 0.6931471805599453f; a.pl[rowidx] = l; }
         }
-        // A 32-column slab of O goes through a private shared-memory tile so that global accesses run along rows.
-        float * tile = reinterpret_cast<float *>(smem + SM_EPI) + warp * (32 * 33);
-        const int c_lo = hf * (DH / 2), c_hi = c_lo + DH / 2;
-        size_t orow[8];
-        bool live[8];
+        float * tile = reinterpret_cast<float *>(smem + SM_EPI) + warp * (32 * EPI_STR);
 #pragma unroll
-        for (int q8 = 0; q8 < 8; ++q8) {
-            const int nr = n0 + (warp & 3) * 32 + 4 * q8 + sub;
-            const int tr = nr / GQA, hr = nr - tr * GQA;
-            live[q8] = nr < R;
-            orow[q8] = piece ? (slot * BM + nr - n0) * DH + col : ((size_t) tr * a.Hq + hk * GQA + hr) * DH + col;
-        }
-        const bool gated = any_gate && !raw;
-        auto gate_at = [&](size_t o) {
-            if (a.gate) return __ldg(reinterpret_cast<const float4 *>(a.gate + o));
-            const uint2 u = __ldg(reinterpret_cast<const uint2 *>(a.gate_b + o));
-            return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
-                               __uint_as_float(u.y & 0xffff0000u));
-        };
-        float4 gn[8];   // gate values of the next slab, requested one slab ahead
-#pragma unroll
-        for (int q8 = 0; q8 < 8; ++q8) gn[q8] = (gated && live[q8]) ? gate_at(orow[q8] + c_lo) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const size_t n_groups = (size_t) a.T * a.Hq * (DH / 32);
-#pragma unroll 1
-        for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
-            float4 gv[8];
-#pragma unroll
-            for (int q8 = 0; q8 < 8; ++q8) {
-                gv[q8] = gn[q8];
-                if (gated && live[q8] && c0 + 32 < c_hi) gn[q8] = gate_at(orow[q8] + c0 + 32);
-            }
+        for (int c0 = 0; c0 < DH / 2; c0 += 32) {
             uint32_t o[32];
             if (have_o) {
-                umma::tmem_ld32(t_O + lane_off + c0, o);
+                umma::tmem_ld32(t_O + lane_off + hf * (DH / 2) + c0, o);
                 umma::tmem_ld_wait();
             } else {
 #pragma unroll
                 for (int c = 0; c < 32; ++c) o[c] = 0u;
             }
 #pragma unroll
-            for (int c = 0; c < 32; ++c) tile[lane * 33 + c] = __uint_as_float(o[c]) * inv;
-            __syncwarp();
-#pragma unroll
-            for (int q8 = 0; q8 < 8; ++q8) {
-                const int rl = 4 * q8 + sub;
-                float4 y = make_float4(tile[rl * 33 + col], tile[rl * 33 + col + 1], tile[rl * 33 + col + 2], tile[rl * 33 + col + 3]);
-                if (gated) {
-                    y.x *= fast_sigmoid(gv[q8].x); y.y *= fast_sigmoid(gv[q8].y);
-                    y.z *= fast_sigmoid(gv[q8].z); y.w *= fast_sigmoid(gv[q8].w);
-                }
-                if (live[q8]) {
-                    if (raw || !a.out_b) *reinterpret_cast<float4 *>((piece ? a.po : a.out) + orow[q8] + c0) = y;
-                    if (!raw && a.out_b) {
-                        const __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
-                        *reinterpret_cast<uint2 *>(a.out_b + orow[q8] + c0) =
-                            make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
-                    }
-                }
-                // the a16 copy for the projection that follows: the eight lanes of a row segment hold one 32-value group
-                if (a.qbuf && !raw) a16_store_lanes8(y, a.qbuf, (orow[q8] + c0) / 32, n_groups, live[q8]);
-            }
-            __syncwarp();
+            for (int c = 0; c < 32; c += 4)
+                *reinterpret_cast<float4 *>(tile + lane * EPI_STR + c0 + c) = make_float4(__uint_as_float(o[c]) * inv, __uint_as_float(o[c + 1]) * inv,
+                                                                                          __uint_as_float(o[c + 2]) * inv, __uint_as_float(o[c + 3]) * inv);
         }
-        umma::fence_async_smem();   // the epilogue tiles lie where the next segment's K images are copied to
+        __syncwarp();
+        const size_t n_groups = (size_t) a.T * a.Hq * (DH / 32);
+#pragma unroll 1
+        for (int i0 = 0; i0 < STEPS; i0 += AHEAD) {
+            float4 y[AHEAD][2];
+            long long o[AHEAD];
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) {
+                o[i] = row_at(i0 + i);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) y[i][h] = *reinterpret_cast<const float4 *>(tile + (2 * (i0 + i) + lr) * EPI_STR + 64 * h + lc);
+            }
+            if (gated) {
+                float4 gv[AHEAD][2];
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t u = __float_as_uint(gn[i][h].x), v = __float_as_uint(gn[i][h].y);
+                        gv[i][h] = gate16 ? make_float4(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u), __uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u))
+                                          : gn[i][h];
+                    }
+                if (i0 + AHEAD < STEPS) gate_ahead(i0 + AHEAD);
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        y[i][h].x *= fast_sigmoid(gv[i][h].x); y[i][h].y *= fast_sigmoid(gv[i][h].y);
+                        y[i][h].z *= fast_sigmoid(gv[i][h].z); y[i][h].w *= fast_sigmoid(gv[i][h].w);
+                    }
+            }
+            if (!raw && a.out_b) {
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const __nv_bfloat162 lo = __floats2bfloat162_rn(y[i][h].x, y[i][h].y), hi = __floats2bfloat162_rn(y[i][h].z, y[i][h].w);
+                        if (o[i] >= 0) *reinterpret_cast<uint2 *>(a.out_b + o[i] + 64 * h) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+                    }
+            } else {
+                float * const p_out = a.po + (slot * BM + (warp & 3) * 32 + 2 * i0 + lr) * DH + hf * (DH / 2) + lc;
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i) {
+                    float * dst = piece ? p_out + 2 * i * DH : a.out + o[i];
+                    if (o[i] >= 0) { *reinterpret_cast<float4 *>(dst) = y[i][0]; *reinterpret_cast<float4 *>(dst + 64) = y[i][1]; }
+                }
+            }
+            // the a16 copy for the projection that follows: eight lanes of a row hold one 32-value group
+            if (a.qbuf && !raw) {
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i) {
+                    a16_store_lanes8(y[i][0], a.qbuf, (size_t) o[i] / 32, n_groups, o[i] >= 0);
+                    a16_store_lanes8(y[i][1], a.qbuf, (size_t) o[i] / 32 + 2, n_groups, o[i] >= 0);
+                }
+            }
+        }
+        umma::fence_async_smem();   // the epilogue tiles lie where the next segment's images are copied to
     }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    g += nsteps; gi += ntiles;
+    g += nsteps; g2 += ntiles >> 1;
     w += nsteps;
     if (w >= w_end) break;
     st0 = 0;
