@@ -734,6 +734,7 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
 }
 
 #include "decode_tc.cuh"
+#include "decode_warp.cuh"
 
 // The kernel.  With a run plan: every segment of the CTA's run one after the other.  Fixed chunks without a plan (one slot;
 // no more chunks than CTAs; more slots than a plan holds): units u = index, + CTAs of the kv head, .., one chunk each, the highest chunk
@@ -1370,13 +1371,13 @@ encode_tiled_fn tensor_map_encoder() {
 }
 // Encoding a map is pure host arithmetic on (base, geometry); the last few are kept, since a serving loop calls with the
 // same caches (one K and one V per layer) every step.
-struct map_entry { const char * base; unsigned long long rowb, pstride, rows; int HB; bool paged; CUtensorMap m; };
+struct map_entry { const char * base; unsigned long long rowb, pstride, rows; int HB, box_rows; bool paged; CUtensorMap m; };
 constexpr int MAP_CACHE = 256;
 map_entry g_maps[MAP_CACHE];
 int g_nmaps = 0, g_map_next = 0;
 std::mutex g_map_mu;
 
-bool make_cache_map(CUtensorMap * m, const char * base, const dec_args & a, int HB) {
+bool make_cache_map(CUtensorMap * m, const char * base, const dec_args & a, int HB, int box_rows = TILE) {
     encode_tiled_fn enc = tensor_map_encoder();
     if (!enc) return false;
     const bool paged = a.g.pt != nullptr;
@@ -1386,7 +1387,7 @@ bool make_cache_map(CUtensorMap * m, const char * base, const dec_args & a, int 
         std::lock_guard<std::mutex> lk(g_map_mu);
         for (int i = 0; i < g_nmaps; ++i) {
             const map_entry & e = g_maps[i];
-            if (e.base == base && e.rowb == a.g.rowb && e.pstride == pstr && e.rows == rows && e.HB == HB && e.paged == paged) {
+            if (e.base == base && e.rowb == a.g.rowb && e.pstride == pstr && e.rows == rows && e.HB == HB && e.box_rows == box_rows && e.paged == paged) {
                 *m = e.m;
                 return true;
             }
@@ -1404,7 +1405,7 @@ bool make_cache_map(CUtensorMap * m, const char * base, const dec_args & a, int 
     } else {
         const cuuint64_t gdim[3] = {a.g.rowb / 2, rows, npages};
         const cuuint64_t gstr[2] = {a.g.rowb, pbytes};
-        const cuuint32_t box[3] = {(cuuint32_t) HB / 2, (cuuint32_t) TILE, 1};
+        const cuuint32_t box[3] = {(cuuint32_t) HB / 2, (cuuint32_t) box_rows, 1};
         rc = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, (void *) base, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
@@ -1413,7 +1414,7 @@ bool make_cache_map(CUtensorMap * m, const char * base, const dec_args & a, int 
     map_entry & e = g_maps[g_map_next];
     g_map_next = (g_map_next + 1) % MAP_CACHE;
     if (g_nmaps < MAP_CACHE) ++g_nmaps;
-    e.base = base; e.rowb = a.g.rowb; e.pstride = pstr; e.rows = rows; e.HB = HB; e.paged = paged; e.m = *m;
+    e.base = base; e.rowb = a.g.rowb; e.pstride = pstr; e.rows = rows; e.HB = HB; e.box_rows = box_rows; e.paged = paged; e.m = *m;
     return true;
 }
 
@@ -1455,6 +1456,29 @@ int launch_part(const dec_args & a_in, unsigned blocks, cudaStream_t s) {
     return B200_OK;
 }
 
+template <uint32_t KT, int NT>
+int launch_warp(const dec_args & a_in, unsigned runs, cudaStream_t s) {
+    dec_args a = a_in;
+    CUtensorMap mapK, mapV;
+    memset(&mapK, 0, sizeof mapK);
+    memset(&mapV, 0, sizeof mapV);
+    a.tiled = 0;
+    if ((!a.g.pt || a.g.psh >= 6) && a.g.rowb % 16 == 0 &&
+        (a.g.pt ? a.g.pstride < ((unsigned long long) 1 << 40) : (a.n_ctx >= 1 && a.g.rowb * (unsigned long long) a.n_ctx < ((unsigned long long) 1 << 40))))
+        a.tiled = make_cache_map(&mapK, a.g.k, a, traits<KT>::HB, WT) && make_cache_map(&mapV, a.g.v, a, traits<KT>::HB, WT);
+    constexpr size_t sm = wk<KT, NT>::smem(wk<KT, NT>::slots());
+    static std::atomic<bool> attr_done[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!attr_done[dev & 63].load(std::memory_order_acquire)) {
+        if (cudaFuncSetAttribute(decode_warp_k<KT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm) != cudaSuccess)
+            return launch_status("attn_decode (shared memory attribute)");
+        cudaFuncSetAttribute(decode_warp_k<KT, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        attr_done[dev & 63].store(true, std::memory_order_release);
+    }
+    decode_warp_k<KT, NT><<<(runs + 1) / 2, WK_THR, sm, s>>>(a, (int) runs, mapK, mapV);
+    return B200_OK;
+}
 template <uint32_t KT, bool RUNS>
 int launch_part_runs(const dec_args & a, unsigned blocks, cudaStream_t s) {
     const int nt = (a.q_len * GQA + 7) / 8;
@@ -1529,6 +1553,16 @@ int resident_ctas(uint32_t type, int q_len) {
     return per_sm * sm_count();
 }
 
+// runs of decode_warp_k that fit the GPU at once, 0 = not its call.  q4_0: only where the runs may be two tiles long.  Shorter ones have nothing to
+// amortise and half the warps per run: 9 slots of up to 3433 keys, two layers, 79 us for 74 (8 slots x 2 rows of 2839 keys 94 for 88); 40 slots of
+// 13880 keys 377 for 419.
+int warp_runs(uint32_t type, int n_slots, int q_len, int max_n, int Hkv) {
+    if (type == B200_KV_Q8_0) return q_len == 1 ? 2 * wk<B200_KV_Q8_0, 1>::CTAS * sm_count() : 0;
+    if (type != B200_KV_Q4_0 || q_len > 2) return 0;
+    const int n = 2 * (q_len == 1 ? wk<B200_KV_Q4_0, 1>::CTAS : wk<B200_KV_Q4_0, 2>::CTAS) * sm_count();
+    return (long long) n_slots * ((max_n + TILE - 1) / TILE) * Hkv >= 2LL * n ? n : 0;
+}
+
 int auto_chunk(long long total_keys, int Hkv) {
     // enough units for several waves over the SMs, chunks between 256 and 4096 keys
     const long long units = 8LL * sm_count();
@@ -1566,11 +1600,11 @@ bool recording_of(cudaStream_t s, unsigned long long & id) {
     if (st == cudaStreamCaptureStatusNone) id = 0;
     return st != cudaStreamCaptureStatusInvalidated;
 }
-struct dec_geom { int CH, max_chunks, R, max_cta, list_cap; size_t units, segs, part_floats, list_ints; bool planned, split, tc; };
+struct dec_geom { int CH, max_chunks, R, max_cta, list_cap; size_t units, segs, part_floats, list_ints; bool planned, split, tc, warp; };
 
-bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int max_n, int n_ctx, int Hkv, int chunk_keys, bool tc = false, bool rows = false) {
+bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int max_n, int n_ctx, int Hkv, int chunk_keys, bool tc = false, bool rows = false, bool warp = true) {
     if (max_n < 1) max_n = 1;
-    g.tc = false;
+    g.tc = g.warp = false;
     g.R = q_len * GQA;
     g.split = chunk_keys < 0 && n_slots > 1 && n_slots <= SPLIT_MAX_SLOTS;
     g.planned = false;
@@ -1579,7 +1613,9 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
         g.CH = TILE;
         g.max_chunks = (max_n + TILE - 1) / TILE;
         g.tc = tc && type == B200_KV_Q8_0 && q_len >= 2;   // the tensor-core kernel: one CTA per SM
-        g.max_cta = std::max(1, std::min(SPLIT_MAX_CTA, (g.tc ? sm_count() : resident_ctas(type, q_len)) / Hkv));
+        const int runs = g.tc || !warp ? 0 : warp_runs(type, n_slots, q_len, max_n, Hkv);
+        g.warp = runs > 0;
+        g.max_cta = std::max(1, std::min(SPLIT_MAX_CTA, (g.tc ? sm_count() : g.warp ? runs : resident_ctas(type, q_len)) / Hkv));
         g.segs = (size_t) g.max_cta + n_slots;
         g.units = g.segs * Hkv;
         g.part_floats = g.units * g.R * (DH + 2);
@@ -1653,6 +1689,7 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     int rc;
     if (gm.split && gm.tc) rc = launch_tc_nc(a, blocks, s);
     else if (c->type == B200_KV_F16) rc = launch_part_nt<B200_KV_F16>(a, blocks, s);
+    else if (gm.warp) rc = c->type == B200_KV_Q8_0 ? launch_warp<B200_KV_Q8_0, 1>(a, blocks, s) : q_len == 1 ? launch_warp<B200_KV_Q4_0, 1>(a, blocks, s) : launch_warp<B200_KV_Q4_0, 2>(a, blocks, s);
     else if (c->type == B200_KV_Q8_0) rc = launch_part_nt<B200_KV_Q8_0>(a, blocks, s);
     else rc = launch_part_nt<B200_KV_Q4_0>(a, blocks, s);
     if (rc != B200_OK) return rc;
@@ -1744,7 +1781,9 @@ int decode_noalloc_impl(const float * q, const b200_kv_cache * c, float * out, c
     const int chk = decode_check(q, c, out, gate, n_slots, q_len, Hq, who);
     if (chk != B200_OK) return chk;
     dec_geom gm;
-    const bool ok = decode_geometry(gm, c->type, n_slots, q_len, max_n, c->n_ctx, c->Hkv, chunk_keys, tc_eligible(*c, q_len));
+    bool ok = decode_geometry(gm, c->type, n_slots, q_len, max_n, c->n_ctx, c->Hkv, chunk_keys, tc_eligible(*c, q_len));
+    if (ok && gm.warp && gm.part_floats + gm.list_ints > NOALLOC_FLOATS)   // decode_part_k takes fewer runs, and with them partials, of q4_0
+        ok = decode_geometry(gm, c->type, n_slots, q_len, max_n, c->n_ctx, c->Hkv, chunk_keys, false, false, false);
     // fixed chunks need no plan; beyond that the kv heads go in as many groups as the array needs (their partials are independent of one another)
     if (ok && gm.planned && gm.part_floats <= NOALLOC_FLOATS && gm.part_floats + gm.list_ints > NOALLOC_FLOATS) { gm.planned = false; gm.list_ints = 0; }
     const size_t per_head = ok ? gm.part_floats / c->Hkv : 0;
