@@ -155,7 +155,7 @@ def test_allocation_free_call_takes_as_many_slots_as_its_array_ever_held(cuda, l
     q = torch.randn(n, hq, D, device=cuda)
     pos = torch.arange(n, dtype=torch.int32, device=cuda) * 9
     a, b = (torch.full_like(q, float("nan")) for _ in range(2))
-    assert fast.attn_decode_slots_noalloc(q, c, a, None, n, 1, pos, 4096, hq, SCALE, -1)
+    assert fast.attn_decode_slots_noalloc(q, c, a, None, n, 1, pos, 4096, hq, SCALE, -1) == 0
     assert fast.attn_decode_slots(q, c, b, None, n, 1, pos, 4096, hq, SCALE, -1)
     torch.cuda.synchronize()
     assert float((a - b).norm() / b.norm()) < 3 ** 0.5 * 2.0 ** -11
