@@ -23,8 +23,8 @@
 // Batched calls of several slots that let the library choose the split (chunk_keys < 0) cut the batch evenly over the CTAs that fit the GPU
 // (decode_split_k; one plan per model step when the caller declares the step, b200_attn_step_begin).  There q8_0 caches
 // with two to four rows per slot run on a second kernel, decode_tc_k (decode_tc.cuh): tcgen05 MMAs with K in tensor
-// memory and V as an f16 image in shared memory, one CTA per SM.  Everything else, and every fixed-chunk call, runs on
-// the kernel described above.
+// memory and V as an f16 image in shared memory, one CTA per SM (one slot of such rows too); q8_0 with one row per slot and q4_0 with one or
+// two on a third, decode_warp_k (decode_warp.cuh).  Everything else, and every fixed-chunk call, runs on the kernel described above.
 //
 // Reference counterpart: dec2_k / attn_decode2 (src/fast/attn_dec2.cu:210-530), fp32 FFMA on sm_60.
 #include "umma.cuh"
@@ -133,6 +133,7 @@ struct dec_args {
     const int4 * segs;                    // (slot, first key, end key, 0) in CTA order; a run that crosses a slot boundary has several
     const int * cta_seg;                  // [n_cta + 1] first segment of each CTA
     const int2 * slot_seg;                // [n_slots] (first segment, segments) of each slot
+    int solo;                             // > 0: one slot in even runs without a plan (solo_runs), at most so many
     const int * n_cta;                    // CTAs (per kv head) that hold work; < 0: -n_cta segments, CTA c takes c, c + CTAs of the head, ..
 };
 
@@ -143,6 +144,18 @@ __device__ __forceinline__ int key_limit(const dec_args & a) {
     const long long lim = chunk_lo(a.CH, a.max_chunks);
     const int l = (int) (lim < 0x7fffffffLL ? lim : 0x7fffffffLL);
     return a.g.pt ? l : min(l, a.n_ctx);
+}
+
+__device__ __forceinline__ int row_pos(const dec_args & a, int slot, int j);
+
+// One slot in an even split: its 64-key tiles (returned) in `runs` runs per kv head, of two tiles (decode_tc_k walks pairs) where there are so few; run c takes tiles [c W / runs, (c + 1) W / runs).  The
+// decode kernel and the merge find this by themselves: a plan kernel would cost the call 3 us.
+__device__ __forceinline__ int solo_runs(const dec_args & a, int & runs) {
+    int n = 0;
+    for (int j = 0; j < a.q_len; ++j) n = max(n, row_pos(a, 0, j) + 1);
+    const int W = (max(0, min(n, key_limit(a))) + TILE - 1) / TILE;
+    runs = min(a.solo, (W + 1) / 2);
+    return W;
 }
 
 // One tiled copy (TMA unit) of a box of a rank-3 tensor into shared memory, completion counted in bytes on an mbarrier.
@@ -860,7 +873,9 @@ __global__ void __launch_bounds__(64) decode_merge_k(const dec_args a, const flo
     int nch;
     size_t unit0, ustr;
     if constexpr (!CHUNKED) {
-        const int2 sg = a.slot_seg[slot];
+        int2 sg;
+        if (a.solo) { sg.x = 0; solo_runs(a, sg.y); }
+        else sg = a.slot_seg[slot];
         nch = pos < 0 ? 0 : sg.y;
         unit0 = (size_t) sg.x * a.nhk + hl; ustr = a.nhk;
     } else {
@@ -918,7 +933,9 @@ __global__ void __launch_bounds__(MERGE_THR, AHEAD > 4 ? 2 : 4) decode_merge_str
         most = a.max_chunks;
         unit0 = ((size_t) slot * a.nhk + hl) * a.max_chunks; ustr = 1;
     } else {
-        const int2 sg = a.slot_seg[slot];
+        int2 sg;
+        if (a.solo) { sg.x = 0; solo_runs(a, sg.y); }
+        else sg = a.slot_seg[slot];
         most = sg.y;
         unit0 = (size_t) sg.x * a.nhk + hl; ustr = a.nhk;
     }
@@ -1506,7 +1523,7 @@ bool tc_eligible(const b200_kv_cache & c, int q_len) {
     return tc_enabled() && c.type == B200_KV_Q8_0 && q_len >= 2 && cache_tiles(view_of(c), c.n_ctx) && tensor_map_encoder() != nullptr;
 }
 
-template <int NC>
+template <int NC, bool EX>
 int launch_tc(const dec_args & a_in, unsigned blocks, cudaStream_t s) {
     dec_args a = a_in;
     CUtensorMap mapK, mapV;
@@ -1520,17 +1537,18 @@ int launch_tc(const dec_args & a_in, unsigned blocks, cudaStream_t s) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_done[dev & 63].load(std::memory_order_acquire)) {
-        if (cudaFuncSetAttribute(decode_tc_k<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm) != cudaSuccess)
+        if (cudaFuncSetAttribute(decode_tc_k<NC, EX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sm) != cudaSuccess)
             return launch_status("attn_decode (shared memory attribute)");
         attr_done[dev & 63].store(true, std::memory_order_release);
     }
     // a step of few rows is short enough for the gap before the kernel to count
-    if (a.n_slots * a.q_len <= 64) launch(decode_tc_k<NC>, blocks, TC_THR, sm, s, a, mapK, mapV);
-    else decode_tc_k<NC><<<blocks, TC_THR, sm, s>>>(a, mapK, mapV);
+    if (a.n_slots * a.q_len <= 64) launch(decode_tc_k<NC, EX>, blocks, TC_THR, sm, s, a, mapK, mapV);
+    else decode_tc_k<NC, EX><<<blocks, TC_THR, sm, s>>>(a, mapK, mapV);
     return B200_OK;
 }
 int launch_tc_nc(const dec_args & a, unsigned blocks, cudaStream_t s) {
-    return a.q_len <= 2 ? launch_tc<16>(a, blocks, s) : launch_tc<32>(a, blocks, s);
+    if (a.solo) return a.q_len <= 2 ? launch_tc<16, true>(a, blocks, s) : launch_tc<32, true>(a, blocks, s);
+    return a.q_len <= 2 ? launch_tc<16, false>(a, blocks, s) : launch_tc<32, false>(a, blocks, s);
 }
 
 int sm_count() {
@@ -1582,13 +1600,14 @@ int single_grid(int max_n, int Hkv) {
 }
 
 // geometry of a call: chunk, chunks per slot, partial floats, work-list ints
-//   split   (chunk chosen from the batch, two to SPLIT_MAX_SLOTS slots): one contiguous run of tiles per resident CTA
+//   split   (chunk chosen from the batch, two to SPLIT_MAX_SLOTS slots; one slot for decode_tc_k): one contiguous run of tiles per resident CTA
 //   planned (fixed chunks of several slots, more units than a wave): the same runs, cut at chunk boundaries
 //   else    see decode_part_k
 // rows: a call of the row entry points (chunk_keys = 0: the position grid).
-// One slot with chunk_keys < 0 (single_grid) stays on decode_part_k, which keeps K integer times fp32 scale (decode_tc_k rounds q * d to f16), in
-// chunks that are nowhere longer than auto_chunk's: their error is that of their reference maxima.  Against 64-bit attention over the stored rows,
-// q8_0, 4 rows at 30011 keys: 3.5e-4, on decode_tc_k 4.2e-4.
+// One slot with chunk_keys < 0: two to four rows of a q8_0 cache run on decode_tc_k in its exact form (K as integers, references renewed every 256 keys),
+// which is no further from 64-bit attention than chunks of 256 keys on decode_part_k (4 rows, 30011 / 65536 keys: 3.48e-4 / 3.50e-4 against 3.54e-4);
+// 16 layers of 1 + 3 rows at 30011 keys, two heads, 587 -> 443 us, 8 layers at 1500 keys 159 -> 139, at 130000 (four heads) 1029 -> 694.  All else stays on decode_part_k in
+// chunks (single_grid) that are nowhere longer than auto_chunk's.
 //   the plan holds `segs` segments, the runs' or (listed) every chunk
 size_t run_list_ints(size_t segs, int max_cta, int n_slots) { return (4 * segs + 2 * (size_t) n_slots + max_cta + 2 + 3) & ~(size_t) 3; }
 static_assert(SCR_PLAN_INTS >= 4 * (SPLIT_MAX_CTA + PLAN_MAX_SLOTS) + 2 * PLAN_MAX_SLOTS + SPLIT_MAX_CTA + 2 &&
@@ -1606,7 +1625,7 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
     if (max_n < 1) max_n = 1;
     g.tc = g.warp = false;
     g.R = q_len * GQA;
-    g.split = chunk_keys < 0 && n_slots > 1 && n_slots <= SPLIT_MAX_SLOTS;
+    g.split = chunk_keys < 0 && (n_slots > 1 || (tc && type == B200_KV_Q8_0 && q_len >= 2)) && n_slots <= SPLIT_MAX_SLOTS;
     g.planned = false;
     g.max_cta = g.list_cap = 0;
     if (g.split) {
@@ -1619,7 +1638,7 @@ bool decode_geometry(dec_geom & g, uint32_t type, int n_slots, int q_len, int ma
         g.segs = (size_t) g.max_cta + n_slots;
         g.units = g.segs * Hkv;
         g.part_floats = g.units * g.R * (DH + 2);
-        g.list_ints = run_list_ints(g.segs, g.max_cta, n_slots);
+        g.list_ints = n_slots > 1 ? run_list_ints(g.segs, g.max_cta, n_slots) : 0;
         return true;
     }
     g.CH = chunk_keys > 0 ? round_tile(chunk_keys) : chunk_keys < 0 && n_slots > 1 ? auto_chunk((long long) n_slots * max_n / 2, Hkv) :
@@ -1669,10 +1688,12 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     a.n_ctx = c->n_ctx; a.tiled = 0;
     a.chunked = gm.split ? 0 : 1;
     a.segs = nullptr; a.cta_seg = nullptr; a.slot_seg = nullptr; a.n_cta = nullptr;
+    a.solo = gm.split && n_slots == 1 ? gm.max_cta : 0;
     int launches = 2;
     // fixed chunks without a plan: at most one wave of CTAs, a multiple of the heads
     unsigned blocks = (unsigned) std::min<size_t>((size_t) n_slots * gm.max_chunks, (size_t) gm.max_cta) * (unsigned) a.nhk;
-    if (gm.split || gm.planned) {
+    if (a.solo) blocks = (unsigned) gm.max_cta * (unsigned) a.nhk;
+    else if (gm.split || gm.planned) {
         if (!list) list = reinterpret_cast<int *>(scr + part_floats);
         int4 * segs = reinterpret_cast<int4 *>(list);
         int2 * slot_seg = reinterpret_cast<int2 *>(list + 4 * gm.segs);
@@ -1728,7 +1749,7 @@ int decode_impl(const float * q, const b200_kv_cache * c, const merge_out & mo, 
     k.max_cta = gm.max_cta; k.Hkv = c->Hkv; k.n_ctx = c->n_ctx; k.paged = c->pt != nullptr; k.part_floats = gm.part_floats;
     k.list_cap = gm.list_cap; k.split = gm.split; k.tc = gm.tc;
     const bool in_step = e->step_mode && pos && (const char *) pos >= e->step_lo && (const char *) pos < e->step_hi;
-    const bool listed = gm.split || gm.planned;
+    const bool listed = (gm.split && n_slots > 1) || gm.planned;
     const bool known = !listed || recording_of(s, k.rec);
     const bool reuse = listed && in_step && known && e->plan_valid && k == e->key;
     int * list = reinterpret_cast<int *>(e->p) + (!known || k.rec ? SCR_PLAN_INTS : 0);
@@ -1882,6 +1903,7 @@ int b200_attn_reserve(uint32_t kv_type, int max_slots, int q_len, int max_n, int
             if (decode_geometry(g1, kv_type, 1, q_len, n1, n1, Hkv, -1)) need = std::max(need, g1.part_floats);
         }
     if (chunk_keys < 0 && max_slots == 1 && decode_geometry(g1, kv_type, 1, q_len, max_n, max_n, Hkv, -1)) need = std::max(need, g1.part_floats);
+    if (chunk_keys < 0 && kv_type == B200_KV_Q8_0 && q_len >= 2 && decode_geometry(g1, kv_type, 1, q_len, max_n, max_n, Hkv, -1, true)) need = std::max(need, g1.part_floats);
     if (chunk_keys < 0 && max_slots > 1 && !gm.split) {
         // a fixed chunk chosen from the batch: smaller batches take smaller chunks; their unit count stays under this bound
         const size_t u = 2 * 8 * (size_t) sm_count() + (size_t) max_slots * Hkv;

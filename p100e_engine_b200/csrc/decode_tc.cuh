@@ -23,20 +23,31 @@
 // of the instruction stream: what the CUDA cores still do is the widening of 2 x 128 x 256 cache values per tile (seven
 // instructions per four values) and 128 x rows exponentials.
 //
+// EX, for one slot, whose results are to be as close to 64-bit attention as those of the mma.sync kernel: K enters as its integers (f16 subnormals, a
+// mask or a byte permute per pair) and each block of 32 dims has a score accumulator of its own, which the workers multiply with the block's
+// scale in fp32; the offset of the integers comes out through one more product, of the block scales with the block sums of Q.  Tensor memory then
+// holds one buffer of K (128 columns) and of S^T (8 x 32 + 32), so the scores are read before K of the next tile is written.  And the reference
+// maxima move to the tile's maximum every 256 keys: the largest P of a stretch is then a power of two, which f16 holds exactly.  Relative error
+// at 65536 keys, 4 rows: 3.58e-4 without the renewal, 3.50e-4 with it, chunks of 256 keys on the mma.sync kernel 3.54e-4; K rounded 4.1e-4.  On
+// batches the exact form is slower (8 x 4 rows 342 -> 374 us, 64 x 4 rows 2010 -> 2199): the double buffers are worth more there.
+//
 // Every wait is bounded (mbar_wait gives up after two seconds and records ST_WAIT_TIMEOUT).
 
 constexpr int UT = 128;                       // keys per tile
 constexpr int TC_WORKERS = 512, TC_THR = TC_WORKERS + 64;   // 16 worker warps, the MMA warp, the TMA warp
 constexpr int TC_NBUF = 4;                    // staging ring, in the order the workers consume: K0, K1, V0, K2, V1, ..
-constexpr int TC_HDR = 2048;                  // barriers, reference maxima, exchange arrays, page entries
-constexpr int TC_PGS = 224;                   // page-table entries of a run kept in shared memory
+constexpr int TC_HDR = 1536;                  // barriers, reference maxima, exchange arrays, page entries
+constexpr int TC_PGS = 64;                    // page-table entries of a run kept in shared memory
 constexpr int TC_VF = UT * DH * 2;            // f16 image of a tile's V rows
 constexpr int TC_QI = 32 * 32 * 16;           // f16 image of up to 32 query rows
 constexpr int TC_PLBO = 528;                  // bytes between the 8-key chunks of the P image (512 + 16: stores of a warp spread over the banks)
 constexpr int TC_PI = 8704;                   // P image: 16 chunks of up to 32 rows
+constexpr int TC_REREF = 2;                   // EX: tiles between two renewals of the reference maxima
+constexpr int TC_QB = 2 * 32 * 16;            // block sums of Q (EX): 16 values of up to 32 rows
 
 constexpr int TC_HB = head_bytes(B200_KV_Q8_0);   // the kernel serves q8_0 rows: 8 f16 block scales, then 256 int8
-constexpr size_t tc_smem_bytes() { return TC_HDR + (size_t) TC_NBUF * UT * TC_HB + TC_VF + TC_QI + TC_PI; }
+constexpr size_t tc_smem_bytes() { return TC_HDR + (size_t) TC_NBUF * UT * TC_HB + TC_VF + TC_QI + TC_PI + TC_QB; }
+static_assert(tc_smem_bytes() <= 227 * 1024, "decode_tc_k shared memory");
 
 __device__ __forceinline__ void tc_arrive(uint64_t * bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -73,7 +84,7 @@ __device__ __forceinline__ void tc_block(const unsigned char * row, int blk, uin
 
 // NC = score columns (16 for up to two verify rows, 32 for up to four): column 8 j + h = verify row j, head h of the group
 // (h < 6); columns with h = 6, 7 are padding (zero query rows).
-template <int NC>
+template <int NC, bool EX>
 __global__ void __launch_bounds__(TC_THR, 1)
 decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV) {
     pdl_enter();
@@ -84,9 +95,19 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
     const bool worker = w < TC_WORKERS / 32;
     const int lq = w & 3, gq = (w >> 2) & 3;     // worker warp: tensor-memory lane quarter, column / block group
     const int hk = (int) (blockIdx.x % (unsigned) a.g.Hkv), ui = (int) (blockIdx.x / (unsigned) a.g.Hkv);
-    if (ui >= *a.n_cta) return;
-    const int s0 = a.cta_seg[ui], s1 = a.cta_seg[ui + 1];
-    if (s0 >= s1) return;
+    int s0, s1;
+    int4 one = make_int4(0, 0, 0, 0);
+    if constexpr (EX) {
+        int runs;
+        const long long W = solo_runs(a, runs);
+        if (ui >= runs) return;
+        one.y = (int) (W * ui / runs) * TILE; one.z = (int) (W * (ui + 1) / runs) * TILE;
+        s0 = ui; s1 = ui + 1;
+    } else {
+        if (ui >= *a.n_cta) return;
+        s0 = a.cta_seg[ui]; s1 = a.cta_seg[ui + 1];
+        if (s0 >= s1) return;
+    }
 
     uint64_t * full = reinterpret_cast<uint64_t *>(smem);                       // [TC_NBUF] staging buffer filled
     uint64_t * s_full = full + 4;                                                // [2] Q K^T of a tile has landed in S^T buffer b
@@ -100,7 +121,8 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
     float * wx = reinterpret_cast<float *>(smem + 384);                          // [4][32] per lane quarter: maxima / sums
     float2 * mm = reinterpret_cast<float2 *>(smem + 896);                        // [32] (reference + REF_GAP, finite reference - PSHIFT)
     int * pgs = reinterpret_cast<int *>(smem + 1152);                            // [TC_PGS]
-    unsigned char * stg = smem + TC_HDR, * VF = stg + TC_NBUF * BUF, * QI = VF + TC_VF, * PI = QI + TC_QI;
+    float * mtop = reinterpret_cast<float *>(smem + 1152 + 4 * TC_PGS);          // [32] EX: largest reference so far
+    unsigned char * stg = smem + TC_HDR, * VF = stg + TC_NBUF * BUF, * QI = VF + TC_VF, * PI = QI + TC_QI, * QBI = PI + TC_PI;
 
     if (tid == 0) {
         for (int b = 0; b < TC_NBUF; ++b) mbar_init(&full[b], 1);
@@ -117,7 +139,8 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
     umma::fence_after_sync();
     const uint32_t tb = *tbase_p;
     // tensor memory: K as f16 pairs (2 x 128 columns), S^T (2 x 32), O^T (two halves of 128 dims, NC columns each)
-    const uint32_t tA = tb, tS = tb + 256, tO = tb + 320;
+    // EX: K as integers (128 columns), S^T of each block (8 x NC), the offsets' part of S^T (NC), O^T, the block scales as f16 pairs (8)
+    const uint32_t tA = tb, tS = tb + (EX ? 128 : 256), tC = tS + 8 * NC, tO = EX ? tC + NC : tb + 320, tD = tO + 2 * NC;
     const uint32_t lane_off = (uint32_t) (32 * lq) << 16;
     const int R = a.q_len * GQA;
     // the O^T columns this worker warp rescales and writes out: half hO of the dims, columns 16 cO .. 16 cO + 15
@@ -126,7 +149,7 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
 
     int g = 0;   // tiles this CTA has walked (parities of the per-tile barriers); 2 g = staging items before the run
     for (int sg = s0; sg < s1; ++sg) {
-        const int4 seg = a.segs[sg];
+        const int4 seg = EX ? one : a.segs[sg];
         const int slot = seg.x, k_lo = seg.y;
         const size_t unit = (size_t) sg * a.g.Hkv + hk;
         int n_slot = 0;
@@ -183,12 +206,37 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                 if (hh < GQA && grp < a.q_len) {
                     const float4 * src = reinterpret_cast<const float4 *>(a.q + ((size_t) (slot * a.q_len + grp) * a.Hq + hk * GQA + hh) * DH + kc * 8);
                     const float4 v0 = src[0], v1 = src[1];
-                    pk = make_uint4(pack_h2(v0.x * a.qscale, v0.y * a.qscale), pack_h2(v0.z * a.qscale, v0.w * a.qscale),
-                                    pack_h2(v1.x * a.qscale, v1.y * a.qscale), pack_h2(v1.z * a.qscale, v1.w * a.qscale));
+                    if constexpr (EX)   // the order in which a word of four cache bytes splits into pairs (k_store)
+                        pk = make_uint4(pack_h2(v0.x * a.qscale, v0.z * a.qscale), pack_h2(v0.y * a.qscale, v0.w * a.qscale),
+                                        pack_h2(v1.x * a.qscale, v1.z * a.qscale), pack_h2(v1.y * a.qscale, v1.w * a.qscale));
+                    else
+                        pk = make_uint4(pack_h2(v0.x * a.qscale, v0.y * a.qscale), pack_h2(v0.z * a.qscale, v0.w * a.qscale),
+                                        pack_h2(v1.x * a.qscale, v1.y * a.qscale), pack_h2(v1.z * a.qscale, v1.w * a.qscale));
                 }
                 *reinterpret_cast<uint4 *>(QI + grp * 128 + kc * (NC * 16) + hh * 16) = pk;
             }
-            if (tid < 32) { mref[tid] = B200_NEG_INF; mm[tid] = make_float2(B200_NEG_INF, -PSHIFT); }
+            if (tid < 32) { mref[tid] = mtop[tid] = B200_NEG_INF; mm[tid] = make_float2(B200_NEG_INF, -PSHIFT); }
+            if constexpr (EX) {
+                // -1/32 of the sum of a block's 32 query values (finite whatever they are), as f16 and what f16 leaves of it: value b and b + 8 of row n of
+                // the K-major B operand of the offsets' product, [d, d] (A, tensor memory) * this * 4096
+                tc_bar_workers();
+                for (int i = tid; i < 8 * NC; i += TC_WORKERS) {
+                    const int n = i & (NC - 1), b = i / NC;
+                    float sum = 0.0f;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint4 x = *reinterpret_cast<const uint4 *>(QI + (n >> 3) * 128 + (4 * b + c) * (NC * 16) + (n & 7) * 16);
+                        const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) { const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&xw[e])); sum += f.x + f.y; }
+                    }
+                    const float y = -0.03125f * sum;
+                    const __half hi = __float2half_rn(y), lo = __float2half_rn(y - __half2float(hi));
+                    unsigned char * dst = QBI + (n >> 3) * 128 + (n & 7) * 16 + b * 2;
+                    *reinterpret_cast<__half *>(dst) = hi;
+                    *reinterpret_cast<__half *>(dst + NC * 16) = lo;
+                }
+            }
             umma::fence_async_smem();
         }
         __syncthreads();
@@ -203,7 +251,7 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
             const int nt_u = __shfl_sync(0xffffffffu, nt, 0), g_u = __shfl_sync(0xffffffffu, g, 0);
             if (w == TC_WORKERS / 32) {
                 const uint32_t tb_u = __shfl_sync(0xffffffffu, tb, 0);
-                const uint32_t tA_u = tb_u, tS_u = tb_u + 256, tO_u = tb_u + 320;
+                const uint32_t tA_u = tb_u, tS_u = tb_u + (EX ? 128 : 256), tC_u = tS_u + 8 * NC, tO_u = EX ? tC_u + NC : tb_u + 320, tD_u = tO_u + 2 * NC;
                 constexpr uint32_t id_qk = umma::idesc_f16(UT, NC, false, false);   // S^T[128 x NC] = K (tensor memory) * Q^T (K-major)
                 constexpr uint32_t id_pv = umma::idesc_f16(UT, NC, true, false);    // O^T[128 x NC] += V^T (MN-major) * P^T (K-major)
                 const uint32_t q_s = smem_u32(QI), p_s = smem_u32(PI), v_s = smem_u32(VF);
@@ -214,7 +262,9 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                     if (lead) {
 #pragma unroll
                         for (int ks = 0; ks < DH / 16; ++ks)
-                            umma::mma_ts(tS_u + 32 * b, tA_u + 128 * b + ks * 8, umma::smem_desc(q_s + ks * 2 * (NC * 16), NC * 16, 128), id_qk, ks > 0);
+                            umma::mma_ts(EX ? tS_u + (ks >> 1) * NC : tS_u + 32 * b, tA_u + (EX ? 0 : 128 * b) + ks * 8,
+                                         umma::smem_desc(q_s + ks * 2 * (NC * 16), NC * 16, 128), id_qk, EX ? ks & 1 : ks > 0);
+                        if constexpr (EX) umma::mma_ts(tC_u, tD_u, umma::smem_desc(smem_u32(QBI), NC * 16, 128), id_qk, 0u);
                         umma::commit(&s_full[b]);
                     }
                 };
@@ -263,11 +313,36 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
 
             // K rows of a tile -> tensor-memory buffer tb_k (lane = key; this warp: blocks 2 gq, 2 gq + 1 of keys 32 lq ..).
             // The stores are left in flight: k_publish waits for them and tells the issuers.
+            uint4 dk = make_uint4(0, 0, 0, 0), dk_next = dk;   // EX: block scales of this thread's key, of the tile whose scores come next and of the one after
             auto k_store = [&](int G) {
                 const int buf = cons & (TC_NBUF - 1);
                 tc_wait(&full[buf], (uint32_t) ((cons >> 2) & 1), a.status, 2);
                 ++cons;
                 const unsigned char * row = krow0 + buf * BUF;
+                if constexpr (EX) {
+                    // the integers as f16 subnormals u * 2^-24, u = q + 128: a mask or a byte permute per pair
+                    dk_next = *reinterpret_cast<const uint4 *>(row);
+#pragma unroll
+                    for (int bb = 0; bb < 2; ++bb) {
+                        uint32_t r[16];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint4 x = *reinterpret_cast<const uint4 *>(row + 16 + 32 * (2 * gq + bb) + 16 * h);
+                            const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                r[8 * h + 2 * j] = (xw[j] & 0x00ff00ffu) ^ 0x00800080u;
+                                r[8 * h + 2 * j + 1] = (xw[j] >> 8 & 0x00ff00ffu) ^ 0x00800080u;
+                            }
+                        }
+                        umma::tmem_st16(tA + lane_off + (2 * gq + bb) * 16, r);
+                    }
+                    if (gq == 0) {
+                        const uint32_t r[8] = {dk_next.x, dk_next.y, dk_next.z, dk_next.w, dk_next.x, dk_next.y, dk_next.z, dk_next.w};
+                        umma::tmem_st8(tD + lane_off, r);
+                    }
+                    return;
+                }
                 const uint32_t sc2 = *reinterpret_cast<const uint32_t *>(row + 4 * gq);   // the two blocks' scales
 #pragma unroll
                 for (int bb = 0; bb < 2; ++bb) {
@@ -287,12 +362,38 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
             k_publish(g);
             for (int i = 0; i < nt; ++i) {
                 const int G = g + i, p_t = k_lo + i * UT;
-                if (i + 1 < nt) k_store(G + 1);
+                if (!EX && i + 1 < nt) k_store(G + 1);
                 // ---- this tile's scores: the load from tensor memory flies during the V phase
                 tc_wait(&s_full[G & 1], (uint32_t) ((G >> 1) & 1), a.status, 5);
                 umma::fence_after_sync();
                 uint32_t sr[8];
-                if (act) umma::tmem_ld8(tS + 32 * (G & 1) + lane_off + 8 * gq, sr);
+                if constexpr (!EX) { if (act) umma::tmem_ld8(tS + 32 * (G & 1) + lane_off + 8 * gq, sr); }
+                else {
+                    // s = 2^24 * sum over blocks of d * (K integers . Q) + the offsets' part; then K and S in tensor memory are free for the next tile
+                    dk = dk_next;
+                    if (act) {
+                        float acc[GQA];
+                        const uint32_t dw[4] = {dk.x, dk.y, dk.z, dk.w};
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            uint32_t c[4][8];
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) umma::tmem_ld8(tS + NC * (4 * h + b) + lane_off + 8 * gq, c[b]);
+                            if (h == 0) umma::tmem_ld8(tC + lane_off + 8 * gq, sr);
+                            umma::tmem_ld_wait();
+#pragma unroll
+                            for (int b = 0; b < 4; ++b) {
+                                const float2 d2 = __half22float2(*reinterpret_cast<const __half2 *>(&dw[2 * h + (b >> 1)]));
+                                const float d = (b & 1 ? d2.y : d2.x) * 16777216.0f;
+#pragma unroll
+                                for (int e = 0; e < GQA; ++e) acc[e] = fmaf(d, __uint_as_float(c[b][e]), h == 0 && b == 0 ? 4096.0f * __uint_as_float(sr[e]) : acc[e]);
+                            }
+                        }
+#pragma unroll
+                        for (int e = 0; e < GQA; ++e) sr[e] = __float_as_uint(acc[e]);
+                    }
+                    if (i + 1 < nt) k_store(G + 1);
+                }
                 // ---- V rows -> f16 image, MN-major: byte(key, d) = (d / 8) * 128 + (key / 8) * 4096 + (key % 8) * 16 + (d % 8) * 2
                 {
                     const int buf = cons & (TC_NBUF - 1);
@@ -316,7 +417,7 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                 float s[GQA], ofs[GQA];
                 int grow = 0;
                 if (act) {
-                    umma::tmem_ld_wait();
+                    if constexpr (!EX) umma::tmem_ld_wait();
                     const float4 m0 = mm4[0], m1 = mm4[1], m2 = mm4[2];
                     const float gap[GQA] = {m0.x, m0.z, m1.x, m1.z, m2.x, m2.z};
                     ofs[0] = m0.y; ofs[1] = m0.w; ofs[2] = m1.y; ofs[3] = m1.w; ofs[4] = m2.y; ofs[5] = m2.w;
@@ -336,8 +437,10 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                     for (int e = 0; e < GQA; ++e) { s[e] = B200_NEG_INF; ofs[e] = 0.0f; }
                 }
                 // A column's reference maximum trails its true maximum by at most REF_GAP; it moves (and O, l are rescaled)
-                // only when some key of the tile outgrows it, which the workers find out with one vote per tile.
-                if (tc_vote_workers(grow)) {
+                // only when some key of the tile outgrows it, which the workers find out with one vote per tile.  EX: every TC_REREF tiles also to
+                // a lower maximum, as long as that is within REF_GAP of the largest reference so far.
+                const bool again = EX && i > 0 && i % TC_REREF == 0;
+                if (tc_vote_workers(grow | again)) {
                     if (act) {
 #pragma unroll
                         for (int e = 0; e < GQA; ++e) {
@@ -353,9 +456,10 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                         if ((tid >> 3) < a.q_len && (tid & 7) < GQA) {
                             const float mx = fmaxf(fmaxf(wx[tid], wx[32 + tid]), fmaxf(wx[64 + tid], wx[96 + tid]));
                             const float m_old = mref[tid];
-                            if (mx > m_old + REF_GAP) {   // mx is finite here
+                            if (mx > m_old + REF_GAP || (again && mx >= mtop[tid] - REF_GAP && mx > B200_NEG_INF)) {   // mx is finite here
                                 f = ex2f(m_old - mx);     // 2^(-inf) = 0 on the first move
                                 mref[tid] = mx;
+                                mtop[tid] = fmaxf(mtop[tid], mx);
                                 mm[tid] = make_float2(mx + REF_GAP, mx - PSHIFT);
                             }
                         }

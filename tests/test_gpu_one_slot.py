@@ -117,3 +117,39 @@ def test_one_slot_after_a_reservation(cuda, lib, hkv):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, w), n
+
+
+@pytest.mark.parametrize("q_len", [2, 4])
+@pytest.mark.parametrize("n", [128, 129, 300, 2049, 20011])
+@pytest.mark.parametrize("trend", ["rising", "falling", "one peak", "large q"])
+def test_one_slot_verify_with_scores_that_drift(cuda, lib, q_len, n, trend):
+    """scores whose maxima move by hundreds over the context, up, down, or at one key only, and query sums beyond f16 times 128: the reference maxima of
+    the exact verify form follow without leaving f16 and fp32"""
+    import torch
+    from p100e_engine_b200 import fast
+    c = fast.kv_alloc(TYPES["q8_0"], n, HKV, D)
+    g = torch.Generator(device="cuda").manual_seed(n + q_len)
+    rn = lambda *s: torch.randn(*s, generator=g, device=cuda)
+    k, q = rn(n, HKV, D), rn(q_len, HQ, D)
+    along = q[0, ::6][None] / 16.0        # a direction that the first head of each group sees
+    ramp = torch.linspace(0.0, 40.0, n, device=cuda)[:, None, None]
+    if trend == "rising":
+        k += ramp * along
+    elif trend == "falling":
+        k += (40.0 - ramp) * along
+    elif trend == "one peak":
+        k[n // 2] += 60.0 * along[0]
+    else:
+        q = q * 40.0 + 300.0
+    assert fast.kv_append(c, k, rn(n, HKV, D), 0, n)
+    pos = torch.arange(n - q_len, n, dtype=torch.int32, device=cuda)
+    one, fixed = (torch.full((q_len, HQ, D), float("nan"), device=cuda) for _ in range(2))
+    assert fast.attn_decode_slots(q, c, one, None, 1, q_len, pos, n, HQ, SCALE, -1)
+    assert fast.attn_decode_slots(q, c, fixed, None, 1, q_len, pos, n, HQ, SCALE, 256)
+    torch.cuda.synchronize()
+    assert fast.device_status() == 0
+    ref = _attention64(q, c, "q8_0", n, n - q_len)
+    err = [float((o.double() - ref).norm() / ref.norm()) for o in (one, fixed)]
+    print("%s n=%d q_len=%d: one slot %.3e, chunks of 256 %.3e" % (trend, n, q_len, *err))
+    # the rounding of Q to f16 (2^-12 rms of scores of up to some hundreds) is common to both; beyond it three roundings of 2^-12 rms
+    assert err[0] <= 1.05 * err[1] + 3 ** 0.5 * 2.0 ** -12
