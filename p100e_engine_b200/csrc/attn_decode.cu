@@ -133,6 +133,7 @@ struct dec_args {
     const int4 * segs;                    // (slot, first key, end key, 0) in CTA order; a run that crosses a slot boundary has several
     const int * cta_seg;                  // [n_cta + 1] first segment of each CTA
     const int2 * slot_seg;                // [n_slots] (first segment, segments) of each slot
+    int max_cta;                          // runs per kv head that a plan may hold
     int solo;                             // > 0: one slot in even runs without a plan (solo_runs), at most so many
     const int * n_cta;                    // CTAs (per kv head) that hold work; < 0: -n_cta segments, CTA c takes c, c + CTAs of the head, ..
 };
@@ -190,19 +191,30 @@ __device__ __forceinline__ void tma_box4(void * dst, const CUtensorMap * map, in
 // unit + 1, ..: sums and references start afresh at every chunk, so a chunk's bits do not depend on where a unit begins or
 // ends. Called by all threads of the CTA.  A CTA that runs several units keeps its ring of copy slots, their barriers and the
 // arrival counters going from one unit to the next: tiles_before is the number of tiles its earlier units walked (two ring
-// items each); the function returns this unit's tile count. t_base: tensor-memory base of the parked accumulators.
+// items each); the function returns this unit's tile count. t_slot: where the tensor-memory base of the parked accumulators is written.
 template <uint32_t KT, int NT, bool RUNS>
 __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, const CUtensorMap & mapK, const CUtensorMap & mapV,
                                            unsigned char * smem, const int hk, const int slot, const int k_lo, const int k_cap,
-                                           unsigned unit, const int tiles_before, const uint32_t t_base) {
+                                           unsigned unit, const int tiles_before, const uint32_t * t_slot) {
     using TR = traits<KT>;
     constexpr int HB = TR::HB, SROW = TR::SROW;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
     const int R = a.q_len * GQA;
 
+    // What the unit reads before its first copy is asked for at once, the positions (lane j: row j), the query rows (this thread's share, in
+    // registers) and the place of the page table; the start of a unit is a chain of such loads, and with one tile per CTA most of the kernel's time.
+    const int posv = lane < a.q_len ? row_pos(a, slot, lane) : -1;
+    const int rt = a.g.pt && a.g.rtab ? a.g.rtab[slot * a.q_len] : 0;
+    constexpr int QN = NT * 8 * (DH / 4) / NTHR;
+    float4 qv[QN];
+#pragma unroll
+    for (int k = 0; k < QN; ++k) {
+        const int i = tid + k * NTHR, r = i / (DH / 4), d4 = (i - r * (DH / 4)) * 4, j = r / GQA, hh = r - j * GQA;
+        qv[k] = r < R ? *reinterpret_cast<const float4 *>(a.q + ((size_t) (slot * a.q_len + j) * a.Hq + hk * GQA + hh) * DH + d4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
     // visible keys of the slot = 1 + the largest row position
-    int n_slot = 0;
-    for (int j = 0; j < a.q_len; ++j) n_slot = max(n_slot, row_pos(a, slot, j) + 1);
+    int n_slot = __reduce_max_sync(0xffffffffu, posv) + 1;
+    const int rmin = __reduce_min_sync(0xffffffffu, lane < a.q_len ? posv : 0x7fffffff);
     {
         const int lim = key_limit(a);
         if (n_slot > lim) { if (tid == 0) atomicOr(a.status, ST_BAD_POS); n_slot = lim; }
@@ -226,7 +238,7 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
     float * wl = wmax + NWARP * NT * 8;                                      // [NWARP][NT*8]
     float4 * Qb = reinterpret_cast<float4 *>(wl + NWARP * NT * 8);           // [NBLK][NT][4] block sums of Q (quantised caches)
 
-    const int32_t * tab = a.g.pt ? a.g.pt + (a.g.rtab ? a.g.rtab[slot * a.q_len] : 0) : nullptr;
+    const int32_t * tab = a.g.pt ? a.g.pt + rt : nullptr;
     const unsigned long long hoff = (unsigned long long) hk * HB;
     // the chunk's page-table entries are staged in shared memory when there are at most PGS of them, so that a refill does
     // not wait for a global load
@@ -241,8 +253,11 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
     // enters P V as zeros.  One warp moving that tile row by row held its CTA for 30 us (q8_0) to 60 us (f16), longer than everything
     // else in a call of 30011 keys (50.2 us in all).  Caches without a tensor map (small pages) are still moved that way, rows past the slot's
     // last key replaced by that key.
-    auto page_of = [&](int p, bool first) { return pg_staged && !first ? pgs[(p >> a.g.psh) - pg0] : tab[p >> a.g.psh]; };
+    // page entries of the first copies: lane q that of item q
+    const int pg_first = w == 0 && tab && lane < nslot && lane < 2 * ntiles ? tab[(k_lo + (lane >> 1) * TILE) >> a.g.psh] : 0;
+    auto page_of = [&](int p) { return pg_staged ? pgs[(p >> a.g.psh) - pg0] : tab[p >> a.g.psh]; };
     auto issue = [&](int q, int s, bool first) {   // s = q mod nslot; called by one whole warp
+        const int zf = first ? __shfl_sync(0xffffffffu, pg_first, q) : 0;
         if (q >= 2 * ntiles) return;
         const int it = q >> 1;
         unsigned char * dst = stg + (size_t) s * TR::SLOT;
@@ -252,7 +267,7 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
             if (lane == 0) {
                 int y = p_t, z = 0;
                 if (tab) {
-                    z = page_of(p_t, first);
+                    z = first ? zf : page_of(p_t);
                     y = p_t & ((1 << a.g.psh) - 1);
                     if (z < 0) { atomicOr(a.status, ST_BAD_PAGE); z = 0; }
                 }
@@ -271,7 +286,7 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
             const int p = min(p_t + row, n_slot - 1);
             unsigned long long off;
             if (tab) {
-                const int pg = page_of(p, first);
+                const int pg = first ? tab[p >> a.g.psh] : page_of(p);
                 if (pg < 0) { atomicOr(a.status, ST_BAD_PAGE); off = 0; }
                 else off = (unsigned long long) pg * a.g.pstride + (unsigned long long) (p & ((1 << a.g.psh) - 1)) * a.g.rowb;
             } else off = (unsigned long long) p * a.g.rowb;
@@ -296,38 +311,38 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
     // Q rows -> shared memory as f16, scaled; row r = j * 6 + hh (verify row j, head hh of the group).  For the quantised
     // caches the middle two of every four dims are swapped (d0 d2 d1 d3): a 32-bit word of cache bytes then splits into the
     // f16 pairs (byte 0, byte 2) and (byte 1, byte 3) with one mask and one byte permute (see the Q K^T loop).
-    for (int i = tid; i < NT * 8 * (DH / 4); i += NTHR) {
-        const int r = i / (DH / 4), d4 = (i - r * (DH / 4)) * 4;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (r < R) {
-            const int j = r / GQA, hh = r - j * GQA;
-            v = *reinterpret_cast<const float4 *>(a.q + ((size_t) (slot * a.q_len + j) * a.Hq + hk * GQA + hh) * DH + d4);
-        }
+    // The cache integers enter the tensor cores as f16 subnormals u * 2^-24 with u = q + 128 (q8_0) or the nibble itself
+    // (q4_0, value = nibble - 8).  The offset is taken out again through the accumulator's starting value: for block b and
+    // row r it is -OFFS * 2^-24 * (sum of the block's 32 scaled f16 query values, which eight neighbouring lanes hold), kept per (block, row tile,
+    // lane quad position) in the order of an accumulator fragment {row 2t, row 2t+1, row 2t, row 2t+1}.
+#pragma unroll
+    for (int k = 0; k < QN; ++k) {
+        const int i = tid + k * NTHR, r = i / (DH / 4), d4 = (i - r * (DH / 4)) * 4;
+        const float4 v = qv[k];
         // four consecutive dims stay together under q_slot (it permutes groups of four): one 8-byte store
         uint2 pk;
         if constexpr (TR::SCALED) pk = make_uint2(pack_h2(v.x * a.qscale, v.z * a.qscale), pack_h2(v.y * a.qscale, v.w * a.qscale));
         else pk = make_uint2(pack_h2(v.x * a.qscale, v.y * a.qscale), pack_h2(v.z * a.qscale, v.w * a.qscale));
         *reinterpret_cast<uint2 *>(Qs + r * QSTR + q_slot<KT>(d4) * 2) = pk;
-    }
-    __syncthreads();
-    if constexpr (TR::SCALED) {
-        // The cache integers enter the tensor cores as f16 subnormals u * 2^-24 with u = q + 128 (q8_0) or the nibble itself
-        // (q4_0, value = nibble - 8).  The offset is taken out again through the accumulator's starting value: for block b and
-        // row r it is -OFFS * 2^-24 * (sum of the block's 32 scaled f16 query values), kept per (block, row tile, lane quad
-        // position) in the order of an accumulator fragment {row 2t, row 2t+1, row 2t, row 2t+1}.
-        constexpr float OFFS = KT == B200_KV_Q8_0 ? 128.0f : 8.0f;
-        for (int i = tid; i < NBLK * NT * 8; i += NTHR) {
-            const int b = i / (NT * 8), r = i - b * (NT * 8);
-            const __half2 * src = reinterpret_cast<const __half2 *>(Qs + r * QSTR + b * 64);   // a block's dims stay inside its 64 bytes
-            float sum = 0.0f;
-#pragma unroll
-            for (int e = 0; e < 16; ++e) { const float2 f = __half22float2(src[e]); sum += f.x + f.y; }
-            const float v = -OFFS * 5.9604644775390625e-8f * sum;
-            float * dst = reinterpret_cast<float *>(Qb + (b * NT + (r >> 3)) * 4 + ((r & 7) >> 1));
-            dst[r & 1] = v; dst[2 + (r & 1)] = v;
+        if constexpr (TR::SCALED) {
+            constexpr float OFFS = KT == B200_KV_Q8_0 ? 128.0f : 8.0f;
+            const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&pk.x)), hi = __half22float2(*reinterpret_cast<const __half2 *>(&pk.y));
+            float sum = (lo.x + lo.y) + (hi.x + hi.y);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+            if ((lane & 7) == 0) {
+                const int b = d4 >> 5;
+                const float x = -OFFS * 5.9604644775390625e-8f * sum;
+                float * dst = reinterpret_cast<float *>(Qb + (b * NT + (r >> 3)) * 4 + ((r & 7) >> 1));
+                dst[r & 1] = x; dst[2 + (r & 1)] = x;
+            }
         }
     }
+    if constexpr (parks<KT, NT>()) umma::fence_before_sync();
     __syncthreads();
+    if constexpr (parks<KT, NT>()) umma::fence_after_sync();
+    const uint32_t t_base = parks<KT, NT>() ? *t_slot : 0u;
 
     // arrive(c): this warp is done with the K (c = 0) or V (c = 1) item of the tile; lane 0 learns whether it was the last of
     // the four warps.  refill_if_last: that warp refills the slot.  The two are apart in the instruction stream so that the
@@ -350,7 +365,8 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int r = 8 * i + 2 * t + e;
-            rpos[i][e] = r < R ? row_pos(a, slot, r / GQA) : -1;
+            const int pr = __shfl_sync(0xffffffffu, posv, min(r / GQA, 31));
+            rpos[i][e] = r < R ? pr : -1;
             m_run[i][e] = B200_NEG_INF;
             l_run[i][e] = 0.0f;
         }
@@ -391,9 +407,7 @@ __device__ __forceinline__ int decode_unit(const dec_args & a, const int nslot, 
     }
 
     const int kA = 16 * w + key_perm<KT>(g), kB = kA + 8;   // this lane's two keys (tile-relative) in the QK phase
-    int rmin = 0x7fffffff;   // the mask is only evaluated in tiles that reach past some row's last key or the chunk's end
-    for (int j = 0; j < a.q_len; ++j) rmin = min(rmin, row_pos(a, slot, j));
-    const int mask_from = min(k_hi, rmin + 1);
+    const int mask_from = min(k_hi, rmin + 1);   // the mask is only evaluated in tiles that reach past some row's last key or the chunk's end
 
     // writes partial `unit` from the accumulators
     auto flush = [&]() {
@@ -763,18 +777,19 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
     // head rows of a position are fetched close together in time
     const int hl = (int) (blockIdx.x % (unsigned) a.nhk), ui = (int) (blockIdx.x / (unsigned) a.nhk);
     int s0, s1, nch = a.max_chunks, step = (int) (gridDim.x / (unsigned) a.nhk);
+    const bool one_wave = (long long) a.max_chunks * a.n_slots <= step;   // no CTA has two chunks: their order does not matter, nor who has how many
     if (a.segs) {
-        const int n = *a.n_cta;
+        const int c = min(ui, a.max_cta - 1), n = *a.n_cta, c0 = a.cta_seg[c], c1 = a.cta_seg[c + 1];   // loads that do not wait for one another
         if (RUNS && n < 0) { s0 = ui; s1 = -n; }
         else {
             if (ui >= n) return;
-            s0 = a.cta_seg[ui]; s1 = a.cta_seg[ui + 1]; step = 1;
+            s0 = c0; s1 = c1; step = 1;
         }
     } else {
-        if (a.n_slots == 1) {   // the chunks the slot has (a position beyond the limit is reported by the unit that runs)
-            int n = 0;
-            for (int j = 0; j < a.q_len; ++j) n = max(n, row_pos(a, 0, j) + 1);
-            n = min(n, key_limit(a));
+        if (one_wave) nch = a.max_chunks;
+        else if (a.n_slots == 1) {   // the chunks the slot has (a position beyond the limit is reported by the unit that runs)
+            const int p = (threadIdx.x & 31) < a.q_len ? row_pos(a, 0, threadIdx.x & 31) : -1;
+            const int n = min(__reduce_max_sync(0xffffffffu, p) + 1, key_limit(a));
             nch = n > 0 ? chunk_of(a.CH, n - 1) + 1 : 0;
         }
         s0 = ui; s1 = (int) min((long long) nch * a.n_slots, 0x7fffffffLL);
@@ -788,17 +803,12 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
         int * cnt = reinterpret_cast<int *>(smem + 96);   // done[2], flag[3]
         cnt[0] = cnt[1] = cnt[2] = cnt[3] = cnt[4] = 0;
     }
-    uint32_t t_base = 0;
+    // (a unit's first barrier makes them and the tensor-memory base known to all; the warp that starts the first copies has made them itself)
     uint32_t * t_slot = reinterpret_cast<uint32_t *>(smem + 120);
     if constexpr (parks<KT, NT>()) {
         if (threadIdx.x >= 32 && threadIdx.x < 64) umma::tmem_alloc(t_slot, PARK_COLS);
-        umma::fence_before_sync();
     }
-    __syncthreads();
-    if constexpr (parks<KT, NT>()) {
-        umma::fence_after_sync();
-        t_base = *t_slot;
-    }
+    __syncwarp();
     int tiles = 0;
     for (int u = s0; u < s1; u += step) {
         int slot, chunk = -1, k_lo, k_cap;
@@ -815,7 +825,7 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
         }
         if (chunk >= 0) unit = ((unsigned) slot * a.nhk + hl) * a.max_chunks + chunk;   // below 2^31 (decode_geometry)
         if (tiles) __syncthreads();   // the previous unit's shared memory is no longer read
-        tiles += decode_unit<KT, NT, RUNS>(a, nslot, mapK, mapV, smem, a.hk0 + hl, slot, k_lo, k_cap, unit, tiles, t_base);
+        tiles += decode_unit<KT, NT, RUNS>(a, nslot, mapK, mapV, smem, a.hk0 + hl, slot, k_lo, k_cap, unit, tiles, t_slot);
         if (u > 0x7fffffff - step) break;
     }
     if constexpr (parks<KT, NT>()) {
@@ -823,7 +833,7 @@ decode_part_k(const dec_args a, const int nslot, const __grid_constant__ CUtenso
         __syncthreads();
         if (threadIdx.x >= 32 && threadIdx.x < 64) {
             umma::fence_after_sync();
-            umma::tmem_dealloc(t_base, PARK_COLS);
+            umma::tmem_dealloc(*t_slot, PARK_COLS);
         }
     }
 }
@@ -1689,6 +1699,7 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     a.chunked = gm.split ? 0 : 1;
     a.segs = nullptr; a.cta_seg = nullptr; a.slot_seg = nullptr; a.n_cta = nullptr;
     a.solo = gm.split && n_slots == 1 ? gm.max_cta : 0;
+    a.max_cta = gm.max_cta;
     int launches = 2;
     // fixed chunks without a plan: at most one wave of CTAs, a multiple of the heads
     unsigned blocks = (unsigned) std::min<size_t>((size_t) n_slots * gm.max_chunks, (size_t) gm.max_cta) * (unsigned) a.nhk;

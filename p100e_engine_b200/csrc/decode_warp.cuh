@@ -112,7 +112,10 @@ decode_warp_k(const dec_args a, const int n_runs, const __grid_constant__ CUtens
     // the run of this pair of warps; kv head = run index mod heads, as in decode_part_k.  n_runs: runs of all heads the grid was made for
     const int vi = (int) blockIdx.x * 2 + v, hl = vi % a.nhk, ui = vi / a.nhk, hk = a.hk0 + hl;
     int s0 = 0, s1 = 0;
-    if (vi < n_runs && ui < *a.n_cta) { s0 = a.cta_seg[ui]; s1 = a.cta_seg[ui + 1]; }
+    {
+        const int c = min(ui, a.max_cta - 1), n = *a.n_cta, c0 = a.cta_seg[c], c1 = a.cta_seg[c + 1];   // loads that do not wait for one another
+        if (vi < n_runs && ui < n) { s0 = c0; s1 = c1; }
+    }
 
     int sc = 0;              // ring slot of the next item to be consumed; a segment starts and ends with an empty ring
     uint32_t ph = 0;         // and the parity of its use
