@@ -123,10 +123,19 @@ __global__ void __launch_bounds__(TOK_WARPS * 32) token_k(const tok_args a) {
     const bool live = it < n_q + 2 * a.Hkv, is_q = it < n_q, is_v = it >= n_q + a.Hkv;
     const int h = is_q ? it : is_v ? it - n_q - a.Hkv : it - n_q;
     int row;
+    // everything that is read is asked for first: the activations, the norm weights, the place of the page table and, behind the position, the page
+    float xv[NF * 4];   // heads that go to the cache as they are: value 32 b + lane
+    if (live && (is_v || !PREP)) {
+        const float * src = is_v ? a.v + (size_t) t * a.ldv + (size_t) h * D : a.k + (size_t) t * a.ldk + (size_t) h * D;
+#pragma unroll
+        for (int b = 0; b < NF * 4; ++b) if (b < nb) xv[b] = src[b * 32 + lane];
+    }
+    const int32_t * tab = kv_tab(a.g, t);
+    int page = 0;
     if constexpr (PREP) {
         const int ppos = a.pos ? a.pos[t] : a.p0 + t;
         row = a.crow ? a.crow[t] : a.p0 < 0 ? ppos : a.p0 + t;
-        float4 x[NF], gt[NF];
+        float4 x[NF], gt[NF], wn[NF];
         const bool rotated = live && !is_v;
         if (rotated) {
             const float4 * src = reinterpret_cast<const float4 *>(is_q ? a.qg + (size_t) t * a.ldq + (size_t) h * 2 * D
@@ -137,13 +146,17 @@ __global__ void __launch_bounds__(TOK_WARPS * 32) token_k(const tok_args a) {
 #pragma unroll
                 for (int j = 0; j < NF; ++j) if (j < nf) gt[j] = src[D / 4 + lane + 32 * j];
             }
+            const float4 * wt = reinterpret_cast<const float4 *>(is_q ? a.qn : a.kn);
+#pragma unroll
+            for (int j = 0; j < NF; ++j) if (j < nf) wn[j] = wt ? wt[lane + 32 * j] : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
         }
-        for (int j = threadIdx.x; j < half; j += TOK_WARPS * 32) {
+        if (tab && row >= 0 && !is_q && live) page = tab[row >> a.g.psh];
+        for (int i = threadIdx.x; i < 2 * half; i += TOK_WARPS * 32) {   // cos and sin of a pair in different threads: the slow range reduction is the longest chain here
+            const int j = i < half ? i : i - half;
             float theta;
             if constexpr (MR) theta = (float) mrope_position(a.mr, t, j) * powf(a.freq_base, -2.0f * j / a.n_rot);
             else theta = (float) ppos * powf(a.freq_base, -2.0f * j / a.n_rot);
-            cs[j] = cosf(theta);
-            cs[half + j] = sinf(theta);
+            cs[i] = i < half ? cosf(theta) : sinf(theta);
         }
         if (rotated) {
             if (is_q) {   // the gate half of the head moves on unchanged
@@ -166,19 +179,19 @@ __global__ void __launch_bounds__(TOK_WARPS * 32) token_k(const tok_args a) {
                 for (int j = 0; j < 8; ++j) part[j] = nx[j];
             }
             const float sc = rsqrtf(part[0] / D + a.eps);
-            const float4 * wt = reinterpret_cast<const float4 *>(is_q ? a.qn : a.kn);
 #pragma unroll
             for (int j = 0; j < NF; ++j)
                 if (j < nf) {
                     float4 o = x[j];
                     o.x *= sc; o.y *= sc; o.z *= sc; o.w *= sc;
-                    if (wt) { const float4 ww = wt[lane + 32 * j]; o.x *= ww.x; o.y *= ww.y; o.z *= ww.z; o.w *= ww.w; }
+                    o.x *= wn[j].x; o.y *= wn[j].y; o.z *= wn[j].z; o.w *= wn[j].w;   // (times 1 without weights: the same value)
                     reinterpret_cast<float4 *>(st)[lane + 32 * j] = o;
                 }
         }
         __syncthreads();
     } else {
         row = (a.p0p ? *a.p0p : a.p0) + t;
+        if (tab && row >= 0 && live) page = tab[row >> a.g.psh];
     }
     if (!live) return;
     if constexpr (PREP) {
@@ -194,19 +207,15 @@ __global__ void __launch_bounds__(TOK_WARPS * 32) token_k(const tok_args a) {
         }
     }
     if (row < 0) return;
-    const int32_t * tab = kv_tab(a.g, t);
-    if (tab && tab[row >> a.g.psh] < 0) { if (lane == 0) atomicOr(a.status, ST_BAD_PAGE); return; }
-    char * head = (is_v ? a.g.v : a.g.k) + kv_off_tab(a.g, tab, row) + (unsigned long long) h * head_bytes(KT, D);
+    if (page < 0) { if (lane == 0) atomicOr(a.status, ST_BAD_PAGE); return; }
+    char * head = (is_v ? a.g.v : a.g.k) + (unsigned long long) h * head_bytes(KT, D) +
+                  (tab ? (unsigned long long) page * a.g.pstride + (unsigned long long) (row & ((1 << a.g.psh) - 1)) * a.g.rowb : (unsigned long long) row * a.g.rowb);
     if (PREP && !is_v) {
 #pragma unroll
         for (int b = 0; b < NF * 4; ++b) if (b < nb) block_to_cache<KT>(st[b * 32 + lane], lane, head, b, nb);
     } else {   // no norm, no rotation: straight from the activations
-        const float * src = is_v ? a.v + (size_t) t * a.ldv + (size_t) h * D : a.k + (size_t) t * a.ldk + (size_t) h * D;
-        float x[NF * 4];
 #pragma unroll
-        for (int b = 0; b < NF * 4; ++b) if (b < nb) x[b] = src[b * 32 + lane];
-#pragma unroll
-        for (int b = 0; b < NF * 4; ++b) if (b < nb) block_to_cache<KT>(x[b], lane, head, b, nb);
+        for (int b = 0; b < NF * 4; ++b) if (b < nb) block_to_cache<KT>(xv[b], lane, head, b, nb);
     }
 }
 
