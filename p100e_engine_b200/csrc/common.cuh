@@ -225,7 +225,8 @@ __device__ __forceinline__ void a16_store_lanes8(const float4 x, __half2 * __res
 // Measured, us: 16 layers of one row at 4096 keys (recorded) 344 -> 314, 1 + 3 rows at 30011 keys 540 -> 434, four layers of 8 x 4 rows
 // 358 -> 345, of a 77-token prompt 139 -> 131.  Plain launches stay where the early CTAs are in the way: grids of many waves (two layers of
 // 64 x 4 rows 2029 -> 2057 with all of them early, no difference without), the mma.sync decode kernel, whose one wave must spread evenly over
-// the SMs (four layers of one row at 131000 keys 364 -> 426), and prefill_k behind kv_tiles_k (48 rows at 100003 keys 421 -> 596).
+// the SMs (four layers of one row at 131000 keys 364 -> 426; 16 layers of one row at 4096 keys, 256 CTAs, 311 -> 319), and prefill_k behind a kv_tiles_k of
+// several waves (48 rows at 100003 keys 421 -> 596).
 // The line is four CTAs per SM of a B200.  Late / early: rope_rows_k of 600 tokens 11.5 / 14.1 us, of 256 4.8 / 4.4; a merge of 768 CTAs behind the verify
 // kernel (8 x 4 rows at 4096 keys, with prep, in a step) 37.8 / 41.7, of 384 (two heads) 32.0 / 30.7 when launched call by call.
 __device__ __forceinline__ void pdl_enter() {
