@@ -150,10 +150,9 @@ __device__ __forceinline__ int key_limit(const dec_args & a) {
 __device__ __forceinline__ int row_pos(const dec_args & a, int slot, int j);
 
 // One slot in an even split: its 64-key tiles (returned) in `runs` runs per kv head, of two tiles (decode_tc_k walks pairs) where there are so few; run c takes tiles [c W / runs, (c + 1) W / runs).  The
-// decode kernel and the merge find this by themselves: a plan kernel would cost the call 3 us.
+// decode kernel and the merge find this by themselves: a plan kernel would cost the call 3 us.  Called by whole warps.
 __device__ __forceinline__ int solo_runs(const dec_args & a, int & runs) {
-    int n = 0;
-    for (int j = 0; j < a.q_len; ++j) n = max(n, row_pos(a, 0, j) + 1);
+    const int lane = threadIdx.x & 31, n = __reduce_max_sync(0xffffffffu, lane < a.q_len ? row_pos(a, 0, lane) : -1) + 1;
     const int W = (max(0, min(n, key_limit(a))) + TILE - 1) / TILE;
     runs = min(a.solo, (W + 1) / 2);
     return W;

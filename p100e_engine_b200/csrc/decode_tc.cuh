@@ -95,6 +95,22 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
     const bool worker = w < TC_WORKERS / 32;
     const int lq = w & 3, gq = (w >> 2) & 3;     // worker warp: tensor-memory lane quarter, column / block group
     const int hk = (int) (blockIdx.x % (unsigned) a.g.Hkv), ui = (int) (blockIdx.x / (unsigned) a.g.Hkv);
+    // The start of a run is a chain of loads (plan, positions, page table, first copies), 5 us of the 14 that one slot of 30011 keys takes: what can be
+    // asked for together is; one slot's query rows go into registers before anything else (16 layers of 1 + 3 rows 435 -> 419 us; 8 x 4 rows at 4000 keys, two
+    // layers, 100 -> 97).  Thread i of the workers takes 8 values of a row; EX: four neighbouring lanes a block of 32.
+    constexpr int QN = NC * 32 / TC_WORKERS;
+    float4 qv[QN][2];
+    auto load_q = [&](int slot) {
+#pragma unroll
+        for (int k = 0; k < QN; ++k) {
+            const int i = tid + k * TC_WORKERS, n = (EX ? i >> 2 : i) & (NC - 1), kc = EX ? (i & 3) | (i / (4 * NC)) << 2 : i / NC, grp = n >> 3, hh = n & 7;
+            const bool have = hh < GQA && grp < a.q_len;
+            const float4 * src = reinterpret_cast<const float4 *>(a.q + ((size_t) (slot * a.q_len + (have ? grp : 0)) * a.Hq + hk * GQA + (have ? hh : 0)) * DH + kc * 8);
+            qv[k][0] = src[0]; qv[k][1] = src[1];
+            if (!have) qv[k][0] = qv[k][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    if (EX && worker) load_q(0);
     int s0, s1;
     int4 one = make_int4(0, 0, 0, 0);
     if constexpr (EX) {
@@ -104,9 +120,9 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
         one.y = (int) (W * ui / runs) * TILE; one.z = (int) (W * (ui + 1) / runs) * TILE;
         s0 = ui; s1 = ui + 1;
     } else {
-        if (ui >= *a.n_cta) return;
-        s0 = a.cta_seg[ui]; s1 = a.cta_seg[ui + 1];
-        if (s0 >= s1) return;
+        const int n = *a.n_cta;
+        s0 = a.cta_seg[ui]; s1 = a.cta_seg[ui + 1];   // (the grid has as many runs as the plan has room for)
+        if (ui >= n || s0 >= s1) return;
     }
 
     uint64_t * full = reinterpret_cast<uint64_t *>(smem);                       // [TC_NBUF] staging buffer filled
@@ -152,8 +168,9 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
         const int4 seg = EX ? one : a.segs[sg];
         const int slot = seg.x, k_lo = seg.y;
         const size_t unit = (size_t) sg * a.g.Hkv + hk;
-        int n_slot = 0;
-        for (int j = 0; j < a.q_len; ++j) n_slot = max(n_slot, row_pos(a, slot, j) + 1);
+        const int posv = lane < a.q_len ? row_pos(a, slot, lane) : -1;   // lane j: row j
+        const int rt = a.g.pt && a.g.rtab ? a.g.rtab[slot * a.q_len] : 0;
+        int n_slot = __reduce_max_sync(0xffffffffu, posv) + 1;
         {
             const int lim = key_limit(a);
             if (n_slot > lim) { if (tid == 0) atomicOr(a.status, ST_BAD_POS); n_slot = lim; }
@@ -161,9 +178,10 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
         const int k_hi = min(seg.z, n_slot);
         const int nt = k_hi > k_lo ? (k_hi - k_lo + UT - 1) / UT : 0;
         if (nt == 0) continue;
-        const int32_t * tab = a.g.pt ? a.g.pt + (a.g.rtab ? a.g.rtab[slot * a.q_len] : 0) : nullptr;
-        const int pg0 = tab ? k_lo >> a.g.psh : 0;
+        const int32_t * tab = a.g.pt ? a.g.pt + rt : nullptr;
+        const int pg0 = tab ? k_lo >> a.g.psh : 0, pg_n = tab ? ((k_hi - 1) >> a.g.psh) - pg0 + 1 : 1;
         const int ib = 2 * g;
+        int pgl = 0;   // TMA warp: lane l holds page entry l of the run, for the first copies
         // Staging item q of the run, in the order the workers consume them (K0, K1, V0, K2, V1, .., K(nt-1), V(nt-2), V(nt-1)):
         // one or two 64-position boxes (boxes past the run's end hold no key) into ring buffer (2 g + q) mod 4.  Called by the
         // whole TMA warp with warp-uniform arguments; the elected lane issues.  staged: page entries come from shared memory.
@@ -181,7 +199,7 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                 int y = p, z = 0;
                 if (tab) {
                     const int idx = (p >> a.g.psh) - pg0;
-                    z = staged && idx < TC_PGS ? pgs[idx] : tab[p >> a.g.psh];
+                    z = !staged ? __shfl_sync(0xffffffffu, pgl, idx) : idx < TC_PGS ? pgs[idx] : tab[p >> a.g.psh];   // the first copies: 384 positions, 7 pages at most
                     y = p & ((1 << a.g.psh) - 1);
                     if (z < 0) { if (lead) atomicOr(a.status, ST_BAD_PAGE); z = 0; }
                 }
@@ -191,52 +209,48 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
         // The ring is empty at the start of a run (the previous run's end barrier): its first items go out now, before the
         // workers stage the page entries and the query rows, so that the copies fly during that prologue.
         if (w == TC_WORKERS / 32 + 1) {
+            if (tab) pgl = tab[pg0 + min(lane, pg_n - 1)];
             const bool lead = umma::elect_one();
             for (int q = 0; q < TC_NBUF && q < 2 * nt; ++q) issue_item(q, lead, false);
         }
         if (worker) {
             if (tab) {
-                const int npg = min(TC_PGS, ((k_hi - 1) >> a.g.psh) - pg0 + 1);
+                const int npg = min(TC_PGS, pg_n);
                 for (int j = tid; j < npg; j += TC_WORKERS) pgs[j] = tab[pg0 + j];
             }
+            if constexpr (!EX) load_q(slot);
             // Q rows -> f16, scaled, as the K-major B operand: byte(n, d) = (n / 8) * 128 + (d / 8) * (NC * 16) + (n % 8) * 16 + (d % 8) * 2
-            for (int i = tid; i < NC * 32; i += TC_WORKERS) {
-                const int n = i & (NC - 1), kc = i / NC, grp = n >> 3, hh = n & 7;
-                uint4 pk = make_uint4(0, 0, 0, 0);
-                if (hh < GQA && grp < a.q_len) {
-                    const float4 * src = reinterpret_cast<const float4 *>(a.q + ((size_t) (slot * a.q_len + grp) * a.Hq + hk * GQA + hh) * DH + kc * 8);
-                    const float4 v0 = src[0], v1 = src[1];
-                    if constexpr (EX)   // the order in which a word of four cache bytes splits into pairs (k_store)
-                        pk = make_uint4(pack_h2(v0.x * a.qscale, v0.z * a.qscale), pack_h2(v0.y * a.qscale, v0.w * a.qscale),
-                                        pack_h2(v1.x * a.qscale, v1.z * a.qscale), pack_h2(v1.y * a.qscale, v1.w * a.qscale));
-                    else
-                        pk = make_uint4(pack_h2(v0.x * a.qscale, v0.y * a.qscale), pack_h2(v0.z * a.qscale, v0.w * a.qscale),
-                                        pack_h2(v1.x * a.qscale, v1.y * a.qscale), pack_h2(v1.z * a.qscale, v1.w * a.qscale));
-                }
+#pragma unroll
+            for (int k = 0; k < QN; ++k) {
+                const int i = tid + k * TC_WORKERS, n = (EX ? i >> 2 : i) & (NC - 1), kc = EX ? (i & 3) | (i / (4 * NC)) << 2 : i / NC, grp = n >> 3, hh = n & 7;
+                const float4 v0 = qv[k][0], v1 = qv[k][1];
+                uint4 pk;
+                if constexpr (EX)   // the order in which a word of four cache bytes splits into pairs (k_store)
+                    pk = make_uint4(pack_h2(v0.x * a.qscale, v0.z * a.qscale), pack_h2(v0.y * a.qscale, v0.w * a.qscale),
+                                    pack_h2(v1.x * a.qscale, v1.z * a.qscale), pack_h2(v1.y * a.qscale, v1.w * a.qscale));
+                else
+                    pk = make_uint4(pack_h2(v0.x * a.qscale, v0.y * a.qscale), pack_h2(v0.z * a.qscale, v0.w * a.qscale),
+                                    pack_h2(v1.x * a.qscale, v1.y * a.qscale), pack_h2(v1.z * a.qscale, v1.w * a.qscale));
                 *reinterpret_cast<uint4 *>(QI + grp * 128 + kc * (NC * 16) + hh * 16) = pk;
-            }
-            if (tid < 32) { mref[tid] = mtop[tid] = B200_NEG_INF; mm[tid] = make_float2(B200_NEG_INF, -PSHIFT); }
-            if constexpr (EX) {
-                // -1/32 of the sum of a block's 32 query values (finite whatever they are), as f16 and what f16 leaves of it: value b and b + 8 of row n of
-                // the K-major B operand of the offsets' product, [d, d] (A, tensor memory) * this * 4096
-                tc_bar_workers();
-                for (int i = tid; i < 8 * NC; i += TC_WORKERS) {
-                    const int n = i & (NC - 1), b = i / NC;
+                if constexpr (EX) {
+                    // -1/32 of the sum of a block's 32 query values (finite whatever they are), as f16 and what f16 leaves of it: value b and b + 8 of row n
+                    // of the K-major B operand of the offsets' product, [d, d] (A, tensor memory) * this * 4096
+                    const uint32_t xw[4] = {pk.x, pk.y, pk.z, pk.w};
                     float sum = 0.0f;
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const uint4 x = *reinterpret_cast<const uint4 *>(QI + (n >> 3) * 128 + (4 * b + c) * (NC * 16) + (n & 7) * 16);
-                        const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) { const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&xw[e])); sum += f.x + f.y; }
+                    for (int e = 0; e < 4; ++e) { const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&xw[e])); sum += f.x + f.y; }
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                    if ((i & 3) == 0) {
+                        const float y = -0.03125f * sum;
+                        const __half hi = __float2half_rn(y), lo = __float2half_rn(y - __half2float(hi));
+                        unsigned char * dst = QBI + grp * 128 + hh * 16 + (kc >> 2) * 2;
+                        *reinterpret_cast<__half *>(dst) = hi;
+                        *reinterpret_cast<__half *>(dst + NC * 16) = lo;
                     }
-                    const float y = -0.03125f * sum;
-                    const __half hi = __float2half_rn(y), lo = __float2half_rn(y - __half2float(hi));
-                    unsigned char * dst = QBI + (n >> 3) * 128 + (n & 7) * 16 + b * 2;
-                    *reinterpret_cast<__half *>(dst) = hi;
-                    *reinterpret_cast<__half *>(dst + NC * 16) = lo;
                 }
             }
+            if (tid < 32) { mref[tid] = mtop[tid] = B200_NEG_INF; mm[tid] = make_float2(B200_NEG_INF, -PSHIFT); }
             umma::fence_async_smem();
         }
         __syncthreads();
