@@ -1541,7 +1541,7 @@ int launch_tc(const dec_args & a_in, unsigned blocks, cudaStream_t s) {
     if (!make_cache_map(&mapK, a.g.k, a, TC_HB) || !make_cache_map(&mapV, a.g.v, a, TC_HB))
         B200_REFUSE(B200_ERR_CUDA, "attn_decode: the cache's tensor map could not be encoded");
     a.tiled = 1;
-    const size_t sm = tc_smem_bytes();
+    constexpr size_t sm = tc_smem_bytes(EX);
     static std::atomic<bool> attr_done[64];
     int dev = 0;
     cudaGetDevice(&dev);

@@ -36,8 +36,8 @@
 constexpr int UT = 128;                       // keys per tile
 constexpr int TC_WORKERS = 512, TC_THR = TC_WORKERS + 64;   // 16 worker warps, the MMA warp, the TMA warp
 constexpr int TC_NBUF = 4;                    // staging ring, in the order the workers consume: K0, K1, V0, K2, V1, ..
-constexpr int TC_HDR = 1536;                  // barriers, reference maxima, exchange arrays, page entries
-constexpr int TC_PGS = 64;                    // page-table entries of a run kept in shared memory
+constexpr int TC_HDR = 2048, TC_HDR_EX = 1536;   // barriers, reference maxima, exchange arrays, page entries
+constexpr int TC_PGS = 224, TC_PGS_EX = 64;      // page-table entries of a run kept in shared memory (a run of one slot is a fraction of 1 / (SMs per kv head) of it)
 constexpr int TC_VF = UT * DH * 2;            // f16 image of a tile's V rows
 constexpr int TC_QI = 32 * 32 * 16;           // f16 image of up to 32 query rows
 constexpr int TC_PLBO = 528;                  // bytes between the 8-key chunks of the P image (512 + 16: stores of a warp spread over the banks)
@@ -46,8 +46,8 @@ constexpr int TC_REREF = 2;                   // EX: tiles between two renewals 
 constexpr int TC_QB = 2 * 32 * 16;            // block sums of Q (EX): 16 values of up to 32 rows
 
 constexpr int TC_HB = head_bytes(B200_KV_Q8_0);   // the kernel serves q8_0 rows: 8 f16 block scales, then 256 int8
-constexpr size_t tc_smem_bytes() { return TC_HDR + (size_t) TC_NBUF * UT * TC_HB + TC_VF + TC_QI + TC_PI + TC_QB; }
-static_assert(tc_smem_bytes() <= 227 * 1024, "decode_tc_k shared memory");
+constexpr size_t tc_smem_bytes(bool ex) { return (ex ? TC_HDR_EX + TC_QB : TC_HDR) + (size_t) TC_NBUF * UT * TC_HB + TC_VF + TC_QI + TC_PI; }
+static_assert(tc_smem_bytes(false) <= 227 * 1024 && tc_smem_bytes(true) <= 227 * 1024, "decode_tc_k shared memory");
 
 __device__ __forceinline__ void tc_arrive(uint64_t * bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -136,9 +136,10 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
     float * fsc = reinterpret_cast<float *>(smem + 256);                         // [32] rescale factor of the last move
     float * wx = reinterpret_cast<float *>(smem + 384);                          // [4][32] per lane quarter: maxima / sums
     float2 * mm = reinterpret_cast<float2 *>(smem + 896);                        // [32] (reference + REF_GAP, finite reference - PSHIFT)
-    int * pgs = reinterpret_cast<int *>(smem + 1152);                            // [TC_PGS]
-    float * mtop = reinterpret_cast<float *>(smem + 1152 + 4 * TC_PGS);          // [32] EX: largest reference so far
-    unsigned char * stg = smem + TC_HDR, * VF = stg + TC_NBUF * BUF, * QI = VF + TC_VF, * PI = QI + TC_QI, * QBI = PI + TC_PI;
+    constexpr int PGS = EX ? TC_PGS_EX : TC_PGS;
+    int * pgs = reinterpret_cast<int *>(smem + 1152);                            // [PGS]
+    float * mtop = reinterpret_cast<float *>(smem + 1152 + 4 * TC_PGS_EX);       // [32] EX: largest reference so far
+    unsigned char * stg = smem + (EX ? TC_HDR_EX : TC_HDR), * VF = stg + TC_NBUF * BUF, * QI = VF + TC_VF, * PI = QI + TC_QI, * QBI = PI + TC_PI;
 
     if (tid == 0) {
         for (int b = 0; b < TC_NBUF; ++b) mbar_init(&full[b], 1);
@@ -199,7 +200,7 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                 int y = p, z = 0;
                 if (tab) {
                     const int idx = (p >> a.g.psh) - pg0;
-                    z = !staged ? __shfl_sync(0xffffffffu, pgl, idx) : idx < TC_PGS ? pgs[idx] : tab[p >> a.g.psh];   // the first copies: 384 positions, 7 pages at most
+                    z = !staged ? __shfl_sync(0xffffffffu, pgl, idx) : idx < PGS ? pgs[idx] : tab[p >> a.g.psh];   // the first copies: 384 positions, 7 pages at most
                     y = p & ((1 << a.g.psh) - 1);
                     if (z < 0) { if (lead) atomicOr(a.status, ST_BAD_PAGE); z = 0; }
                 }
@@ -215,7 +216,7 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
         }
         if (worker) {
             if (tab) {
-                const int npg = min(TC_PGS, pg_n);
+                const int npg = min(PGS, pg_n);
                 for (int j = tid; j < npg; j += TC_WORKERS) pgs[j] = tab[pg0 + j];
             }
             if constexpr (!EX) load_q(slot);
@@ -250,7 +251,7 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                     }
                 }
             }
-            if (tid < 32) { mref[tid] = mtop[tid] = B200_NEG_INF; mm[tid] = make_float2(B200_NEG_INF, -PSHIFT); }
+            if (tid < 32) { mref[tid] = B200_NEG_INF; if constexpr (EX) mtop[tid] = B200_NEG_INF; mm[tid] = make_float2(B200_NEG_INF, -PSHIFT); }
             umma::fence_async_smem();
         }
         __syncthreads();
@@ -470,10 +471,10 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                         if ((tid >> 3) < a.q_len && (tid & 7) < GQA) {
                             const float mx = fmaxf(fmaxf(wx[tid], wx[32 + tid]), fmaxf(wx[64 + tid], wx[96 + tid]));
                             const float m_old = mref[tid];
-                            if (mx > m_old + REF_GAP || (again && mx >= mtop[tid] - REF_GAP && mx > B200_NEG_INF)) {   // mx is finite here
+                            if (mx > m_old + REF_GAP || (EX && again && mx >= mtop[tid] - REF_GAP && mx > B200_NEG_INF)) {   // mx is finite here
                                 f = ex2f(m_old - mx);     // 2^(-inf) = 0 on the first move
                                 mref[tid] = mx;
-                                mtop[tid] = fmaxf(mtop[tid], mx);
+                                if constexpr (EX) mtop[tid] = fmaxf(mtop[tid], mx);
                                 mm[tid] = make_float2(mx + REF_GAP, mx - PSHIFT);
                             }
                         }
