@@ -6,8 +6,8 @@
 //   K rows (TMA -> staging) --16 worker warps: int8 -> f16 * block scale--> tensor memory, lane = key
 //   S^T[128 keys x rows]   = K (A operand in tensor memory) * Q^T (B operand, K-major image in shared memory)
 //   V rows (TMA -> staging) --workers--> f16 image [key][dim] in shared memory
-//   workers: S^T -> mask -> P = 2^(S - reference maximum + 8) as f16 -> P image [row][key] in shared memory
-//   O^T[256 dims x rows]  += V^T (A operand, the MN-major image, two halves of 128 dims) * P^T (B operand, K-major image)
+//   workers: S^T -> mask -> P = 2^(S - reference maximum + 8) as f16 -> P image [key][row] in shared memory
+//   O^T[256 dims x rows]  += V^T (A operand, the MN-major image, two halves of 128 dims) * P^T (B operand, MN-major image)
 // Two more warps issue: warp 16 the MMAs, warp 17 the TMA copies (a TMA instruction can hold its thread while the copy
 // unit's queue is full, which must not delay an MMA).  Both walk their loops with all 32 lanes and let one elected lane
 // issue, so that tensor-memory addresses and descriptors are warp-uniform values: the MMA and TMA instructions take their
@@ -40,8 +40,8 @@ constexpr int TC_HDR = 2048, TC_HDR_EX = 1536;   // barriers, reference maxima, 
 constexpr int TC_PGS = 224, TC_PGS_EX = 64;      // page-table entries of a run kept in shared memory (a run of one slot is a fraction of 1 / (SMs per kv head) of it)
 constexpr int TC_VF = UT * DH * 2;            // f16 image of a tile's V rows
 constexpr int TC_QI = 32 * 32 * 16;           // f16 image of up to 32 query rows
-constexpr int TC_PLBO = 528;                  // bytes between the 8-key chunks of the P image (512 + 16: stores of a warp spread over the banks)
-constexpr int TC_PI = 8704;                   // P image: 16 chunks of up to 32 rows
+constexpr int TC_PSBO = UT * 16;              // P image: 8 rows (a verify row's six heads and two of padding) of 128 keys
+constexpr int TC_PI = 4 * TC_PSBO;
 constexpr int TC_REREF = 2;                   // EX: tiles between two renewals of the reference maxima
 constexpr int TC_QB = 2 * 32 * 16;            // block sums of Q (EX): 16 values of up to 32 rows
 
@@ -268,7 +268,7 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                 const uint32_t tb_u = __shfl_sync(0xffffffffu, tb, 0);
                 const uint32_t tA_u = tb_u, tS_u = tb_u + (EX ? 128 : 256), tC_u = tS_u + 8 * NC, tO_u = EX ? tC_u + NC : tb_u + 320, tD_u = tO_u + 2 * NC;
                 constexpr uint32_t id_qk = umma::idesc_f16(UT, NC, false, false);   // S^T[128 x NC] = K (tensor memory) * Q^T (K-major)
-                constexpr uint32_t id_pv = umma::idesc_f16(UT, NC, true, false);    // O^T[128 x NC] += V^T (MN-major) * P^T (K-major)
+                constexpr uint32_t id_pv = umma::idesc_f16(UT, NC, true, true);     // O^T[128 x NC] += V^T (MN-major) * P^T (MN-major)
                 const uint32_t q_s = smem_u32(QI), p_s = smem_u32(PI), v_s = smem_u32(VF);
                 auto qk = [&](int j) {   // tile j: waits for its K in tensor memory, queues Q K^T
                     const int G = g_u + j, b = G & 1;
@@ -293,9 +293,9 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
 #pragma unroll
                         for (int ks = 0; ks < UT / 16; ++ks)
 #pragma unroll
-                            for (int h = 0; h < 2; ++h)   // V image: 8-key groups 4096 apart (LBO), 8-dim groups 128 apart (SBO); P: 8-key chunks TC_PLBO apart
+                            for (int h = 0; h < 2; ++h)   // V image: 8-key groups 4096 apart (LBO), 8-dim groups 128 apart (SBO); P: 8-key groups 128 apart, 8-row groups TC_PSBO
                                 umma::mma_ss(tO_u + h * NC, umma::smem_desc(v_s + ks * 2 * 4096 + h * 2048, 4096, 128),
-                                             umma::smem_desc(p_s + ks * 2 * TC_PLBO, TC_PLBO, 128), id_pv, (i > 0 || ks > 0) ? 1u : 0u);
+                                             umma::smem_desc(p_s + ks * 2 * 128, 128, TC_PSBO), id_pv, (i > 0 || ks > 0) ? 1u : 0u);
                         umma::commit(pv_done);
                     }
                 }
@@ -319,7 +319,7 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
             const int vkey = tid & (UT - 1), vb = tid >> 7;         // and its key / first block in the V phase
             const unsigned char * const krow0 = stg + kk * HB, * const vrow0 = stg + vkey * HB;
             unsigned char * const vdst = VF + vb * 512 + (vkey >> 3) * 4096 + (vkey & 7) * 16;
-            unsigned char * const pdst = PI + gq * 128 + (kk >> 3) * TC_PLBO + (kk & 7) * 2;
+            unsigned char * const pdst = PI + gq * TC_PSBO + kk * 16;
             const float4 * mm4 = reinterpret_cast<const float4 *>(mm) + 4 * gq;
             float l_acc[GQA];
 #pragma unroll
@@ -505,14 +505,13 @@ decode_tc_k(const dec_args a, const __grid_constant__ CUtensorMap mapK, const __
                         }
                     }
                 }
-                // ---- P = 2^(S - reference + 8) as f16 into the K-major image: byte(row, key) = (row / 8) * 128 + (key / 8) * TC_PLBO + (row % 8) * 16 + (key % 8) * 2
+                // ---- P = 2^(S - reference + 8) as f16 into the MN-major image: byte(row, key) = (row / 8) * TC_PSBO + key * 16 + (row % 8) * 2: this key's
+                // six heads of verify row gq are one store (six 2-byte stores into a K-major image: 64 x 4 rows, two layers, 2017 -> 2006 us)
                 if (act) {
+                    float p[GQA];
 #pragma unroll
-                    for (int e = 0; e < GQA; ++e) {
-                        const float p = ex2f(s[e] - ofs[e]);
-                        l_acc[e] += p;
-                        *reinterpret_cast<__half *>(pdst + e * 16) = __float2half_rn(p);
-                    }
+                    for (int e = 0; e < GQA; ++e) { p[e] = ex2f(s[e] - ofs[e]); l_acc[e] += p[e]; }
+                    *reinterpret_cast<uint4 *>(pdst) = make_uint4(pack_h2(p[0], p[1]), pack_h2(p[2], p[3]), pack_h2(p[4], p[5]), 0u);
                 }
                 umma::fence_async_smem();
                 umma::fence_before_sync();
