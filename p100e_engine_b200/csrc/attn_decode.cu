@@ -1732,7 +1732,9 @@ int decode_launch(const float * q, const b200_kv_cache * c, const merge_out & mo
     const long long grid = (long long) mg.x * mg.y;
     const bool one = gm.split ? parts <= 8 : parts <= 4 || (parts <= MERGE_STREAMS && grid > 8LL * sms);
     if (one) launch(gm.split ? decode_merge_k<false> : decode_merge_k<true>, mg, 64, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
-    else launch(parts > 4 * MERGE_STREAMS && grid * (DH / 4 / MERGE_DL) <= 2LL * sms ? decode_merge_streams_k<8> : decode_merge_streams_k<4>, dim3(mg.x, mg.y, DH / 4 / MERGE_DL), MERGE_THR, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
+    // (early up to eight CTAs per SM: they are small and behind kernels of one wave; 768 CTAs, four layers of 8 rows of up to
+    // 16384 keys 306 -> 302 us, of up to 4000 keys 158 -> 149)
+    else launch_if(grid * (DH / 4 / MERGE_DL) < 2 * (long long) PDL_MAX_CTAS, parts > 4 * MERGE_STREAMS && grid * (DH / 4 / MERGE_DL) <= 2LL * sms ? decode_merge_streams_k<8> : decode_merge_streams_k<4>, dim3(mg.x, mg.y, DH / 4 / MERGE_DL), MERGE_THR, 0, s, a, mo.gate, mo.out, mo.fo, mo.fm, mo.fl, (__half2 *) mo.qbuf);
     count_launch(launches);
     return launch_status(who);
 }

@@ -235,14 +235,18 @@ __device__ __forceinline__ void pdl_enter() {
 }
 constexpr size_t PDL_MAX_CTAS = 4 * 148;
 template <typename... P, typename... A>
-inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&... args) {
+inline void launch_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&... args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = (size_t) grid.x * grid.y * grid.z < PDL_MAX_CTAS ? 1 : 0;
+    at[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
     cfg.attrs = at; cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // a failure is found by launch_status
+}
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&... args) {
+    launch_if((size_t) grid.x * grid.y * grid.z < PDL_MAX_CTAS, kernel, grid, block, smem, s, args...);
 }
 
 inline bool aligned16(const void * p) { return ((uintptr_t) p & 15) == 0; }
